@@ -22,6 +22,20 @@ struct Coef {
   double ltau_lo, ltau_hi;
 };
 
+// kappa log2 e = kappa2 + kappa2_lo with kappa2_lo > 0: kappa2 the FP32 value at
+// or below the FP64 one, kappa2_lo the FP32 remainder (a tiny positive value when
+// kappa2 is exact), so that -hi * inf - lo * inf of a +inf padding cost entry is
+// -inf, never NaN.
+__host__ __device__ inline void coef_kappa2(Coef& c) {
+  const double k2 = c.kappa * 1.4426950408889634074;
+  float hi = (float)k2;
+  if ((double)hi > k2) hi = nextafterf(hi, 0.f);
+  float lo = (float)(k2 - (double)hi);
+  if (!(lo > 0.f)) lo = 1e-30f;
+  c.kappa2 = hi;
+  c.kappa2_lo = lo;
+}
+
 // The reference's exponents alpha1 = lambda1 / (lambda1 + eps) and
 // alpha2 = lambda2 / (lambda2 + eps) (optimal_transport.py:119-121 / :201-203)
 // and the constants the log-domain updates need.
@@ -41,16 +55,7 @@ __host__ __device__ inline Coef make_coef(double eps, double lambda1, double lam
   c.q = q;
   c.logq = log(q);
   c.kappa = cost_scale / eps;
-  // kappa2 = hi + lo with lo > 0: hi the FP32 value at or below the FP64 one, lo
-  // the FP32 remainder (a tiny positive value when hi is exact), so that
-  // -hi * inf - lo * inf of a +inf padding cost entry is -inf, never NaN
-  const double k2 = cost_scale / eps * 1.4426950408889634074;
-  float hi = (float)k2;
-  if ((double)hi > k2) hi = nextafterf(hi, 0.f);
-  float lo = (float)(k2 - (double)hi);
-  if (!(lo > 0.f)) lo = 1e-30f;
-  c.kappa2 = hi;
-  c.kappa2_lo = lo;
+  coef_kappa2(c);
   c.ltau_lo = -INFINITY;
   c.ltau_hi = INFINITY;
   return c;

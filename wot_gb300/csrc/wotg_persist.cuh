@@ -1,0 +1,673 @@
+// wotg_persist.cuh — a whole materialised-cost solve in one persistent kernel.
+//
+// Every CTA owns a contiguous block of rows and of columns (their FP64 state,
+// merges and updates) and takes its share of the column pass; an iteration is
+//   row phase      a warp per owned row: the online LSE of the row (row_lse),
+//                  merged as FP32 pairs; then a thread per row: log2 and the
+//                  FP64 a-update                                        | grid barrier
+//   column phase   a warp per (128 columns, row block): col_lse partials  | grid barrier
+//   merge phase    a warp per owned float4 column: its row blocks' partials
+//                  merged as FP32 pairs; then a thread per column: log2 and
+//                  the FP64 b-update                                    | grid barrier
+// and the stages, batches, absorptions, stage-exit tests and duality-gap tests
+// of the reference run in the same kernel: every CTA sums the same partial sums
+// in the same order and so takes the same decisions.
+//
+// What bounds it. At the sizes of a day pair (up to a few 1e7 entries, C in L2)
+// an iteration used to be four launches of 2 to 37 us each, and most of that was
+// FP64: one instruction holds a sub-partition's FP64 unit 64 cycles
+// (wotg_df.cuh), and a row's merge and update took some 85 of them on one lane.
+// Here the merges are FP32 pairs, the updates take one instruction for up to 32
+// rows, and a grid barrier (2300 cycles) stands where a launch did.
+//
+// The element arithmetic, its order within a lane and the row blocks of the
+// column pass are those of the standalone passes, so the sums of exponentials
+// are the same bits whatever the grid.
+//
+// Barriers: one CTA per SM, launched cooperatively, so that all are resident;
+// each wait is bounded and a CTA that gives up raises *err, on which the others
+// give up as well. A launch runs at most `budget` iterations and leaves its
+// state in PersistCtl, so that no launch is long.
+#pragma once
+
+#include "wotg_df.cuh"
+#include "wotg_state.cuh"
+
+namespace wotg {
+
+constexpr int kPersistThreads = 512;
+constexpr int kPersistWarps = kPersistThreads / 32;
+constexpr int kPersistBlk = 512;      // rows (columns) of a CTA merged per round
+constexpr int kScalings = 5;          // n_scalings of the duality-gap solver (optimal_transport.py:105)
+constexpr uint32_t kBarrierTries = 40000000;  // polls of about 0.3 us
+
+enum PersistMode : int { kModeGap = 0, kModeFixed = 1, kModeRefine = 2 };
+enum PersistStatus : int { kRunning = 0, kConverged = 1, kMaxIter = 2, kNonfinite = 3 };
+
+struct PersistCtl {
+  double eps, q, sumk;            // current epsilon, mean(p), sum exp(-C/eps) / (I J) at the final stage
+  double gap_num, gap_den;        // the last relative gap as a quotient
+  long long it, checks, absorptions;
+  int stage, status, lrow_valid, started, since, index, pad_[2];
+  unsigned long long bar;         // arrivals (low word) and absorption flags (high word); zeroed per launch
+  int err, pad2_;                 // zeroed per launch
+};
+
+struct PersistArgs {
+  const float* C;
+  Geom g;
+  Vecs V;
+  PersistCtl* ctl;
+  double epsilon, lambda1, lambda2, epsilon0, tau, tolerance, max_iter, cost_scale;
+  double scale_factor;            // exp(-log(epsilon) / kScalings)
+  int batch_size, scaling_iter, inner_iter_max, extra_iter, n_iter, mode;
+  long long budget;               // iterations of this launch (a batch is not split)
+};
+
+struct PersistShared {
+  float4 tab[kLogTable];
+  float4 res[kPersistBlk];        // merged (m, h, l) per row or column of a round
+  double sums[8][kNq];
+  double tot[kNq];
+  Coef c;
+  double a1ln2, a1logj, ku, a2ln2, bconst, kv, iel2;   // folded update coefficients
+  double consts[4];               // log I, log J, log q, log tau
+  unsigned long long bar;
+  int ticket, ok, decision;
+};
+
+// Weight and offset of a point from FP64: as split_weight / grid_value, with the
+// rounding to the 2^-14 grid by one FP64 addition of 1.5 * 2^38 (the same
+// nearest-even value) for |w| < 2^10.
+__device__ __forceinline__ bool below_1024(double w) { return (__double2hiint(w) & 0x7FFFFFFF) < 0x40900000; }
+constexpr double kGridMagic = 412316860416.0;   // 1.5 * 2^38: ulp 2^-14
+
+__device__ __forceinline__ float2 split_pair(double w) {
+  if (below_1024(w)) {
+    const double h = (w + kGridMagic) - kGridMagic;
+    return make_float2((float)h, (float)(w - h));
+  }
+  float2 r;
+  split_weight(w, &r.x, &r.y, 0);
+  return r;
+}
+__device__ __forceinline__ float grid_near(double x) {
+  return below_1024(x) ? (float)((x + kGridMagic) - kGridMagic) : grid_value(x);
+}
+
+struct Persist {
+  const PersistArgs& A;
+  PersistShared& sh;
+  unsigned long long target;      // arrivals that complete the next barrier
+  unsigned int flags;             // absorption flags seen so far
+  int r0, r1, c0, c1;             // owned rows, owned float4 columns
+  float* orow;                    // I   row offsets (on the weight grid); rowc's memory, free during the solve
+  float2* l2col;                  // J   base-2 log-sum-exp of each column: offset on the grid + remainder (Lcol's memory)
+
+  // All CTAs arrive; `flag` is added up over the CTAs (returned in `flagged`).
+  __device__ bool sync(bool flag, bool* flagged = nullptr) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.ctl->bar),
+                   "l"(1ull + ((unsigned long long)(flag ? 1 : 0) << 32))
+                   : "memory");
+      unsigned long long v = 0;
+      bool done = false;
+      for (uint32_t t = 0; t < kBarrierTries; ++t) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.ctl->bar) : "memory");
+        if ((v & 0xFFFFFFFFull) >= target) {
+          done = true;
+          break;
+        }
+        if ((t & 255) == 255 && *(volatile int*)&A.ctl->err) break;
+      }
+      if (!done) atomicExch(&A.ctl->err, 1);
+      sh.ok = done;
+      sh.bar = v;
+    }
+    __syncthreads();
+    target += gridDim.x;
+    const unsigned int hi = (unsigned int)(sh.bar >> 32);
+    if (flagged) *flagged = hi != flags;
+    flags = hi;
+    return sh.ok != 0;
+  }
+
+  // Coefficients of the updates at `eps` (make_coef's, its divisions one per lane).
+  __device__ void set_coef(double eps) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int l = threadIdx.x;
+      const double num = l == 1 ? A.lambda1 : l == 2 ? A.lambda2 : l == 5 ? A.cost_scale : 1.0;
+      const double den = l == 1 || l == 3 ? A.lambda1 + eps : l == 2 || l == 4 ? A.lambda2 + eps : eps;
+      const double x = num / den;
+      Coef c;
+      c.eps = eps;
+      c.inv_eps = __shfl_sync(0xffffffffu, x, 0);
+      c.alpha1 = __shfl_sync(0xffffffffu, x, 1);
+      c.alpha2 = __shfl_sync(0xffffffffu, x, 2);
+      c.inv_l1e = __shfl_sync(0xffffffffu, x, 3);
+      c.inv_l2e = __shfl_sync(0xffffffffu, x, 4);
+      c.kappa = __shfl_sync(0xffffffffu, x, 5);
+      if (l == 0) {
+        c.lambda1 = A.lambda1;
+        c.lambda2 = A.lambda2;
+        c.logI = sh.consts[0];
+        c.logJ = sh.consts[1];
+        c.logq = sh.consts[2];
+        c.q = A.ctl->q;
+        coef_kappa2(c);
+        c.ltau_lo = sh.consts[3] - 1e-9;
+        c.ltau_hi = sh.consts[3] + 1e-9;
+        sh.c = c;
+        sh.a1ln2 = c.alpha1 * kLn2;
+        sh.a1logj = c.alpha1 * c.logJ;
+        sh.ku = -(c.alpha1 * c.inv_eps + c.inv_l1e);
+        sh.a2ln2 = c.alpha2 * kLn2;
+        sh.bconst = c.alpha2 * (c.logq + c.logI);
+        sh.kv = -(c.alpha2 * c.inv_eps + c.inv_l2e);
+        sh.iel2 = c.inv_eps * kLog2e;
+      }
+    }
+    __syncthreads();
+  }
+
+  __device__ __forceinline__ bool over_tau(double l) const {
+    if (l < sh.c.ltau_lo) return false;
+    if (l > sh.c.ltau_hi) return INFINITY > A.tau;
+    return exp(l) > A.tau;
+  }
+
+  // The reference's a-update (optimal_transport.py:133) of row i from its base-2
+  // log-sum-exp; true when a_i > tau.
+  __device__ __forceinline__ bool update_row(int64_t i, double L2) const {
+    const double ui = A.V.u[i];
+    const double la = fma(-sh.a1ln2, L2, fma(sh.c.alpha1, A.V.logp[i], fma(ui, sh.ku, sh.a1logj)));
+    A.V.la_old[i] = A.V.la[i];
+    A.V.la[i] = la;
+    const float2 w = split_pair(fma(la, kLog2e, ui * sh.iel2));
+    A.V.wrow[i] = w.x;
+    A.V.wrow_lo[i] = w.y;
+    return over_tau(la);
+  }
+  __device__ __forceinline__ bool update_col(int64_t j, double L2) const {
+    const double vj = A.V.v[j];
+    const double lb = fma(-sh.a2ln2, L2, fma(vj, sh.kv, sh.bconst));
+    A.V.lb_old[j] = A.V.lb[j];
+    A.V.lb[j] = lb;
+    const float2 w = split_pair(fma(lb, kLog2e, vj * sh.iel2));
+    A.V.wcol[j] = w.x;
+    A.V.wcol_lo[j] = w.y;
+    return over_tau(lb);
+  }
+
+  // Row phase. FRESH: the row sums with the current b only (a gap check), kept
+  // for the a-update of the next iteration.
+  template <bool FRESH>
+  __device__ bool row_phase() {
+    const int lane = threadIdx.x & 31;
+    const float k2 = sh.c.kappa2, k2l = sh.c.kappa2_lo;
+    const float4* w4 = reinterpret_cast<const float4*>(A.V.wcol);
+    const float4* wl4 = reinterpret_cast<const float4*>(A.V.wcol_lo);
+    bool over = false;
+    for (int b = r0; b < r1; b += kPersistBlk) {
+      const int e = min(r1, b + kPersistBlk);
+      if (threadIdx.x == 0) sh.ticket = b;
+      __syncthreads();
+      for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&sh.ticket, 1);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= e) break;
+        float m, s, cmp, h, l;
+        row_lse<true>(reinterpret_cast<const float4*>(A.C + (int64_t)i * A.g.ldc), w4, wl4, A.g.ldc >> 2, lane,
+                      orow[i], k2, k2l, m, s, cmp);
+        two_sum(s, -cmp, h, l);
+        df_merge_lanes<16, 1>(m, h, l);
+        if (lane == 0) sh.res[i - b] = make_float4(m, h, l, 0.f);
+      }
+      __syncthreads();
+      for (int i = b + threadIdx.x; i < e; i += kPersistThreads) {
+        const float4 r = sh.res[i - b];
+        const double L2 = lse2_pair(orow[i], r.x, r.y, r.z, sh.tab);
+        orow[i] = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
+        if (FRESH)
+          A.V.Lrow[i] = L2 * kLn2;
+        else
+          over |= update_row(i, L2);
+      }
+    }
+    return over;
+  }
+
+  // The a-update from the row sums of the preceding check.
+  __device__ bool row_update_cached() {
+    bool over = false;
+    for (int i = r0 + threadIdx.x; i < r1; i += kPersistThreads) over |= update_row(i, A.V.Lrow[i] * kLog2e);
+    return over;
+  }
+
+  // Column phase: partials of (float4 column, row block) at part[(c4 nrb + r) 4 + q].
+  __device__ void col_phase() {
+    const int lane = threadIdx.x & 31;
+    const int nv = (int)(A.g.ldc >> 2), ncg = (nv + 31) >> 5;
+    const int units = ncg * A.g.nrb, nw = gridDim.x * kPersistWarps;
+    const float k2 = sh.c.kappa2, k2l = sh.c.kappa2_lo;
+    for (int u = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; u < units; u += nw) {
+      const int r = u / ncg, c4 = (u % ncg) * 32 + lane;
+      if (c4 >= nv) continue;
+      float o[4], m[4], s[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A.g.J ? l2col[c4 * 4 + q].x : 0.f;
+      const int64_t a = (int64_t)r * A.g.rows_per;
+      col_lse<true>(A.C, A.g.ldc, c4, a, min(A.g.I, a + A.g.rows_per), A.V.wrow, A.V.wrow_lo, o, k2, k2l, m, s);
+      float4* out = reinterpret_cast<float4*>(A.V.part + ((int64_t)c4 * A.g.nrb + r) * 4);
+      out[0] = make_float4(m[0], s[0], m[1], s[1]);
+      out[1] = make_float4(m[2], s[2], m[3], s[3]);
+    }
+  }
+
+  // Merge phase: eight lanes per column over its row blocks, then the b-update.
+  __device__ bool merge_phase() {
+    const int lane = threadIdx.x & 31, q = lane & 3, rl = lane >> 2;
+    constexpr int kCols4 = kPersistBlk / 4;
+    bool over = false;
+    for (int b = c0; b < c1; b += kCols4) {
+      const int e = min(c1, b + kCols4);
+      for (int c4 = b + (threadIdx.x >> 5); c4 < e; c4 += kPersistWarps) {
+        const float2* p = A.V.part + (int64_t)c4 * A.g.nrb * 4 + q;
+        float m = kNegBig, h = 0.f, l = 0.f;
+#pragma unroll 4
+        for (int r = rl; r < A.g.nrb; r += 8) m = fmaxf(m, p[(int64_t)r * 4].x);
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll 4
+        for (int r = rl; r < A.g.nrb; r += 8) {
+          const float2 ps = p[(int64_t)r * 4];
+          const float f = ex2(ps.x - m);
+          const float x = __fmul_rn(ps.y, f);
+          df_add(h, l, x, __fmaf_rn(ps.y, f, -x));
+        }
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) {
+          const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+          df_add(h, l, h2, l2);
+        }
+        if (rl == 0) sh.res[(c4 - b) * 4 + q] = make_float4(m, h, l, 0.f);
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < (e - b) * 4; t += kPersistThreads) {
+        const int j = b * 4 + t;
+        if (j >= A.g.J) break;
+        const float4 r = sh.res[t];
+        const double L2 = lse2_pair(l2col[j].x, r.x, r.y, r.z, sh.tab);
+        const float o = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
+        l2col[j] = make_float2(o, (float)(L2 - (double)o));
+        over |= update_col(j, L2);
+      }
+      __syncthreads();
+    }
+    return over;
+  }
+
+  // u += eps log a, a = 1 (and for v, b): tau-absorption (optimal_transport.py:
+  // 137-141), or with RESCALE the start of a stage (:118-125), whose weights
+  // are for the new epsilon. The caller separates it from the next pass.
+  template <bool RESCALE>
+  __device__ void absorb(double eps_old) {
+    for (int i = r0 + threadIdx.x; i < r1; i += kPersistThreads) {
+      const double un = A.V.u[i] + eps_old * A.V.la[i];
+      A.V.u[i] = un;
+      A.V.la[i] = 0.0;
+      if (RESCALE) A.V.la_old[i] = 0.0;
+      split_weight(un * sh.c.inv_eps * kLog2e, A.V.wrow, A.V.wrow_lo, i);
+    }
+    const int j1 = (int)min((int64_t)c1 * 4, A.g.J);
+    for (int j = c0 * 4 + threadIdx.x; j < j1; j += kPersistThreads) {
+      const double vn = A.V.v[j] + eps_old * A.V.lb[j];
+      A.V.v[j] = vn;
+      A.V.lb[j] = 0.0;
+      if (RESCALE) A.V.lb_old[j] = 0.0;
+      split_weight(vn * sh.c.inv_eps * kLog2e, A.V.wcol, A.V.wcol_lo, j);
+    }
+  }
+
+  // One iteration; *absorb_now when max(a, b) > tau.
+  __device__ bool iterate(bool lrow_valid, bool* absorb_now) {
+    bool over = lrow_valid ? row_update_cached() : row_phase<false>();
+    if (!sync(false)) return false;
+    col_phase();
+    if (!sync(false)) return false;
+    over |= merge_phase();
+    over = __syncthreads_or(over);
+    return sync(over, absorb_now);
+  }
+
+  // Sums over all CTAs of per-thread values (threads 0..127 hold row terms,
+  // 128..255 column terms, the others none): every thread ends with the totals
+  // in sh.tot. One barrier.
+  template <int NQ>
+  __device__ bool total(double (&acc)[NQ], bool any) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < 8) {
+      if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) acc[q] = warp_sum(acc[q]);
+      }
+      if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) sh.sums[w][q] = acc[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < NQ) {
+      double t = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t += sh.sums[k][threadIdx.x];
+      A.V.red[blockIdx.x * kNq + threadIdx.x] = t;
+    }
+    if (!sync(false)) return false;
+    if (w < NQ) {
+      double t = 0.0;
+      for (int b = lane; b < (int)gridDim.x; b += 32) t += A.V.red[b * kNq + w];
+      t = warp_sum(t);
+      if (lane == 0) sh.tot[w] = t;
+    }
+    __syncthreads();
+    return true;
+  }
+
+  // Stage-exit test (optimal_transport.py:158-160) in the reference's expressions.
+  __device__ bool stage_test(bool* go_on) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    bool any = false;
+    const bool rows = threadIdx.x < 128;
+    const double* u = rows ? A.V.u : A.V.v;
+    const double* la = rows ? A.V.la : A.V.lb;
+    const double* lo = rows ? A.V.la_old : A.V.lb_old;
+    const int n0 = rows ? r0 : c0 * 4, n1 = rows ? r1 : (int)min((int64_t)c1 * 4, A.g.J);
+    if (threadIdx.x < 256) {
+      double d2 = 0.0, a2 = 0.0;
+      for (int k = n0 + (threadIdx.x & 127); k < n1; k += 128) {
+        const double e = exp(u[k] * sh.c.inv_eps);
+        const double ta = exp(la[k]) * e;
+        const double d = ta - exp(lo[k]) * e;
+        d2 += d * d;
+        a2 += ta * ta;
+        any = true;
+      }
+      acc[rows ? 0 : 2] = d2;
+      acc[rows ? 1 : 3] = a2;
+    }
+    if (!total<4>(acc, any)) return false;
+    if (threadIdx.x < 32) {
+      const double r = sqrt(sh.tot[threadIdx.x & 3]);
+      const double n = __shfl_sync(0xffffffffu, r, (threadIdx.x & 1) * 2);
+      const double d = __shfl_sync(0xffffffffu, r, (threadIdx.x & 1) * 2 + 1);
+      const double g = n / (1.0 + d);
+      const double ga = __shfl_sync(0xffffffffu, g, 0), gb = __shfl_sync(0xffffffffu, g, 1);
+      const double gap = gb > ga ? gb : ga;   // Python's max: the first unless the second is larger
+      if (threadIdx.x == 0) {
+        sh.decision = gap > 1e-6;
+        if (blockIdx.x == 0) {
+          A.ctl->gap_num = gap;
+          A.ctl->gap_den = 1.0;
+        }
+      }
+    }
+    __syncthreads();
+    *go_on = sh.decision != 0;
+    return true;
+  }
+
+  // Duality-gap test in O(I + J) (see wotg_sinkhorn.cu) after a fresh row phase.
+  __device__ bool gap_test(double sumk, bool* go_on, bool* nan) {
+    double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const Coef& c = sh.c;
+    bool any = false;
+    if (threadIdx.x < 128) {
+      for (int i = r0 + threadIdx.x; i < r1; i += 128) {
+        const double ui = A.V.u[i], la = A.V.la[i];
+        const double ue = ui * c.inv_eps, ub = ui + c.eps * la;
+        double x, f, conj;
+        gap_terms(la + ue + A.V.Lrow[i] - c.logJ, la, ue, A.V.p[i], A.V.logp[i], c.lambda1, c.eps, &x, &f, &conj);
+        acc[0] += c.lambda1 * f + conj + ub * x;
+        acc[2] += f;
+        acc[4] += ub * x;
+        acc[6] += x;
+        any = true;
+      }
+    } else if (threadIdx.x < 256) {
+      const int j1 = (int)min((int64_t)c1 * 4, A.g.J);
+      for (int j = c0 * 4 + threadIdx.x - 128; j < j1; j += 128) {
+        const double vj = A.V.v[j], lb = A.V.lb[j];
+        const double ve = vj * c.inv_eps, vb = vj + c.eps * lb;
+        const float2 l2 = l2col[j];
+        double y, f, conj;
+        gap_terms(lb + ve + ((double)l2.x + (double)l2.y) * kLn2 - c.logI, lb, ve, c.q, c.logq, c.lambda2, c.eps, &y,
+                  &f, &conj);
+        acc[1] += c.lambda2 * f + conj + vb * y;
+        acc[3] += f;
+        acc[5] += vb * y;
+        any = true;
+      }
+    }
+    if (!total<7>(acc, any)) return false;
+    if (threadIdx.x == 0) {
+      const double* h = sh.tot;
+      const double dx = 1.0 / (double)A.g.I, dy = 1.0 / (double)A.g.J;
+      const double num = dx * h[0] + dy * h[1];
+      const double pri = c.lambda1 * dx * h[2] + c.lambda2 * dy * h[3] + dx * h[4] + dy * h[5] +
+                         c.eps * (sumk - dx * h[6]);
+      const double den = fabs(pri);
+      // gap = num / den, as a comparison (the quotient is formed once, on the host)
+      const bool isnan_ = num != num || den != den || (num == 0.0 && den == 0.0) || (isinf(num) && isinf(den));
+      sh.decision = isnan_ ? 2 : num > A.tolerance * den ? 1 : 0;
+      if (blockIdx.x == 0) {
+        A.ctl->gap_num = num;
+        A.ctl->gap_den = den;
+      }
+    }
+    __syncthreads();
+    *go_on = sh.decision == 1;
+    *nan = sh.decision == 2;
+    return true;
+  }
+
+  // sum_ij exp(-kappa C_ij) / (I J) (the reference's sum of its _K).
+  __device__ bool sum_exp(double* out) {
+    const int lane = threadIdx.x & 31;
+    const float k2 = sh.c.kappa2;
+    const int64_t nv = A.g.ldc >> 2;
+    float h = 0.f, l = 0.f;
+    for (int i = r0 + (threadIdx.x >> 5); i < r1; i += kPersistWarps) {
+      const float4* row = reinterpret_cast<const float4*>(A.C + (int64_t)i * A.g.ldc);
+      for (int64_t k = lane; k < nv; k += 32) {
+        const float4 cc = ld_stream(row + k);   // padding is +inf: exp2(-inf) = 0
+        df_add(h, l, (ex2(-k2 * cc.x) + ex2(-k2 * cc.y)) + (ex2(-k2 * cc.z) + ex2(-k2 * cc.w)), 0.f);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+      df_add(h, l, h2, l2);
+    }
+    __syncthreads();
+    if (lane == 0) sh.res[threadIdx.x >> 5] = make_float4(h, l, 0.f, 0.f);
+    __syncthreads();
+    double acc[1] = {0.0};
+    if (threadIdx.x < kPersistWarps) {
+      const float4 r = sh.res[threadIdx.x];
+      acc[0] = (double)r.x + (double)r.y;
+    }
+    __syncthreads();
+    if (!total<1>(acc, threadIdx.x < kPersistWarps)) return false;
+    *out = sh.tot[0] / ((double)A.g.I * (double)A.g.J);
+    return true;
+  }
+
+  __device__ bool mean_growth() {
+    double acc[1] = {0.0};
+    bool any = false;
+    if (threadIdx.x < 128)
+      for (int i = r0 + threadIdx.x; i < r1; i += 128) {
+        acc[0] += A.V.p[i];
+        any = true;
+      }
+    if (!total<1>(acc, any)) return false;
+    if (threadIdx.x == 0 && blockIdx.x == 0) A.ctl->q = sh.tot[0] / (double)A.g.I;
+    return sync(false);
+  }
+
+  // Absorbs with the old epsilon and starts a stage at `eps`.
+  __device__ bool start_stage(double eps_old, double eps) {
+    set_coef(eps);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      A.ctl->gap_num = INFINITY;
+      A.ctl->gap_den = 1.0;
+    }
+    absorb<true>(eps_old);
+    return sync(false);
+  }
+
+  __device__ void run() {
+    PersistCtl* ctl = A.ctl;
+    const int n = gridDim.x, b = blockIdx.x;
+    target = n;
+    flags = 0;
+    r0 = (int)(A.g.I * b / n);
+    r1 = (int)(A.g.I * (b + 1) / n);
+    const int64_t nv = A.g.ldc >> 2;
+    c0 = (int)(nv * b / n);
+    c1 = (int)(nv * (b + 1) / n);
+    orow = reinterpret_cast<float*>(A.V.rowc);
+    l2col = reinterpret_cast<float2*>(A.V.Lcol);
+    for (int i = threadIdx.x; i < kLogTable; i += kPersistThreads) sh.tab[i] = log_table_entry(i);
+    // the state this launch starts from (CTA 0 writes it back at the end, after
+    // barriers that every CTA has passed)
+    double eps = ctl->eps, sumk = ctl->sumk;
+    long long it = ctl->it, checks = ctl->checks, absorptions = ctl->absorptions;
+    int stage = ctl->stage, status = ctl->status, lrow_valid = ctl->lrow_valid, since = ctl->since,
+        index = ctl->index;
+    const int started = ctl->started;
+    if (status != kRunning) return;
+    if (!started && !mean_growth()) return;
+    if (threadIdx.x < 32) {
+      const double x = threadIdx.x == 0 ? (double)A.g.I : threadIdx.x == 1 ? (double)A.g.J
+                       : threadIdx.x == 2 ? *(volatile double*)&ctl->q : A.tau;
+      const double y = log(x);
+      if (threadIdx.x < 4) sh.consts[threadIdx.x] = y;
+    }
+    if (started) set_coef(eps);
+    long long used = 0;
+    bool ok = true, absorb_now = false;
+    if (A.mode == kModeGap) {
+      if (!started) {
+        // epsilon0 * factor / factor, as the reference's arithmetic
+        const double old = A.epsilon0 * A.scale_factor;
+        eps = old / A.scale_factor;
+        ok = start_stage(old, eps);
+      }
+      bool stage_done = false;
+      while (ok && status == kRunning && used < A.budget) {
+        if (stage_done) {
+          const double old = eps;
+          eps = eps / A.scale_factor;
+          ++stage;
+          lrow_valid = 0;
+          stage_done = false;
+          if (!(ok = start_stage(old, eps))) break;
+          if (stage == kScalings && !(ok = sum_exp(&sumk))) break;
+        }
+        const int nb = stage == kScalings ? A.batch_size : 5;
+        for (int t = 0; t < nb; ++t) {
+          ++it;
+          ++used;
+          if (!(ok = iterate(lrow_valid != 0, &absorb_now))) break;
+          lrow_valid = 0;
+          if (absorb_now) {
+            ++absorptions;
+            absorb<false>(eps);
+            if (!(ok = sync(false))) break;
+          }
+          if ((double)it >= A.max_iter) {
+            status = kMaxIter;
+            break;
+          }
+        }
+        if (!ok) break;
+        if (status == kMaxIter) {
+          row_phase<true>();
+          break;
+        }
+        ++checks;
+        bool go_on = true, nan = false;
+        if (stage == kScalings) {
+          row_phase<true>();
+          lrow_valid = 1;
+          __syncthreads();
+          if (!(ok = gap_test(sumk, &go_on, &nan))) break;
+          if (!go_on) status = nan ? kNonfinite : kConverged;
+        } else {
+          if (!(ok = stage_test(&go_on))) break;
+          stage_done = !go_on;
+          if (stage_done && used >= A.budget) used = A.budget - 1;   // the next launch starts inside a stage
+        }
+      }
+    } else {
+      const bool fixed = A.mode == kModeFixed;
+      if (!started) {
+        eps = fixed ? A.epsilon0 : A.epsilon;
+        if (fixed) {
+          ok = start_stage(0.0, eps);
+        } else {
+          set_coef(eps);   // potentials loaded with a = b = 1
+        }
+      }
+      const long long with_absorb = fixed ? A.scaling_iter : A.n_iter;
+      const long long total_it = with_absorb + (fixed ? A.extra_iter : 0);
+      while (ok && it < total_it && used < A.budget) {
+        ++used;
+        if (!(ok = iterate(false, &absorb_now))) break;
+        if (it < with_absorb && absorb_now) {
+          ++absorptions;
+          absorb<false>(eps);
+          if (!(ok = sync(false))) break;
+        }
+        ++it;
+        if (fixed && it <= with_absorb && ++since == A.inner_iter_max) {
+          ++index;
+          since = 0;
+          const double eps_new = (A.epsilon0 - A.epsilon) * exp(-(double)index) + A.epsilon;
+          const double old = eps;
+          eps = eps_new;
+          if (!(ok = start_stage(old, eps))) break;
+        }
+      }
+      if (ok && it >= total_it) {
+        if (fixed) row_phase<true>();
+        status = kConverged;
+      }
+    }
+    if (ok && b == 0 && threadIdx.x == 0) {
+      ctl->eps = eps;
+      ctl->sumk = sumk;
+      ctl->it = it;
+      ctl->checks = checks;
+      ctl->absorptions = absorptions;
+      ctl->stage = stage;
+      ctl->status = status;
+      ctl->lrow_valid = lrow_valid;
+      ctl->started = 1;
+      ctl->since = since;
+      ctl->index = index;
+    }
+  }
+};
+
+__global__ void __launch_bounds__(kPersistThreads, 1) persist_kernel(PersistArgs A) {
+  __shared__ PersistShared sh;
+  Persist p{A, sh, 0, 0, 0, 0, 0, 0, nullptr, nullptr};
+  p.run();
+}
+
+}  // namespace wotg

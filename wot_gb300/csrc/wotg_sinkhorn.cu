@@ -35,37 +35,11 @@
 #include "wotg_coef.cuh"
 #include "wotg_common.cuh"
 #include "wotg_onthefly.cuh"
+#include "wotg_persist.cuh"
+#include "wotg_state.cuh"
 #include "wotg_tc_kernel.cuh"
 
 namespace wotg {
-
-// Per-solve vectors in the caller's workspace.
-struct Vecs {
-  double* u;       // I   absorbed potential (reference u)
-  double* v;       // J
-  double* la;      // I   log a
-  double* lb;      // J   log b
-  double* la_old;  // I   log a at the start of the last iteration (stage-exit test)
-  double* lb_old;  // J
-  double* logp;    // I   log p (p = G of this growth iteration)
-  double* p;       // I
-  double* Lrow;    // I   log sum_j exp(v_j/eps + lb_j - kappa C_ij)
-  double* Lcol;    // J   log sum_i exp(u_i/eps + la_i - kappa C_ij)
-  float* wrow;     // I   (u_i/eps + la_i) * log2(e), FP32 operand of the column pass (hi part, see split_weight)
-  float* wcol;     // ldc (v_j/eps + lb_j) * log2(e), zero in padding columns (hi part)
-  float* wrow_lo;  // I   remainders of the weights (lo parts)
-  float* wcol_lo;  // ldc
-  float4* rowc;    // I   per-row constants of the dense coupling (coupling_rows_kernel)
-  float2* part;    // nrb x ldc column-pass partials (m, s) in base 2
-  unsigned long long* maxslot;  // 2 slots of max(a, b) bits, alternating per iteration
-  double* red;     // kRedBlocks x kNq reduction partials
-  double* scal;    // kNq final sums + misc scalars
-  int* counters;   // [0] absorptions
-};
-
-constexpr int kNq = 8;
-constexpr int kRedBlocks = 296;
-
 
 // Buffers of the on-the-fly (tensor-core) form.
 struct TcState {
@@ -104,25 +78,8 @@ struct TcState {
   bool xb_ok, yb_ok;
 };
 
-struct Geom {
-  int64_t I, J, ldc;
-  int row_grid;
-  int ncb, nrb;             // column-pass grid: column blocks x row blocks
-  int64_t rows_per;
-};
-
-// The reference's a-update for row i; returns the new a_i (for the
-// absorption test, reduced per block by the caller).
-// exp(la) as the absorption test needs it: the test only compares the largest
-// exp(la) with tau, so away from log(tau) the value is 0 (below) or +inf
-// (above) with the same outcome, and the FP64 exp (slow on this part) is formed
-// only within 1e-9 of log(tau). NaN stays NaN.
-__device__ __forceinline__ double absorb_key(double la, const Coef& c) {
-  if (la < c.ltau_lo) return 0.0;
-  if (la > c.ltau_hi) return INFINITY;
-  return exp(la);
-}
-
+// The reference's a-update for row i; returns the key of the new a_i for the
+// absorption test (reduced per block by the caller).
 __device__ __forceinline__ double a_update(int64_t i, double L, const Vecs& V, const Coef& c) {
   const double ui = V.u[i];
   const double logs = ui * c.inv_eps + L - c.logJ;                 // log (K (b dy))_i
@@ -157,108 +114,20 @@ __device__ __forceinline__ void block_max_to_slot(double v, unsigned long long* 
   }
 }
 
-// Exponent of one element: plain (w - k2 C, one rounding) or precise (relative
-// to the grid offset o with the weight's and kappa2's low parts, see
-// split_weight).
-template <bool PREC>
-__device__ __forceinline__ float expo(float cc, float w, float wl, float o, float k2, float k2l) {
-  if (PREC) return fmaf(-k2, cc, w - o) + fmaf(-k2l, cc, wl);
-  return fmaf(-k2, cc, w);
-}
-
-// Row pass: one warp per row, 128-bit streaming loads of C, online base-2 LSE.
-// UPDATE_A additionally applies the a-update to the row (first half-step).
-// PREC: the solver's precise form (weights hi + lo in V.wcol / V.wcol_lo, the
-// row's previous log-sum-exp in V.Lrow as its offset); otherwise the plain form
-// on one FP32 weight vector (the standalone half-step).
-template <bool UPDATE_A, bool PREC>
-__global__ void __launch_bounds__(256) row_pass_kernel(const float* __restrict__ C, Geom g,
-                                                       Vecs V, Coef c, int parity) {
+// Standalone row pass: one warp per row, 128-bit streaming loads of C, online
+// base-2 LSE of one FP32 weight vector.
+__global__ void __launch_bounds__(256) row_pass_kernel(const float* __restrict__ C, Geom g, const float* w, float k2,
+                                                       double* __restrict__ L) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t nv = g.ldc >> 2;
-  const float4* __restrict__ w4 = reinterpret_cast<const float4*>(V.wcol);
-  const float4* __restrict__ wl4 = reinterpret_cast<const float4*>(PREC ? V.wcol_lo : V.wcol);
-  const float k2 = c.kappa2, k2l = c.kappa2_lo;
-  double amax = 0.0;
+  const float4* w4 = reinterpret_cast<const float4*>(w);
   for (int64_t i = warp; i < g.I; i += nwarps) {
-    const float4* __restrict__ row = reinterpret_cast<const float4*>(C + i * g.ldc);
-    const float o = PREC ? grid_offset(V.Lrow[i]) : 0.f;
-    float m = kNegBig, s = 0.f, cmp = 0.f;   // PREC: compensated sum s - cmp
-    int64_t k = lane;
-    // the cost loads of the next 128-float4 chunk are issued before this
-    // chunk's arithmetic (two chunks of loads in flight per lane)
-    float4 cn[4];
-    if (k + 96 < nv) {
-#pragma unroll
-      for (int t = 0; t < 4; ++t) cn[t] = ld_stream(row + k + 32 * t);
-    }
-    for (; k + 96 < nv; k += 128) {
-      float4 cc[4], ww[4], wl[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) cc[t] = cn[t];
-      if (k + 128 + 96 < nv) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) cn[t] = ld_stream(row + k + 128 + 32 * t);
-      }
-#pragma unroll
-      for (int t = 0; t < 4; ++t) ww[t] = __ldg(w4 + k + 32 * t);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) wl[t] = PREC ? __ldg(wl4 + k + 32 * t) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float x0 = expo<PREC>(cc[t].x, ww[t].x, wl[t].x, o, k2, k2l);
-        const float x1 = expo<PREC>(cc[t].y, ww[t].y, wl[t].y, o, k2, k2l);
-        const float x2 = expo<PREC>(cc[t].z, ww[t].z, wl[t].z, o, k2, k2l);
-        const float x3 = expo<PREC>(cc[t].w, ww[t].w, wl[t].w, o, k2, k2l);
-        const float mn = fmaxf(m, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
-        const float r = ex2(m - mn);
-        const float v = (ex2(x0 - mn) + ex2(x1 - mn)) + (ex2(x2 - mn) + ex2(x3 - mn));
-        if (PREC) {
-          s = __fmul_rn(s, r);
-          cmp = __fmul_rn(cmp, r);
-          kahan_add(s, cmp, v);
-        } else {
-          s = s * r + v;
-        }
-        m = mn;
-      }
-    }
-    for (; k < nv; k += 32) {
-      const float4 cc = ld_stream(row + k);
-      const float4 ww = __ldg(w4 + k);
-      const float4 wl = PREC ? __ldg(wl4 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float x0 = expo<PREC>(cc.x, ww.x, wl.x, o, k2, k2l);
-      const float x1 = expo<PREC>(cc.y, ww.y, wl.y, o, k2, k2l);
-      const float x2 = expo<PREC>(cc.z, ww.z, wl.z, o, k2, k2l);
-      const float x3 = expo<PREC>(cc.w, ww.w, wl.w, o, k2, k2l);
-      const float mn = fmaxf(m, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
-      const float r = ex2(m - mn);
-      const float v = (ex2(x0 - mn) + ex2(x1 - mn)) + (ex2(x2 - mn) + ex2(x3 - mn));
-      if (PREC) {
-        s = __fmul_rn(s, r);
-        cmp = __fmul_rn(cmp, r);
-        kahan_add(s, cmp, v);
-      } else {
-        s = s * r + v;
-      }
-      m = mn;
-    }
-    double S = (double)s - (double)cmp;
-    if (PREC) {
-      warp_lse_f64(m, S);
-    } else {
-      warp_lse(m, s);
-      S = (double)s;
-    }
-    if (lane == 0) {
-      const double L = ((double)o + (double)m + log2(S)) * kLn2;
-      V.Lrow[i] = L;
-      if (UPDATE_A) amax = fmax(amax, a_update(i, L, V, c));
-    }
+    float m, s, cmp;
+    row_lse<false>(reinterpret_cast<const float4*>(C + i * g.ldc), w4, w4, g.ldc >> 2, lane, 0.f, k2, 0.f, m, s, cmp);
+    warp_lse(m, s);
+    if (lane == 0) L[i] = ((double)m + log2((double)s)) * kLn2;
   }
-  if (UPDATE_A) block_max_to_slot(amax, V.maxslot + parity);
 }
 
 // a-update from a cached row LSE (the row pass of the preceding gap check).
@@ -270,150 +139,36 @@ __global__ void a_update_kernel(Geom g, Vecs V, Coef c, int parity) {
   block_max_to_slot(amax, V.maxslot + parity);
 }
 
-// Column pass, phase 1: CTA = 1024 columns (float4 per thread) x rows_per rows;
-// writes one (m, s) base-2 LSE partial per column and row block.
-constexpr int kColRowChunk = 4;
-
-// Offset of column j of the precise column pass (0 in padding columns); the
-// combine recomputes the same value from the same V.Lcol.
-__device__ __forceinline__ float col_offset(const Vecs& V, const Geom& g, int64_t j) {
-  return j < g.J ? grid_offset(V.Lcol[j]) : 0.f;
-}
-
-template <bool PREC>
-__global__ void __launch_bounds__(256) col_partial_kernel(const float* __restrict__ C, Geom g,
-                                                          Vecs V, Coef c) {
+// Standalone column pass, phase 1: CTA = 1024 columns (float4 per thread) x
+// rows_per rows; writes one (m, s) base-2 LSE partial per column and row block.
+__global__ void __launch_bounds__(256) col_partial_kernel(const float* __restrict__ C, Geom g, const float* w, float k2,
+                                                          float2* __restrict__ part) {
   const int64_t c4 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nv = g.ldc >> 2;
   const int64_t r0 = (int64_t)blockIdx.y * g.rows_per;
-  const int64_t r1 = min(g.I, r0 + g.rows_per);
-  if (c4 >= nv) return;
-  const float k2 = c.kappa2, k2l = c.kappa2_lo;
-  float o[4] = {0.f, 0.f, 0.f, 0.f};
-  if (PREC) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) o[q] = col_offset(V, g, c4 * 4 + q);
-  }
-  float m[4] = {kNegBig, kNegBig, kNegBig, kNegBig};
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
-  float cmp[4] = {0.f, 0.f, 0.f, 0.f};   // PREC: compensated sums s - cmp
-  int64_t i = r0;
-  // the next chunk's cost loads are issued before this chunk's arithmetic
-  float4 cn[kColRowChunk];
-  if (i + kColRowChunk <= r1) {
-#pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) cn[t] = ld_stream(reinterpret_cast<const float4*>(C + (i + t) * g.ldc) + c4);
-  }
-  for (; i + kColRowChunk <= r1; i += kColRowChunk) {
-    float4 cc[kColRowChunk];
-    float w[kColRowChunk], wl[kColRowChunk];
-#pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) cc[t] = cn[t];
-    if (i + 2 * kColRowChunk <= r1) {
-#pragma unroll
-      for (int t = 0; t < kColRowChunk; ++t)
-        cn[t] = ld_stream(reinterpret_cast<const float4*>(C + (i + kColRowChunk + t) * g.ldc) + c4);
-    }
-#pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) w[t] = __ldg(V.wrow + i + t);
-#pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) wl[t] = PREC ? __ldg(V.wrow_lo + i + t) : 0.f;
-    float x[4][kColRowChunk];
-#pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) {
-      x[0][t] = expo<PREC>(cc[t].x, w[t], wl[t], o[0], k2, k2l);
-      x[1][t] = expo<PREC>(cc[t].y, w[t], wl[t], o[1], k2, k2l);
-      x[2][t] = expo<PREC>(cc[t].z, w[t], wl[t], o[2], k2, k2l);
-      x[3][t] = expo<PREC>(cc[t].w, w[t], wl[t], o[3], k2, k2l);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float mx = x[q][0];
-#pragma unroll
-      for (int t = 1; t < kColRowChunk; ++t) mx = fmaxf(mx, x[q][t]);
-      const float mn = fmaxf(m[q], mx);
-      const float r = ex2(m[q] - mn);
-      float v = 0.f;
-#pragma unroll
-      for (int t = 0; t < kColRowChunk; ++t) v += ex2(x[q][t] - mn);
-      if (PREC) {
-        s[q] = __fmul_rn(s[q], r);
-        cmp[q] = __fmul_rn(cmp[q], r);
-        kahan_add(s[q], cmp[q], v);
-      } else {
-        s[q] = s[q] * r + v;
-      }
-      m[q] = mn;
-    }
-  }
-  for (; i < r1; ++i) {
-    const float4 cc = ld_stream(reinterpret_cast<const float4*>(C + i * g.ldc) + c4);
-    const float w = __ldg(V.wrow + i);
-    const float wl = PREC ? __ldg(V.wrow_lo + i) : 0.f;
-    const float xs[4] = {expo<PREC>(cc.x, w, wl, o[0], k2, k2l), expo<PREC>(cc.y, w, wl, o[1], k2, k2l),
-                         expo<PREC>(cc.z, w, wl, o[2], k2, k2l), expo<PREC>(cc.w, w, wl, o[3], k2, k2l)};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float mn = fmaxf(m[q], xs[q]);
-      const float r = ex2(m[q] - mn);
-      if (PREC) {
-        s[q] = __fmul_rn(s[q], r);
-        cmp[q] = __fmul_rn(cmp[q], r);
-        kahan_add(s[q], cmp[q], ex2(xs[q] - mn));
-      } else {
-        s[q] = s[q] * r + ex2(xs[q] - mn);
-      }
-      m[q] = mn;
-    }
-  }
-  if (PREC) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s[q] -= cmp[q];
-  }
-  float4* out = reinterpret_cast<float4*>(V.part + (int64_t)blockIdx.y * g.ldc + c4 * 4);
+  if (c4 >= g.ldc >> 2) return;
+  const float o[4] = {0.f, 0.f, 0.f, 0.f};
+  float m[4], s[4];
+  col_lse<false>(C, g.ldc, c4, r0, min(g.I, r0 + g.rows_per), w, w, o, k2, 0.f, m, s);
+  float4* out = reinterpret_cast<float4*>(part + (int64_t)blockIdx.y * g.ldc + c4 * 4);
   out[0] = make_float4(m[0], s[0], m[1], s[1]);
   out[1] = make_float4(m[2], s[2], m[3], s[3]);
 }
 
-// Column pass, phase 2: merge the row-block partials of each column in FP64,
-// then (UPDATE_B) the reference's b-update.
-template <bool UPDATE_B, bool PREC>
-__global__ void col_combine_kernel(Geom g, Vecs V, Coef c, int parity) {
+// Phase 2: the row-block partials of each column.
+__global__ void col_combine_kernel(Geom g, const float2* __restrict__ part, double* __restrict__ L) {
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double bmax = 0.0;
-  if (j < g.J) {
-    const float o = PREC ? col_offset(V, g, j) : 0.f;
-    double L;
-    if (PREC) {
-      // the row-block partials merged in FP64 against their largest exponent
-      // (FP32 scale factors, 2 ulp; two passes: measured faster than one pass
-      // with a running maximum, whose rescaling lengthens the FP64 chain)
-      float m = kNegBig;
-      for (int r = 0; r < g.nrb; ++r) m = fmaxf(m, V.part[(int64_t)r * g.ldc + j].x);
-      double S = 0.0;
-      for (int r = 0; r < g.nrb; ++r) {
-        const float2 ps = V.part[(int64_t)r * g.ldc + j];
-        S += (double)ps.y * (double)ex2(ps.x - m);
-      }
-      L = ((double)o + (double)m + log2(S)) * kLn2;
-    } else {
-      float m = kNegBig, s = 0.f;
-      for (int r = 0; r < g.nrb; ++r) {
-        const float2 ps = V.part[(int64_t)r * g.ldc + j];
-        lse_merge(m, s, ps.x, ps.y);
-      }
-      L = lse2(m, s) * kLn2;
-    }
-    V.Lcol[j] = L;
-    if (UPDATE_B) bmax = b_update(j, L, V, c);
+  if (j >= g.J) return;
+  float m = kNegBig, s = 0.f;
+  for (int r = 0; r < g.nrb; ++r) {
+    const float2 ps = part[(int64_t)r * g.ldc + j];
+    lse_merge(m, s, ps.x, ps.y);
   }
-  if (UPDATE_B) block_max_to_slot(bmax, V.maxslot + parity);
+  L[j] = lse2(m, s) * kLn2;
 }
 
 // tau-absorption (optimal_transport.py:137-141 / :211-216): if max(a, b) > tau,
 // u += eps log a, v += eps log b, a = b = 1. Also clears the other max slot.
-// The on-the-fly form also rewrites the column-form biases of the absorbed
-// points (bx, by; tiles = nullptr in the materialised form).
+// Also rewrites the column-form biases of the absorbed points (bx, by).
 __global__ void absorb_kernel(Geom g, Vecs V, Coef c, double tau, int parity, TcBias bx, TcBias by) {
   pdl_wait();
   pdl_trigger();
@@ -481,6 +236,7 @@ __global__ void init_kernel(Geom g, Vecs V, const double* __restrict__ G) {
     V.wrow[idx] = 0.f;
     V.wrow_lo[idx] = 0.f;
     V.Lrow[idx] = 0.0;
+    reinterpret_cast<float*>(V.rowc)[idx] = 0.f;   // row offsets of the persistent solver
   }
   if (idx < g.ldc) {
     V.wcol[idx] = 0.f;
@@ -611,29 +367,6 @@ __global__ void stage_test_kernel(Geom g, Vecs V, Coef c, double* red) {
 //   acc[2] = sum_i (x log(x/p) - x + p)       acc[3] = sum_j (y log(y/q) - y + q)
 //   acc[4] = sum_i ubar x                      acc[5] = sum_j vbar y
 //   acc[6] = sum_i x
-// The gap terms of one point: x = exp(t) its marginal sum (t = log x), p its
-// target, the scaling a~ = exp(la) exp(u/eps) evaluated as the reference does.
-// Where nothing overflows or underflows, log(x / p) = t - log p and
-// log a~ = la + u/eps (to an ulp), which saves four of the six FP64
-// transcendentals per point (slow on this part); at the edges the reference's
-// own expressions run, so overflow, 0 log 0 and NaN behave as in the reference.
-__device__ __forceinline__ void gap_terms(double t, double la, double ue, double p, double logp, double lambda,
-                                          double eps, double* x_out, double* f_out, double* conj_out) {
-  const double x = exp(t);
-  double f, conj;
-  if (x > 0.0 && fabs(t) < 700.0 && fabs(la) < 700.0 && fabs(ue) < 700.0 && fabs(la + ue) < 700.0 && p > 0.0) {
-    f = x * (t - logp) - x + p;
-    conj = lambda * p * (exp(-eps * (la + ue) / lambda) - 1.0);
-  } else {
-    const double at = exp(la) * exp(ue);
-    f = x * log(x / p) - x + p;
-    conj = lambda * p * (exp(-eps * log(at) / lambda) - 1.0);
-  }
-  *x_out = x;
-  *f_out = f;
-  *conj_out = conj;
-}
-
 __global__ void gap_partial_kernel(Geom g, Vecs V, Coef c, double* red) {
   double acc[kNq];
 #pragma unroll
@@ -931,7 +664,6 @@ struct Solver {
   // both stay in median-normalised units whatever the units of the input points
   // (FP16 range); their product is gamma x . y.
   int tc_prepare(const Coef& c) {
-    if (!tc.on) return WOTG_OK;
     tc.off_row_ok = false;  // a new epsilon: the offsets and biases of both sides are stale
     tc.off_col_ok = false;
     tc.xb_ok = tc.yb_ok = false;
@@ -1029,39 +761,23 @@ struct Solver {
     return WOTG_OK;
   }
 
-  int iteration(const Coef& c, bool lrow_valid, int parity, bool update_b_only = false) {
-    (void)update_b_only;
-    if (tc.on) {
-      int s;
-      if (lrow_valid) {
-        a_update_kernel<<<vec_blocks(g.I), 256, 0, st>>>(g, V, c, parity);
-        WOTG_LAUNCHED();
-        tc.xb_ok = false;  // la changed without its biases: the column pass packs them
-      } else {
-        s = tc_row_pass<true>(c, parity);
-        if (s) return s;
-      }
-      return tc_col_pass(c, parity);
-    }
+  // One on-the-fly iteration (the materialised form iterates in persist_kernel).
+  int iteration(const Coef& c, bool lrow_valid, int parity) {
+    int s;
     if (lrow_valid) {
       a_update_kernel<<<vec_blocks(g.I), 256, 0, st>>>(g, V, c, parity);
+      WOTG_LAUNCHED();
+      tc.xb_ok = false;  // la changed without its biases: the column pass packs them
     } else {
-      row_pass_kernel<true, true><<<g.row_grid, 256, 0, st>>>(C, g, V, c, parity);
+      s = tc_row_pass<true>(c, parity);
+      if (s) return s;
     }
-    WOTG_LAUNCHED();
-    col_partial_kernel<true><<<dim3(g.ncb, g.nrb), 256, 0, st>>>(C, g, V, c);
-    WOTG_LAUNCHED();
-    col_combine_kernel<true, true><<<vec_blocks(g.J), 256, 0, st>>>(g, V, c, parity);
-    WOTG_LAUNCHED();
-    return WOTG_OK;
+    return tc_col_pass(c, parity);
   }
 
   int absorb(const Coef& c, double tau, int parity) {
-    if (tc.on)
-      WOTG_CUDA(launch_dependent(absorb_kernel, dim3(vec_blocks(g.I + g.J)), dim3(256), 0, st, g, V, c, tau, parity,
-                                 bias_x(), bias_y()));
-    else
-      absorb_kernel<<<vec_blocks(g.I + g.J), 256, 0, st>>>(g, V, c, tau, parity, TcBias{}, TcBias{});
+    WOTG_CUDA(launch_dependent(absorb_kernel, dim3(vec_blocks(g.I + g.J)), dim3(256), 0, st, g, V, c, tau, parity,
+                               bias_x(), bias_y()));
     WOTG_LAUNCHED();
     return WOTG_OK;
   }
@@ -1100,12 +816,7 @@ struct Solver {
     return WOTG_OK;
   }
 
-  int fresh_lrow(const Coef& c) {
-    if (tc.on) return tc_row_pass<false>(c, 0);
-    row_pass_kernel<false, true><<<g.row_grid, 256, 0, st>>>(C, g, V, c, 0);
-    WOTG_LAUNCHED();
-    return WOTG_OK;
-  }
+  int fresh_lrow(const Coef& c) { return tc_row_pass<false>(c, 0); }
 
   // CUDA-graph replay of the final stage's batches between duality-gap checks.
   // In that stage a batch starts right after a check (L_row fresh) with both
@@ -1123,7 +834,7 @@ struct Solver {
   cudaEvent_t gev[2] = {nullptr, nullptr};
   bool graphs_off = false;                   // no private stream: plain launches
 
-  bool steady() const { return !tc.on || (tc.off_row_ok && tc.off_col_ok && tc.xb_ok && tc.yb_ok); }
+  bool steady() const { return tc.off_row_ok && tc.off_col_ok && tc.xb_ok && tc.yb_ok; }
 
   void drop_graphs() {
     for (auto& b : bg) {
@@ -1243,14 +954,80 @@ struct SolveResult {
   bool max_iter = false;
   int64_t iterations = 0;
   int64_t checks = 0;
+  int64_t absorptions = 0;
   double gap = NAN;
   double eps = 0.0;
   Coef final_coef{};
 };
 
+// A materialised solve (mode kModeGap / kModeFixed) or n_iter refinement
+// iterations at epsilon `eps` (kModeRefine): launches of persist_kernel until
+// it reports an end. A launch is kept to some 20 ms (its iterations cost about
+// 8 us and 2.5 ps per entry), so that a long solve stays a sequence of short
+// kernels.
+static int solve_persistent(Solver& S, const wotg_params& P, int mode, double eps, int n_iter, SolveResult& res) {
+  static_assert(sizeof(PersistCtl) <= 16 * sizeof(double), "PersistCtl lives in Vecs::scal");
+  PersistArgs A{};
+  A.C = S.C;
+  A.g = S.g;
+  A.V = S.V;
+  A.ctl = reinterpret_cast<PersistCtl*>(S.V.scal);
+  A.epsilon = eps;
+  A.lambda1 = P.lambda1;
+  A.lambda2 = P.lambda2;
+  A.epsilon0 = P.epsilon0;
+  A.tau = P.tau;
+  A.tolerance = P.tolerance;
+  A.max_iter = P.max_iter;
+  A.cost_scale = S.cost_scale;
+  A.scale_factor = std::exp(-std::log(P.epsilon) / kScalings);
+  A.batch_size = P.batch_size;
+  A.scaling_iter = P.scaling_iter;
+  A.inner_iter_max = P.inner_iter_max;
+  A.extra_iter = P.extra_iter;
+  A.n_iter = n_iter;
+  A.mode = mode;
+  const double per_iter = 8e-6 + 2.5e-12 * (double)S.g.I * (double)S.g.J;
+  A.budget = std::max<long long>(8, std::min<long long>(2000, (long long)(0.02 / per_iter)));
+  WOTG_CUDA(cudaMemsetAsync(A.ctl, 0, sizeof(PersistCtl), S.st));
+  // one CTA per SM; fewer only where the device grants the process fewer SMs
+  int grid = std::min(sm_count(), kRedBlocks);
+  PersistCtl h{};
+  for (;;) {
+    WOTG_CUDA(cudaMemsetAsync(&A.ctl->bar, 0, 2 * sizeof(unsigned long long), S.st));
+    void* args[] = {&A};
+    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(persist_kernel), dim3(grid),
+                                                dim3(kPersistThreads), args, 0, S.st);
+    while (e == cudaErrorCooperativeLaunchTooLarge && grid > 1) {
+      cudaGetLastError();
+      grid /= 2;
+      e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(persist_kernel), dim3(grid),
+                                      dim3(kPersistThreads), args, 0, S.st);
+    }
+    WOTG_CUDA(e);
+    WOTG_LAUNCHED();
+    WOTG_CUDA(cudaMemcpyAsync(&h, A.ctl, sizeof(h), cudaMemcpyDeviceToHost, S.st));
+    WOTG_CUDA(cudaStreamSynchronize(S.st));
+    if (h.err) {
+      set_last_message("persistent solver: a bounded grid barrier ran out");
+      return WOTG_CUDA_ERROR;
+    }
+    if (h.status != kRunning) break;
+  }
+  res.iterations = h.it;
+  res.checks = h.checks;
+  res.absorptions = h.absorptions;
+  res.gap = mode == kModeGap ? h.gap_num / h.gap_den : NAN;
+  res.eps = h.eps;
+  res.max_iter = h.status == kMaxIter;
+  res.final_coef = S.coef(h.eps, P, h.q);
+  return h.status == kNonfinite ? WOTG_NONFINITE : WOTG_OK;
+}
+
 // Python's max(x, y): returns x unless y > x (so a NaN in first position wins).
 static inline double py_max(double x, double y) { return (y > x) ? y : x; }
 
+// The on-the-fly form's duality-gap solver: the control on the host.
 static int solve_duality_gap(Solver& S, const wotg_params& P, double q, SolveResult& res) {
   const int n_scalings = 5;
   const double scale_factor = std::exp(-std::log(P.epsilon) / n_scalings);
@@ -1388,13 +1165,10 @@ static int solve_fixed_iters(Solver& S, const wotg_params& P, double q, SolveRes
   return WOTG_OK;
 }
 
-// Resident 256-thread CTAs per SM of a kernel (6 when the query fails).
-template <class K>
-static int occupancy(K kernel) {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 256, 0) != cudaSuccess || n <= 0) return 6;
-  return n;
-}
+// Row blocks of the column pass: about kColCtasPerSm CTAs of 1024 columns per
+// SM. The partition fixes the order of a column's sum, so it stays the same for
+// every kernel that walks it. kRowCtasPerSm sizes the standalone row pass.
+constexpr int kRowCtasPerSm = 3, kColCtasPerSm = 4;
 
 static Geom make_geom(int64_t I, int64_t J, int64_t ldc) {
   Geom g;
@@ -1402,15 +1176,13 @@ static Geom make_geom(int64_t I, int64_t J, int64_t ldc) {
   g.J = J;
   g.ldc = ldc;
   const int sms = sm_count();
-  static const int occ_row = occupancy(row_pass_kernel<true, true>);
-  static const int occ_col = occupancy(col_partial_kernel<true>);
-  const int64_t max_warps = (int64_t)sms * occ_row * 8;
+  const int64_t max_warps = (int64_t)sms * kRowCtasPerSm * 8;
   const int64_t rows_per_warp = (I + max_warps - 1) / max_warps;
   const int64_t warps = (I + rows_per_warp - 1) / rows_per_warp;
   g.row_grid = (int)std::max<int64_t>(1, (warps + 7) / 8);
   const int64_t nv = ldc >> 2;
   g.ncb = (int)std::max<int64_t>(1, (nv + 255) / 256);
-  int64_t nrb = std::max<int64_t>(1, ((int64_t)sms * occ_col) / g.ncb);
+  int64_t nrb = std::max<int64_t>(1, ((int64_t)sms * kColCtasPerSm) / g.ncb);
   nrb = std::min<int64_t>(nrb, std::max<int64_t>(1, I / 8));
   int64_t rows_per = (I + nrb - 1) / nrb;
   rows_per = (rows_per + kColRowChunk - 1) / kColRowChunk * kColRowChunk;
@@ -1440,7 +1212,6 @@ static size_t layout(Bump& b, const Geom& g, Vecs& V) {
   V.red = b.take<double>((size_t)kRedBlocks * kNq);
   V.scal = b.take<double>(16);
   V.counters = b.take<int>(8);
-  V.scal = V.scal;
   return b.off + 256;
 }
 
@@ -1460,24 +1231,17 @@ extern "C" int wotg_lse_matvec(const float* C, int64_t I, int64_t J, int64_t ldc
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (axis == 0 && (reinterpret_cast<uintptr_t>(w) & 15)))
     return WOTG_BADARG;
   Geom g = make_geom(I, J, ldc);
-  Vecs V{};
-  Coef c{};
-  c.kappa2 = kappa2;
   cudaStream_t st = (cudaStream_t)stream;
   if (axis == 0) {
-    V.wcol = const_cast<float*>(w);
-    V.Lrow = L;
-    row_pass_kernel<false, false><<<g.row_grid, 256, 0, st>>>(C, g, V, c, 0);
+    row_pass_kernel<<<g.row_grid, 256, 0, st>>>(C, g, w, kappa2, L);
     WOTG_LAUNCHED();
     return WOTG_OK;
   }
   if (!workspace || workspace_bytes < wotg_lse_matvec_workspace_bytes(I, J, ldc)) return WOTG_WORKSPACE;
-  V.wrow = const_cast<float*>(w);
-  V.Lcol = L;
-  V.part = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  col_partial_kernel<false><<<dim3(g.ncb, g.nrb), 256, 0, st>>>(C, g, V, c);
+  float2* part = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
+  col_partial_kernel<<<dim3(g.ncb, g.nrb), 256, 0, st>>>(C, g, w, kappa2, part);
   WOTG_LAUNCHED();
-  col_combine_kernel<false, false><<<(unsigned)((J + 255) / 256), 256, 0, st>>>(g, V, c, 0);
+  col_combine_kernel<<<(unsigned)((J + 255) / 256), 256, 0, st>>>(g, part, L);
   WOTG_LAUNCHED();
   return WOTG_OK;
 }
@@ -1604,17 +1368,22 @@ extern "C" int wotg_compute_transport_matrix(const wotg_problem* prob, const wot
     }
     init_kernel<<<S.vec_blocks(std::max(I, ldc)), 256, 0, st>>>(g, V, G);
     WOTG_LAUNCHED();
-    double q = 0.0;
-    int s = S.mean_of(V.p, I, &q);
-    if (s) return s;
     SolveResult res;
-    s = (P.solver == WOTG_SOLVER_DUALITY_GAP) ? solve_duality_gap(S, P, q, res)
-                                              : solve_fixed_iters(S, P, q, res);
-    int absorptions = 0;
-    WOTG_CUDA(cudaMemcpyAsync(&absorptions, V.counters, sizeof(int), cudaMemcpyDeviceToHost, st));
-    WOTG_CUDA(cudaStreamSynchronize(st));
+    int s;
+    if (S.tc.on) {
+      double q = 0.0;
+      s = S.mean_of(V.p, I, &q);
+      if (s) return s;
+      s = (P.solver == WOTG_SOLVER_DUALITY_GAP) ? solve_duality_gap(S, P, q, res) : solve_fixed_iters(S, P, q, res);
+      int absorptions = 0;
+      WOTG_CUDA(cudaMemcpyAsync(&absorptions, V.counters, sizeof(int), cudaMemcpyDeviceToHost, st));
+      WOTG_CUDA(cudaStreamSynchronize(st));
+      res.absorptions = absorptions;
+    } else {
+      s = solve_persistent(S, P, P.solver == WOTG_SOLVER_DUALITY_GAP ? kModeGap : kModeFixed, P.epsilon, 0, res);
+    }
     total.iterations += res.iterations;
-    total.absorptions += absorptions;
+    total.absorptions += res.absorptions;
     total.checks += res.checks;
     total.gap = res.gap;
     total.final_epsilon = res.eps;
@@ -1690,21 +1459,34 @@ extern "C" int wotg_refine_potentials(const wotg_problem* prob, const wotg_param
   }
   init_kernel<<<S.vec_blocks(std::max(I, ldc)), 256, 0, st>>>(g, V, prob->G);
   WOTG_LAUNCHED();
-  double q = 0.0;
-  int s = S.mean_of(V.p, I, &q);
-  if (s) return s;
-  const Coef c = S.coef(epsilon, P, q);
-  load_potentials_kernel<<<S.vec_blocks(I + J), 256, 0, st>>>(g, V, u_bar, v_bar, c.inv_eps);
-  WOTG_LAUNCHED();
-  s = S.tc_prepare(c);
-  if (s) return s;
-  int parity = 0;
-  for (int it = 0; it < n_iter; ++it) {
-    s = S.iteration(c, false, parity);
+  int s;
+  Coef c{};
+  int64_t absorptions = 0;
+  if (S.tc.on) {
+    double q = 0.0;
+    s = S.mean_of(V.p, I, &q);
     if (s) return s;
-    s = S.absorb(c, P.tau, parity);
+    c = S.coef(epsilon, P, q);
+    load_potentials_kernel<<<S.vec_blocks(I + J), 256, 0, st>>>(g, V, u_bar, v_bar, c.inv_eps);
+    WOTG_LAUNCHED();
+    s = S.tc_prepare(c);
     if (s) return s;
-    parity ^= 1;
+    int parity = 0;
+    for (int it = 0; it < n_iter; ++it) {
+      s = S.iteration(c, false, parity);
+      if (s) return s;
+      s = S.absorb(c, P.tau, parity);
+      if (s) return s;
+      parity ^= 1;
+    }
+  } else {
+    load_potentials_kernel<<<S.vec_blocks(I + J), 256, 0, st>>>(g, V, u_bar, v_bar, 1.0 / epsilon);
+    WOTG_LAUNCHED();
+    SolveResult res;
+    s = solve_persistent(S, P, kModeRefine, epsilon, n_iter, res);
+    if (s) return s;
+    c = res.final_coef;
+    absorptions = res.absorptions;
   }
   s = S.outputs(c, false, nullptr, nullptr, u_bar, v_bar);
   if (s) return s;
@@ -1713,12 +1495,11 @@ extern "C" int wotg_refine_potentials(const wotg_problem* prob, const wotg_param
   out.iterations = n_iter;
   out.final_epsilon = epsilon;
   out.gap = NAN;
-  {
-    int absorptions = 0;
-    WOTG_CUDA(cudaMemcpy(&absorptions, V.counters, sizeof(int), cudaMemcpyDeviceToHost));
-    out.absorptions = absorptions;
-  }
+  out.absorptions = absorptions;
   if (S.tc.on) {
+    int absorbed = 0;
+    WOTG_CUDA(cudaMemcpy(&absorbed, V.counters, sizeof(int), cudaMemcpyDeviceToHost));
+    out.absorptions = absorbed;
     int err = 0;
     WOTG_CUDA(cudaMemcpy(&err, S.tc.err, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) {
