@@ -39,7 +39,7 @@ constexpr int kPersistThreads = 512;
 constexpr int kPersistWarps = kPersistThreads / 32;
 constexpr int kPersistBlk = 512;      // rows (columns) of a CTA merged per round
 constexpr int kScalings = 5;          // n_scalings of the duality-gap solver (optimal_transport.py:105)
-constexpr uint32_t kBarrierTries = 40000000;  // polls of about 0.3 us
+constexpr uint32_t kBarrierTries = 10000000;  // polls of about 0.3 us
 
 enum PersistMode : int { kModeGap = 0, kModeFixed = 1, kModeRefine = 2 };
 enum PersistStatus : int { kRunning = 0, kConverged = 1, kMaxIter = 2, kNonfinite = 3 };
@@ -48,7 +48,7 @@ struct PersistCtl {
   double eps, q, sumk;            // current epsilon, mean(p), sum exp(-C/eps) / (I J) at the final stage
   double gap_num, gap_den;        // the last relative gap as a quotient
   long long it, checks, absorptions;
-  int stage, status, lrow_valid, started, since, index, pad_[2];
+  int stage, status, lrow_valid, started, since, index, epoch, pad_;
   unsigned long long bar;         // arrivals (low word) and absorption flags (high word); zeroed per launch
   int err, pad2_;                 // zeroed per launch
 };
@@ -64,6 +64,14 @@ struct PersistArgs {
   long long budget;               // iterations of this launch (a batch is not split)
 };
 
+// The solver's control state during a launch; thread 0 of every CTA keeps the
+// same copy in shared memory (in registers it would crowd out the passes).
+struct RunState {
+  double eps, sumk;
+  long long it, checks, absorptions, used;
+  int stage, status, lrow_valid, since, index, stage_done;
+};
+
 struct PersistShared {
   float4 tab[kLogTable];
   float4 res[kPersistBlk];        // merged (m, h, l) per row or column of a round
@@ -71,8 +79,12 @@ struct PersistShared {
   double tot[kNq];
   Coef c;
   double a1ln2, a1logj, ku, a2ln2, bconst, kv, iel2;   // folded update coefficients
+  float a1h, a1l, a2h, a2l;       // alpha1, alpha2 as pairs
   double consts[4];               // log I, log J, log q, log tau
+  double dx, dy;                  // 1 / I, 1 / J
+  RunState rs;
   unsigned long long bar;
+  int off[32];                    // resident variant: its arrays' places in dynamic shared memory
   int ticket, ok, decision;
 };
 
@@ -95,14 +107,18 @@ __device__ __forceinline__ float grid_near(double x) {
   return below_1024(x) ? (float)((x + kGridMagic) - kGridMagic) : grid_value(x);
 }
 
-struct Persist {
+struct PersistBase {
   const PersistArgs& A;
   PersistShared& sh;
   unsigned long long target;      // arrivals that complete the next barrier
   unsigned int flags;             // absorption flags seen so far
-  int r0, r1, c0, c1;             // owned rows, owned float4 columns
-  float* orow;                    // I   row offsets (on the weight grid); rowc's memory, free during the solve
-  float2* l2col;                  // J   base-2 log-sum-exp of each column: offset on the grid + remainder (Lcol's memory)
+
+  __device__ PersistBase(const PersistArgs& args, PersistShared& shared) : A(args), sh(shared) {
+    target = gridDim.x;
+    flags = 0;
+    if (threadIdx.x == 0) sh.ok = 1;
+    for (int i = threadIdx.x; i < kLogTable; i += blockDim.x) sh.tab[i] = log_table_entry(i);
+  }
 
   // All CTAs arrive; `flag` is added up over the CTAs (returned in `flagged`).
   __device__ bool sync(bool flag, bool* flagged = nullptr) {
@@ -122,7 +138,7 @@ struct Persist {
         if ((t & 255) == 255 && *(volatile int*)&A.ctl->err) break;
       }
       if (!done) atomicExch(&A.ctl->err, 1);
-      sh.ok = done;
+      if (!done) sh.ok = 0;
       sh.bar = v;
     }
     __syncthreads();
@@ -167,6 +183,10 @@ struct Persist {
         sh.bconst = c.alpha2 * (c.logq + c.logI);
         sh.kv = -(c.alpha2 * c.inv_eps + c.inv_l2e);
         sh.iel2 = c.inv_eps * kLog2e;
+        sh.a1h = (float)c.alpha1;
+        sh.a1l = (float)(c.alpha1 - (double)sh.a1h);
+        sh.a2h = (float)c.alpha2;
+        sh.a2l = (float)(c.alpha2 - (double)sh.a2h);
       }
     }
     __syncthreads();
@@ -176,6 +196,131 @@ struct Persist {
     if (l < sh.c.ltau_lo) return false;
     if (l > sh.c.ltau_hi) return INFINITY > A.tau;
     return exp(l) > A.tau;
+  }
+
+  // Cross-CTA sums of the NQ values that every CTA has written to its place in
+  // V.red: one barrier, then every CTA adds them in the same order into sh.tot.
+  template <int NQ>
+  __device__ bool reduce_ctas() {
+    if (!sync(false)) return false;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < NQ) {
+      double t = 0.0;
+      for (int b = lane; b < (int)gridDim.x; b += 32) t += A.V.red[b * kNq + w];
+      t = warp_sum(t);
+      if (lane == 0) sh.tot[w] = t;
+    }
+    __syncthreads();
+    return true;
+  }
+
+  // Sum over all threads of the pairs h + l, over I J.
+  __device__ bool total_pairs(float h, float l, double* out) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+      df_add(h, l, h2, l2);
+    }
+    __syncthreads();
+    if (lane == 0) sh.res[w] = make_float4(h, l, 0.f, 0.f);
+    __syncthreads();
+    if (w == 0) {
+      const float4 r = lane < (int)(blockDim.x >> 5) ? sh.res[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const double t = warp_sum((double)r.x + (double)r.y);
+      if (lane == 0) A.V.red[blockIdx.x * kNq] = t;
+    }
+    if (!reduce_ctas<1>()) return false;
+    *out = sh.tot[0] / ((double)A.g.I * (double)A.g.J);
+    return true;
+  }
+
+  // Stage-exit decision from |a~ - old|^2, |a~|^2 and the same of b in sh.tot.
+  __device__ bool stage_decision(bool* go_on) {
+    if (threadIdx.x < 32) {
+      // ga = sqrt(h0) / (1 + sqrt(h1)), gb likewise; Python's max (the first unless
+      // the second is larger) and the comparison with 1e-6 as products
+      const double r = sqrt(sh.tot[threadIdx.x & 3]);
+      const double na = __shfl_sync(0xffffffffu, r, 0), nb = __shfl_sync(0xffffffffu, r, 2);
+      const double da = 1.0 + __shfl_sync(0xffffffffu, r, 1), db = 1.0 + __shfl_sync(0xffffffffu, r, 3);
+      const bool b = nb * da > na * db;
+      const double num = b ? nb : na, den = b ? db : da;
+      if (threadIdx.x == 0) {
+        sh.decision = num > 1e-6 * den;
+        if (blockIdx.x == 0) {
+          A.ctl->gap_num = num;
+          A.ctl->gap_den = den;
+        }
+      }
+    }
+    __syncthreads();
+    *go_on = sh.decision != 0;
+    return true;
+  }
+
+  // Duality-gap decision from the sums of gap_test in sh.tot.
+  __device__ bool gap_decision(double sumk, bool* go_on, bool* nan) {
+    if (threadIdx.x == 0) {
+      const double* h = sh.tot;
+      const Coef& c = sh.c;
+      const double dx = sh.dx, dy = sh.dy;
+      const double num = dx * h[0] + dy * h[1];
+      const double pri = c.lambda1 * dx * h[2] + c.lambda2 * dy * h[3] + dx * h[4] + dy * h[5] +
+                         c.eps * (sumk - dx * h[6]);
+      const double den = fabs(pri);
+      // gap = num / den, as a comparison (the quotient is formed once, on the host)
+      const bool isnan_ = num != num || den != den || (num == 0.0 && den == 0.0) || (isinf(num) && isinf(den));
+      sh.decision = isnan_ ? 2 : num > A.tolerance * den ? 1 : 0;
+      if (blockIdx.x == 0) {
+        A.ctl->gap_num = num;
+        A.ctl->gap_den = den;
+      }
+    }
+    __syncthreads();
+    *go_on = sh.decision == 1;
+    *nan = sh.decision == 2;
+    return true;
+  }
+
+  // q = mean(p) from its sum, and the constants of the coefficients.
+  __device__ bool publish_mean() {
+    if (threadIdx.x == 0 && blockIdx.x == 0) A.ctl->q = sh.tot[0] / (double)A.g.I;
+    return sync(false);
+  }
+  __device__ void constants() {
+    if (threadIdx.x < 32) {
+      const double x = threadIdx.x == 0 ? (double)A.g.I : threadIdx.x == 1 ? (double)A.g.J
+                       : threadIdx.x == 2 ? *(volatile double*)&A.ctl->q : A.tau;
+      const double y = log(x), z = 1.0 / x;
+      if (threadIdx.x < 4) sh.consts[threadIdx.x] = y;
+      if (threadIdx.x == 0) sh.dx = z;
+      if (threadIdx.x == 1) sh.dy = z;
+    }
+  }
+  __device__ void reset_gap() {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      A.ctl->gap_num = INFINITY;
+      A.ctl->gap_den = 1.0;
+    }
+  }
+};
+
+// The streamed variant: C read from L2 or HBM in both passes, the FP64 state in
+// global memory (own rows and columns only), any size.
+struct Streamed : PersistBase {
+  int r0, r1, c0, c1;             // owned rows, owned float4 columns
+  float* orow;                    // I   row offsets (on the weight grid); rowc's memory, free during the solve
+  float2* l2col;                  // J   base-2 log-sum-exp of each column: offset on the grid + remainder (Lcol's memory)
+
+  __device__ Streamed(const PersistArgs& args, PersistShared& shared) : PersistBase(args, shared) {
+    const int n = gridDim.x, b = blockIdx.x;
+    r0 = (int)(A.g.I * b / n);
+    r1 = (int)(A.g.I * (b + 1) / n);
+    const int64_t nv = A.g.ldc >> 2;
+    c0 = (int)(nv * b / n);
+    c1 = (int)(nv * (b + 1) / n);
+    orow = reinterpret_cast<float*>(A.V.rowc);
+    l2col = reinterpret_cast<float2*>(A.V.Lcol);
   }
 
   // The reference's a-update (optimal_transport.py:133) of row i from its base-2
@@ -220,8 +365,10 @@ struct Persist {
         i = __shfl_sync(0xffffffffu, i, 0);
         if (i >= e) break;
         float m, s, cmp, h, l;
-        row_lse<true>(reinterpret_cast<const float4*>(A.C + (int64_t)i * A.g.ldc), w4, wl4, A.g.ldc >> 2, lane,
-                      orow[i], k2, k2l, m, s, cmp);
+        // plain loads of the weights: other CTAs wrote them before the last barrier
+        const float4* row = reinterpret_cast<const float4*>(A.C + (int64_t)i * A.g.ldc);
+        row_lse<true>([row](int k) { return ld_stream(row + k); }, [w4](int k) { return w4[k]; },
+                      [wl4](int k) { return wl4[k]; }, (int)(A.g.ldc >> 2), lane, orow[i], k2, k2l, m, s, cmp);
         two_sum(s, -cmp, h, l);
         df_merge_lanes<16, 1>(m, h, l);
         if (lane == 0) sh.res[i - b] = make_float4(m, h, l, 0.f);
@@ -260,7 +407,11 @@ struct Persist {
 #pragma unroll
       for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A.g.J ? l2col[c4 * 4 + q].x : 0.f;
       const int64_t a = (int64_t)r * A.g.rows_per;
-      col_lse<true>(A.C, A.g.ldc, c4, a, min(A.g.I, a + A.g.rows_per), A.V.wrow, A.V.wrow_lo, o, k2, k2l, m, s);
+      const float4* col = reinterpret_cast<const float4*>(A.C) + c4;
+      const int64_t ld4 = A.g.ldc >> 2;
+      const float *wr = A.V.wrow, *wrl = A.V.wrow_lo;
+      col_lse<true>([=](int64_t i) { return ld_stream(col + i * ld4); }, [wr](int64_t i) { return wr[i]; },
+                    [wrl](int64_t i) { return wrl[i]; }, a, min(A.g.I, a + A.g.rows_per), o, k2, k2l, m, s);
       float4* out = reinterpret_cast<float4*>(A.V.part + ((int64_t)c4 * A.g.nrb + r) * 4);
       out[0] = make_float4(m[0], s[0], m[1], s[1]);
       out[1] = make_float4(m[2], s[2], m[3], s[3]);
@@ -365,15 +516,7 @@ struct Persist {
       for (int k = 0; k < 8; ++k) t += sh.sums[k][threadIdx.x];
       A.V.red[blockIdx.x * kNq + threadIdx.x] = t;
     }
-    if (!sync(false)) return false;
-    if (w < NQ) {
-      double t = 0.0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) t += A.V.red[b * kNq + w];
-      t = warp_sum(t);
-      if (lane == 0) sh.tot[w] = t;
-    }
-    __syncthreads();
-    return true;
+    return reduce_ctas<NQ>();
   }
 
   // Stage-exit test (optimal_transport.py:158-160) in the reference's expressions.
@@ -399,24 +542,7 @@ struct Persist {
       acc[rows ? 1 : 3] = a2;
     }
     if (!total<4>(acc, any)) return false;
-    if (threadIdx.x < 32) {
-      const double r = sqrt(sh.tot[threadIdx.x & 3]);
-      const double n = __shfl_sync(0xffffffffu, r, (threadIdx.x & 1) * 2);
-      const double d = __shfl_sync(0xffffffffu, r, (threadIdx.x & 1) * 2 + 1);
-      const double g = n / (1.0 + d);
-      const double ga = __shfl_sync(0xffffffffu, g, 0), gb = __shfl_sync(0xffffffffu, g, 1);
-      const double gap = gb > ga ? gb : ga;   // Python's max: the first unless the second is larger
-      if (threadIdx.x == 0) {
-        sh.decision = gap > 1e-6;
-        if (blockIdx.x == 0) {
-          A.ctl->gap_num = gap;
-          A.ctl->gap_den = 1.0;
-        }
-      }
-    }
-    __syncthreads();
-    *go_on = sh.decision != 0;
-    return true;
+    return stage_decision(go_on);
   }
 
   // Duality-gap test in O(I + J) (see wotg_sinkhorn.cu) after a fresh row phase.
@@ -452,25 +578,7 @@ struct Persist {
       }
     }
     if (!total<7>(acc, any)) return false;
-    if (threadIdx.x == 0) {
-      const double* h = sh.tot;
-      const double dx = 1.0 / (double)A.g.I, dy = 1.0 / (double)A.g.J;
-      const double num = dx * h[0] + dy * h[1];
-      const double pri = c.lambda1 * dx * h[2] + c.lambda2 * dy * h[3] + dx * h[4] + dy * h[5] +
-                         c.eps * (sumk - dx * h[6]);
-      const double den = fabs(pri);
-      // gap = num / den, as a comparison (the quotient is formed once, on the host)
-      const bool isnan_ = num != num || den != den || (num == 0.0 && den == 0.0) || (isinf(num) && isinf(den));
-      sh.decision = isnan_ ? 2 : num > A.tolerance * den ? 1 : 0;
-      if (blockIdx.x == 0) {
-        A.ctl->gap_num = num;
-        A.ctl->gap_den = den;
-      }
-    }
-    __syncthreads();
-    *go_on = sh.decision == 1;
-    *nan = sh.decision == 2;
-    return true;
+    return gap_decision(sumk, go_on, nan);
   }
 
   // sum_ij exp(-kappa C_ij) / (I J) (the reference's sum of its _K).
@@ -486,23 +594,7 @@ struct Persist {
         df_add(h, l, (ex2(-k2 * cc.x) + ex2(-k2 * cc.y)) + (ex2(-k2 * cc.z) + ex2(-k2 * cc.w)), 0.f);
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
-      df_add(h, l, h2, l2);
-    }
-    __syncthreads();
-    if (lane == 0) sh.res[threadIdx.x >> 5] = make_float4(h, l, 0.f, 0.f);
-    __syncthreads();
-    double acc[1] = {0.0};
-    if (threadIdx.x < kPersistWarps) {
-      const float4 r = sh.res[threadIdx.x];
-      acc[0] = (double)r.x + (double)r.y;
-    }
-    __syncthreads();
-    if (!total<1>(acc, threadIdx.x < kPersistWarps)) return false;
-    *out = sh.tot[0] / ((double)A.g.I * (double)A.g.J);
-    return true;
+    return total_pairs(h, l, out);
   }
 
   __device__ bool mean_growth() {
@@ -514,160 +606,193 @@ struct Persist {
         any = true;
       }
     if (!total<1>(acc, any)) return false;
-    if (threadIdx.x == 0 && blockIdx.x == 0) A.ctl->q = sh.tot[0] / (double)A.g.I;
-    return sync(false);
+    return publish_mean();
   }
 
   // Absorbs with the old epsilon and starts a stage at `eps`.
   __device__ bool start_stage(double eps_old, double eps) {
     set_coef(eps);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      A.ctl->gap_num = INFINITY;
-      A.ctl->gap_den = 1.0;
-    }
+    reset_gap();
     absorb<true>(eps_old);
     return sync(false);
   }
-
-  __device__ void run() {
-    PersistCtl* ctl = A.ctl;
-    const int n = gridDim.x, b = blockIdx.x;
-    target = n;
-    flags = 0;
-    r0 = (int)(A.g.I * b / n);
-    r1 = (int)(A.g.I * (b + 1) / n);
-    const int64_t nv = A.g.ldc >> 2;
-    c0 = (int)(nv * b / n);
-    c1 = (int)(nv * (b + 1) / n);
-    orow = reinterpret_cast<float*>(A.V.rowc);
-    l2col = reinterpret_cast<float2*>(A.V.Lcol);
-    for (int i = threadIdx.x; i < kLogTable; i += kPersistThreads) sh.tab[i] = log_table_entry(i);
-    // the state this launch starts from (CTA 0 writes it back at the end, after
-    // barriers that every CTA has passed)
-    double eps = ctl->eps, sumk = ctl->sumk;
-    long long it = ctl->it, checks = ctl->checks, absorptions = ctl->absorptions;
-    int stage = ctl->stage, status = ctl->status, lrow_valid = ctl->lrow_valid, since = ctl->since,
-        index = ctl->index;
-    const int started = ctl->started;
-    if (status != kRunning) return;
-    if (!started && !mean_growth()) return;
-    if (threadIdx.x < 32) {
-      const double x = threadIdx.x == 0 ? (double)A.g.I : threadIdx.x == 1 ? (double)A.g.J
-                       : threadIdx.x == 2 ? *(volatile double*)&ctl->q : A.tau;
-      const double y = log(x);
-      if (threadIdx.x < 4) sh.consts[threadIdx.x] = y;
-    }
-    if (started) set_coef(eps);
-    long long used = 0;
-    bool ok = true, absorb_now = false;
-    if (A.mode == kModeGap) {
-      if (!started) {
-        // epsilon0 * factor / factor, as the reference's arithmetic
-        const double old = A.epsilon0 * A.scale_factor;
-        eps = old / A.scale_factor;
-        ok = start_stage(old, eps);
-      }
-      bool stage_done = false;
-      while (ok && status == kRunning && used < A.budget) {
-        if (stage_done) {
-          const double old = eps;
-          eps = eps / A.scale_factor;
-          ++stage;
-          lrow_valid = 0;
-          stage_done = false;
-          if (!(ok = start_stage(old, eps))) break;
-          if (stage == kScalings && !(ok = sum_exp(&sumk))) break;
-        }
-        const int nb = stage == kScalings ? A.batch_size : 5;
-        for (int t = 0; t < nb; ++t) {
-          ++it;
-          ++used;
-          if (!(ok = iterate(lrow_valid != 0, &absorb_now))) break;
-          lrow_valid = 0;
-          if (absorb_now) {
-            ++absorptions;
-            absorb<false>(eps);
-            if (!(ok = sync(false))) break;
-          }
-          if ((double)it >= A.max_iter) {
-            status = kMaxIter;
-            break;
-          }
-        }
-        if (!ok) break;
-        if (status == kMaxIter) {
-          row_phase<true>();
-          break;
-        }
-        ++checks;
-        bool go_on = true, nan = false;
-        if (stage == kScalings) {
-          row_phase<true>();
-          lrow_valid = 1;
-          __syncthreads();
-          if (!(ok = gap_test(sumk, &go_on, &nan))) break;
-          if (!go_on) status = nan ? kNonfinite : kConverged;
-        } else {
-          if (!(ok = stage_test(&go_on))) break;
-          stage_done = !go_on;
-          if (stage_done && used >= A.budget) used = A.budget - 1;   // the next launch starts inside a stage
-        }
-      }
-    } else {
-      const bool fixed = A.mode == kModeFixed;
-      if (!started) {
-        eps = fixed ? A.epsilon0 : A.epsilon;
-        if (fixed) {
-          ok = start_stage(0.0, eps);
-        } else {
-          set_coef(eps);   // potentials loaded with a = b = 1
-        }
-      }
-      const long long with_absorb = fixed ? A.scaling_iter : A.n_iter;
-      const long long total_it = with_absorb + (fixed ? A.extra_iter : 0);
-      while (ok && it < total_it && used < A.budget) {
-        ++used;
-        if (!(ok = iterate(false, &absorb_now))) break;
-        if (it < with_absorb && absorb_now) {
-          ++absorptions;
-          absorb<false>(eps);
-          if (!(ok = sync(false))) break;
-        }
-        ++it;
-        if (fixed && it <= with_absorb && ++since == A.inner_iter_max) {
-          ++index;
-          since = 0;
-          const double eps_new = (A.epsilon0 - A.epsilon) * exp(-(double)index) + A.epsilon;
-          const double old = eps;
-          eps = eps_new;
-          if (!(ok = start_stage(old, eps))) break;
-        }
-      }
-      if (ok && it >= total_it) {
-        if (fixed) row_phase<true>();
-        status = kConverged;
-      }
-    }
-    if (ok && b == 0 && threadIdx.x == 0) {
-      ctl->eps = eps;
-      ctl->sumk = sumk;
-      ctl->it = it;
-      ctl->checks = checks;
-      ctl->absorptions = absorptions;
-      ctl->stage = stage;
-      ctl->status = status;
-      ctl->lrow_valid = lrow_valid;
-      ctl->started = 1;
-      ctl->since = since;
-      ctl->index = index;
-    }
+  __device__ bool absorb_now(double eps) {
+    absorb<false>(eps);
+    return sync(false);
   }
+  __device__ void fresh() {
+    row_phase<true>();
+    __syncthreads();
+  }
+  // Refinement starts from loaded potentials and weights.
+  __device__ bool start_refine(double eps) {
+    set_coef(eps);
+    return true;
+  }
+  __device__ bool resume(double eps) {
+    set_coef(eps);
+    return true;
+  }
+  __device__ bool save(bool done) { return true; }
 };
 
-__global__ void __launch_bounds__(kPersistThreads, 1) persist_kernel(PersistArgs A) {
+// The reference's control (stages, batches, tests) over a variant's phases.
+// Every CTA runs it on its own copy of the state (sh.rs).
+template <bool GAP, class P>
+__device__ void persist_run(P& p) {
+  const PersistArgs& A = p.A;
+  PersistCtl* ctl = A.ctl;
+  RunState& rs = p.sh.rs;
+  // one thread changes the state, between two barriers of the CTA
+  auto change = [&](auto f) {
+    __syncthreads();
+    if (threadIdx.x == 0) f();
+    __syncthreads();
+  };
+  // the state this launch starts from (CTA 0 writes it back at the end, after
+  // barriers that every CTA has passed)
+  const int started = ctl->started;
+  change([&] {
+    rs.eps = ctl->eps;
+    rs.sumk = ctl->sumk;
+    rs.it = ctl->it;
+    rs.checks = ctl->checks;
+    rs.absorptions = ctl->absorptions;
+    rs.used = 0;
+    rs.stage = ctl->stage;
+    rs.status = ctl->status;
+    rs.lrow_valid = ctl->lrow_valid;
+    rs.since = ctl->since;
+    rs.index = ctl->index;
+    rs.stage_done = 0;
+  });
+  if (rs.status != kRunning) return;
+  if (!started && !p.mean_growth()) return;
+  p.constants();
+  if (started && !p.resume(rs.eps)) return;
+  if constexpr (GAP) {
+    if (!started) {
+      // epsilon0 * factor / factor, as the reference's arithmetic
+      const double old = A.epsilon0 * A.scale_factor;
+      change([&] { rs.eps = old / A.scale_factor; });
+      if (!p.start_stage(old, rs.eps)) return;
+    }
+    while (rs.status == kRunning && rs.used < A.budget) {
+      if (rs.stage_done) {
+        const double old = rs.eps;
+        change([&] {
+          rs.eps = old / A.scale_factor;
+          ++rs.stage;
+          rs.lrow_valid = 0;
+          rs.stage_done = 0;
+        });
+        if (!p.start_stage(old, rs.eps)) return;
+        if (rs.stage == kScalings) {
+          double sumk;
+          if (!p.sum_exp(&sumk)) return;
+          change([&] { rs.sumk = sumk; });
+        }
+      }
+      const int nb = rs.stage == kScalings ? A.batch_size : 5;
+      bool cached = rs.lrow_valid != 0, last = false;
+      int t = 0;
+      while (t < nb && !last) {
+        bool over = false;
+        if (!p.iterate(cached, &over)) return;
+        cached = false;
+        ++t;
+        if (over) {
+          change([&] { ++rs.absorptions; });
+          if (!p.absorb_now(rs.eps)) return;
+        }
+        last = (double)(rs.it + t) >= A.max_iter;
+      }
+      change([&] {
+        rs.it += t;
+        rs.used += t;
+        rs.lrow_valid = 0;
+        if (last)
+          rs.status = kMaxIter;
+        else
+          ++rs.checks;
+      });
+      if (last) {
+        p.fresh();
+        break;
+      }
+      bool go_on = true, nan = false;
+      if (rs.stage == kScalings) {
+        p.fresh();
+        if (!p.gap_test(rs.sumk, &go_on, &nan)) return;
+        change([&] {
+          rs.lrow_valid = 1;
+          if (!go_on) rs.status = nan ? kNonfinite : kConverged;
+        });
+      } else {
+        if (!p.stage_test(&go_on)) return;
+        change([&] {
+          rs.stage_done = !go_on;
+          if (!go_on && rs.used >= A.budget) rs.used = A.budget - 1;   // the next launch starts inside a stage
+        });
+      }
+    }
+  } else {
+    const bool fixed = A.mode == kModeFixed;
+    if (!started) {
+      change([&] { rs.eps = fixed ? A.epsilon0 : A.epsilon; });
+      if (!(fixed ? p.start_stage(0.0, rs.eps) : p.start_refine(rs.eps))) return;
+    }
+    const long long with_absorb = fixed ? A.scaling_iter : A.n_iter;
+    const long long total_it = with_absorb + (fixed ? A.extra_iter : 0);
+    while (rs.it < total_it && rs.used < A.budget) {
+      bool over = false;
+      if (!p.iterate(false, &over)) return;
+      if (over && rs.it < with_absorb) {
+        change([&] { ++rs.absorptions; });
+        if (!p.absorb_now(rs.eps)) return;
+      }
+      const double old = rs.eps;
+      bool new_eps = false;
+      if (fixed && rs.it < with_absorb) new_eps = rs.since + 1 == A.inner_iter_max;
+      change([&] {
+        ++rs.it;
+        ++rs.used;
+        if (fixed) ++rs.since;
+        if (new_eps) {
+          ++rs.index;
+          rs.since = 0;
+          rs.eps = (A.epsilon0 - A.epsilon) * exp(-(double)rs.index) + A.epsilon;
+        }
+      });
+      if (new_eps && !p.start_stage(old, rs.eps)) return;
+    }
+    if (rs.it >= total_it) {
+      if (fixed) p.fresh();
+      change([&] { rs.status = kConverged; });
+    }
+  }
+  if (!p.save(rs.status != kRunning)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->eps = rs.eps;
+    ctl->sumk = rs.sumk;
+    ctl->it = rs.it;
+    ctl->checks = rs.checks;
+    ctl->absorptions = rs.absorptions;
+    ctl->stage = rs.stage;
+    ctl->status = rs.status;
+    ctl->lrow_valid = rs.lrow_valid;
+    ctl->started = 1;
+    ctl->since = rs.since;
+    ctl->index = rs.index;
+  }
+}
+
+// GAP: the duality-gap solver (kModeGap); else kModeFixed or kModeRefine.
+template <bool GAP>
+__global__ void __launch_bounds__(kPersistThreads, 1) persist_kernel(const __grid_constant__ PersistArgs A) {
   __shared__ PersistShared sh;
-  Persist p{A, sh, 0, 0, 0, 0, 0, 0, nullptr, nullptr};
-  p.run();
+  Streamed p(A, sh);
+  persist_run<GAP>(p);
 }
 
 }  // namespace wotg

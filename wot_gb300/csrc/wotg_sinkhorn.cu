@@ -36,6 +36,7 @@
 #include "wotg_common.cuh"
 #include "wotg_onthefly.cuh"
 #include "wotg_persist.cuh"
+#include "wotg_resident.cuh"
 #include "wotg_state.cuh"
 #include "wotg_tc_kernel.cuh"
 
@@ -124,7 +125,9 @@ __global__ void __launch_bounds__(256) row_pass_kernel(const float* __restrict__
   const float4* w4 = reinterpret_cast<const float4*>(w);
   for (int64_t i = warp; i < g.I; i += nwarps) {
     float m, s, cmp;
-    row_lse<false>(reinterpret_cast<const float4*>(C + i * g.ldc), w4, w4, g.ldc >> 2, lane, 0.f, k2, 0.f, m, s, cmp);
+    const float4* row = reinterpret_cast<const float4*>(C + i * g.ldc);
+    auto wk = [w4](int k) { return __ldg(w4 + k); };
+    row_lse<false>([row](int k) { return ld_stream(row + k); }, wk, wk, (int)(g.ldc >> 2), lane, 0.f, k2, 0.f, m, s, cmp);
     warp_lse(m, s);
     if (lane == 0) L[i] = ((double)m + log2((double)s)) * kLn2;
   }
@@ -148,7 +151,11 @@ __global__ void __launch_bounds__(256) col_partial_kernel(const float* __restric
   if (c4 >= g.ldc >> 2) return;
   const float o[4] = {0.f, 0.f, 0.f, 0.f};
   float m[4], s[4];
-  col_lse<false>(C, g.ldc, c4, r0, min(g.I, r0 + g.rows_per), w, w, o, k2, 0.f, m, s);
+  const float4* col = reinterpret_cast<const float4*>(C) + c4;
+  const int64_t ld4 = g.ldc >> 2;
+  auto wi = [w](int64_t i) { return __ldg(w + i); };
+  col_lse<false>([=](int64_t i) { return ld_stream(col + i * ld4); }, wi, wi, r0, min(g.I, r0 + g.rows_per), o, k2, 0.f,
+                 m, s);
   float4* out = reinterpret_cast<float4*>(part + (int64_t)blockIdx.y * g.ldc + c4 * 4);
   out[0] = make_float4(m[0], s[0], m[1], s[1]);
   out[1] = make_float4(m[2], s[2], m[3], s[3]);
@@ -960,6 +967,25 @@ struct SolveResult {
   Coef final_coef{};
 };
 
+// Shared memory the resident kernels may use beside their static part; their
+// limit is raised to it once per device.
+static int resident_room(int* room) {
+  static std::atomic<int> known[64] = {};
+  int dev = 0;
+  WOTG_CUDA(cudaGetDevice(&dev));
+  if (dev < 64 && (*room = known[dev].load(std::memory_order_acquire)) > 0) return WOTG_OK;
+  int limit = 0;
+  cudaFuncAttributes a{}, b{};
+  WOTG_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  WOTG_CUDA(cudaFuncGetAttributes(&a, resident_kernel<true>));
+  WOTG_CUDA(cudaFuncGetAttributes(&b, resident_kernel<false>));
+  *room = limit - (int)std::max(a.sharedSizeBytes, b.sharedSizeBytes);
+  WOTG_CUDA(cudaFuncSetAttribute(resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, *room));
+  WOTG_CUDA(cudaFuncSetAttribute(resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, *room));
+  if (dev < 64) known[dev].store(*room, std::memory_order_release);
+  return WOTG_OK;
+}
+
 // A materialised solve (mode kModeGap / kModeFixed) or n_iter refinement
 // iterations at epsilon `eps` (kModeRefine): launches of persist_kernel until
 // it reports an end. A launch is kept to some 20 ms (its iterations cost about
@@ -992,17 +1018,42 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
   WOTG_CUDA(cudaMemsetAsync(A.ctl, 0, sizeof(PersistCtl), S.st));
   // one CTA per SM; fewer only where the device grants the process fewer SMs
   int grid = std::min(sm_count(), kRedBlocks);
+  bool resident = false;
+  int rows_cap = 0, cols_cap = 0;
+  size_t smem = 0;
+  {
+    const ResidentPlan plan = resident_plan(S.g, grid);
+    int room = 0;
+    int s = resident_room(&room);
+    if (s) return s;
+    resident = resident_fits(plan, S.g, (size_t)room);
+    if (resident) {
+      grid = plan.grid;
+      rows_cap = plan.rows;
+      cols_cap = plan.cols4 * 4;
+      smem = plan.bytes;
+    }
+  }
+  const bool gap = mode == kModeGap;
+  const void* streamed = gap ? reinterpret_cast<const void*>(persist_kernel<true>)
+                             : reinterpret_cast<const void*>(persist_kernel<false>);
+  const void* kernel = !resident ? streamed
+                       : gap     ? reinterpret_cast<const void*>(resident_kernel<true>)
+                                 : reinterpret_cast<const void*>(resident_kernel<false>);
   PersistCtl h{};
   for (;;) {
     WOTG_CUDA(cudaMemsetAsync(&A.ctl->bar, 0, 2 * sizeof(unsigned long long), S.st));
-    void* args[] = {&A};
-    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(persist_kernel), dim3(grid),
-                                                dim3(kPersistThreads), args, 0, S.st);
-    while (e == cudaErrorCooperativeLaunchTooLarge && grid > 1) {
+    void* args[] = {&A, &rows_cap, &cols_cap};
+    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid),
+                                                dim3(kernel == streamed ? kPersistThreads : kResidentThreads), args,
+                                                smem, S.st);
+    while (e == cudaErrorCooperativeLaunchTooLarge && (kernel != streamed || grid > 1)) {
+      // fewer SMs than the device has: the streamed variant runs on any number
       cudaGetLastError();
-      grid /= 2;
-      e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(persist_kernel), dim3(grid),
-                                      dim3(kPersistThreads), args, 0, S.st);
+      if (kernel == streamed) grid /= 2;
+      kernel = streamed;
+      smem = 0;
+      e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kPersistThreads), args, smem, S.st);
     }
     WOTG_CUDA(e);
     WOTG_LAUNCHED();

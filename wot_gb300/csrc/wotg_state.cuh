@@ -64,121 +64,106 @@ __device__ __forceinline__ float expo(float cc, float w, float wl, float o, floa
   return fmaf(-k2, cc, w);
 }
 
-// One lane's share of a row's online base-2 LSE: float4 columns lane, lane + 32,
-// ... of the row against the weights w4 (+ wl4); (m, s) as partial s 2^m, with
-// PREC the sum compensated, s - cmp. The loads of the weights are plain ones:
-// in the persistent solver other CTAs wrote them before the last grid barrier.
+// One step of an online base-2 LSE: the partial (m, s) (with PREC the sum
+// compensated, s - cmp) takes in the four exponents x.
 template <bool PREC>
-__device__ __forceinline__ void row_lse(const float4* __restrict__ row, const float4* w4, const float4* wl4,
-                                        int64_t nv, int lane, float o, float k2, float k2l, float& m, float& s,
-                                        float& cmp) {
+__device__ __forceinline__ void lse_step(float x0, float x1, float x2, float x3, float& m, float& s, float& cmp) {
+  const float mn = fmaxf(m, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
+  const float r = ex2(m - mn);
+  const float v = (ex2(x0 - mn) + ex2(x1 - mn)) + (ex2(x2 - mn) + ex2(x3 - mn));
+  if (PREC) {
+    s = __fmul_rn(s, r);
+    cmp = __fmul_rn(cmp, r);
+    kahan_add(s, cmp, v);
+  } else {
+    s = s * r + v;
+  }
+  m = mn;
+}
+
+// One lane's share of a row's online base-2 LSE: float4 columns lane, lane + 32,
+// ... < nv, in order; (m, s) as partial s 2^m, with PREC the sum compensated,
+// s - cmp. cost(k), w(k), wl(k) load float4 k of the row, the weights and their
+// low parts (from global or shared memory).
+template <bool PREC, class Cost, class W, class Wl>
+__device__ __forceinline__ void row_lse(const Cost& cost, const W& w, const Wl& wl, int nv, int lane, float o, float k2,
+                                        float k2l, float& m, float& s, float& cmp) {
   m = kNegBig;
   s = 0.f;
   cmp = 0.f;
-  int64_t k = lane;
+  auto step = [&](const float4& cc, const float4& ww, const float4& wlo) {
+    lse_step<PREC>(expo<PREC>(cc.x, ww.x, wlo.x, o, k2, k2l), expo<PREC>(cc.y, ww.y, wlo.y, o, k2, k2l),
+                   expo<PREC>(cc.z, ww.z, wlo.z, o, k2, k2l), expo<PREC>(cc.w, ww.w, wlo.w, o, k2, k2l), m, s, cmp);
+  };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   // the cost loads of the next 128-float4 chunk are issued before this
   // chunk's arithmetic (two chunks of loads in flight per lane)
   float4 cn[4];
-  if (k + 96 < nv) {
 #pragma unroll
-    for (int t = 0; t < 4; ++t) cn[t] = ld_stream(row + k + 32 * t);
-  }
-  for (; k + 96 < nv; k += 128) {
-    float4 cc[4], ww[4], wl[4];
+  for (int t = 0; t < 4; ++t)
+    if (lane + 32 * t < nv) cn[t] = cost(lane + 32 * t);
+  int k = lane;
+  const int full = nv & ~127;   // whole chunks; the last, partial one follows
+  for (; k < full; k += 128) {
+    float4 cc[4], ww[4], wlo[4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) cc[t] = cn[t];
-    if (k + 128 + 96 < nv) {
 #pragma unroll
-      for (int t = 0; t < 4; ++t) cn[t] = ld_stream(row + k + 128 + 32 * t);
-    }
+    for (int t = 0; t < 4; ++t)
+      if (k + 128 + 32 * t < nv) cn[t] = cost(k + 128 + 32 * t);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) ww[t] = w4[k + 32 * t];
+    for (int t = 0; t < 4; ++t) ww[t] = w(k + 32 * t);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) wl[t] = PREC ? wl4[k + 32 * t] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = 0; t < 4; ++t) wlo[t] = PREC ? wl(k + 32 * t) : zero;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float x0 = expo<PREC>(cc[t].x, ww[t].x, wl[t].x, o, k2, k2l);
-      const float x1 = expo<PREC>(cc[t].y, ww[t].y, wl[t].y, o, k2, k2l);
-      const float x2 = expo<PREC>(cc[t].z, ww[t].z, wl[t].z, o, k2, k2l);
-      const float x3 = expo<PREC>(cc[t].w, ww[t].w, wl[t].w, o, k2, k2l);
-      const float mn = fmaxf(m, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
-      const float r = ex2(m - mn);
-      const float v = (ex2(x0 - mn) + ex2(x1 - mn)) + (ex2(x2 - mn) + ex2(x3 - mn));
-      if (PREC) {
-        s = __fmul_rn(s, r);
-        cmp = __fmul_rn(cmp, r);
-        kahan_add(s, cmp, v);
-      } else {
-        s = s * r + v;
-      }
-      m = mn;
-    }
+    for (int t = 0; t < 4; ++t) step(cc[t], ww[t], wlo[t]);
   }
-  for (; k < nv; k += 32) {
-    const float4 cc = ld_stream(row + k);
-    const float4 ww = w4[k];
-    const float4 wl = PREC ? wl4[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float x0 = expo<PREC>(cc.x, ww.x, wl.x, o, k2, k2l);
-    const float x1 = expo<PREC>(cc.y, ww.y, wl.y, o, k2, k2l);
-    const float x2 = expo<PREC>(cc.z, ww.z, wl.z, o, k2, k2l);
-    const float x3 = expo<PREC>(cc.w, ww.w, wl.w, o, k2, k2l);
-    const float mn = fmaxf(m, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
-    const float r = ex2(m - mn);
-    const float v = (ex2(x0 - mn) + ex2(x1 - mn)) + (ex2(x2 - mn) + ex2(x3 - mn));
-    if (PREC) {
-      s = __fmul_rn(s, r);
-      cmp = __fmul_rn(cmp, r);
-      kahan_add(s, cmp, v);
-    } else {
-      s = s * r + v;
-    }
-    m = mn;
-  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (k + 32 * t < nv) step(cn[t], w(k + 32 * t), PREC ? wl(k + 32 * t) : zero);
 }
 
-// One thread's share of a column pass: the online base-2 LSE of the 4 columns
-// of float4 column c4 over rows [r0, r1), in chunks of kColRowChunk rows; the
-// row weights are wrow (+ wrow_lo), o the columns' offsets (PREC).
+// One thread's share of a column pass: the online base-2 LSE of 4 columns over
+// rows [r0, r1), in chunks of kColRowChunk rows. cost(i) loads the columns'
+// float4 of row i, w(i) and wl(i) the row's weight; o the columns' offsets (PREC).
 constexpr int kColRowChunk = 4;
 
-template <bool PREC>
-__device__ __forceinline__ void col_lse(const float* __restrict__ C, int64_t ldc, int64_t c4, int64_t r0, int64_t r1,
-                                        const float* wrow, const float* wrow_lo, const float (&o)[4], float k2,
-                                        float k2l, float (&m)[4], float (&s)[4]) {
+template <bool PREC, class I, class Cost, class W, class Wl>
+__device__ __forceinline__ void col_lse(const Cost& cost, const W& w, const Wl& wl, I r0, I r1, const float (&o)[4],
+                                        float k2, float k2l, float (&m)[4], float (&s)[4]) {
   float cmp[4] = {0.f, 0.f, 0.f, 0.f};   // PREC: compensated sums s - cmp
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     m[q] = kNegBig;
     s[q] = 0.f;
   }
-  int64_t i = r0;
+  I i = r0;
   // the next chunk's cost loads are issued before this chunk's arithmetic
   float4 cn[kColRowChunk];
   if (i + kColRowChunk <= r1) {
 #pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) cn[t] = ld_stream(reinterpret_cast<const float4*>(C + (i + t) * ldc) + c4);
+    for (int t = 0; t < kColRowChunk; ++t) cn[t] = cost(i + t);
   }
   for (; i + kColRowChunk <= r1; i += kColRowChunk) {
     float4 cc[kColRowChunk];
-    float w[kColRowChunk], wl[kColRowChunk];
+    float ww[kColRowChunk], wlo[kColRowChunk];
 #pragma unroll
     for (int t = 0; t < kColRowChunk; ++t) cc[t] = cn[t];
     if (i + 2 * kColRowChunk <= r1) {
 #pragma unroll
-      for (int t = 0; t < kColRowChunk; ++t)
-        cn[t] = ld_stream(reinterpret_cast<const float4*>(C + (i + kColRowChunk + t) * ldc) + c4);
+      for (int t = 0; t < kColRowChunk; ++t) cn[t] = cost(i + kColRowChunk + t);
     }
 #pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) w[t] = wrow[i + t];
+    for (int t = 0; t < kColRowChunk; ++t) ww[t] = w(i + t);
 #pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) wl[t] = PREC ? wrow_lo[i + t] : 0.f;
+    for (int t = 0; t < kColRowChunk; ++t) wlo[t] = PREC ? wl(i + t) : 0.f;
     float x[4][kColRowChunk];
 #pragma unroll
     for (int t = 0; t < kColRowChunk; ++t) {
-      x[0][t] = expo<PREC>(cc[t].x, w[t], wl[t], o[0], k2, k2l);
-      x[1][t] = expo<PREC>(cc[t].y, w[t], wl[t], o[1], k2, k2l);
-      x[2][t] = expo<PREC>(cc[t].z, w[t], wl[t], o[2], k2, k2l);
-      x[3][t] = expo<PREC>(cc[t].w, w[t], wl[t], o[3], k2, k2l);
+      x[0][t] = expo<PREC>(cc[t].x, ww[t], wlo[t], o[0], k2, k2l);
+      x[1][t] = expo<PREC>(cc[t].y, ww[t], wlo[t], o[1], k2, k2l);
+      x[2][t] = expo<PREC>(cc[t].z, ww[t], wlo[t], o[2], k2, k2l);
+      x[3][t] = expo<PREC>(cc[t].w, ww[t], wlo[t], o[3], k2, k2l);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -201,11 +186,11 @@ __device__ __forceinline__ void col_lse(const float* __restrict__ C, int64_t ldc
     }
   }
   for (; i < r1; ++i) {
-    const float4 cc = ld_stream(reinterpret_cast<const float4*>(C + i * ldc) + c4);
-    const float w = wrow[i];
-    const float wl = PREC ? wrow_lo[i] : 0.f;
-    const float xs[4] = {expo<PREC>(cc.x, w, wl, o[0], k2, k2l), expo<PREC>(cc.y, w, wl, o[1], k2, k2l),
-                         expo<PREC>(cc.z, w, wl, o[2], k2, k2l), expo<PREC>(cc.w, w, wl, o[3], k2, k2l)};
+    const float4 cc = cost(i);
+    const float ww = w(i);
+    const float wlo = PREC ? wl(i) : 0.f;
+    const float xs[4] = {expo<PREC>(cc.x, ww, wlo, o[0], k2, k2l), expo<PREC>(cc.y, ww, wlo, o[1], k2, k2l),
+                         expo<PREC>(cc.z, ww, wlo, o[2], k2, k2l), expo<PREC>(cc.w, ww, wlo, o[3], k2, k2l)};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float mn = fmaxf(m[q], xs[q]);
