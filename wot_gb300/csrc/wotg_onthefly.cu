@@ -106,24 +106,10 @@ __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restric
 // ---------------------------------------------------------------------------
 __global__ void tc_pack_kernel(const float* __restrict__ X, int64_t n, int64_t ldx, int d, int kp, float scale,
                                int row_form, __half* __restrict__ tiles, double* __restrict__ norm) {
-  const int64_t ntiles = (n + 127) / 128;
-  const int64_t total = ntiles * 128 * kp;
-  const int64_t tile_halfs = (int64_t)2 * 128 * kp;
+  const int64_t total = (n + 127) / 128 * 128 * kp;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = idx / kp;
-    const int k = (int)(idx % kp);
-    float x = 0.f;
-    if (k < d) x = i < n ? scale * X[i * ldx + k] : 0.f;
-    else if (row_form && k < d + 2) x = 1.f;
-    else if (!row_form && i >= n && k == d) x = -60000.f;
-    __half h, l;
-    tc::split_f16(x, h, l);
-    __half* tile = tiles + (i / 128) * tile_halfs;
-    const uint32_t off = tc::core_offset((int)(i % 128), k, kp) >> 1;
-    tile[off] = h;
-    tile[128 * kp + off] = l;
-  }
+       idx += (int64_t)gridDim.x * blockDim.x)
+    tc_pack_entry(X, n, ldx, d, kp, scale, row_form, tiles, idx);
   if (norm) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
       double s = 0.0;

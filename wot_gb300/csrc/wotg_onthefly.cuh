@@ -31,16 +31,18 @@ int tc_pack_bias(int64_t n, const double* pot, const double* lsc, const double* 
 __device__ __forceinline__ void tc_write_bias(int64_t i, double beta, int d, int kp, __half* tiles) {
   __half h1, l1, h2, l2;
   const __half zero = __float2half_rn(0.f);
-  if (beta != beta || beta == INFINITY) {
+  const float b1 = (float)beta;
+  if (!(b1 < INFINITY)) {   // NaN or +inf
     h1 = __float2half_rn(NAN);
     l1 = h2 = l2 = zero;
-  } else if (beta < -60000.0) {
+  } else if (b1 < -60000.f) {
     h1 = __float2half_rn(-60000.f);
     l1 = h2 = l2 = zero;
   } else {
-    const float b1 = (float)beta;
+    // h1 + l1 is exact in FP32 (a multiple of b1's last bit), so one conversion and one
+    // difference give the exact remainder (an FP64 instruction is 64 cycles on this part)
     tc::split_f16(b1, h1, l1);
-    const float b2 = (float)(beta - (double)__half2float(h1) - (double)__half2float(l1));
+    const float b2 = (float)(beta - (double)(__half2float(h1) + __half2float(l1)));
     tc::split_f16(b2, h2, l2);
   }
   __half* tile = tiles + (i / 128) * ((int64_t)2 * 128 * kp);
@@ -52,14 +54,24 @@ __device__ __forceinline__ void tc_write_bias(int64_t i, double beta, int d, int
   tile[128 * kp + o2] = l2;
 }
 
-// Where a kernel that changes the potential or the log-scaling of a point
-// writes that point's column-form bias (tiles = nullptr: nowhere):
-//   bias_i = (pot_i / eps + lsc_i) log2 e - kappa log2 e |x_i|^2.
-struct TcBias {
-  __half* tiles;
-  const double* norm;
-  int d, kp;
-};
+// Entry k of the packing of n points (K-major core matrices, FP16 hi then lo
+// blocks per 128-point tile; see the packing kernel): row form [scale x, 1, 1],
+// column form [scale x, bias columns], points past n zero with the bias of weight 0.
+__device__ __forceinline__ void tc_pack_entry(const float* __restrict__ X, int64_t n, int64_t ldx, int d, int kp,
+                                              float scale, int row_form, __half* __restrict__ tiles, int64_t idx) {
+  const int64_t i = idx / kp;
+  const int k = (int)(idx % kp);
+  float x = 0.f;
+  if (k < d) x = i < n ? scale * X[i * ldx + k] : 0.f;
+  else if (row_form && k < d + 2) x = 1.f;
+  else if (!row_form && i >= n && k == d) x = -60000.f;
+  __half h, l;
+  tc::split_f16(x, h, l);
+  __half* tile = tiles + (i / 128) * ((int64_t)2 * 128 * kp);
+  const uint32_t off = tc::core_offset((int)(i % 128), k, kp) >> 1;
+  tile[off] = h;
+  tile[128 * kp + off] = l;
+}
 
 // Resident CTAs per SM of the tensor-core half-step kernel.
 int tc_ctas_per_sm(int kp);

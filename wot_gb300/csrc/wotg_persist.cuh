@@ -30,6 +30,8 @@
 // state in PersistCtl, so that no launch is long.
 #pragma once
 
+#include <stddef.h>
+
 #include "wotg_df.cuh"
 #include "wotg_state.cuh"
 
@@ -49,7 +51,7 @@ struct PersistCtl {
   double gap_num, gap_den;        // the last relative gap as a quotient
   long long it, checks, absorptions;
   int stage, status, lrow_valid, started, since, index, epoch, pad_;
-  unsigned long long bar;         // arrivals (low word) and absorption flags (high word); zeroed per launch
+  unsigned long long bar;         // grid barrier: arrivals and flags (PersistBase::sync); zeroed per launch
   int err, pad2_;                 // zeroed per launch
 };
 
@@ -72,21 +74,60 @@ struct RunState {
   int stage, status, lrow_valid, since, index, stage_done;
 };
 
+// A virtual CTA's tiles in a tensor-core half-step (wotg_tc_persist.cuh).
+struct TcStretch {
+  int n, t, q, nseg, nq;
+};
+
+// A CTA's working state, at the start of its dynamic shared memory (hdr()). The
+// variants are stateless: what they keep between phases is here, and not in an
+// object on the stack, because the phases are functions of their own and a
+// stack access after a grid barrier (whose acquire empties L1) is a trip to L2.
 struct PersistShared {
-  float4 tab[kLogTable];
-  float4 res[kPersistBlk];        // merged (m, h, l) per row or column of a round
+  float2 pairs[32];               // a pair sum per warp
   double sums[8][kNq];
   double tot[kNq];
   Coef c;
   double a1ln2, a1logj, ku, a2ln2, bconst, kv, iel2;   // folded update coefficients
-  float a1h, a1l, a2h, a2l;       // alpha1, alpha2 as pairs
   double consts[4];               // log I, log J, log q, log tau
   double dx, dy;                  // 1 / I, 1 / J
+  float a1h, a1l, a2h, a2l;       // alpha1, alpha2 as pairs
   RunState rs;
-  unsigned long long bar;
-  int off[32];                    // resident variant: its arrays' places in dynamic shared memory
-  int ticket, ok, decision;
+  unsigned int target;            // barrier arrivals that complete the next barrier
+  unsigned int flags, flags2;     // barrier flags seen so far (absorption; rows to recompute)
+  int flagged, flagged2;          // raised at the last barrier
+  int ok, decision, ticket;
+  int r0, r1, j0, j1, c0, c1;     // owned rows, columns, float4 columns
+  int row_flag, over_flag;        // a row to recompute / a scaling above tau, since the half-step began
+  int row_ok, col_ok;             // on-the-fly: offsets of the side exist for this epsilon
+  int jbase[2], segbase[2];       // on-the-fly, per half: tiles and segments of the half-steps before
+  int copied[2], copied_seg[2];   // and the producer's own count
+  TcStretch stretch[2][2];        // on-the-fly: of either side, per half
+  unsigned int epoch;             // resident: the iteration
+  int row_over;                   // resident: an owned row is above tau
+  int off[32];                    // resident: its arrays' places
 };
+
+// What the variants that merge sums themselves keep beside it.
+struct MergeShared {
+  float4 tab[kLogTable];          // log2_pair's table
+  float4 res[kPersistBlk];        // merged (m, h, l) per row or column of a round
+};
+
+// The header of dynamic shared memory: the state, a copy of the kernel's arguments
+// (a parameter reached by reference from a function would be a load through L2)
+// and, where a variant merges, MergeShared.
+constexpr int kPersistArgBytes = 640;
+struct PersistHeader {
+  PersistShared sh;
+  alignas(16) unsigned char args[kPersistArgBytes];
+  alignas(16) MergeShared mg;     // streamed and resident variants only
+};
+constexpr size_t kMergeHeaderBytes = (sizeof(PersistHeader) + 1023) & ~size_t(1023);
+constexpr size_t kPlainHeaderBytes = (offsetof(PersistHeader, mg) + 1023) & ~size_t(1023);
+
+extern __shared__ __align__(1024) unsigned char persist_smem[];
+__device__ __forceinline__ PersistHeader& persist_hdr() { return *reinterpret_cast<PersistHeader*>(persist_smem); }
 
 // Weight and offset of a point from FP64: as split_weight / grid_value, with the
 // rounding to the 2^-14 grid by one FP64 addition of 1.5 * 2^38 (the same
@@ -108,54 +149,90 @@ __device__ __forceinline__ float grid_near(double x) {
 }
 
 struct PersistBase {
-  const PersistArgs& A;
-  PersistShared& sh;
-  unsigned long long target;      // arrivals that complete the next barrier
-  unsigned int flags;             // absorption flags seen so far
-
-  __device__ PersistBase(const PersistArgs& args, PersistShared& shared) : A(args), sh(shared) {
-    target = gridDim.x;
-    flags = 0;
-    if (threadIdx.x == 0) sh.ok = 1;
-    for (int i = threadIdx.x; i < kLogTable; i += blockDim.x) sh.tab[i] = log_table_entry(i);
+  __device__ static __forceinline__ PersistShared& sh() { return persist_hdr().sh; }
+  __device__ static __forceinline__ MergeShared& mg() { return persist_hdr().mg; }
+  __device__ static __forceinline__ const PersistArgs& A() {
+    return *reinterpret_cast<const PersistArgs*>(persist_hdr().args);
   }
 
-  // All CTAs arrive; `flag` is added up over the CTAs (returned in `flagged`).
-  __device__ bool sync(bool flag, bool* flagged = nullptr) {
+  // Copies the arguments, resets the state; a CTA's shares of rows and columns.
+  template <class Args>
+  __device__ static void begin(const Args& args) {
+    static_assert(sizeof(Args) % 4 == 0 && sizeof(Args) <= kPersistArgBytes, "copied by words into the header");
+    for (int k = threadIdx.x; k < (int)(sizeof(Args) / 4); k += blockDim.x)
+      reinterpret_cast<uint32_t*>(persist_hdr().args)[k] = reinterpret_cast<const uint32_t*>(&args)[k];
     __syncthreads();
     if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.ctl->bar),
-                   "l"(1ull + ((unsigned long long)(flag ? 1 : 0) << 32))
+      PersistShared& s = sh();
+      const Geom& g = A().g;
+      const int n = gridDim.x, b = blockIdx.x;
+      s.target = n;
+      s.flags = s.flags2 = 0;
+      s.ok = 1;
+      s.r0 = (int)(g.I * b / n);
+      s.r1 = (int)(g.I * (b + 1) / n);
+      s.j0 = (int)(g.J * b / n);
+      s.j1 = (int)(g.J * (b + 1) / n);
+      s.jbase[0] = s.jbase[1] = s.segbase[0] = s.segbase[1] = 0;
+      s.copied[0] = s.copied[1] = s.copied_seg[0] = s.copied_seg[1] = 0;
+    }
+    __syncthreads();
+  }
+  __device__ static void fill_table() {
+    for (int i = threadIdx.x; i < kLogTable; i += blockDim.x) mg().tab[i] = log_table_entry(i);
+  }
+
+  // All CTAs arrive; `flag` and `flag2` are or-ed over the CTAs into *flagged and
+  // *flagged2. The word counts arrivals in its low 24 bits and flags in 20 bits
+  // each above: enough for the 2000 iterations of a launch at 304 CTAs.
+  __device__ static __noinline__ bool barrier(bool flag, bool flag2) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      PersistShared& s = sh();
+      PersistCtl* ctl = A().ctl;
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->bar),
+                   "l"(1ull + ((unsigned long long)(flag ? 1 : 0) << 24) + ((unsigned long long)(flag2 ? 1 : 0) << 44))
                    : "memory");
       unsigned long long v = 0;
+      const unsigned int want = s.target;
       bool done = false;
       for (uint32_t t = 0; t < kBarrierTries; ++t) {
-        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.ctl->bar) : "memory");
-        if ((v & 0xFFFFFFFFull) >= target) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&ctl->bar) : "memory");
+        if (((unsigned int)v & 0xFFFFFFu) >= want) {
           done = true;
           break;
         }
-        if ((t & 255) == 255 && *(volatile int*)&A.ctl->err) break;
+        if ((t & 255) == 255 && *(volatile int*)&ctl->err) break;
       }
-      if (!done) atomicExch(&A.ctl->err, 1);
-      if (!done) sh.ok = 0;
-      sh.bar = v;
+      if (!done) {
+        atomicExch(&ctl->err, 1);
+        s.ok = 0;
+      }
+      const unsigned int f = (unsigned int)(v >> 24) & 0xFFFFFu, f2 = (unsigned int)(v >> 44);
+      s.flagged = f != s.flags;
+      s.flagged2 = f2 != s.flags2;
+      s.flags = f;
+      s.flags2 = f2;
+      s.target = want + gridDim.x;
     }
     __syncthreads();
-    target += gridDim.x;
-    const unsigned int hi = (unsigned int)(sh.bar >> 32);
-    if (flagged) *flagged = hi != flags;
-    flags = hi;
-    return sh.ok != 0;
+    return sh().ok != 0;
+  }
+  __device__ static __forceinline__ bool sync(bool flag, bool* flagged = nullptr, bool flag2 = false,
+                                              bool* flagged2 = nullptr) {
+    const bool ok = barrier(flag, flag2);
+    if (flagged) *flagged = sh().flagged != 0;
+    if (flagged2) *flagged2 = sh().flagged2 != 0;
+    return ok;
   }
 
   // Coefficients of the updates at `eps` (make_coef's, its divisions one per lane).
-  __device__ void set_coef(double eps) {
+  __device__ static void set_coef(double eps) {
     __syncthreads();
     if (threadIdx.x < 32) {
       const int l = threadIdx.x;
-      const double num = l == 1 ? A.lambda1 : l == 2 ? A.lambda2 : l == 5 ? A.cost_scale : 1.0;
-      const double den = l == 1 || l == 3 ? A.lambda1 + eps : l == 2 || l == 4 ? A.lambda2 + eps : eps;
+      const double num = l == 1 ? A().lambda1 : l == 2 ? A().lambda2 : l == 5 ? A().cost_scale : 1.0;
+      const double den = l == 1 || l == 3 ? A().lambda1 + eps : l == 2 || l == 4 ? A().lambda2 + eps : eps;
       const double x = num / den;
       Coef c;
       c.eps = eps;
@@ -166,56 +243,56 @@ struct PersistBase {
       c.inv_l2e = __shfl_sync(0xffffffffu, x, 4);
       c.kappa = __shfl_sync(0xffffffffu, x, 5);
       if (l == 0) {
-        c.lambda1 = A.lambda1;
-        c.lambda2 = A.lambda2;
-        c.logI = sh.consts[0];
-        c.logJ = sh.consts[1];
-        c.logq = sh.consts[2];
-        c.q = A.ctl->q;
+        c.lambda1 = A().lambda1;
+        c.lambda2 = A().lambda2;
+        c.logI = sh().consts[0];
+        c.logJ = sh().consts[1];
+        c.logq = sh().consts[2];
+        c.q = A().ctl->q;
         coef_kappa2(c);
-        c.ltau_lo = sh.consts[3] - 1e-9;
-        c.ltau_hi = sh.consts[3] + 1e-9;
-        sh.c = c;
-        sh.a1ln2 = c.alpha1 * kLn2;
-        sh.a1logj = c.alpha1 * c.logJ;
-        sh.ku = -(c.alpha1 * c.inv_eps + c.inv_l1e);
-        sh.a2ln2 = c.alpha2 * kLn2;
-        sh.bconst = c.alpha2 * (c.logq + c.logI);
-        sh.kv = -(c.alpha2 * c.inv_eps + c.inv_l2e);
-        sh.iel2 = c.inv_eps * kLog2e;
-        sh.a1h = (float)c.alpha1;
-        sh.a1l = (float)(c.alpha1 - (double)sh.a1h);
-        sh.a2h = (float)c.alpha2;
-        sh.a2l = (float)(c.alpha2 - (double)sh.a2h);
+        c.ltau_lo = sh().consts[3] - 1e-9;
+        c.ltau_hi = sh().consts[3] + 1e-9;
+        sh().c = c;
+        sh().a1ln2 = c.alpha1 * kLn2;
+        sh().a1logj = c.alpha1 * c.logJ;
+        sh().ku = -(c.alpha1 * c.inv_eps + c.inv_l1e);
+        sh().a2ln2 = c.alpha2 * kLn2;
+        sh().bconst = c.alpha2 * (c.logq + c.logI);
+        sh().kv = -(c.alpha2 * c.inv_eps + c.inv_l2e);
+        sh().iel2 = c.inv_eps * kLog2e;
+        sh().a1h = (float)c.alpha1;
+        sh().a1l = (float)(c.alpha1 - (double)sh().a1h);
+        sh().a2h = (float)c.alpha2;
+        sh().a2l = (float)(c.alpha2 - (double)sh().a2h);
       }
     }
     __syncthreads();
   }
 
-  __device__ __forceinline__ bool over_tau(double l) const {
-    if (l < sh.c.ltau_lo) return false;
-    if (l > sh.c.ltau_hi) return INFINITY > A.tau;
-    return exp(l) > A.tau;
+  __device__ static __forceinline__ bool over_tau(double l) {
+    if (l < sh().c.ltau_lo) return false;
+    if (l > sh().c.ltau_hi) return INFINITY > A().tau;
+    return exp(l) > A().tau;
   }
 
   // Cross-CTA sums of the NQ values that every CTA has written to its place in
-  // V.red: one barrier, then every CTA adds them in the same order into sh.tot.
+  // V.red: one barrier, then every CTA adds them in the same order into sh().tot.
   template <int NQ>
-  __device__ bool reduce_ctas() {
+  __device__ static bool reduce_ctas() {
     if (!sync(false)) return false;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w < NQ) {
       double t = 0.0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) t += A.V.red[b * kNq + w];
+      for (int b = lane; b < (int)gridDim.x; b += 32) t += A().V.red[b * kNq + w];
       t = warp_sum(t);
-      if (lane == 0) sh.tot[w] = t;
+      if (lane == 0) sh().tot[w] = t;
     }
     __syncthreads();
     return true;
   }
 
   // Sum over all threads of the pairs h + l, over I J.
-  __device__ bool total_pairs(float h, float l, double* out) {
+  __device__ static bool total_pairs(float h, float l, double* out) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -223,282 +300,101 @@ struct PersistBase {
       df_add(h, l, h2, l2);
     }
     __syncthreads();
-    if (lane == 0) sh.res[w] = make_float4(h, l, 0.f, 0.f);
+    if (lane == 0) sh().pairs[w] = make_float2(h, l);
     __syncthreads();
     if (w == 0) {
-      const float4 r = lane < (int)(blockDim.x >> 5) ? sh.res[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float2 r = lane < (int)(blockDim.x >> 5) ? sh().pairs[lane] : make_float2(0.f, 0.f);
       const double t = warp_sum((double)r.x + (double)r.y);
-      if (lane == 0) A.V.red[blockIdx.x * kNq] = t;
+      if (lane == 0) A().V.red[blockIdx.x * kNq] = t;
     }
     if (!reduce_ctas<1>()) return false;
-    *out = sh.tot[0] / ((double)A.g.I * (double)A.g.J);
+    *out = sh().tot[0] / ((double)A().g.I * (double)A().g.J);
     return true;
   }
 
-  // Stage-exit decision from |a~ - old|^2, |a~|^2 and the same of b in sh.tot.
-  __device__ bool stage_decision(bool* go_on) {
+  // Stage-exit decision from |a~ - old|^2, |a~|^2 and the same of b in sh().tot.
+  __device__ static bool stage_decision(bool* go_on) {
     if (threadIdx.x < 32) {
       // ga = sqrt(h0) / (1 + sqrt(h1)), gb likewise; Python's max (the first unless
       // the second is larger) and the comparison with 1e-6 as products
-      const double r = sqrt(sh.tot[threadIdx.x & 3]);
+      const double r = sqrt(sh().tot[threadIdx.x & 3]);
       const double na = __shfl_sync(0xffffffffu, r, 0), nb = __shfl_sync(0xffffffffu, r, 2);
       const double da = 1.0 + __shfl_sync(0xffffffffu, r, 1), db = 1.0 + __shfl_sync(0xffffffffu, r, 3);
       const bool b = nb * da > na * db;
       const double num = b ? nb : na, den = b ? db : da;
       if (threadIdx.x == 0) {
-        sh.decision = num > 1e-6 * den;
+        sh().decision = num > 1e-6 * den;
         if (blockIdx.x == 0) {
-          A.ctl->gap_num = num;
-          A.ctl->gap_den = den;
+          A().ctl->gap_num = num;
+          A().ctl->gap_den = den;
         }
       }
     }
     __syncthreads();
-    *go_on = sh.decision != 0;
+    *go_on = sh().decision != 0;
     return true;
   }
 
-  // Duality-gap decision from the sums of gap_test in sh.tot.
-  __device__ bool gap_decision(double sumk, bool* go_on, bool* nan) {
+  // Duality-gap decision from the sums of gap_test in sh().tot.
+  __device__ static bool gap_decision(double sumk, bool* go_on, bool* nan) {
     if (threadIdx.x == 0) {
-      const double* h = sh.tot;
-      const Coef& c = sh.c;
-      const double dx = sh.dx, dy = sh.dy;
+      const double* h = sh().tot;
+      const Coef& c = sh().c;
+      const double dx = sh().dx, dy = sh().dy;
       const double num = dx * h[0] + dy * h[1];
       const double pri = c.lambda1 * dx * h[2] + c.lambda2 * dy * h[3] + dx * h[4] + dy * h[5] +
                          c.eps * (sumk - dx * h[6]);
       const double den = fabs(pri);
       // gap = num / den, as a comparison (the quotient is formed once, on the host)
       const bool isnan_ = num != num || den != den || (num == 0.0 && den == 0.0) || (isinf(num) && isinf(den));
-      sh.decision = isnan_ ? 2 : num > A.tolerance * den ? 1 : 0;
+      sh().decision = isnan_ ? 2 : num > A().tolerance * den ? 1 : 0;
       if (blockIdx.x == 0) {
-        A.ctl->gap_num = num;
-        A.ctl->gap_den = den;
+        A().ctl->gap_num = num;
+        A().ctl->gap_den = den;
       }
     }
     __syncthreads();
-    *go_on = sh.decision == 1;
-    *nan = sh.decision == 2;
+    *go_on = sh().decision == 1;
+    *nan = sh().decision == 2;
     return true;
   }
 
   // q = mean(p) from its sum, and the constants of the coefficients.
-  __device__ bool publish_mean() {
-    if (threadIdx.x == 0 && blockIdx.x == 0) A.ctl->q = sh.tot[0] / (double)A.g.I;
+  __device__ static bool publish_mean() {
+    if (threadIdx.x == 0 && blockIdx.x == 0) A().ctl->q = sh().tot[0] / (double)A().g.I;
     return sync(false);
   }
-  __device__ void constants() {
+  __device__ static void constants() {
     if (threadIdx.x < 32) {
-      const double x = threadIdx.x == 0 ? (double)A.g.I : threadIdx.x == 1 ? (double)A.g.J
-                       : threadIdx.x == 2 ? *(volatile double*)&A.ctl->q : A.tau;
+      const double x = threadIdx.x == 0 ? (double)A().g.I : threadIdx.x == 1 ? (double)A().g.J
+                       : threadIdx.x == 2 ? *(volatile double*)&A().ctl->q : A().tau;
       const double y = log(x), z = 1.0 / x;
-      if (threadIdx.x < 4) sh.consts[threadIdx.x] = y;
-      if (threadIdx.x == 0) sh.dx = z;
-      if (threadIdx.x == 1) sh.dy = z;
+      if (threadIdx.x < 4) sh().consts[threadIdx.x] = y;
+      if (threadIdx.x == 0) sh().dx = z;
+      if (threadIdx.x == 1) sh().dy = z;
     }
   }
-  __device__ void reset_gap() {
+  __device__ static void reset_gap() {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-      A.ctl->gap_num = INFINITY;
-      A.ctl->gap_den = 1.0;
+      A().ctl->gap_num = INFINITY;
+      A().ctl->gap_den = 1.0;
     }
   }
 };
 
-// The streamed variant: C read from L2 or HBM in both passes, the FP64 state in
-// global memory (own rows and columns only), any size.
-struct Streamed : PersistBase {
-  int r0, r1, c0, c1;             // owned rows, owned float4 columns
-  float* orow;                    // I   row offsets (on the weight grid); rowc's memory, free during the solve
-  float2* l2col;                  // J   base-2 log-sum-exp of each column: offset on the grid + remainder (Lcol's memory)
-
-  __device__ Streamed(const PersistArgs& args, PersistShared& shared) : PersistBase(args, shared) {
-    const int n = gridDim.x, b = blockIdx.x;
-    r0 = (int)(A.g.I * b / n);
-    r1 = (int)(A.g.I * (b + 1) / n);
-    const int64_t nv = A.g.ldc >> 2;
-    c0 = (int)(nv * b / n);
-    c1 = (int)(nv * (b + 1) / n);
-    orow = reinterpret_cast<float*>(A.V.rowc);
-    l2col = reinterpret_cast<float2*>(A.V.Lcol);
-  }
-
-  // The reference's a-update (optimal_transport.py:133) of row i from its base-2
-  // log-sum-exp; true when a_i > tau.
-  __device__ __forceinline__ bool update_row(int64_t i, double L2) const {
-    const double ui = A.V.u[i];
-    const double la = fma(-sh.a1ln2, L2, fma(sh.c.alpha1, A.V.logp[i], fma(ui, sh.ku, sh.a1logj)));
-    A.V.la_old[i] = A.V.la[i];
-    A.V.la[i] = la;
-    const float2 w = split_pair(fma(la, kLog2e, ui * sh.iel2));
-    A.V.wrow[i] = w.x;
-    A.V.wrow_lo[i] = w.y;
-    return over_tau(la);
-  }
-  __device__ __forceinline__ bool update_col(int64_t j, double L2) const {
-    const double vj = A.V.v[j];
-    const double lb = fma(-sh.a2ln2, L2, fma(vj, sh.kv, sh.bconst));
-    A.V.lb_old[j] = A.V.lb[j];
-    A.V.lb[j] = lb;
-    const float2 w = split_pair(fma(lb, kLog2e, vj * sh.iel2));
-    A.V.wcol[j] = w.x;
-    A.V.wcol_lo[j] = w.y;
-    return over_tau(lb);
-  }
-
-  // Row phase. FRESH: the row sums with the current b only (a gap check), kept
-  // for the a-update of the next iteration.
-  template <bool FRESH>
-  __device__ bool row_phase() {
-    const int lane = threadIdx.x & 31;
-    const float k2 = sh.c.kappa2, k2l = sh.c.kappa2_lo;
-    const float4* w4 = reinterpret_cast<const float4*>(A.V.wcol);
-    const float4* wl4 = reinterpret_cast<const float4*>(A.V.wcol_lo);
-    bool over = false;
-    for (int b = r0; b < r1; b += kPersistBlk) {
-      const int e = min(r1, b + kPersistBlk);
-      if (threadIdx.x == 0) sh.ticket = b;
-      __syncthreads();
-      for (;;) {
-        int i = 0;
-        if (lane == 0) i = atomicAdd(&sh.ticket, 1);
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i >= e) break;
-        float m, s, cmp, h, l;
-        // plain loads of the weights: other CTAs wrote them before the last barrier
-        const float4* row = reinterpret_cast<const float4*>(A.C + (int64_t)i * A.g.ldc);
-        row_lse<true>([row](int k) { return ld_stream(row + k); }, [w4](int k) { return w4[k]; },
-                      [wl4](int k) { return wl4[k]; }, (int)(A.g.ldc >> 2), lane, orow[i], k2, k2l, m, s, cmp);
-        two_sum(s, -cmp, h, l);
-        df_merge_lanes<16, 1>(m, h, l);
-        if (lane == 0) sh.res[i - b] = make_float4(m, h, l, 0.f);
-      }
-      __syncthreads();
-      for (int i = b + threadIdx.x; i < e; i += kPersistThreads) {
-        const float4 r = sh.res[i - b];
-        const double L2 = lse2_pair(orow[i], r.x, r.y, r.z, sh.tab);
-        orow[i] = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
-        if (FRESH)
-          A.V.Lrow[i] = L2 * kLn2;
-        else
-          over |= update_row(i, L2);
-      }
-    }
-    return over;
-  }
-
-  // The a-update from the row sums of the preceding check.
-  __device__ bool row_update_cached() {
-    bool over = false;
-    for (int i = r0 + threadIdx.x; i < r1; i += kPersistThreads) over |= update_row(i, A.V.Lrow[i] * kLog2e);
-    return over;
-  }
-
-  // Column phase: partials of (float4 column, row block) at part[(c4 nrb + r) 4 + q].
-  __device__ void col_phase() {
-    const int lane = threadIdx.x & 31;
-    const int nv = (int)(A.g.ldc >> 2), ncg = (nv + 31) >> 5;
-    const int units = ncg * A.g.nrb, nw = gridDim.x * kPersistWarps;
-    const float k2 = sh.c.kappa2, k2l = sh.c.kappa2_lo;
-    for (int u = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; u < units; u += nw) {
-      const int r = u / ncg, c4 = (u % ncg) * 32 + lane;
-      if (c4 >= nv) continue;
-      float o[4], m[4], s[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A.g.J ? l2col[c4 * 4 + q].x : 0.f;
-      const int64_t a = (int64_t)r * A.g.rows_per;
-      const float4* col = reinterpret_cast<const float4*>(A.C) + c4;
-      const int64_t ld4 = A.g.ldc >> 2;
-      const float *wr = A.V.wrow, *wrl = A.V.wrow_lo;
-      col_lse<true>([=](int64_t i) { return ld_stream(col + i * ld4); }, [wr](int64_t i) { return wr[i]; },
-                    [wrl](int64_t i) { return wrl[i]; }, a, min(A.g.I, a + A.g.rows_per), o, k2, k2l, m, s);
-      float4* out = reinterpret_cast<float4*>(A.V.part + ((int64_t)c4 * A.g.nrb + r) * 4);
-      out[0] = make_float4(m[0], s[0], m[1], s[1]);
-      out[1] = make_float4(m[2], s[2], m[3], s[3]);
-    }
-  }
-
-  // Merge phase: eight lanes per column over its row blocks, then the b-update.
-  __device__ bool merge_phase() {
-    const int lane = threadIdx.x & 31, q = lane & 3, rl = lane >> 2;
-    constexpr int kCols4 = kPersistBlk / 4;
-    bool over = false;
-    for (int b = c0; b < c1; b += kCols4) {
-      const int e = min(c1, b + kCols4);
-      for (int c4 = b + (threadIdx.x >> 5); c4 < e; c4 += kPersistWarps) {
-        const float2* p = A.V.part + (int64_t)c4 * A.g.nrb * 4 + q;
-        float m = kNegBig, h = 0.f, l = 0.f;
-#pragma unroll 4
-        for (int r = rl; r < A.g.nrb; r += 8) m = fmaxf(m, p[(int64_t)r * 4].x);
-#pragma unroll
-        for (int o = 16; o >= 4; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-#pragma unroll 4
-        for (int r = rl; r < A.g.nrb; r += 8) {
-          const float2 ps = p[(int64_t)r * 4];
-          const float f = ex2(ps.x - m);
-          const float x = __fmul_rn(ps.y, f);
-          df_add(h, l, x, __fmaf_rn(ps.y, f, -x));
-        }
-#pragma unroll
-        for (int o = 16; o >= 4; o >>= 1) {
-          const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
-          df_add(h, l, h2, l2);
-        }
-        if (rl == 0) sh.res[(c4 - b) * 4 + q] = make_float4(m, h, l, 0.f);
-      }
-      __syncthreads();
-      for (int t = threadIdx.x; t < (e - b) * 4; t += kPersistThreads) {
-        const int j = b * 4 + t;
-        if (j >= A.g.J) break;
-        const float4 r = sh.res[t];
-        const double L2 = lse2_pair(l2col[j].x, r.x, r.y, r.z, sh.tab);
-        const float o = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
-        l2col[j] = make_float2(o, (float)(L2 - (double)o));
-        over |= update_col(j, L2);
-      }
-      __syncthreads();
-    }
-    return over;
-  }
-
-  // u += eps log a, a = 1 (and for v, b): tau-absorption (optimal_transport.py:
-  // 137-141), or with RESCALE the start of a stage (:118-125), whose weights
-  // are for the new epsilon. The caller separates it from the next pass.
-  template <bool RESCALE>
-  __device__ void absorb(double eps_old) {
-    for (int i = r0 + threadIdx.x; i < r1; i += kPersistThreads) {
-      const double un = A.V.u[i] + eps_old * A.V.la[i];
-      A.V.u[i] = un;
-      A.V.la[i] = 0.0;
-      if (RESCALE) A.V.la_old[i] = 0.0;
-      split_weight(un * sh.c.inv_eps * kLog2e, A.V.wrow, A.V.wrow_lo, i);
-    }
-    const int j1 = (int)min((int64_t)c1 * 4, A.g.J);
-    for (int j = c0 * 4 + threadIdx.x; j < j1; j += kPersistThreads) {
-      const double vn = A.V.v[j] + eps_old * A.V.lb[j];
-      A.V.v[j] = vn;
-      A.V.lb[j] = 0.0;
-      if (RESCALE) A.V.lb_old[j] = 0.0;
-      split_weight(vn * sh.c.inv_eps * kLog2e, A.V.wcol, A.V.wcol_lo, j);
-    }
-  }
-
-  // One iteration; *absorb_now when max(a, b) > tau.
-  __device__ bool iterate(bool lrow_valid, bool* absorb_now) {
-    bool over = lrow_valid ? row_update_cached() : row_phase<false>();
-    if (!sync(false)) return false;
-    col_phase();
-    if (!sync(false)) return false;
-    over |= merge_phase();
-    over = __syncthreads_or(over);
-    return sync(over, absorb_now);
-  }
+// A CTA's share of the O(I + J) work, state in global memory: rows [r0, r1),
+// columns [j0, j1).
+struct Owned : PersistBase {
+  __device__ static __forceinline__ int r0() { return sh().r0; }
+  __device__ static __forceinline__ int r1() { return sh().r1; }
+  __device__ static __forceinline__ int j0() { return sh().j0; }
+  __device__ static __forceinline__ int j1() { return sh().j1; }
 
   // Sums over all CTAs of per-thread values (threads 0..127 hold row terms,
   // 128..255 column terms, the others none): every thread ends with the totals
-  // in sh.tot. One barrier.
+  // in sh().tot. One barrier.
   template <int NQ>
-  __device__ bool total(double (&acc)[NQ], bool any) {
+  __device__ static bool total(double (&acc)[NQ], bool any) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w < 8) {
       if (__any_sync(0xffffffffu, any)) {
@@ -507,31 +403,31 @@ struct Streamed : PersistBase {
       }
       if (lane == 0)
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) sh.sums[w][q] = acc[q];
+        for (int q = 0; q < NQ; ++q) sh().sums[w][q] = acc[q];
     }
     __syncthreads();
     if (threadIdx.x < NQ) {
       double t = 0.0;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) t += sh.sums[k][threadIdx.x];
-      A.V.red[blockIdx.x * kNq + threadIdx.x] = t;
+      for (int k = 0; k < 8; ++k) t += sh().sums[k][threadIdx.x];
+      A().V.red[blockIdx.x * kNq + threadIdx.x] = t;
     }
     return reduce_ctas<NQ>();
   }
 
   // Stage-exit test (optimal_transport.py:158-160) in the reference's expressions.
-  __device__ bool stage_test(bool* go_on) {
+  __device__ static bool stage_test(bool* go_on) {
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     bool any = false;
     const bool rows = threadIdx.x < 128;
-    const double* u = rows ? A.V.u : A.V.v;
-    const double* la = rows ? A.V.la : A.V.lb;
-    const double* lo = rows ? A.V.la_old : A.V.lb_old;
-    const int n0 = rows ? r0 : c0 * 4, n1 = rows ? r1 : (int)min((int64_t)c1 * 4, A.g.J);
+    const double* u = rows ? A().V.u : A().V.v;
+    const double* la = rows ? A().V.la : A().V.lb;
+    const double* lo = rows ? A().V.la_old : A().V.lb_old;
+    const int n0 = rows ? r0() : j0(), n1 = rows ? r1() : j1();
     if (threadIdx.x < 256) {
       double d2 = 0.0, a2 = 0.0;
       for (int k = n0 + (threadIdx.x & 127); k < n1; k += 128) {
-        const double e = exp(u[k] * sh.c.inv_eps);
+        const double e = exp(u[k] * sh().c.inv_eps);
         const double ta = exp(la[k]) * e;
         const double d = ta - exp(lo[k]) * e;
         d2 += d * d;
@@ -546,16 +442,18 @@ struct Streamed : PersistBase {
   }
 
   // Duality-gap test in O(I + J) (see wotg_sinkhorn.cu) after a fresh row phase.
-  __device__ bool gap_test(double sumk, bool* go_on, bool* nan) {
+  // lcol(j): the column's log-sum-exp (natural).
+  template <class Lcol>
+  __device__ static bool gap_test_with(const Lcol& lcol, double sumk, bool* go_on, bool* nan) {
     double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const Coef& c = sh.c;
+    const Coef& c = sh().c;
     bool any = false;
     if (threadIdx.x < 128) {
-      for (int i = r0 + threadIdx.x; i < r1; i += 128) {
-        const double ui = A.V.u[i], la = A.V.la[i];
+      for (int i = r0() + threadIdx.x; i < r1(); i += 128) {
+        const double ui = A().V.u[i], la = A().V.la[i];
         const double ue = ui * c.inv_eps, ub = ui + c.eps * la;
         double x, f, conj;
-        gap_terms(la + ue + A.V.Lrow[i] - c.logJ, la, ue, A.V.p[i], A.V.logp[i], c.lambda1, c.eps, &x, &f, &conj);
+        gap_terms(la + ue + A().V.Lrow[i] - c.logJ, la, ue, A().V.p[i], A().V.logp[i], c.lambda1, c.eps, &x, &f, &conj);
         acc[0] += c.lambda1 * f + conj + ub * x;
         acc[2] += f;
         acc[4] += ub * x;
@@ -563,14 +461,11 @@ struct Streamed : PersistBase {
         any = true;
       }
     } else if (threadIdx.x < 256) {
-      const int j1 = (int)min((int64_t)c1 * 4, A.g.J);
-      for (int j = c0 * 4 + threadIdx.x - 128; j < j1; j += 128) {
-        const double vj = A.V.v[j], lb = A.V.lb[j];
+      for (int j = j0() + threadIdx.x - 128; j < j1(); j += 128) {
+        const double vj = A().V.v[j], lb = A().V.lb[j];
         const double ve = vj * c.inv_eps, vb = vj + c.eps * lb;
-        const float2 l2 = l2col[j];
         double y, f, conj;
-        gap_terms(lb + ve + ((double)l2.x + (double)l2.y) * kLn2 - c.logI, lb, ve, c.q, c.logq, c.lambda2, c.eps, &y,
-                  &f, &conj);
+        gap_terms(lb + ve + lcol(j) - c.logI, lb, ve, c.q, c.logq, c.lambda2, c.eps, &y, &f, &conj);
         acc[1] += c.lambda2 * f + conj + vb * y;
         acc[3] += f;
         acc[5] += vb * y;
@@ -582,13 +477,13 @@ struct Streamed : PersistBase {
   }
 
   // sum_ij exp(-kappa C_ij) / (I J) (the reference's sum of its _K).
-  __device__ bool sum_exp(double* out) {
+  __device__ static bool sum_exp(double* out) {
     const int lane = threadIdx.x & 31;
-    const float k2 = sh.c.kappa2;
-    const int64_t nv = A.g.ldc >> 2;
+    const float k2 = sh().c.kappa2;
+    const int64_t nv = A().g.ldc >> 2;
     float h = 0.f, l = 0.f;
-    for (int i = r0 + (threadIdx.x >> 5); i < r1; i += kPersistWarps) {
-      const float4* row = reinterpret_cast<const float4*>(A.C + (int64_t)i * A.g.ldc);
+    for (int i = r0() + (threadIdx.x >> 5); i < r1(); i += (int)(blockDim.x >> 5)) {
+      const float4* row = reinterpret_cast<const float4*>(A().C + (int64_t)i * A().g.ldc);
       for (int64_t k = lane; k < nv; k += 32) {
         const float4 cc = ld_stream(row + k);   // padding is +inf: exp2(-inf) = 0
         df_add(h, l, (ex2(-k2 * cc.x) + ex2(-k2 * cc.y)) + (ex2(-k2 * cc.z) + ex2(-k2 * cc.w)), 0.f);
@@ -597,52 +492,253 @@ struct Streamed : PersistBase {
     return total_pairs(h, l, out);
   }
 
-  __device__ bool mean_growth() {
+  __device__ static bool mean_growth() {
     double acc[1] = {0.0};
     bool any = false;
     if (threadIdx.x < 128)
-      for (int i = r0 + threadIdx.x; i < r1; i += 128) {
-        acc[0] += A.V.p[i];
+      for (int i = r0() + threadIdx.x; i < r1(); i += 128) {
+        acc[0] += A().V.p[i];
         any = true;
       }
     if (!total<1>(acc, any)) return false;
     return publish_mean();
   }
+};
+
+// The streamed variant: C read from L2 or HBM in both passes, the FP64 state in
+// global memory (own rows and columns only), any size.
+struct Streamed : Owned {
+  __device__ static __forceinline__ int c0() { return sh().c0; }
+  __device__ static __forceinline__ int c1() { return sh().c1; }
+  // I row offsets (on the weight grid) in rowc's memory, free during the solve; J
+  // base-2 log-sum-exps of the columns (offset on the grid + remainder) in Lcol's.
+  __device__ static __forceinline__ float* orow() { return reinterpret_cast<float*>(A().V.rowc); }
+  __device__ static __forceinline__ float2* l2col() { return reinterpret_cast<float2*>(A().V.Lcol); }
+
+  __device__ Streamed() {
+    fill_table();
+    if (threadIdx.x == 0) {
+      PersistShared& s = sh();
+      const Geom& g = A().g;
+      const int64_t nv = g.ldc >> 2;
+      s.c0 = (int)(nv * blockIdx.x / gridDim.x);
+      s.c1 = (int)(nv * (blockIdx.x + 1) / gridDim.x);
+      s.j0 = (int)min((int64_t)s.c0 * 4, g.J);
+      s.j1 = (int)min((int64_t)s.c1 * 4, g.J);
+    }
+    __syncthreads();
+  }
+
+  // The reference's a-update (optimal_transport.py:133) of row i from its base-2
+  // log-sum-exp; true when a_i > tau.
+  __device__ static __forceinline__ bool update_row(int64_t i, double L2) {
+    const double ui = A().V.u[i];
+    const double la = fma(-sh().a1ln2, L2, fma(sh().c.alpha1, A().V.logp[i], fma(ui, sh().ku, sh().a1logj)));
+    A().V.la_old[i] = A().V.la[i];
+    A().V.la[i] = la;
+    const float2 w = split_pair(fma(la, kLog2e, ui * sh().iel2));
+    A().V.wrow[i] = w.x;
+    A().V.wrow_lo[i] = w.y;
+    return over_tau(la);
+  }
+  __device__ static __forceinline__ bool update_col(int64_t j, double L2) {
+    const double vj = A().V.v[j];
+    const double lb = fma(-sh().a2ln2, L2, fma(vj, sh().kv, sh().bconst));
+    A().V.lb_old[j] = A().V.lb[j];
+    A().V.lb[j] = lb;
+    const float2 w = split_pair(fma(lb, kLog2e, vj * sh().iel2));
+    A().V.wcol[j] = w.x;
+    A().V.wcol_lo[j] = w.y;
+    return over_tau(lb);
+  }
+
+  // Row phase. FRESH: the row sums with the current b only (a gap check), kept
+  // for the a-update of the next iteration.
+  template <bool FRESH>
+  __device__ static bool row_phase() {
+    const int lane = threadIdx.x & 31;
+    const float k2 = sh().c.kappa2, k2l = sh().c.kappa2_lo;
+    const float4* w4 = reinterpret_cast<const float4*>(A().V.wcol);
+    const float4* wl4 = reinterpret_cast<const float4*>(A().V.wcol_lo);
+    bool over = false;
+    for (int b = r0(); b < r1(); b += kPersistBlk) {
+      const int e = min(r1(), b + kPersistBlk);
+      if (threadIdx.x == 0) sh().ticket = b;
+      __syncthreads();
+      for (;;) {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&sh().ticket, 1);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= e) break;
+        float m, s, cmp, h, l;
+        // plain loads of the weights: other CTAs wrote them before the last barrier
+        const float4* row = reinterpret_cast<const float4*>(A().C + (int64_t)i * A().g.ldc);
+        row_lse<true>([row](int k) { return ld_stream(row + k); }, [w4](int k) { return w4[k]; },
+                      [wl4](int k) { return wl4[k]; }, (int)(A().g.ldc >> 2), lane, orow()[i], k2, k2l, m, s, cmp);
+        two_sum(s, -cmp, h, l);
+        df_merge_lanes<16, 1>(m, h, l);
+        if (lane == 0) mg().res[i - b] = make_float4(m, h, l, 0.f);
+      }
+      __syncthreads();
+      for (int i = b + threadIdx.x; i < e; i += kPersistThreads) {
+        const float4 r = mg().res[i - b];
+        const double L2 = lse2_pair(orow()[i], r.x, r.y, r.z, mg().tab);
+        orow()[i] = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
+        if (FRESH)
+          A().V.Lrow[i] = L2 * kLn2;
+        else
+          over |= update_row(i, L2);
+      }
+    }
+    return over;
+  }
+
+  // The a-update from the row sums of the preceding check.
+  __device__ static bool row_update_cached() {
+    bool over = false;
+    for (int i = r0() + threadIdx.x; i < r1(); i += kPersistThreads) over |= update_row(i, A().V.Lrow[i] * kLog2e);
+    return over;
+  }
+
+  // Column phase: partials of (float4 column, row block) at part[(c4 nrb + r) 4 + q].
+  __device__ static void col_phase() {
+    const int lane = threadIdx.x & 31;
+    const int nv = (int)(A().g.ldc >> 2), ncg = (nv + 31) >> 5;
+    const int units = ncg * A().g.nrb, nw = gridDim.x * kPersistWarps;
+    const float k2 = sh().c.kappa2, k2l = sh().c.kappa2_lo;
+    for (int u = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; u < units; u += nw) {
+      const int r = u / ncg, c4 = (u % ncg) * 32 + lane;
+      if (c4 >= nv) continue;
+      float o[4], m[4], s[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A().g.J ? l2col()[c4 * 4 + q].x : 0.f;
+      const int64_t a = (int64_t)r * A().g.rows_per;
+      const float4* col = reinterpret_cast<const float4*>(A().C) + c4;
+      const int64_t ld4 = A().g.ldc >> 2;
+      const float *wr = A().V.wrow, *wrl = A().V.wrow_lo;
+      col_lse<true>([=](int64_t i) { return ld_stream(col + i * ld4); }, [wr](int64_t i) { return wr[i]; },
+                    [wrl](int64_t i) { return wrl[i]; }, a, min(A().g.I, a + A().g.rows_per), o, k2, k2l, m, s);
+      float4* out = reinterpret_cast<float4*>(A().V.part + ((int64_t)c4 * A().g.nrb + r) * 4);
+      out[0] = make_float4(m[0], s[0], m[1], s[1]);
+      out[1] = make_float4(m[2], s[2], m[3], s[3]);
+    }
+  }
+
+  // Merge phase: eight lanes per column over its row blocks, then the b-update.
+  __device__ static bool merge_phase() {
+    const int lane = threadIdx.x & 31, q = lane & 3, rl = lane >> 2;
+    constexpr int kCols4 = kPersistBlk / 4;
+    bool over = false;
+    for (int b = c0(); b < c1(); b += kCols4) {
+      const int e = min(c1(), b + kCols4);
+      for (int c4 = b + (threadIdx.x >> 5); c4 < e; c4 += kPersistWarps) {
+        const float2* p = A().V.part + (int64_t)c4 * A().g.nrb * 4 + q;
+        float m = kNegBig, h = 0.f, l = 0.f;
+#pragma unroll 4
+        for (int r = rl; r < A().g.nrb; r += 8) m = fmaxf(m, p[(int64_t)r * 4].x);
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll 4
+        for (int r = rl; r < A().g.nrb; r += 8) {
+          const float2 ps = p[(int64_t)r * 4];
+          const float f = ex2(ps.x - m);
+          const float x = __fmul_rn(ps.y, f);
+          df_add(h, l, x, __fmaf_rn(ps.y, f, -x));
+        }
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) {
+          const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+          df_add(h, l, h2, l2);
+        }
+        if (rl == 0) mg().res[(c4 - b) * 4 + q] = make_float4(m, h, l, 0.f);
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < (e - b) * 4; t += kPersistThreads) {
+        const int j = b * 4 + t;
+        if (j >= A().g.J) break;
+        const float4 r = mg().res[t];
+        const double L2 = lse2_pair(l2col()[j].x, r.x, r.y, r.z, mg().tab);
+        const float o = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
+        l2col()[j] = make_float2(o, (float)(L2 - (double)o));
+        over |= update_col(j, L2);
+      }
+      __syncthreads();
+    }
+    return over;
+  }
+
+  // u += eps log a, a = 1 (and for v, b): tau-absorption (optimal_transport.py:
+  // 137-141), or with RESCALE the start of a stage (:118-125), whose weights
+  // are for the new epsilon. The caller separates it from the next pass.
+  template <bool RESCALE>
+  __device__ static void absorb(double eps_old) {
+    for (int i = r0() + threadIdx.x; i < r1(); i += kPersistThreads) {
+      const double un = A().V.u[i] + eps_old * A().V.la[i];
+      A().V.u[i] = un;
+      A().V.la[i] = 0.0;
+      if (RESCALE) A().V.la_old[i] = 0.0;
+      split_weight(un * sh().c.inv_eps * kLog2e, A().V.wrow, A().V.wrow_lo, i);
+    }
+    for (int j = j0() + threadIdx.x; j < j1(); j += kPersistThreads) {
+      const double vn = A().V.v[j] + eps_old * A().V.lb[j];
+      A().V.v[j] = vn;
+      A().V.lb[j] = 0.0;
+      if (RESCALE) A().V.lb_old[j] = 0.0;
+      split_weight(vn * sh().c.inv_eps * kLog2e, A().V.wcol, A().V.wcol_lo, j);
+    }
+  }
+
+  // One iteration; *absorb_now when max(a, b) > tau.
+  __device__ static bool iterate(bool lrow_valid, bool* absorb_now) {
+    bool over = lrow_valid ? row_update_cached() : row_phase<false>();
+    if (!sync(false)) return false;
+    col_phase();
+    if (!sync(false)) return false;
+    over |= merge_phase();
+    over = __syncthreads_or(over);
+    return sync(over, absorb_now);
+  }
+
+  __device__ static bool gap_test(double sumk, bool* go_on, bool* nan) {
+    const float2* l2 = l2col();
+    return gap_test_with([l2](int j) { return ((double)l2[j].x + (double)l2[j].y) * kLn2; }, sumk, go_on, nan);
+  }
 
   // Absorbs with the old epsilon and starts a stage at `eps`.
-  __device__ bool start_stage(double eps_old, double eps) {
+  __device__ static bool start_stage(double eps_old, double eps) {
     set_coef(eps);
     reset_gap();
     absorb<true>(eps_old);
     return sync(false);
   }
-  __device__ bool absorb_now(double eps) {
+  __device__ static bool absorb_now(double eps) {
     absorb<false>(eps);
     return sync(false);
   }
-  __device__ void fresh() {
+  __device__ static bool fresh() {
     row_phase<true>();
     __syncthreads();
+    return true;
   }
   // Refinement starts from loaded potentials and weights.
-  __device__ bool start_refine(double eps) {
+  __device__ static bool start_refine(double eps) {
     set_coef(eps);
     return true;
   }
-  __device__ bool resume(double eps) {
+  __device__ static bool resume(double eps) {
     set_coef(eps);
     return true;
   }
-  __device__ bool save(bool done) { return true; }
+  __device__ static bool save(bool done) { return true; }
 };
 
 // The reference's control (stages, batches, tests) over a variant's phases.
-// Every CTA runs it on its own copy of the state (sh.rs).
+// Every CTA runs it on its own copy of the state (sh().rs).
 template <bool GAP, class P>
 __device__ void persist_run(P& p) {
-  const PersistArgs& A = p.A;
+  const PersistArgs& A = P::A();
   PersistCtl* ctl = A.ctl;
-  RunState& rs = p.sh.rs;
+  RunState& rs = P::sh().rs;
   // one thread changes the state, between two barriers of the CTA
   auto change = [&](auto f) {
     __syncthreads();
@@ -717,12 +813,12 @@ __device__ void persist_run(P& p) {
           ++rs.checks;
       });
       if (last) {
-        p.fresh();
+        if (!p.fresh()) return;
         break;
       }
       bool go_on = true, nan = false;
       if (rs.stage == kScalings) {
-        p.fresh();
+        if (!p.fresh()) return;
         if (!p.gap_test(rs.sumk, &go_on, &nan)) return;
         change([&] {
           rs.lrow_valid = 1;
@@ -767,7 +863,7 @@ __device__ void persist_run(P& p) {
       if (new_eps && !p.start_stage(old, rs.eps)) return;
     }
     if (rs.it >= total_it) {
-      if (fixed) p.fresh();
+      if (fixed && !p.fresh()) return;
       change([&] { rs.status = kConverged; });
     }
   }
@@ -790,8 +886,8 @@ __device__ void persist_run(P& p) {
 // GAP: the duality-gap solver (kModeGap); else kModeFixed or kModeRefine.
 template <bool GAP>
 __global__ void __launch_bounds__(kPersistThreads, 1) persist_kernel(const __grid_constant__ PersistArgs A) {
-  __shared__ PersistShared sh;
-  Streamed p(A, sh);
+  PersistBase::begin(A);
+  Streamed p;
   persist_run<GAP>(p);
 }
 

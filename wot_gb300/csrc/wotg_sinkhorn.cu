@@ -39,6 +39,7 @@
 #include "wotg_resident.cuh"
 #include "wotg_state.cuh"
 #include "wotg_tc_kernel.cuh"
+#include "wotg_tc_persist.cuh"
 
 namespace wotg {
 
@@ -64,56 +65,14 @@ struct TcState {
   // Speculative half-steps: each row's base-2 log-sum-exp of the MMA exponents
   // from the previous half-step (row side offX, column side offY), valid while
   // epsilon is unchanged; rows whose sum left the safe range are listed in
-  // redoX / redoY = [count, rows...] (row and column passes) and recomputed
-  // exactly; each side's half-step empties the other side's list.
+  // redoX / redoY = [count, rows...] (row and column passes) and recomputed exactly.
   float* offX;
   float* offY;
   int* redoX;
   int* redoY;
-  int* tile_ctr;                   // per (row tile, lane quarter): partials written (CombineFin)
+  int* tile_ctr;                   // per (row tile, lane quarter): partials written
   unsigned long long* redo_total;  // rows recomputed exactly, over the solve (diagnostic)
-  bool off_row_ok, off_col_ok;
-  // Column-form biases of X (read by column passes) and Y (row passes) match
-  // the current potentials: written by the row-tile finish of the half-step that
-  // updated them, else packed before the pass that reads them.
-  bool xb_ok, yb_ok;
 };
-
-// The reference's a-update for row i; returns the key of the new a_i for the
-// absorption test (reduced per block by the caller).
-__device__ __forceinline__ double a_update(int64_t i, double L, const Vecs& V, const Coef& c) {
-  const double ui = V.u[i];
-  const double logs = ui * c.inv_eps + L - c.logJ;                 // log (K (b dy))_i
-  const double la_new = c.alpha1 * (V.logp[i] - logs) - ui * c.inv_l1e;
-  V.la_old[i] = V.la[i];
-  V.la[i] = la_new;
-  split_weight((ui * c.inv_eps + la_new) * kLog2e, V.wrow, V.wrow_lo, i);
-  return absorb_key(la_new, c);
-}
-
-__device__ __forceinline__ double b_update(int64_t j, double L, const Vecs& V, const Coef& c) {
-  const double vj = V.v[j];
-  const double logt = vj * c.inv_eps + L - c.logI;                 // log (K^T (a dx))_j
-  const double lb_new = c.alpha2 * (c.logq - logt) - vj * c.inv_l2e;
-  V.lb_old[j] = V.lb[j];
-  V.lb[j] = lb_new;
-  split_weight((vj * c.inv_eps + lb_new) * kLog2e, V.wcol, V.wcol_lo, j);
-  return absorb_key(lb_new, c);
-}
-
-// Block-wide max of the threads' values, folded into the absorption slot with
-// one atomic per block (every thread of the block must call it).
-__device__ __forceinline__ void block_max_to_slot(double v, unsigned long long* slot) {
-  __shared__ double sh[32];
-  v = warp_maxd(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double w = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-    w = warp_maxd(w);
-    if (threadIdx.x == 0) atomic_max_nonneg(slot, w);
-  }
-}
 
 // Standalone row pass: one warp per row, 128-bit streaming loads of C, online
 // base-2 LSE of one FP32 weight vector.
@@ -131,15 +90,6 @@ __global__ void __launch_bounds__(256) row_pass_kernel(const float* __restrict__
     warp_lse(m, s);
     if (lane == 0) L[i] = ((double)m + log2((double)s)) * kLn2;
   }
-}
-
-// a-update from a cached row LSE (the row pass of the preceding gap check).
-__global__ void a_update_kernel(Geom g, Vecs V, Coef c, int parity) {
-  double amax = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.I;
-       i += (int64_t)gridDim.x * blockDim.x)
-    amax = fmax(amax, a_update(i, V.Lrow[i], V, c));
-  block_max_to_slot(amax, V.maxslot + parity);
 }
 
 // Standalone column pass, phase 1: CTA = 1024 columns (float4 per thread) x
@@ -171,58 +121,6 @@ __global__ void col_combine_kernel(Geom g, const float2* __restrict__ part, doub
     lse_merge(m, s, ps.x, ps.y);
   }
   L[j] = lse2(m, s) * kLn2;
-}
-
-// tau-absorption (optimal_transport.py:137-141 / :211-216): if max(a, b) > tau,
-// u += eps log a, v += eps log b, a = b = 1. Also clears the other max slot.
-// Also rewrites the column-form biases of the absorbed points (bx, by).
-__global__ void absorb_kernel(Geom g, Vecs V, Coef c, double tau, int parity, TcBias bx, TcBias by) {
-  pdl_wait();
-  pdl_trigger();
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const double mx = __longlong_as_double((long long)V.maxslot[parity]);
-  if (idx == 0) V.maxslot[parity ^ 1] = 0ull;
-  if (!(mx > tau)) return;
-  if (idx == 0) V.counters[0] += 1;
-  const double k2d = c.kappa * kLog2e;
-  if (idx < g.I) {
-    const double un = V.u[idx] + c.eps * V.la[idx];
-    V.u[idx] = un;
-    V.la[idx] = 0.0;
-    split_weight(un * c.inv_eps * kLog2e, V.wrow, V.wrow_lo, idx);
-    if (bx.tiles) tc_write_bias(idx, (un * c.inv_eps + 0.0) * kLog2e - k2d * bx.norm[idx], bx.d, bx.kp, bx.tiles);
-  } else if (idx < g.I + g.J) {
-    const int64_t j = idx - g.I;
-    const double vn = V.v[j] + c.eps * V.lb[j];
-    V.v[j] = vn;
-    V.lb[j] = 0.0;
-    split_weight(vn * c.inv_eps * kLog2e, V.wcol, V.wcol_lo, j);
-    if (by.tiles) tc_write_bias(j, (vn * c.inv_eps + 0.0) * kLog2e - k2d * by.norm[j], by.d, by.kp, by.tiles);
-  }
-}
-
-// Absorb with the old epsilon, switch to the new one, reset a = b = 1
-// (stage start, optimal_transport.py:118-125; epsilon step, :218-228).
-__global__ void rescale_kernel(Geom g, Vecs V, double eps_old, double inv_eps_new) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx == 0) {
-    V.maxslot[0] = 0ull;
-    V.maxslot[1] = 0ull;
-  }
-  if (idx < g.I) {
-    const double un = V.u[idx] + eps_old * V.la[idx];
-    V.u[idx] = un;
-    V.la[idx] = 0.0;
-    V.la_old[idx] = 0.0;
-    split_weight(un * inv_eps_new * kLog2e, V.wrow, V.wrow_lo, idx);
-  } else if (idx < g.I + g.J) {
-    const int64_t j = idx - g.I;
-    const double vn = V.v[j] + eps_old * V.lb[j];
-    V.v[j] = vn;
-    V.lb[j] = 0.0;
-    V.lb_old[j] = 0.0;
-    split_weight(vn * inv_eps_new * kLog2e, V.wcol, V.wcol_lo, j);
-  }
 }
 
 // Zero state for a new solve; p = G; padding of wcol = 0.
@@ -275,132 +173,6 @@ __global__ void load_potentials_kernel(Geom g, Vecs V, const double* __restrict_
     V.Lcol[j] = 0.0;
     split_weight(vbar[j] * inv_eps * kLog2e, V.wcol, V.wcol_lo, j);
   }
-}
-
-// ---------------------------------------------------------------------------
-// Deterministic two-level FP64 reductions: kRedBlocks blocks write partials,
-// one block sums them.
-// ---------------------------------------------------------------------------
-template <int NQ>
-__device__ __forceinline__ void block_reduce_store(double (&acc)[NQ], double* out) {
-  __shared__ double sh[32][NQ];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = warp_sum(acc[q]);
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) sh[wid][q] = acc[q];
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      double t = lane < nw ? sh[lane][q] : 0.0;
-      t = warp_sum(t);
-      if (lane == 0) out[q] = t;
-    }
-  }
-}
-
-__global__ void finalize_kernel(const double* __restrict__ red, int nblocks, double* out) {
-  double acc[kNq];
-#pragma unroll
-  for (int q = 0; q < kNq; ++q) acc[q] = 0.0;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-#pragma unroll
-    for (int q = 0; q < kNq; ++q) acc[q] += red[b * kNq + q];
-  block_reduce_store<kNq>(acc, out);
-}
-
-// sum_ij exp(-kappa C_ij) over valid entries (the reference's sum of _K, used
-// in the primal objective at the final stage).
-__global__ void __launch_bounds__(256) sum_exp_kernel(const float* __restrict__ C, Geom g, float kappa2,
-                                                      double* red) {
-  const int64_t nv = g.ldc >> 2;
-  double acc[kNq];
-#pragma unroll
-  for (int q = 0; q < kNq; ++q) acc[q] = 0.0;
-  for (int64_t i = blockIdx.x; i < g.I; i += gridDim.x) {
-    const float4* row = reinterpret_cast<const float4*>(C + i * g.ldc);
-    float s = 0.f;
-    for (int64_t k = threadIdx.x; k < nv; k += blockDim.x) {
-      const float4 cc = ld_stream(row + k);
-      s += (ex2(-kappa2 * cc.x) + ex2(-kappa2 * cc.y)) + (ex2(-kappa2 * cc.z) + ex2(-kappa2 * cc.w));
-    }
-    acc[0] += (double)s;  // padding is +inf -> exp2(-inf) = 0
-  }
-  block_reduce_store<kNq>(acc, red + blockIdx.x * kNq);
-}
-
-// mean(G) (q = ones(J) * np.average(G), optimal_transport.py:108 / :192).
-__global__ void sum_vec_kernel(const double* __restrict__ x, int64_t n, double* red) {
-  double acc[kNq];
-#pragma unroll
-  for (int q = 0; q < kNq; ++q) acc[q] = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    acc[0] += x[i];
-  block_reduce_store<kNq>(acc, red + blockIdx.x * kNq);
-}
-
-// Stage-exit test (optimal_transport.py:158-160), FP64, as the reference
-// evaluates it: a~ = a * exp(u/eps), old = old_a * exp(u/eps).
-//   acc[0] = |a~ - old|^2, acc[1] = |a~|^2, acc[2], acc[3] likewise for b.
-__global__ void stage_test_kernel(Geom g, Vecs V, Coef c, double* red) {
-  double acc[kNq];
-#pragma unroll
-  for (int q = 0; q < kNq; ++q) acc[q] = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.I; i += stride) {
-    const double e = exp(V.u[i] * c.inv_eps);
-    const double ta = exp(V.la[i]) * e;
-    const double d = ta - exp(V.la_old[i]) * e;
-    acc[0] += d * d;
-    acc[1] += ta * ta;
-  }
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < g.J; j += stride) {
-    const double e = exp(V.v[j] * c.inv_eps);
-    const double tb = exp(V.lb[j]) * e;
-    const double d = tb - exp(V.lb_old[j]) * e;
-    acc[2] += d * d;
-    acc[3] += tb * tb;
-  }
-  block_reduce_store<kNq>(acc, red + blockIdx.x * kNq);
-}
-
-// Duality-gap terms (final stage). Needs Lrow with the current b and Lcol
-// with the current a.
-//   acc[0] = sum_i [lambda1 (x log(x/p) - x + p) + lambda1 p (exp(-eps log a~/lambda1) - 1) + ubar x]
-//   acc[1] = same over j with lambda2, q, b~, vbar, y
-//   acc[2] = sum_i (x log(x/p) - x + p)       acc[3] = sum_j (y log(y/q) - y + q)
-//   acc[4] = sum_i ubar x                      acc[5] = sum_j vbar y
-//   acc[6] = sum_i x
-__global__ void gap_partial_kernel(Geom g, Vecs V, Coef c, double* red) {
-  double acc[kNq];
-#pragma unroll
-  for (int q = 0; q < kNq; ++q) acc[q] = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.I; i += stride) {
-    const double ui = V.u[i], lai = V.la[i], pi = V.p[i];
-    const double ue = ui * c.inv_eps;
-    double x, f, conj;
-    gap_terms(lai + ue + V.Lrow[i] - c.logJ, lai, ue, pi, V.logp[i], c.lambda1, c.eps, &x, &f, &conj);
-    const double ub = ui + c.eps * lai;
-    acc[0] += c.lambda1 * f + conj + ub * x;
-    acc[2] += f;
-    acc[4] += ub * x;
-    acc[6] += x;
-  }
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < g.J; j += stride) {
-    const double vj = V.v[j], lbj = V.lb[j];
-    const double ve = vj * c.inv_eps;
-    double y, f, conj;
-    gap_terms(lbj + ve + V.Lcol[j] - c.logI, lbj, ve, c.q, c.logq, c.lambda2, c.eps, &y, &f, &conj);
-    const double vb = vj + c.eps * lbj;
-    acc[1] += c.lambda2 * f + conj + vb * y;
-    acc[3] += f;
-    acc[5] += vb * y;
-  }
-  block_reduce_store<kNq>(acc, red + blockIdx.x * kNq);
 }
 
 // Outputs. `log_scale` is the log of the factor applied to R = diag(a) K diag(b):
@@ -496,153 +268,29 @@ __global__ void __launch_bounds__(256) coupling_kernel(const float* __restrict__
   }
 }
 
-// ---------------------------------------------------------------------------
-// On-the-fly form: the FP64 finish of the tensor-core kernel's partials. The
-// exponent of element (i, j) is split as
-//   bias_j + gamma (x_i . y_j) - kappa2 |x_i|^2,   gamma = 2 kappa2,
-//   bias_j = (v_j / eps + lb_j) log2 e - kappa2 |y_j|^2     (FP64, carried by the MMA),
-// i.e. (v_j/eps + lb_j - kappa C_ij) in base 2 with C = |x|^2 + |y|^2 - 2 x.y; the
-// tensor-core kernel produces the first two terms, its row-tile finish
-// (CombineFin, below) adds the third.
-// ---------------------------------------------------------------------------
-// Column-form bias of point i of the side a half-step just updated (ROW: a row
-// point with its new log-scaling la, for the next column pass; else a column
-// point with its new lb, for the next row pass).
-template <bool ROW>
-__device__ __forceinline__ void write_bias(int64_t i, const Vecs& V, const Coef& c, const TcBias& b) {
-  const double pot = ROW ? V.u[i] : V.v[i];
-  const double lsc = ROW ? V.la[i] : V.lb[i];
-  tc_write_bias(i, (pot * c.inv_eps + lsc) * kLog2e - (c.kappa * kLog2e) * b.norm[i], b.d, b.kp, b.tiles);
-}
-
-// Exact half-step of the rows listed by a speculative half-step (a warp per row):
-// L_i = log sum_j exp(w_j - kappa |x_i - y_j|^2) from the FP32 points with a
-// running maximum, then the same update and offset as the row-tile finish.
-template <bool ROW, bool UPDATE>
-__global__ void tc_exact_rows_kernel(Geom g, Vecs V, Coef c, const float* __restrict__ P, int64_t ldp,
-                                     const float* __restrict__ Q, int64_t ldq, int d, const double* __restrict__ norm,
-                                     float* __restrict__ off, int* __restrict__ redo,
-                                     unsigned long long* __restrict__ total, int parity, TcBias bias) {
-  pdl_wait();
-  pdl_trigger();
-  const int cnt = redo[0];
-  if (blockIdx.x == 0 && threadIdx.x == 0 && cnt > 0) atomicAdd(total, (unsigned long long)cnt);
+// Sum of n values on kRedBlocks + 1 blocks of 256 threads, in a fixed order (the
+// growth's mean of the on-the-fly solver; its last bit reaches the results).
+__device__ __forceinline__ void block_sum_store(double acc, double* out) {
+  __shared__ double sh[8];
   const int lane = threadIdx.x & 31;
-  const int64_t m_cols = ROW ? g.J : g.I;
-  const double* pot = ROW ? V.v : V.u;
-  const double* lsc = ROW ? V.lb : V.la;
-  const float k2 = (float)(c.kappa * kLog2e);
-  for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < cnt; w += (int)((gridDim.x * blockDim.x) >> 5)) {
-    const int64_t i = redo[1 + w];
-    const float* x = P + i * ldp;
-    float m = kNegBig, s = 0.f;
-    for (int64_t j = lane; j < m_cols; j += 32) {
-      const float* y = Q + j * ldq;
-      float cc = 0.f;
-      for (int t = 0; t < d; ++t) {
-        const float df = x[t] - y[t];
-        cc = fmaf(df, df, cc);
-      }
-      const float tt = (float)((pot[j] * c.inv_eps + lsc[j]) * kLog2e) - k2 * cc;
-      const float mn = fmaxf(m, tt);
-      s = s * ex2(m - mn) + ex2(tt - mn);
-      m = mn;
-    }
-    warp_lse(m, s);
-    if (lane == 0) {
-      const double L2 = lse2(m, s);
-      off[i] = (float)(L2 + (double)k2 * norm[i]);
-      const double L = L2 * kLn2;
-      double v = 0.0;
-      if (ROW) {
-        V.Lrow[i] = L;
-        if (UPDATE) v = a_update(i, L, V, c);
-      } else {
-        V.Lcol[i] = L;
-        if (UPDATE) v = b_update(i, L, V, c);
-      }
-      if (UPDATE) atomic_max_nonneg(V.maxslot + parity, v);
-      if (UPDATE && bias.tiles) write_bias<ROW>(i, V, c, bias);
-    }
+  acc = warp_sum(acc);
+  if (lane == 0) sh[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const double t = warp_sum(lane < 8 ? sh[lane] : 0.0);
+    if (lane == 0) *out = t;
   }
 }
-
-// Row-tile finish of an on-the-fly half-step inside lse_tc_kernel: the warp
-// that writes the last partial of 32 rows (over the CTAs and column halves that
-// covered their row tile) merges them in a fixed order (FP32 LSE merge), then
-// per row either lists it for the exact recompute (a speculative sum outside
-// [2^-80, 2^100]) or writes its offset and log-sum-exp and, with UPDATE, the
-// FP64 a- or b-update, the point's column-form bias for the other side's next
-// pass and the absorption maximum (the work of a separate merge pass, without
-// its launch and its wait on the whole kernel). Ordering: every lane fences its partial, the warp synchronises, one
-// atomic per warp counts it; the finishing warp fences again and reads the
-// partials from L2.
-template <bool ROW, bool UPDATE>
-struct CombineFin {
-  static constexpr bool kActive = true;
-  Geom g;
-  Vecs V;
-  Coef c;
-  const double* norm;
-  float* off;
-  int* redo;
-  int* redo_other;
-  TcBias bias;
-  int* ctr;  // per (row tile, lane quarter): partials written so far
-  int nq, ctas, parity, spec;
-
-  // the other side's exact-row list was consumed by its last half-step
-  __device__ __forceinline__ void start() const { redo_other[0] = 0; }
-
-  __device__ void quarter_done(const float2* part, int t, int wq, int lane) const {
-    __threadfence();
-    __syncwarp();
-    const int64_t n = ROW ? g.I : g.J;
-    const int64_t total = ((n + 127) >> 7) * (int64_t)nq;
-    const int64_t c_lo = tc_cta_of((int64_t)t * nq, total, ctas);
-    const int64_t c_hi = tc_cta_of(((int64_t)t + 1) * nq - 1, total, ctas);
-    const int expect = 2 * (int)(c_hi - c_lo + 1);
-    int old = 0;
-    if (lane == 0) old = atomicAdd(ctr + 4 * t + wq, 1);
-    old = __shfl_sync(0xffffffffu, old, 0);
-    if (old != expect - 1) return;
-    if (lane == 0) ctr[4 * t + wq] = 0;   // for the next launch
-    __threadfence();
-    const int64_t i = (int64_t)t * 128 + 32 * wq + lane;
-    double vmax = 0.0;
-    if (i < n) {
-      float m = kNegBig, s = 0.f;
-      for (int64_t cc = c_lo; cc <= c_hi; ++cc) {
-        const float2* pp = part + ((cc + t) * 128 + (i & 127)) * kTcParts;
-#pragma unroll
-        for (int k = 0; k < kTcParts; ++k) {
-          const float2 u = __ldcg(pp + k);
-          lse_merge(m, s, u.x, u.y);
-        }
-      }
-      if (spec && !(s >= 0x1p-80f && s <= 0x1p100f)) {
-        const int k = atomicAdd(redo, 1);
-        redo[1 + k] = (int)i;
-      } else {
-        const double D = lse2(m, s);
-        off[i] = (float)D;
-        const double L = D * kLn2 - c.kappa * norm[i];
-        if (ROW) {
-          V.Lrow[i] = L;
-          if (UPDATE) vmax = a_update(i, L, V, c);
-        } else {
-          V.Lcol[i] = L;
-          if (UPDATE) vmax = b_update(i, L, V, c);
-        }
-        if (UPDATE && bias.tiles) write_bias<ROW>(i, V, c, bias);
-      }
-    }
-    if (UPDATE) {
-      vmax = warp_maxd(vmax);
-      if (lane == 0) atomic_max_nonneg(V.maxslot + parity, vmax);
-    }
-  }
-};
+__global__ void __launch_bounds__(256) sum_vec_kernel(const double* __restrict__ x, int64_t n, double* red) {
+  double acc = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) acc += x[i];
+  block_sum_store(acc, red + blockIdx.x);
+}
+__global__ void __launch_bounds__(256) finalize_sum_kernel(const double* __restrict__ red, int n, double* out) {
+  double acc = 0.0;
+  for (int b = threadIdx.x; b < n; b += 256) acc += red[b];
+  block_sum_store(acc, out);
+}
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -653,269 +301,32 @@ struct Solver {
   Vecs V;
   cudaStream_t st;
   double cost_scale;
-  int small_grid;  // grid for O(I+J) kernels
   TcState tc;
 
   Coef coef(double eps, const wotg_params& P, double q) const {
-    Coef c = make_coef(eps, P.lambda1, P.lambda2, cost_scale, g.I, g.J, q);
-    c.ltau_lo = std::log(P.tau) - 1e-9;
-    c.ltau_hi = std::log(P.tau) + 1e-9;
-    return c;
+    return make_coef(eps, P.lambda1, P.lambda2, cost_scale, g.I, g.J, q);
   }
 
   int vec_blocks(int64_t n) const { return (int)std::max<int64_t>(1, (n + 255) / 256); }
 
-  // On-the-fly row pass (K (b dy)) / column pass (K^T (a dx)).
-  // Row forms carry gamma = 2 kappa2, which changes with epsilon. Column forms
-  // hold sqrt(cost_scale) y and row forms (gamma / sqrt(cost_scale)) x, so that
-  // both stay in median-normalised units whatever the units of the input points
-  // (FP16 range); their product is gamma x . y.
-  int tc_prepare(const Coef& c) {
-    tc.off_row_ok = false;  // a new epsilon: the offsets and biases of both sides are stale
-    tc.off_col_ok = false;
-    tc.xb_ok = tc.yb_ok = false;
-    WOTG_CUDA(cudaMemsetAsync(tc.redoX, 0, sizeof(int), st));
-    WOTG_CUDA(cudaMemsetAsync(tc.redoY, 0, sizeof(int), st));
-    WOTG_CUDA(cudaMemsetAsync(tc.tile_ctr, 0, sizeof(int) * 4 * std::max(tc.n_xt, tc.n_yt), st));
-    const float gamma = (float)(2.0 * c.kappa * kLog2e / std::sqrt(cost_scale));
-    int s = tc_pack_points(tc.X, g.I, tc.ldx, tc.d, tc.kp, gamma, 1, tc.Xa, nullptr, st);
-    if (s) return s;
-    return tc_pack_points(tc.Y, g.J, tc.ldy, tc.d, tc.kp, gamma, 1, tc.Ya, nullptr, st);
-  }
-
-  // The half-steps run in the speculative form once the offsets of their side
-  // exist for the current epsilon (the first half-step of each side after an
-  // epsilon change or a new solve runs the exact form and writes them).
-  TcBias bias_x() const { return TcBias{tc.Xb, tc.normX, tc.d, tc.kp}; }
-  TcBias bias_y() const { return TcBias{tc.Yb, tc.normY, tc.d, tc.kp}; }
-
-  // One on-the-fly half-step with its row-tile finish inside the kernel
-  // (CombineFin), launched as a dependent of the previous kernel.
-  template <bool ROW, bool UPDATE>
-  int tc_fused_pass(const Coef& c, int parity, bool spec) {
-    using F = CombineFin<ROW, UPDATE>;
-    F fin;
-    fin.g = g;
-    fin.V = V;
-    fin.c = c;
-    fin.norm = ROW ? tc.normX : tc.normY;
-    fin.off = ROW ? tc.offX : tc.offY;
-    fin.redo = ROW ? tc.redoX : tc.redoY;
-    fin.redo_other = ROW ? tc.redoY : tc.redoX;
-    fin.bias = UPDATE ? (ROW ? bias_x() : bias_y()) : TcBias{};
-    fin.ctr = tc.tile_ctr;
-    fin.nq = ROW ? tc.n_yt : tc.n_xt;
-    fin.ctas = ROW ? tc.ctas_row : tc.ctas_col;
-    fin.parity = parity;
-    fin.spec = spec ? 1 : 0;
-    const __half* Pt = ROW ? tc.Xa : tc.Ya;
-    const __half* Qt = ROW ? tc.Yb : tc.Xb;
-    const int n_pt = ROW ? tc.n_xt : tc.n_yt;
-    const float* offp = spec ? fin.off : nullptr;
-    const float* no_w = nullptr;
-    float* no_s = nullptr;
-    if (tc.kp == 32) {
-      WOTG_CUDA((tc_set_smem_attr<32, 0, F>()));
-      WOTG_CUDA(launch_dependent(lse_tc_kernel<32, 0, F>, dim3(fin.ctas), dim3(kTcThreads), TcSmem<32>::kAlloc, st,
-                                 Pt, Qt, n_pt, fin.nq, tc.part, offp, tc.err, kTcWaitTries, no_w, 0, 0, no_s, fin));
-    } else {
-      WOTG_CUDA((tc_set_smem_attr<64, 0, F>()));
-      WOTG_CUDA(launch_dependent(lse_tc_kernel<64, 0, F>, dim3(fin.ctas), dim3(kTcThreads), TcSmem<64>::kAlloc, st,
-                                 Pt, Qt, n_pt, fin.nq, tc.part, offp, tc.err, kTcWaitTries, no_w, 0, 0, no_s, fin));
-    }
-    WOTG_LAUNCHED();
-    return WOTG_OK;
-  }
-
-  template <bool UPDATE>
-  int tc_row_pass(const Coef& c, int parity) {
-    if (!tc.yb_ok) {
-      int s = tc_pack_bias(g.J, V.v, V.lb, tc.normY, c.inv_eps, c.kappa * kLog2e, tc.d, tc.kp, tc.Yb, st);
-      if (s) return s;
-      tc.yb_ok = true;
-    }
-    const bool spec = tc.off_row_ok;
-    int s = tc_fused_pass<true, UPDATE>(c, parity, spec);
-    if (s) return s;
-    const TcBias bx = UPDATE ? bias_x() : TcBias{};
-    if (spec) {
-      WOTG_CUDA(launch_dependent(tc_exact_rows_kernel<true, UPDATE>, dim3(2 * sm_count()), dim3(256), 0, st, g, V, c,
-                                 (const float*)tc.X, tc.ldx, (const float*)tc.Y, tc.ldy, tc.d,
-                                 (const double*)tc.normX, tc.offX, tc.redoX, tc.redo_total, parity, bx));
-      WOTG_LAUNCHED();
-    }
-    tc.off_row_ok = true;
-    if (UPDATE) tc.xb_ok = true;
-    return WOTG_OK;
-  }
-  int tc_col_pass(const Coef& c, int parity) {
-    if (!tc.xb_ok) {
-      int s = tc_pack_bias(g.I, V.u, V.la, tc.normX, c.inv_eps, c.kappa * kLog2e, tc.d, tc.kp, tc.Xb, st);
-      if (s) return s;
-      tc.xb_ok = true;
-    }
-    const bool spec = tc.off_col_ok;
-    int s = tc_fused_pass<false, true>(c, parity, spec);
-    if (s) return s;
-    if (spec) {
-      WOTG_CUDA(launch_dependent(tc_exact_rows_kernel<false, true>, dim3(2 * sm_count()), dim3(256), 0, st, g, V, c,
-                                 (const float*)tc.Y, tc.ldy, (const float*)tc.X, tc.ldx, tc.d,
-                                 (const double*)tc.normY, tc.offY, tc.redoY, tc.redo_total, parity, bias_y()));
-      WOTG_LAUNCHED();
-    }
-    tc.off_col_ok = true;
-    tc.yb_ok = true;
-    return WOTG_OK;
-  }
-
-  // One on-the-fly iteration (the materialised form iterates in persist_kernel).
-  int iteration(const Coef& c, bool lrow_valid, int parity) {
-    int s;
-    if (lrow_valid) {
-      a_update_kernel<<<vec_blocks(g.I), 256, 0, st>>>(g, V, c, parity);
-      WOTG_LAUNCHED();
-      tc.xb_ok = false;  // la changed without its biases: the column pass packs them
-    } else {
-      s = tc_row_pass<true>(c, parity);
-      if (s) return s;
-    }
-    return tc_col_pass(c, parity);
-  }
-
-  int absorb(const Coef& c, double tau, int parity) {
-    WOTG_CUDA(launch_dependent(absorb_kernel, dim3(vec_blocks(g.I + g.J)), dim3(256), 0, st, g, V, c, tau, parity,
-                               bias_x(), bias_y()));
-    WOTG_LAUNCHED();
-    return WOTG_OK;
-  }
-
-  int rescale(double eps_old, double eps_new) {
-    rescale_kernel<<<vec_blocks(g.I + g.J), 256, 0, st>>>(g, V, eps_old, 1.0 / eps_new);
-    WOTG_LAUNCHED();
-    return WOTG_OK;
-  }
-
-  int reduce_to_host(double* host8) {
-    finalize_kernel<<<1, 256, 0, st>>>(V.red, kRedBlocks, V.scal);
-    WOTG_LAUNCHED();
-    WOTG_CUDA(cudaMemcpyAsync(host8, V.scal, kNq * sizeof(double), cudaMemcpyDeviceToHost, st));
+  // Rows that the speculative on-the-fly half-steps recomputed exactly; synchronises.
+  int exact_rows(int32_t* out) const {
+    if (!tc.on) return WOTG_OK;
+    unsigned long long redo = 0;
+    WOTG_CUDA(cudaMemcpyAsync(&redo, tc.redo_total, sizeof(redo), cudaMemcpyDeviceToHost, st));
     WOTG_CUDA(cudaStreamSynchronize(st));
+    *out = (int32_t)std::min<unsigned long long>(redo, 0x7fffffffull);
     return WOTG_OK;
   }
 
-  int mean_of(const double* x, int64_t n, double* out) {
+  int mean_of(const double* x, int64_t n, double* out) const {
     sum_vec_kernel<<<kRedBlocks, 256, 0, st>>>(x, n, V.red);
+    finalize_sum_kernel<<<1, 256, 0, st>>>(V.red, kRedBlocks, V.scal);
     WOTG_LAUNCHED();
-    double h[kNq];
-    int s = reduce_to_host(h);
-    if (s) return s;
-    *out = h[0] / (double)n;
-    return WOTG_OK;
-  }
-
-  int sum_exp(const Coef& c, double* out) {
-    sum_exp_kernel<<<kRedBlocks, 256, 0, st>>>(C, g, c.kappa2, V.red);
-    WOTG_LAUNCHED();
-    double h[kNq];
-    int s = reduce_to_host(h);
-    if (s) return s;
-    *out = h[0];
-    return WOTG_OK;
-  }
-
-  int fresh_lrow(const Coef& c) { return tc_row_pass<false>(c, 0); }
-
-  // CUDA-graph replay of the final stage's batches between duality-gap checks.
-  // In that stage a batch starts right after a check (L_row fresh) with both
-  // sides' speculative offsets and column-form biases current, and ends in the
-  // same host state, so its launches (nb iterations with their absorption
-  // tests, all arguments fixed for the stage) are captured once per starting
-  // parity and replayed; a new epsilon drops them.
-  struct BatchGraph {
-    cudaGraphExec_t exec = nullptr;
-    unsigned long long launches = 0;
-    int nb = 0;
-  };
-  BatchGraph bg[2] = {};
-  cudaStream_t gs = nullptr;                 // private stream of the captures and replays
-  cudaEvent_t gev[2] = {nullptr, nullptr};
-  bool graphs_off = false;                   // no private stream: plain launches
-
-  bool steady() const { return tc.off_row_ok && tc.off_col_ok && tc.xb_ok && tc.yb_ok; }
-
-  void drop_graphs() {
-    for (auto& b : bg) {
-      if (b.exec) cudaGraphExecDestroy(b.exec);
-      b = BatchGraph{};
-    }
-  }
-  void release_graphs() {
-    drop_graphs();
-    for (auto& e : gev)
-      if (e) cudaEventDestroy(e);
-    gev[0] = gev[1] = nullptr;
-    if (gs) cudaStreamDestroy(gs);
-    gs = nullptr;
-  }
-
-  // One batch of nb iterations from a fresh L_row at `parity`, as a graph;
-  // *used = false when graphs are unavailable (the caller launches plainly).
-  int batch_graph(const Coef& c, int nb, int parity, double tau, bool* used) {
-    *used = false;
-    if (graphs_off) return WOTG_OK;
-    if (!gs) {
-      if (cudaStreamCreateWithFlags(&gs, cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&gev[0], cudaEventDisableTiming) != cudaSuccess ||
-          cudaEventCreateWithFlags(&gev[1], cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        release_graphs();
-        graphs_off = true;
-        return WOTG_OK;
-      }
-    }
-    BatchGraph& G = bg[parity & 1];
-    if (G.exec && G.nb != nb) {
-      cudaGraphExecDestroy(G.exec);
-      G = BatchGraph{};
-    }
-    bool fresh = false;
-    if (!G.exec) {
-      const unsigned long long before = launches_so_far();
-      WOTG_CUDA(cudaStreamBeginCapture(gs, cudaStreamCaptureModeThreadLocal));
-      const cudaStream_t user = st;
-      st = gs;
-      int s = WOTG_OK;
-      int p = parity;
-      for (int t = 0; t < nb && s == WOTG_OK; ++t) {
-        s = iteration(c, t == 0, p);
-        if (s == WOTG_OK) s = absorb(c, tau, p);
-        p ^= 1;
-      }
-      st = user;
-      cudaGraph_t graph = nullptr;
-      const cudaError_t e = cudaStreamEndCapture(gs, &graph);
-      cudaError_t ei = e;
-      if (s == WOTG_OK && e == cudaSuccess) ei = cudaGraphInstantiate(&G.exec, graph, 0);
-      if (graph) cudaGraphDestroy(graph);
-      if (s != WOTG_OK || ei != cudaSuccess) {
-        // nothing of the batch ran (capture only) and the host state is the one
-        // it started from: fall back to plain launches for the rest of the solve
-        G = BatchGraph{};
-        cudaGetLastError();
-        graphs_off = true;
-        return WOTG_OK;
-      }
-      G.launches = launches_so_far() - before;   // counted at capture, for the first replay
-      G.nb = nb;
-      fresh = true;
-    }
-    WOTG_CUDA(cudaEventRecord(gev[0], st));
-    WOTG_CUDA(cudaStreamWaitEvent(gs, gev[0], 0));
-    WOTG_CUDA(cudaGraphLaunch(G.exec, gs));
-    WOTG_CUDA(cudaEventRecord(gev[1], gs));
-    WOTG_CUDA(cudaStreamWaitEvent(st, gev[1], 0));
-    if (!fresh) count_launches(G.launches);
-    *used = true;
+    double h;
+    WOTG_CUDA(cudaMemcpyAsync(&h, V.scal, sizeof(h), cudaMemcpyDeviceToHost, st));
+    WOTG_CUDA(cudaStreamSynchronize(st));
+    *out = h / (double)n;
     return WOTG_OK;
   }
 
@@ -943,18 +354,6 @@ struct Solver {
     return WOTG_OK;
   }
 };
-
-// Frees a solver's captured graphs, stream and events when its entry point
-// returns (every replay has completed by then: each batch is followed by a
-// duality-gap check that synchronises the stream).
-struct SolverGraphs {
-  Solver& s;
-  ~SolverGraphs() { s.release_graphs(); }
-};
-
-// Set for the duration of a no-alloc call: its solver creates no stream, event
-// or graph of its own (plain launches on the caller's stream only).
-static thread_local bool t_plain_launches = false;
 
 struct SolveResult {
   int status = WOTG_OK;
@@ -986,11 +385,11 @@ static int resident_room(int* room) {
   return WOTG_OK;
 }
 
-// A materialised solve (mode kModeGap / kModeFixed) or n_iter refinement
-// iterations at epsilon `eps` (kModeRefine): launches of persist_kernel until
-// it reports an end. A launch is kept to some 20 ms (its iterations cost about
-// 8 us and 2.5 ps per entry), so that a long solve stays a sequence of short
-// kernels.
+// A solve (mode kModeGap / kModeFixed) or n_iter refinement iterations at epsilon
+// `eps` (kModeRefine): launches of the form's persistent kernel until it reports an
+// end. A launch is kept to some 20 ms (an iteration costs about 8 us and 2.5 ps per
+// entry streamed, 0.4 ps per entry on the tensor cores), so that a long solve
+// stays a sequence of short kernels.
 static int solve_persistent(Solver& S, const wotg_params& P, int mode, double eps, int n_iter, SolveResult& res) {
   static_assert(sizeof(PersistCtl) <= 16 * sizeof(double), "PersistCtl lives in Vecs::scal");
   PersistArgs A{};
@@ -1013,54 +412,88 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
   A.extra_iter = P.extra_iter;
   A.n_iter = n_iter;
   A.mode = mode;
-  const double per_iter = 8e-6 + 2.5e-12 * (double)S.g.I * (double)S.g.J;
+  const double per_iter = 8e-6 + (S.tc.on ? 4e-13 : 2.5e-12) * (double)S.g.I * (double)S.g.J;
   A.budget = std::max<long long>(8, std::min<long long>(2000, (long long)(0.02 / per_iter)));
-  WOTG_CUDA(cudaMemsetAsync(A.ctl, 0, sizeof(PersistCtl), S.st));
+  PersistCtl h{};
+  if (S.tc.on) {
+    int s = S.mean_of(S.V.p, S.g.I, &h.q);
+    if (s) return s;
+  }
+  WOTG_CUDA(cudaMemcpyAsync(A.ctl, &h, sizeof(h), cudaMemcpyHostToDevice, S.st));
   // one CTA per SM; fewer only where the device grants the process fewer SMs
   int grid = std::min(sm_count(), kRedBlocks);
-  bool resident = false;
   int rows_cap = 0, cols_cap = 0;
-  size_t smem = 0;
-  {
+  size_t smem = kMergeHeaderBytes;
+  const bool gap = mode == kModeGap;
+  const void* streamed = gap ? reinterpret_cast<const void*>(persist_kernel<true>)
+                             : reinterpret_cast<const void*>(persist_kernel<false>);
+  const void* kernel = streamed;
+  TcPersistArgs T{};
+  int threads = kPersistThreads;
+  if (S.tc.on) {
+    const TcState& t = S.tc;
+    T.p = A;
+    T.x = TcSide{t.Xa, t.Xb, t.X, t.ldx, S.g.I, t.normX, t.offX, t.redoX, t.n_xt};
+    T.y = TcSide{t.Ya, t.Yb, t.Y, t.ldy, S.g.J, t.normY, t.offY, t.redoY, t.n_yt};
+    T.d = t.d;
+    T.part = t.part;
+    T.redo_total = t.redo_total;
+    const Coef c = S.coef(eps, P, h.q);
+    T.logs[0] = c.logI;
+    T.logs[1] = c.logJ;
+    T.logs[2] = c.logq;
+    T.logs[3] = std::log(P.tau);
+    WOTG_CUDA(cudaMemsetAsync(t.redoX, 0, sizeof(int), S.st));
+    WOTG_CUDA(cudaMemsetAsync(t.redoY, 0, sizeof(int), S.st));
+    kernel = t.kp == 32 ? (gap ? reinterpret_cast<const void*>(tc_persist_kernel<32, true>)
+                               : reinterpret_cast<const void*>(tc_persist_kernel<32, false>))
+                        : (gap ? reinterpret_cast<const void*>(tc_persist_kernel<64, true>)
+                               : reinterpret_cast<const void*>(tc_persist_kernel<64, false>));
+    smem = t.kp == 32 ? TcPersist<32>::kAlloc : TcPersist<64>::kAlloc;
+    WOTG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    T.vctas = t.ctas_row;
+    grid = std::min(grid, t.ctas_row);
+    threads = kTcPersistThreads;
+  } else {
     const ResidentPlan plan = resident_plan(S.g, grid);
     int room = 0;
     int s = resident_room(&room);
     if (s) return s;
-    resident = resident_fits(plan, S.g, (size_t)room);
-    if (resident) {
+    if (resident_fits(plan, S.g, (size_t)room)) {
       grid = plan.grid;
       rows_cap = plan.rows;
       cols_cap = plan.cols4 * 4;
       smem = plan.bytes;
+      threads = kResidentThreads;
+      kernel = gap ? reinterpret_cast<const void*>(resident_kernel<true>)
+                   : reinterpret_cast<const void*>(resident_kernel<false>);
     }
   }
-  const bool gap = mode == kModeGap;
-  const void* streamed = gap ? reinterpret_cast<const void*>(persist_kernel<true>)
-                             : reinterpret_cast<const void*>(persist_kernel<false>);
-  const void* kernel = !resident ? streamed
-                       : gap     ? reinterpret_cast<const void*>(resident_kernel<true>)
-                                 : reinterpret_cast<const void*>(resident_kernel<false>);
-  PersistCtl h{};
   for (;;) {
     WOTG_CUDA(cudaMemsetAsync(&A.ctl->bar, 0, 2 * sizeof(unsigned long long), S.st));
-    void* args[] = {&A, &rows_cap, &cols_cap};
-    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid),
-                                                dim3(kernel == streamed ? kPersistThreads : kResidentThreads), args,
-                                                smem, S.st);
-    while (e == cudaErrorCooperativeLaunchTooLarge && (kernel != streamed || grid > 1)) {
-      // fewer SMs than the device has: the streamed variant runs on any number
+    void* args[] = {S.tc.on ? (void*)&T : (void*)&A, &rows_cap, &cols_cap};
+    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, S.st);
+    while (e == cudaErrorCooperativeLaunchTooLarge && (threads == kResidentThreads || grid > 1)) {
+      // fewer SMs than the device has: a smaller grid, which the streamed and the
+      // on-the-fly kernels run on as well
       cudaGetLastError();
-      if (kernel == streamed) grid /= 2;
-      kernel = streamed;
-      smem = 0;
-      e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kPersistThreads), args, smem, S.st);
+      if (threads == kResidentThreads) {
+        kernel = streamed;
+        threads = kPersistThreads;
+        smem = kMergeHeaderBytes;
+      } else {
+        grid /= 2;
+        T.vctas = std::min(T.vctas, kTcHalves * grid);
+      }
+      e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, S.st);
     }
     WOTG_CUDA(e);
     WOTG_LAUNCHED();
     WOTG_CUDA(cudaMemcpyAsync(&h, A.ctl, sizeof(h), cudaMemcpyDeviceToHost, S.st));
     WOTG_CUDA(cudaStreamSynchronize(S.st));
     if (h.err) {
-      set_last_message("persistent solver: a bounded grid barrier ran out");
+      set_last_message(S.tc.on ? "tensor-core solver: a bounded wait timed out"
+                               : "persistent solver: a bounded grid barrier ran out");
       return WOTG_CUDA_ERROR;
     }
     if (h.status != kRunning) break;
@@ -1073,147 +506,6 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
   res.max_iter = h.status == kMaxIter;
   res.final_coef = S.coef(h.eps, P, h.q);
   return h.status == kNonfinite ? WOTG_NONFINITE : WOTG_OK;
-}
-
-// Python's max(x, y): returns x unless y > x (so a NaN in first position wins).
-static inline double py_max(double x, double y) { return (y > x) ? y : x; }
-
-// The on-the-fly form's duality-gap solver: the control on the host.
-static int solve_duality_gap(Solver& S, const wotg_params& P, double q, SolveResult& res) {
-  const int n_scalings = 5;
-  const double scale_factor = std::exp(-std::log(P.epsilon) / n_scalings);
-  double eps_i = P.epsilon0 * scale_factor;
-  int64_t it = 0;
-  int parity = 0;
-  double gap = INFINITY;
-  Coef c{};
-  bool lrow_valid = false;
-  for (int stage = 0; stage <= n_scalings; ++stage) {
-    gap = INFINITY;
-    const double eps_old = eps_i;
-    eps_i = eps_i / scale_factor;
-    c = S.coef(eps_i, P, q);
-    int s = S.rescale(eps_old, eps_i);
-    if (s) return s;
-    s = S.tc_prepare(c);
-    if (s) return s;
-    parity = 0;
-    lrow_valid = false;
-    const bool final = stage == n_scalings;
-    const double threshold = final ? P.tolerance : 1e-6;
-    double sumK = 0.0;
-    if (final) {
-      s = S.sum_exp(c, &sumK);
-      if (s) return s;
-    }
-    S.drop_graphs();
-    while (gap > threshold) {
-      const int nb = final ? P.batch_size : 5;
-      bool replayed = false;
-      if (final && lrow_valid && S.steady() && (double)(it + nb) < P.max_iter) {
-        s = S.batch_graph(c, nb, parity, P.tau, &replayed);
-        if (s) return s;
-      }
-      if (replayed) {
-        it += nb;
-        lrow_valid = false;
-        parity ^= (nb & 1);
-      }
-      for (int t = 0; t < nb && !replayed; ++t) {
-        ++it;
-        s = S.iteration(c, lrow_valid, parity);
-        if (s) return s;
-        lrow_valid = false;
-        s = S.absorb(c, P.tau, parity);
-        if (s) return s;
-        parity ^= 1;
-        if ((double)it >= P.max_iter) {
-          res.max_iter = true;
-          res.iterations = it;
-          res.gap = gap;
-          res.eps = eps_i;
-          res.final_coef = c;
-          s = S.fresh_lrow(c);
-          if (s) return s;
-          return WOTG_OK;
-        }
-      }
-      double h[kNq];
-      ++res.checks;
-      if (final) {
-        s = S.fresh_lrow(c);
-        if (s) return s;
-        lrow_valid = true;
-        gap_partial_kernel<<<kRedBlocks, 256, 0, S.st>>>(S.g, S.V, c, S.V.red);
-        WOTG_LAUNCHED();
-        s = S.reduce_to_host(h);
-        if (s) return s;
-        const double I = (double)S.g.I, J = (double)S.g.J;
-        const double dx = 1.0 / I, dy = 1.0 / J;
-        const double gap_abs = dx * h[0] + dy * h[1];
-        const double pri = P.lambda1 * dx * h[2] + P.lambda2 * dy * h[3] + dx * h[4] + dy * h[5] +
-                           eps_i * (sumK / (I * J) - dx * h[6]);
-        gap = gap_abs / std::fabs(pri);
-      } else {
-        stage_test_kernel<<<kRedBlocks, 256, 0, S.st>>>(S.g, S.V, c, S.V.red);
-        WOTG_LAUNCHED();
-        s = S.reduce_to_host(h);
-        if (s) return s;
-        const double ga = std::sqrt(h[0]) / (1.0 + std::sqrt(h[1]));
-        const double gb = std::sqrt(h[2]) / (1.0 + std::sqrt(h[3]));
-        gap = py_max(ga, gb);
-      }
-    }
-  }
-  res.iterations = it;
-  res.gap = gap;
-  res.eps = eps_i;
-  res.final_coef = c;
-  if (std::isnan(gap)) return WOTG_NONFINITE;
-  // Lrow is valid (last gap check ran with the current b).
-  return WOTG_OK;
-}
-
-static int solve_fixed_iters(Solver& S, const wotg_params& P, double q, SolveResult& res) {
-  const double eps_final = P.epsilon;
-  double eps_i = P.epsilon0;  // tau is never None here (the host rejects it)
-  Coef c = S.coef(eps_i, P, q);
-  int s = S.rescale(0.0, eps_i);
-  if (s) return s;
-  s = S.tc_prepare(c);
-  if (s) return s;
-  int parity = 0;
-  int since = 0, index = 0;
-  for (int it = 0; it < P.scaling_iter; ++it) {
-    s = S.iteration(c, false, parity);
-    if (s) return s;
-    ++since;
-    s = S.absorb(c, P.tau, parity);
-    if (s) return s;
-    parity ^= 1;
-    if (since == P.inner_iter_max) {
-      ++index;
-      since = 0;
-      const double eps_new = (P.epsilon0 - eps_final) * std::exp(-(double)index) + eps_final;
-      s = S.rescale(eps_i, eps_new);
-      if (s) return s;
-      parity = 0;
-      eps_i = eps_new;
-      c = S.coef(eps_i, P, q);
-      s = S.tc_prepare(c);
-      if (s) return s;
-    }
-  }
-  for (int it = 0; it < P.extra_iter; ++it) {
-    s = S.iteration(c, false, parity);
-    if (s) return s;
-  }
-  s = S.fresh_lrow(c);
-  if (s) return s;
-  res.iterations = (int64_t)P.scaling_iter + P.extra_iter;
-  res.eps = eps_i;
-  res.final_coef = c;
-  return WOTG_OK;
 }
 
 // Row blocks of the column pass: about kColCtasPerSm CTAs of 1024 columns per
@@ -1338,8 +630,17 @@ static void tc_layout(Bump& b, const wotg_problem* prob, TcState& tc) {
   tc.redoY = b.take<int>(2 + prob->J);
   tc.tile_ctr = b.take<int>((size_t)4 * std::max(tc.n_xt, tc.n_yt));
   tc.redo_total = b.take<unsigned long long>(1);
-  tc.off_row_ok = tc.off_col_ok = false;
-  tc.xb_ok = tc.yb_ok = false;
+}
+
+// The on-the-fly form's buffers; column forms (coordinates; the bias columns are
+// written by the solver) and norms.
+static int tc_setup(Bump& b, const wotg_problem* prob, Solver& S) {
+  tc_layout(b, prob, S.tc);
+  WOTG_CUDA(cudaMemsetAsync(S.tc.redo_total, 0, sizeof(unsigned long long), S.st));
+  const float sigma = (float)std::sqrt(prob->cost_scale);
+  int s = tc_pack_points(prob->X, prob->I, prob->ldx, prob->d, S.tc.kp, sigma, 0, S.tc.Xb, S.tc.normX, S.st);
+  if (s) return s;
+  return tc_pack_points(prob->Y, prob->J, prob->ldy, prob->d, S.tc.kp, sigma, 0, S.tc.Yb, S.tc.normY, S.st);
 }
 
 extern "C" size_t wotg_problem_workspace_bytes(const wotg_problem* prob) {
@@ -1394,18 +695,9 @@ extern "C" int wotg_compute_transport_matrix(const wotg_problem* prob, const wot
   Vecs V{};
   layout(b, g, V);
   cudaStream_t st = (cudaStream_t)stream;
-  Solver S{prob->C, g, V, st, prob->cost_scale, 0, TcState{}};
-  SolverGraphs graphs_guard{S};
-  S.graphs_off = t_plain_launches;
+  Solver S{prob->C, g, V, st, prob->cost_scale, TcState{}};
   if (tc_requested(prob)) {
-    tc_layout(b, prob, S.tc);
-    WOTG_CUDA(cudaMemsetAsync(S.tc.err, 0, sizeof(int), st));
-    WOTG_CUDA(cudaMemsetAsync(S.tc.redo_total, 0, sizeof(unsigned long long), st));
-    // column forms (coordinates; bias columns written per half-step) and norms
-    const float sigma = (float)std::sqrt(prob->cost_scale);
-    int s = tc_pack_points(prob->X, I, prob->ldx, prob->d, S.tc.kp, sigma, 0, S.tc.Xb, S.tc.normX, st);
-    if (s) return s;
-    s = tc_pack_points(prob->Y, J, prob->ldy, prob->d, S.tc.kp, sigma, 0, S.tc.Yb, S.tc.normY, st);
+    int s = tc_setup(b, prob, S);
     if (s) return s;
   }
 
@@ -1420,19 +712,7 @@ extern "C" int wotg_compute_transport_matrix(const wotg_problem* prob, const wot
     init_kernel<<<S.vec_blocks(std::max(I, ldc)), 256, 0, st>>>(g, V, G);
     WOTG_LAUNCHED();
     SolveResult res;
-    int s;
-    if (S.tc.on) {
-      double q = 0.0;
-      s = S.mean_of(V.p, I, &q);
-      if (s) return s;
-      s = (P.solver == WOTG_SOLVER_DUALITY_GAP) ? solve_duality_gap(S, P, q, res) : solve_fixed_iters(S, P, q, res);
-      int absorptions = 0;
-      WOTG_CUDA(cudaMemcpyAsync(&absorptions, V.counters, sizeof(int), cudaMemcpyDeviceToHost, st));
-      WOTG_CUDA(cudaStreamSynchronize(st));
-      res.absorptions = absorptions;
-    } else {
-      s = solve_persistent(S, P, P.solver == WOTG_SOLVER_DUALITY_GAP ? kModeGap : kModeFixed, P.epsilon, 0, res);
-    }
+    int s = solve_persistent(S, P, P.solver == WOTG_SOLVER_DUALITY_GAP ? kModeGap : kModeFixed, P.epsilon, 0, res);
     total.iterations += res.iterations;
     total.absorptions += res.absorptions;
     total.checks += res.checks;
@@ -1458,17 +738,8 @@ extern "C" int wotg_compute_transport_matrix(const wotg_problem* prob, const wot
     }
   }
   WOTG_CUDA(cudaStreamSynchronize(st));
-  if (S.tc.on) {
-    int err = 0;
-    WOTG_CUDA(cudaMemcpy(&err, S.tc.err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (err) {
-      set_last_message("tensor-core half-step: a bounded wait timed out");
-      return WOTG_CUDA_ERROR;
-    }
-    unsigned long long redo = 0;
-    WOTG_CUDA(cudaMemcpy(&redo, S.tc.redo_total, sizeof(redo), cudaMemcpyDeviceToHost));
-    total.exact_rows = (int32_t)std::min<unsigned long long>(redo, 0x7fffffffull);
-  }
+  int s = S.exact_rows(&total.exact_rows);
+  if (s) return s;
   if (stats) *stats = total;
   return status;
 }
@@ -1495,50 +766,19 @@ extern "C" int wotg_refine_potentials(const wotg_problem* prob, const wotg_param
   Vecs V{};
   layout(b, g, V);
   cudaStream_t st = (cudaStream_t)stream;
-  Solver S{prob->C, g, V, st, prob->cost_scale, 0, TcState{}};
-  SolverGraphs graphs_guard{S};
-  S.graphs_off = t_plain_launches;
+  Solver S{prob->C, g, V, st, prob->cost_scale, TcState{}};
   if (tc_requested(prob)) {
-    tc_layout(b, prob, S.tc);
-    WOTG_CUDA(cudaMemsetAsync(S.tc.err, 0, sizeof(int), st));
-    WOTG_CUDA(cudaMemsetAsync(S.tc.redo_total, 0, sizeof(unsigned long long), st));
-    const float sigma = (float)std::sqrt(prob->cost_scale);
-    int s = tc_pack_points(prob->X, I, prob->ldx, prob->d, S.tc.kp, sigma, 0, S.tc.Xb, S.tc.normX, st);
-    if (s) return s;
-    s = tc_pack_points(prob->Y, J, prob->ldy, prob->d, S.tc.kp, sigma, 0, S.tc.Yb, S.tc.normY, st);
+    int s = tc_setup(b, prob, S);
     if (s) return s;
   }
   init_kernel<<<S.vec_blocks(std::max(I, ldc)), 256, 0, st>>>(g, V, prob->G);
   WOTG_LAUNCHED();
-  int s;
-  Coef c{};
-  int64_t absorptions = 0;
-  if (S.tc.on) {
-    double q = 0.0;
-    s = S.mean_of(V.p, I, &q);
-    if (s) return s;
-    c = S.coef(epsilon, P, q);
-    load_potentials_kernel<<<S.vec_blocks(I + J), 256, 0, st>>>(g, V, u_bar, v_bar, c.inv_eps);
-    WOTG_LAUNCHED();
-    s = S.tc_prepare(c);
-    if (s) return s;
-    int parity = 0;
-    for (int it = 0; it < n_iter; ++it) {
-      s = S.iteration(c, false, parity);
-      if (s) return s;
-      s = S.absorb(c, P.tau, parity);
-      if (s) return s;
-      parity ^= 1;
-    }
-  } else {
-    load_potentials_kernel<<<S.vec_blocks(I + J), 256, 0, st>>>(g, V, u_bar, v_bar, 1.0 / epsilon);
-    WOTG_LAUNCHED();
-    SolveResult res;
-    s = solve_persistent(S, P, kModeRefine, epsilon, n_iter, res);
-    if (s) return s;
-    c = res.final_coef;
-    absorptions = res.absorptions;
-  }
+  load_potentials_kernel<<<S.vec_blocks(I + J), 256, 0, st>>>(g, V, u_bar, v_bar, 1.0 / epsilon);
+  WOTG_LAUNCHED();
+  SolveResult res;
+  int s = solve_persistent(S, P, kModeRefine, epsilon, n_iter, res);
+  if (s) return s;
+  const Coef c = res.final_coef;
   s = S.outputs(c, false, nullptr, nullptr, u_bar, v_bar);
   if (s) return s;
   WOTG_CUDA(cudaStreamSynchronize(st));
@@ -1546,21 +786,9 @@ extern "C" int wotg_refine_potentials(const wotg_problem* prob, const wotg_param
   out.iterations = n_iter;
   out.final_epsilon = epsilon;
   out.gap = NAN;
-  out.absorptions = absorptions;
-  if (S.tc.on) {
-    int absorbed = 0;
-    WOTG_CUDA(cudaMemcpy(&absorbed, V.counters, sizeof(int), cudaMemcpyDeviceToHost));
-    out.absorptions = absorbed;
-    int err = 0;
-    WOTG_CUDA(cudaMemcpy(&err, S.tc.err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (err) {
-      set_last_message("tensor-core half-step: a bounded wait timed out");
-      return WOTG_CUDA_ERROR;
-    }
-    unsigned long long redo = 0;
-    WOTG_CUDA(cudaMemcpy(&redo, S.tc.redo_total, sizeof(redo), cudaMemcpyDeviceToHost));
-    out.exact_rows = (int32_t)std::min<unsigned long long>(redo, 0x7fffffffull);
-  }
+  out.absorptions = res.absorptions;
+  s = S.exact_rows(&out.exact_rows);
+  if (s) return s;
   if (stats) *stats = out;
   return WOTG_OK;
 }
@@ -1628,10 +856,6 @@ extern "C" int wotg_compute_transport_matrix_noalloc(const wotg_problem* prob, c
     WOTG_CUDA(cudaGetSymbolAddress(&scratch, g_noalloc_scratch));
     g_noalloc_ptr[dev].store(scratch, std::memory_order_release);
   }
-  struct Plain {
-    Plain() { t_plain_launches = true; }
-    ~Plain() { t_plain_launches = false; }
-  } plain;
   return wotg_compute_transport_matrix(prob, params, tmap, learned_growth, row_sums, u_bar, v_bar, stats,
                                        scratch, kNoAllocScratchBytes, stream);
 }
