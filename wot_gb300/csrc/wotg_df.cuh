@@ -67,10 +67,12 @@ __device__ __forceinline__ float4 log_table_entry(int i) {
   return make_float4(rc, th, (float)(t - (double)th), 0.f);
 }
 
-// log2(h + l) = c + d for h in [2^-100, 2^100]: table-driven (P. T. P. Tang, ACM
+// log2(h + l) = c + d + f for h in [2^-100, 2^100]: table-driven (P. T. P. Tang, ACM
 // TOMS 16, 1990): h + l = 2^e mant, r = mant / c - 1 with |r| < 1/255, the series
-// of log(1 + r) with its first two terms as pairs. Absolute error below 2^-42.
-__device__ __forceinline__ void log2_pair(float h, float l, const float4* tab, float& c, float& d) {
+// of log(1 + r) with its first two terms as pairs. Absolute error about 2^-48 (as a
+// pair, c + d rounded, it was 2^-44: enough to move a weight's low part, of 2^-39
+// units, in every fourth iteration, and with it single FP32 exponents).
+__device__ __forceinline__ void log2_pair(float h, float l, const float4* tab, float& c, float& d, float& f) {
   const int b = __float_as_int(h);
   const int e = (b >> 23) - 127;
   const float scale = __int_as_float((127 - e) << 23);
@@ -94,15 +96,17 @@ __device__ __forceinline__ void log2_pair(float h, float l, const float4* tab, f
   two_sum(t.y, x, s, sl);
   two_sum((float)e, s, u, ul);
   c = u;
-  d = __fadd_rn(ul, __fadd_rn(sl, __fadd_rn(t.z, xl)));
+  float v, vl;
+  two_sum(ul, sl, v, vl);
+  fast_two_sum(v, __fadd_rn(vl, __fadd_rn(t.z, xl)), d, f);
 }
 
 // Base-2 log-sum-exp o + m + log2(h + l) in FP64.
 __device__ __forceinline__ double lse2_pair(float o, float m, float h, float l, const float4* tab) {
   if (!(h >= 0x1p-100f && h <= 0x1p100f)) return (double)o + (double)m + log2((double)h + (double)l);
-  float c, d;
-  log2_pair(h, l, tab, c, d);
-  return ((double)o + (double)m) + ((double)c + (double)d);
+  float c, d, f;
+  log2_pair(h, l, tab, c, d, f);
+  return ((double)o + (double)m) + ((double)c + ((double)d + (double)f));
 }
 
 }  // namespace wotg

@@ -105,7 +105,7 @@ struct PersistShared {
   TcStretch stretch[2][2];        // on-the-fly: of either side, per half
   unsigned int epoch;             // resident: the iteration
   int row_over;                   // resident: an owned row is above tau
-  int off[32];                    // resident: its arrays' places
+  int off[34];                    // resident: its arrays' places
 };
 
 // What the variants that merge sums themselves keep beside it.

@@ -52,7 +52,7 @@ inline ResidentPlan resident_plan(const Geom& g, int sms) {
   const int64_t nv = g.ldc >> 2;
   p.cols4 = (int)((nv + p.grid - 1) / p.grid);
   const size_t rows = (size_t)p.rows, cols = (size_t)p.cols4 * 4;
-  p.bytes = kMergeHeaderBytes + rows * g.ldc * 4 + (size_t)g.ldc * 12 + (rows + cols) * ((7 + 4) * 8 + 16) + rows * 8;
+  p.bytes = kMergeHeaderBytes + rows * g.ldc * 4 + (size_t)g.ldc * 12 + (rows + cols) * ((7 + 4) * 8 + 16 + 4) + rows * 8;
   return p;
 }
 inline bool resident_fits(const ResidentPlan& p, const Geom& g, size_t smem_limit) {
@@ -99,7 +99,8 @@ struct Resident : PersistBase {
   enum : int { kWhi, kWlo, kOcols, kRhi, kRlo,                                                  // floats (C is at kC4)
                kPr, kPc,                                                                      // float4 points
                kU, kLa, kLao, kLogp, kAr, kWr, kKr, kV, kLb, kLbo, kAc, kWc, kKc, kLc, kEx };   // doubles
-  static_assert(kEx < 22, "sh().off[22] on holds the CTA's share");
+  static_assert(kEx < 22, "sh().off[22 .. 30] hold the CTA's share");
+  enum : int { kRp = 32, kCp = 33 };   // floats: the points' third parts
   static constexpr int kC4 = (int)(kMergeHeaderBytes / 16);   // the owned rows of C, in float4s
   static constexpr int kLr = kLao;   // the old scalings are dead in the final stage, where a check keeps its row sums
 
@@ -109,7 +110,8 @@ struct Resident : PersistBase {
   __device__ static __forceinline__ float& F(int array, int t) { return F(sh().off[array] + t); }
   __device__ static __forceinline__ double& D(int array, int t) { return D(sh().off[array] + t); }
   // A row's (column's) point: offset o on the grid; P = W + (A - alpha o ln 2) log2 e as
-  // grid value and remainder, so that its next weight is P - alpha (L2 - o); W.
+  // grid value and remainder (a third part, below the remainder's 2^-39 units, in kRp
+  // and kCp), so that its next weight is P - alpha (L2 - o); W.
   __device__ static __forceinline__ float4& pr(int t) { return F4(sh().off[kPr] + t); }
   __device__ static __forceinline__ float4& pc(int t) { return F4(sh().off[kPc] + t); }
 
@@ -151,6 +153,8 @@ struct Resident : PersistBase {
       at <<= 1;                           // floats
       sh().off[kRhi] = at;
       sh().off[kRlo] = at + rows_cap;
+      sh().off[kRp] = at + 2 * rows_cap;
+      sh().off[kCp] = at + 3 * rows_cap;
       const int nv = (int)(A().g.ldc >> 2), n = gridDim.x, b = blockIdx.x;
       const int b0 = (int)((int64_t)A().g.nrb * b / n), b1 = (int)((int64_t)A().g.nrb * (b + 1) / n);
       const int c0 = (int)((int64_t)nv * b / n), c1 = (int)((int64_t)nv * (b + 1) / n);
@@ -223,17 +227,19 @@ struct Resident : PersistBase {
   // Base-2 log-sum-exp o + m + log2(h + l) in FP64.
   __device__ static __forceinline__ double lse2_own(float o, const float4& r) {
     if (!(r.y >= 0x1p-100f && r.y <= 0x1p100f)) return (double)o + (double)r.x + log2((double)r.y + (double)r.z);
-    float c, d, a, b;
-    log2_pair(r.y, r.z, mg().tab, c, d);
+    float c, d, f, a, b;
+    log2_pair(r.y, r.z, mg().tab, c, d, f);
     two_sum(r.x, c, a, b);
-    return (double)o + ((double)a + (double)__fadd_rn(b, d));
+    return (double)o + ((double)a + ((double)b + ((double)d + (double)f)));
   }
-  // P of a point whose offset is now o (see pr), from K = W + A log2 e.
-  __device__ static __forceinline__ void point_at(float4& p, float o, double K, double alpha) {
-    const float2 w = split(fma(-alpha, (double)o, K));
+  // P of a point whose offset is now o (see pr), from K = W + A log2 e; its third part.
+  __device__ static __forceinline__ void point_at(float4& p, float& third, float o, double K, double alpha) {
+    const double x = fma(-alpha, (double)o, K);
+    const float2 w = split(x);
     p.x = o;
     p.y = w.x;
     p.z = w.y;
+    third = (float)((x - (double)w.x) - (double)w.y);
   }
   // Coefficients folded per stage: log a = A - alpha ln 2 L2, weight = W + log a log2 e = K - alpha L2.
   __device__ static __forceinline__ void fold_row(int t) {
@@ -242,7 +248,7 @@ struct Resident : PersistBase {
     D(kWr, t) = w;
     D(kKr, t) = fma(a, kLog2e, w);
     pr(t).w = (float)w;
-    point_at(pr(t), pr(t).x, D(kKr, t), sh().c.alpha1);
+    point_at(pr(t), F(kRp, t), pr(t).x, D(kKr, t), sh().c.alpha1);
   }
   __device__ static __forceinline__ void fold_col(int t) {
     const double a = fma(D(kV, t), sh().kv, sh().bconst), w = D(kV, t) * sh().iel2;
@@ -250,7 +256,7 @@ struct Resident : PersistBase {
     D(kWc, t) = w;
     D(kKc, t) = fma(a, kLog2e, w);
     pc(t).w = (float)w;
-    point_at(pc(t), pc(t).x, D(kKc, t), sh().c.alpha2);
+    point_at(pc(t), F(kCp, t), pc(t).x, D(kKc, t), sh().c.alpha2);
   }
   __device__ static __noinline__ void fold_all() {
     for (int t = threadIdx.x; t < nr(); t += kResidentThreads) fold_row(t);
@@ -262,13 +268,15 @@ struct Resident : PersistBase {
   // the critical path of the exchange; the FP64 state follows beside it (settle).
   // False where the FP64 path has to decide: sums or values out of range, or a
   // scaling within 1e-3 of tau. On success r becomes (delta, flag, old offset).
-  __device__ static __forceinline__ bool quick(const float4& p, float4& r, float ah, float al, float& o, float& hi, float& lo,
+  __device__ static __forceinline__ bool quick(const float4& p, float third, float4& r, float ah, float al, float& o, float& hi, float& lo,
                                         bool& over) {
     if (!(r.y >= 0x1p-100f && r.y <= 0x1p100f)) return false;
-    float c, d, a, b;
-    log2_pair(r.y, r.z, mg().tab, c, d);
+    float c, d, f, a, b, e;
+    log2_pair(r.y, r.z, mg().tab, c, d, f);
     two_sum(r.x, c, a, b);
-    fast_two_sum(a, __fadd_rn(b, d), a, b);
+    two_sum(b, d, b, e);
+    two_sum(a, b, a, b);
+    fast_two_sum(a, __fadd_rn(b, __fadd_rn(e, f)), a, b);
     float n = rintf(a * 0x1p14f);
     n += rintf(__fmaf_rn(b, 0x1p14f, __fmaf_rn(a, 0x1p14f, -n)));
     o = __fmaf_rn(n, 0x1p-14f, p.x);
@@ -276,7 +284,7 @@ struct Resident : PersistBase {
     const float ze = __fmaf_rn(ah, a, -z) + __fmaf_rn(ah, b, __fmul_rn(al, a));
     float q, ql;
     two_sum(p.z, -z, q, ql);
-    fast_two_sum(q, __fsub_rn(ql, ze), q, ql);
+    fast_two_sum(q, __fadd_rn(__fsub_rn(ql, ze), third), q, ql);
     float k = rintf(q * 0x1p14f);
     k += rintf(__fmaf_rn(ql, 0x1p14f, __fmaf_rn(q, 0x1p14f, -k)));
     hi = __fmaf_rn(k, 0x1p-14f, p.y);
@@ -296,7 +304,7 @@ struct Resident : PersistBase {
     const double L2 = (double)r.w + ((double)r.x + (double)r.y);
     D(kLao, t) = D(kLa, t);
     D(kLa, t) = fma(-sh().a1ln2, L2, D(kAr, t));
-    point_at(pr(t), pr(t).x, D(kKr, t), sh().c.alpha1);
+    point_at(pr(t), F(kRp, t), pr(t).x, D(kKr, t), sh().c.alpha1);
   }
   __device__ static __forceinline__ void settle_col(int t) {
     const float4 r = mg().res[kPersistBlk / 2 + t];
@@ -305,7 +313,7 @@ struct Resident : PersistBase {
     D(kLc, t) = L2;
     D(kLbo, t) = D(kLb, t);
     D(kLb, t) = fma(-sh().a2ln2, L2, D(kAc, t));
-    point_at(pc(t), pc(t).x, D(kKc, t), sh().c.alpha2);
+    point_at(pc(t), F(kCp, t), pc(t).x, D(kKc, t), sh().c.alpha2);
   }
 
   __device__ static __forceinline__ bool update_row(int t, double L2) {
@@ -413,11 +421,11 @@ struct Resident : PersistBase {
         A().V.Lrow[r0() + t] = L2 * kLn2;
         float o;
         near(L2, &o);
-        point_at(F4(p4 + t), o, D(kKr, t), sh().c.alpha1);
+        point_at(F4(p4 + t), F(kRp, t), o, D(kKr, t), sh().c.alpha1);
       } else {
         float o, hi, lo;
         bool ov;
-        if (quick(p, r, sh().a1h, sh().a1l, o, hi, lo, ov)) {
+        if (quick(p, F(kRp, t), r, sh().a1h, sh().a1l, o, hi, lo, ov)) {
           F(kRhi, t) = hi;
           F(kRlo, t) = lo;
           F4(p4 + t).x = o;
@@ -427,7 +435,7 @@ struct Resident : PersistBase {
           const double L2 = lse2_own(p.x, r);
           over |= update_row(t, L2);
           near(L2, &o);
-          point_at(F4(p4 + t), o, D(kKr, t), sh().c.alpha1);
+          point_at(F4(p4 + t), F(kRp, t), o, D(kKr, t), sh().c.alpha1);
           mg().res[t].z = 0.f;
         }
       }
@@ -541,7 +549,7 @@ struct Resident : PersistBase {
       const bool row_flag = r.w != 0.f;
       float o, hi, lo;
       bool ov;
-      if (quick(p, r, sh().a2h, sh().a2l, o, hi, lo, ov)) {
+      if (quick(p, F(kCp, t), r, sh().a2h, sh().a2l, o, hi, lo, ov)) {
         publish(t, hi, lo, o, ov || row_flag);
         F4(p4 + t).x = o;
         mg().res[kPersistBlk / 2 + t] = r;
@@ -554,7 +562,7 @@ struct Resident : PersistBase {
         D(kLc, t) = L2;
         D(kLbo, t) = D(kLb, t);
         D(kLb, t) = x;
-        point_at(F4(p4 + t), o, D(kKc, t), sh().c.alpha2);
+        point_at(F4(p4 + t), F(kCp, t), o, D(kKc, t), sh().c.alpha2);
         mg().res[kPersistBlk / 2 + t].z = 0.f;
       }
     }
