@@ -44,6 +44,7 @@
 
 #include "wotg_coef.cuh"
 #include "wotg_common.cuh"
+#include "wotg_state.cuh"
 
 namespace wotg {
 namespace batch {
@@ -146,6 +147,9 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
 __device__ __forceinline__ void cp_async16(uint32_t saddr, const void* g, uint32_t bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr), "l"(g), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async8(uint32_t saddr, const void* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(saddr), "l"(g) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
@@ -209,38 +213,45 @@ __device__ __forceinline__ double item_b_update(Item& it, int64_t j, double L) {
   return lb_new;
 }
 
-// L2 = base-2 log-sum-exp of row r for entry e; returns the log-scaling whose
-// maximum over rows feeds the absorption test (log a_i or log b_j), else -inf.
-__device__ __forceinline__ double entry_epilogue(Item* items, const Entry& e, int64_t r, double L2) {
+// A log-scaling near or above log tau goes to the item's absorption slot (the test
+// is exp of its maximum > tau; below ltau_lo it cannot be). True when it went.
+__device__ __forceinline__ bool note_scaling(Item& it, double l) {
+  if (!(l > it.c.ltau_lo)) return false;
+  atomic_max_nonneg(&it.maxslot[it.parity], exp(l));
+  return true;
+}
+
+// L2 = base-2 log-sum-exp of row r for entry e; true when an absorption may be due.
+__device__ __forceinline__ bool entry_epilogue(Item* items, const Entry& e, int64_t r, double L2) {
   const double L = L2 * kLn2;
   switch (e.mode) {
     case kOut:
       e.out[r] = L;
       if (e.o) e.o[r] = (float)L2;
-      return -INFINITY;
+      return false;
     case kFresh: {
       Item& it = items[e.item];
       it.Lrow[r] = L;
       it.orow[r] = (float)L2;
-      return -INFINITY;
+      return false;
     }
     case kSumK:
       items[e.item].rsum[r] = exp(L);
-      return -INFINITY;
+      return false;
     case kRowA: {
       Item& it = items[e.item];
       it.Lrow[r] = L;
       it.orow[r] = (float)L2;
-      return item_a_update(it, r, L);
+      return note_scaling(it, item_a_update(it, r, L));
     }
     case kColB: {
       Item& it = items[e.item];
       it.Lcol[r] = L;
       it.ocol[r] = (float)L2;
-      return item_b_update(it, r, L);
+      return note_scaling(it, item_b_update(it, r, L));
     }
     default:
-      return -INFINITY;
+      return false;
   }
 }
 
@@ -292,7 +303,8 @@ __device__ __forceinline__ float4 load_cost(const float4* crow, int64_t q, int64
 // row0 + w * RW + [0, RW)). SPEC: offset sums with exact fallback; else running max.
 template <int KG, int RW, bool SPEC>
 __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int row0, int ng, const Entry* gp,
-                                          float (*sW)[KG][kChunk], double (*s_vmax)[KG], int warp, int lane) {
+                                          float (*sW)[KG][kChunk], float2 (*s_ms)[KG], int* s_over, int warp,
+                                          int lane) {
   float nk2[KG];
   float acc[RW][KG], off[RW][KG];
   bool valid[RW];
@@ -392,8 +404,7 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
           warp_lse(off[rr][k], acc[rr][k]);
       }
     }
-  // Lane k finishes entry k.
-  double vmax = -INFINITY;
+  // Lane k holds entry k.
 #pragma unroll
   for (int rr = 0; rr < RW; ++rr) {
     float s = 0.f, o = 0.f;
@@ -417,25 +428,31 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
         }
       }
     }
-    if (mine) {
-      vmax = fmax(vmax, entry_epilogue(A.items, gp[lane], row[rr], lse2(o, s)));
-    }
+    if (mine) s_ms[warp * RW + rr][lane] = make_float2(o, s);
   }
-  if (lane < KG) s_vmax[warp][lane] = vmax;
+  __syncthreads();
+  // The FP64 updates, a thread per (row, entry): an FP64 instruction takes 64 cycles
+  // however few of a warp's lanes are active, so ten entries of each warp's rows in
+  // turn cost three times as much.
+  const int total = min(kWarps * RW, sg.rows - row0) * ng;
+  for (int idx = threadIdx.x; idx < total; idx += kThreads) {
+    const int r = idx / ng, k = idx - r * ng;
+    const float2 ms = s_ms[r][k];
+    if (entry_epilogue(A.items, gp[k], row0 + r, lse2(ms.x, ms.y))) *s_over = 1;
+  }
 }
 
 // One entry over the tile's rows (a pair with a single active item, as in the
 // tail of a batch): each warp streams its rows with 128-bit loads of the cost
 // and the weights (L1/L2-resident), no shared-memory staging and no barrier.
 // Columns past `cols` in the last float4 meet the cost's +inf padding.
-template <int RW, int KG>
-__device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int row0, const Entry* gp,
-                                           double (*s_vmax)[KG], int warp, int lane) {
+template <int RW>
+__device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int row0, const Entry* gp, int* s_over,
+                                           int warp, int lane) {
   const Entry e = gp[0];
   const float nk2 = e.nk2;
-  const float4* __restrict__ w4 = reinterpret_cast<const float4*>(e.w);
+  const float4* w4 = reinterpret_cast<const float4*>(e.w);
   const int64_t nq = ((int64_t)sg.cols + 3) >> 2;
-  double vmax = -INFINITY;
 #pragma unroll 1
   for (int rr = 0; rr < RW; ++rr) {
     const int64_t row = (int64_t)row0 + warp * RW + rr;
@@ -450,7 +467,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
 #pragma unroll
       for (int t = 0; t < 4; ++t) cc[t] = ld_stream(crow + q + 32 * t);
 #pragma unroll
-      for (int t = 0; t < 4; ++t) ww[t] = __ldg(w4 + q + 32 * t);
+      for (int t = 0; t < 4; ++t) ww[t] = w4[q + 32 * t];   // not __ldg: written by other CTAs before a barrier
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         const uint64_t e01 = ex2_off(fma2(kk, pk(cc[t].x, cc[t].y), pk(ww[t].x, ww[t].y)), mo);
@@ -462,7 +479,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
     }
     for (; q < nq; q += 32) {
       const float4 cc = ld_stream(crow + q);
-      const float4 ww = __ldg(w4 + q);
+      const float4 ww = w4[q];
       s0 += ex2(fmaf(nk2, cc.x, ww.x) - o) + ex2(fmaf(nk2, cc.y, ww.y) - o);
       s1 += ex2(fmaf(nk2, cc.z, ww.z) - o) + ex2(fmaf(nk2, cc.w, ww.w) - o);
     }
@@ -473,17 +490,16 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
       oo = ms.x;
       s = ms.y;
     }
-    if (lane == 0) vmax = fmax(vmax, entry_epilogue(A.items, e, row, lse2(oo, s)));
+    if (lane == 0 && entry_epilogue(A.items, e, row, lse2(oo, s))) *s_over = 1;
   }
-  if (lane == 0) s_vmax[warp][0] = vmax;
 }
 
 template <int KG, int RW, bool SPEC>
 __global__ void __launch_bounds__(kThreads) pass_kernel(PassArgs A) {
   __shared__ __align__(16) float sW[2][KG][kChunk];
   __shared__ Entry gp[KG];
-  __shared__ double s_vmax[kWarps][KG];
-  __shared__ int s_tile;
+  __shared__ float2 s_ms[kWarps * RW][KG];
+  __shared__ int s_tile, s_over;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
     if (threadIdx.x == 0) s_tile = atomicAdd(A.counter, 1);
@@ -500,21 +516,9 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(PassArgs A) {
       if (threadIdx.x < ng) gp[threadIdx.x] = lst[g0 + threadIdx.x];
       __syncthreads();
       if (SPEC && ng == 1)
-        run_single<RW, KG>(A, sg, tile.row0, gp, s_vmax, warp, lane);
+        run_single<RW>(A, sg, tile.row0, gp, &s_over, warp, lane);
       else
-        run_group<KG, RW, SPEC>(A, sg, tile.row0, ng, gp, sW, s_vmax, warp, lane);
-      __syncthreads();
-      // absorption maxima of this group: one atomic per item
-      if (threadIdx.x < ng) {
-        const Entry& e = gp[threadIdx.x];
-        if (e.mode == kRowA || e.mode == kColB) {
-          double v = -INFINITY;
-#pragma unroll
-          for (int w = 0; w < kWarps; ++w) v = fmax(v, s_vmax[w][threadIdx.x]);
-          Item& it = A.items[e.item];
-          atomic_max_nonneg(&it.maxslot[it.parity], exp(v));
-        }
-      }
+        run_group<KG, RW, SPEC>(A, sg, tile.row0, ng, gp, sW, s_ms, &s_over, warp, lane);
       __syncthreads();
     }
   }
@@ -531,43 +535,33 @@ enum Action : int { kActNone = 0, kActCont = 1, kActStage = 2, kActFinish = 3, k
 #define ITEM_LOOP(var, n) \
   for (int var = rank * kThreads + (int)threadIdx.x; var < (n); var += nblk * kThreads)
 
+// Barrier of the kThreads threads that do an item's work (all of a per-item kernel's
+// CTA, the first of the loop kernel's).
+__device__ __forceinline__ void item_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); }
+
+// Sums over the CTA's item threads of the quantities in `used`; the others stay 0.
 template <int NQ>
-__device__ void block_sum(double (&acc)[NQ]) {
+__device__ void block_sum(double (&acc)[NQ], unsigned used = ~0u) {
   __shared__ double sh[kWarps][NQ];
   __shared__ double tot[NQ];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = warp_sum(acc[q]);
+  for (int q = 0; q < NQ; ++q)
+    if (used >> q & 1) acc[q] = warp_sum(acc[q]);
   if (lane == 0)
 #pragma unroll
     for (int q = 0; q < NQ; ++q) sh[wid][q] = acc[q];
-  __syncthreads();
+  item_sync();
   if (threadIdx.x < NQ) {
     double t = 0.0;
-    for (int w = 0; w < kWarps; ++w) t += sh[w][threadIdx.x];
+    if (used >> threadIdx.x & 1)
+      for (int w = 0; w < kWarps; ++w) t += sh[w][threadIdx.x];
     tot[threadIdx.x] = t;
   }
-  __syncthreads();
+  item_sync();
 #pragma unroll
   for (int q = 0; q < NQ; ++q) acc[q] = tot[q];
-  __syncthreads();
-}
-
-__device__ double block_max(double v) {
-  __shared__ double sh[kWarps];
-  __shared__ double tot;
-  v = warp_maxd(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = -INFINITY;
-    for (int w = 0; w < kWarps; ++w) t = fmax(t, sh[w]);
-    tot = t;
-  }
-  __syncthreads();
-  v = tot;
-  __syncthreads();
-  return v;
+  item_sync();
 }
 
 // True in every thread of the last CTA (of `expected`) to arrive at *ctr; all
@@ -575,13 +569,13 @@ __device__ double block_max(double v) {
 __device__ bool arrive_last(int* ctr, int expected) {
   __shared__ bool last;
   __threadfence();
-  __syncthreads();
+  item_sync();
   if (threadIdx.x == 0) {
     const int t = atomicAdd(ctr, 1);
     last = (t == expected - 1);
     if (last) *ctr = 0;
   }
-  __syncthreads();
+  item_sync();
   if (last) __threadfence();
   return last;
 }
@@ -677,6 +671,7 @@ __device__ void start_solve(Item& it) {
   eps = eps / it.scale_factor;
   it.eps_i = eps;
   it.c = make_coef(eps, it.lambda1, it.lambda2, it.cost_scale, it.I, it.J, it.q);
+  it.c.ltau_lo = it.tau > 0.0 ? log(it.tau) - 1e-9 : -INFINITY;
   it.maxslot[0] = 0ull;
   it.maxslot[1] = 0ull;
   it.parity = 0;
@@ -718,8 +713,15 @@ __device__ double reset_slice(Item& it, const double* G, int rank, int nblk) {
 
 // Deterministic total of the item's per-CTA partials (fixed order).
 __device__ __forceinline__ double item_total(const BatchArgs& B, const Item& it, int q) {
+  const double* p = B.part + (int64_t)it.first_blk * kNq + q;
   double t = 0.0;
-  for (int b = 0; b < it.nblk; ++b) t += __ldcg(&B.part[(int64_t)(it.first_blk + b) * kNq + q]);
+  for (int b0 = 0; b0 < it.nblk; b0 += 8) {   // eight loads at a time, in the same order
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = b0 + k < it.nblk ? __ldcg(p + (int64_t)(b0 + k) * kNq) : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += v[k];
+  }
   return t;
 }
 
@@ -755,8 +757,9 @@ __global__ void __launch_bounds__(kThreads) init_kernel(BatchArgs B, const doubl
 
 // After the two half-steps: tau-absorption (optimal_transport.py:137-141),
 // iteration / batch counting, max_iter (:143-145).
-__global__ void __launch_bounds__(kThreads) item_kernel(BatchArgs B) {
-  const ItemBlock ib = B.blk[blockIdx.x];
+// (plain: iterations since the last one that came here, which had nothing to do).
+__device__ void item_body(const BatchArgs& B, int b, int plain) {
+  const ItemBlock ib = B.blk[b];
   Item& it = B.items[ib.item];
   const int rank = ib.rank, nblk = it.nblk;
   if (it.status == kActive) {
@@ -782,9 +785,9 @@ __global__ void __launch_bounds__(kThreads) item_kernel(BatchArgs B) {
       it.maxslot[par ^ 1] = 0ull;
       if (absorb) it.absorptions += 1;
       it.skip_row = 0;
-      it.it += 1;
+      it.it += plain + 1;
       it.parity = par ^ 1;
-      it.batch_cnt += 1;
+      it.batch_cnt += plain + 1;
       const int nb = it.stage == kScalings ? it.batch_size : 5;
       if ((double)it.it >= it.max_iter) {
         it.status = kMaxIterPending;
@@ -794,6 +797,9 @@ __global__ void __launch_bounds__(kThreads) item_kernel(BatchArgs B) {
       }
     }
   }
+}
+__global__ void __launch_bounds__(kThreads) item_kernel(BatchArgs B) {
+  item_body(B, blockIdx.x, 0);
   if (arrive_last(B.counters + 3, gridDim.x)) {
     build_check_lists(B);
     if (threadIdx.x == 0) B.counters[2] = 0;
@@ -807,8 +813,8 @@ __device__ __forceinline__ double py_max(double x, double y) { return (y > x) ? 
 // of a new final stage, and the decision that follows (applied by apply_kernel).
 // Partials: [0..6] gap terms or [0..3] stage-test terms, [7] sum of the row
 // sums of the current coupling (next growth), [8] sum exp(-C/eps).
-__global__ void __launch_bounds__(kThreads) test_kernel(BatchArgs B) {
-  const ItemBlock ib = B.blk[blockIdx.x];
+__device__ void test_body(const BatchArgs& B, int b) {
+  const ItemBlock ib = B.blk[b];
   Item& it = B.items[ib.item];
   const int rank = ib.rank, nblk = it.nblk;
   const int st = it.status;
@@ -825,24 +831,18 @@ __global__ void __launch_bounds__(kThreads) test_kernel(BatchArgs B) {
       ITEM_LOOP(i, it.I) acc[7] += exp(it.la[i] + it.u[i] * c.inv_eps + it.Lrow[i]);
     } else if (due && final) {
       ITEM_LOOP(i, it.I) {
-        const double ui = it.u[i], lai = it.la[i], pi = it.p[i];
-        const double x = exp(lai + ui * c.inv_eps + it.Lrow[i] - c.logJ);
-        const double ub = ui + c.eps * lai;
-        const double at = exp(lai) * exp(ui * c.inv_eps);
-        const double f = x * log(x / pi) - x + pi;
-        const double conj = c.lambda1 * pi * (exp(-c.eps * log(at) / c.lambda1) - 1.0);
+        const double ui = it.u[i], lai = it.la[i], ue = ui * c.inv_eps, ub = ui + c.eps * lai;
+        double x, f, conj;
+        gap_terms(lai + ue + it.Lrow[i] - c.logJ, lai, ue, it.p[i], it.logp[i], c.lambda1, c.eps, &x, &f, &conj);
         acc[0] += c.lambda1 * f + conj + ub * x;
         acc[2] += f;
         acc[4] += ub * x;
         acc[6] += x;
       }
       ITEM_LOOP(j, it.J) {
-        const double vj = it.v[j], lbj = it.lb[j];
-        const double y = exp(lbj + vj * c.inv_eps + it.Lcol[j] - c.logI);
-        const double vb = vj + c.eps * lbj;
-        const double bt = exp(lbj) * exp(vj * c.inv_eps);
-        const double f = y * log(y / c.q) - y + c.q;
-        const double conj = c.lambda2 * c.q * (exp(-c.eps * log(bt) / c.lambda2) - 1.0);
+        const double vj = it.v[j], lbj = it.lb[j], ve = vj * c.inv_eps, vb = vj + c.eps * lbj;
+        double y, f, conj;
+        gap_terms(lbj + ve + it.Lcol[j] - c.logI, lbj, ve, c.q, c.logq, c.lambda2, c.eps, &y, &f, &conj);
         acc[1] += c.lambda2 * f + conj + vb * y;
         acc[3] += f;
         acc[5] += vb * y;
@@ -864,11 +864,15 @@ __global__ void __launch_bounds__(kThreads) test_kernel(BatchArgs B) {
         acc[3] += tb * tb;
       }
     }
-    block_sum<kNq>(acc);
-    if (threadIdx.x < kNq) B.part[(int64_t)blockIdx.x * kNq + threadIdx.x] = acc[threadIdx.x];
-    if (arrive_last(B.item_ctr + ib.item, nblk) && threadIdx.x == 0) {
-      double t[kNq];
-      for (int q = 0; q < kNq; ++q) t[q] = item_total(B, it, q);
+    const unsigned used = (sumk ? 1u << 8 : 0u) | (st == kMaxIterPending ? 1u << 7 : !due ? 0u : final ? 0xFFu : 0xFu);
+    block_sum<kNq>(acc, used);
+    if (threadIdx.x < kNq) B.part[(int64_t)b * kNq + threadIdx.x] = acc[threadIdx.x];
+    const bool last = arrive_last(B.item_ctr + ib.item, nblk);
+    __shared__ double totals[kNq];
+    if (last && threadIdx.x < kNq) totals[threadIdx.x] = used >> threadIdx.x & 1 ? item_total(B, it, threadIdx.x) : 0.0;
+    if (last && threadIdx.x < 32) __syncwarp();
+    if (last && threadIdx.x == 0) {
+      const double* t = totals;
       if (sumk) {
         it.sumK = t[8];
         it.need_sumk = 0;
@@ -904,6 +908,7 @@ __global__ void __launch_bounds__(kThreads) test_kernel(BatchArgs B) {
           it.eps_prev = it.eps_i;
           it.eps_i = it.eps_i / it.scale_factor;
           it.c = make_coef(it.eps_i, it.lambda1, it.lambda2, it.cost_scale, it.I, it.J, it.q);
+          it.c.ltau_lo = it.tau > 0.0 ? log(it.tau) - 1e-9 : -INFINITY;
           it.maxslot[0] = 0ull;
           it.maxslot[1] = 0ull;
           it.parity = 0;
@@ -925,19 +930,18 @@ __global__ void __launch_bounds__(kThreads) test_kernel(BatchArgs B) {
   }
 }
 
+__global__ void __launch_bounds__(kThreads) test_kernel(BatchArgs B) { test_body(B, blockIdx.x); }
+
 // The vector work of test_kernel's decisions, then the next iteration's lists.
-__global__ void __launch_bounds__(kThreads) apply_kernel(BatchArgs B) {
-  const ItemBlock ib = B.blk[blockIdx.x];
+__device__ void apply_body(const BatchArgs& B, int b) {
+  const ItemBlock ib = B.blk[b];
   Item& it = B.items[ib.item];
   const int rank = ib.rank, nblk = it.nblk;
   const int act = it.action;
   if (act != kActNone) {
     const Coef c = it.c;
     if (act == kActCont) {
-      double lmax = -INFINITY;
-      ITEM_LOOP(i, it.I) lmax = fmax(lmax, item_a_update(it, i, it.Lrow[i]));
-      lmax = block_max(lmax);
-      if (threadIdx.x == 0) atomic_max_nonneg(&it.maxslot[it.parity], exp(lmax));
+      ITEM_LOOP(i, it.I) note_scaling(it, item_a_update(it, i, it.Lrow[i]));
     } else if (act == kActStage) {
       // absorb with the old epsilon, a = b = 1; offsets scale with 1/eps
       const double eps_old = it.eps_prev;
@@ -989,7 +993,572 @@ __global__ void __launch_bounds__(kThreads) apply_kernel(BatchArgs B) {
       it.action = kActNone;
     }
   }
+}
+__global__ void __launch_bounds__(kThreads) apply_kernel(BatchArgs B) {
+  apply_body(B, blockIdx.x);
   if (arrive_last(B.counters + 7, gridDim.x)) finish_body(B);
+}
+
+// ---------------------------------------------------------------------------
+// Small batches: the whole loop in one cooperative kernel.
+//
+// What bounds it: an iteration of a day's sweep (ten items on a 1250 x 1800 cost) is 3 us
+// of exponentials per pass, but its six launches took 71 us: about 3 us each to start
+// and drain, two staged passes of 12 to 20 us, and test, apply and item kernels that have
+// nothing to do in four iterations of five (all items' batches end together). Here grid
+// barriers take the place of launches, and an iteration in which no item's batch
+// ends and no scaling nears tau (a plain one) is two passes and two barriers. The
+// lists are not built by a last CTA either: each tile picks its pair's entries from
+// the items' state.
+// ---------------------------------------------------------------------------
+//
+// One CTA of 20 warps per SM: two rows per warp (the rows of a direction are dealt out
+// evenly), the weights of all columns in shared memory at once, so that a pass has no
+// barriers between column chunks; one FP64 update per (row, entry) on state read ahead
+// of the sums. (In double-buffered chunks of 128 columns a pass took 2000 cycles per
+// chunk, waiting.) Column sums keep the order of run_group and run_single.
+// ---------------------------------------------------------------------------
+constexpr int kLoopThreads = 640, kLoopWarps = kLoopThreads / 32;
+constexpr int kLoopRW = 2, kLoopRows = kLoopRW * kLoopWarps;   // rows of a warp, of a round
+constexpr int kLoopKG = 8;          // entries of a register group
+constexpr int kLoopAhead = 3;       // cost loads in flight per lane and row
+constexpr int kLoopMaxItems = 32;   // items of a pair: a warp picks from them
+constexpr int kLoopMaxPairs = 1 << 14;
+constexpr int kLoopIters = 200;     // iterations of a launch: its barrier's flag counts stay below 2^20
+constexpr uint32_t kLoopTries = 6000000;   // polls of a barrier
+
+// rows [row0, row0 + rows) of a pair
+struct LoopTile {
+  int pair_rows, row0;   // pair | rows << 14
+};
+struct LoopDir {
+  const LoopTile* tiles;   // CTA b's tile at b
+  int ntiles;
+  int kg;   // the tuned pass's group: an entry alone in its group is summed by run_single
+};
+struct LoopArgs {
+  BatchArgs B;
+  const Seg* segs;
+  LoopDir dir[2];
+  unsigned long long* bar;   // arrivals (24 bits), two flag counts (20 bits each)
+  int* err;
+  int wcap;                  // floats of the weights' shared memory
+};
+// An entry with its item's pointers and coefficients for the update, cached between
+// the iterations that change them.
+struct LoopEntry {
+  Entry e;
+  const double *pot, *logp;
+  double *ls, *ls_old, *L;
+  float* wout;
+  double inv_eps, alpha, logn, inv_le, logq, ltau_lo;
+};
+struct LoopShared {
+  LoopEntry list[2][kLoopMaxItems];
+  Entry chk[2 * kLoopMaxItems];
+  double state[3][kLoopRows * kLoopKG];   // potential, log-scaling, log p of the (row, entry) pairs in hand
+  float2 ms[kLoopRows][kLoopKG];     // their (offset, sum)
+  float2 nko[kLoopRows][kLoopKG];    // (-kappa2, -offset)
+  int n[3];                          // entries of the row, column and check lists
+  int pair[2], row0[2], rows[2];     // the CTA's tiles
+  Seg seg[2];                        // their costs
+  int kg[2], wcap;
+  int over, ok;
+  unsigned int target, seen, seen2, any, any2;
+};
+static_assert(sizeof(LoopTile) == sizeof(Tile), "kept in the tiles' memory");
+constexpr size_t kLoopHeader = (sizeof(LoopShared) + 127) / 128 * 128;
+extern __shared__ __align__(128) unsigned char loop_smem[];
+
+// All CTAs arrive; the flags of any CTA come back in sh.any and sh.any2.
+__device__ bool loop_barrier(const LoopArgs& A, LoopShared& sh, bool flag, bool flag2) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(A.bar),
+                 "l"(1ull + ((unsigned long long)(flag ? 1 : 0) << 24) + ((unsigned long long)(flag2 ? 1 : 0) << 44))
+                 : "memory");
+    sh.target += gridDim.x;
+    unsigned long long v = 0;
+    bool done = false;
+    for (uint32_t t = 0; t < kLoopTries && !done; ++t) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(A.bar) : "memory");
+      done = (v & 0xFFFFFFu) >= sh.target;
+      if ((t & 255) == 255 && *(volatile int*)A.err) break;
+    }
+    const unsigned int f = (unsigned int)(v >> 24) & 0xFFFFFu, f2 = (unsigned int)(v >> 44);
+    sh.any = f != sh.seen;
+    sh.any2 = f2 != sh.seen2;
+    sh.seen = f;
+    sh.seen2 = f2;
+    if (!done) {
+      atomicExch(A.err, 1);
+      sh.ok = 0;
+    }
+  }
+  __syncthreads();
+  return sh.ok != 0;
+}
+
+// The entries of a pass on the CTA's pair, in the order of its items (warp 0).
+__device__ void pick_entries(const BatchArgs& B, int p, int mode, LoopShared& sh) {
+  const int lane = threadIdx.x & 31, off = B.pair_off[p], k = off + lane;
+  bool one = false, two = false;
+  int item = 0;
+  if (k < B.pair_off[p + 1]) {
+    item = B.pair_items[k];
+    const Item& it = B.items[item];
+    const int st = __ldcg(&it.status), skip = __ldcg(&it.skip_row), due = __ldcg(&it.due), stage = __ldcg(&it.stage),
+              sumk = __ldcg(&it.need_sumk);
+    if (mode == kColB) {
+      one = st == kActive;
+    } else if (mode == kRowA) {
+      one = st == kActive && !skip;
+    } else {
+      one = st == kMaxIterPending || (st == kActive && due && stage == kScalings);
+      two = st == kActive && sumk == 1;
+    }
+  }
+  const unsigned m1 = __ballot_sync(0xffffffffu, one), m2 = __ballot_sync(0xffffffffu, two);
+  const unsigned lt = (1u << lane) - 1;
+  int at = __popc(m1 & lt) + __popc(m2 & lt);
+  if (mode == kFresh) {
+    if (one) sh.chk[at++] = make_entry(B.items, item, mode, B.zeros);
+    if (two) sh.chk[at] = make_entry(B.items, item, kSumK, B.zeros);
+  } else if (one) {
+    const Item& it = B.items[item];
+    const Coef& c = it.c;
+    LoopEntry& e = sh.list[mode == kColB][at];
+    e.e = make_entry(B.items, item, mode, B.zeros);
+    const bool row = mode == kRowA;
+    e.pot = row ? it.u : it.v;
+    e.logp = row ? it.logp : nullptr;
+    e.ls = row ? it.la : it.lb;
+    e.ls_old = row ? it.la_old : it.lb_old;
+    e.L = row ? it.Lrow : it.Lcol;
+    e.wout = row ? it.wrow : it.wcol;
+    e.inv_eps = c.inv_eps;
+    e.alpha = row ? c.alpha1 : c.alpha2;
+    e.logn = row ? c.logJ : c.logI;
+    e.inv_le = row ? c.inv_l1e : c.inv_l2e;
+    e.logq = c.logq;
+    e.ltau_lo = c.ltau_lo;
+  }
+  if (lane == 0) sh.n[mode == kRowA ? 0 : mode == kColB ? 1 : 2] = __popc(m1) + __popc(m2);
+}
+__device__ __forceinline__ const Entry& loop_entry(const LoopShared& sh, int which, int k) {
+  return which == 2 ? sh.chk[k] : sh.list[which][k].e;
+}
+
+// Weights of columns [c0, c0 + cs) of ng entries into W[k cs + c]; zero past `cols`.
+__device__ __forceinline__ void loop_stage(float* W, const LoopShared& sh, int which, int g0, int ng, int c0, int cs,
+                                           int cols) {
+  const int q4 = cs >> 2;
+  for (int idx = threadIdx.x; idx < ng * q4; idx += kLoopThreads) {
+    const int k = idx / q4, q = idx - k * q4;
+    const int left = cols - (c0 + q * 4);
+    const uint32_t bytes = left >= 4 ? 16u : (left > 0 ? (uint32_t)left * 4u : 0u);
+    const float* w = loop_entry(sh, which, g0 + k).w;
+    cp_async16(smem_addr(W + k * cs + q * 4), bytes ? w + c0 + q * 4 : w, bytes);
+  }
+  cp_async_commit();
+}
+__device__ __forceinline__ void loop_staged() {
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+}
+
+// The pass works in functions of their own that share little but shared memory: a
+// register spilled around a call is a local load, and the barrier's acquire empties
+// L1, so that each would be a trip to L2.
+struct LoopGroup {
+  int dir, which, g0, ng, r0;   // entries [g0, g0 + ng), rows from r0 of the tile on
+};
+// Rows of this warp: r0 + warp + r kLoopWarps.
+__device__ __forceinline__ int loop_row_of(const LoopGroup& g, int r) {
+  return g.r0 + ((int)threadIdx.x >> 5) + r * kLoopWarps;
+}
+// Offsets of a warp's rows: lane k has entry k's.
+__device__ __forceinline__ void loop_offsets(const LoopGroup& g, LoopShared& sh, float (&o)[kLoopRW]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < kLoopRW; ++r) {
+    const int i = loop_row_of(g, r);
+    o[r] = 0.f;
+    if (lane < g.ng && i < sh.rows[g.dir]) {
+      const Entry& e = loop_entry(sh, g.which, g.g0 + lane);
+      if (e.o) o[r] = e.o[sh.row0[g.dir] + i];
+    }
+  }
+}
+// Lane k holds entry k's sum of each row: out of range exactly, then into sh.ms.
+__device__ __noinline__ void loop_redo(const LoopGroup g, LoopShared& sh, int r, float s) {
+  const int lane = threadIdx.x & 31, i = loop_row_of(g, r);
+  unsigned redo = __ballot_sync(0xffffffffu, lane < g.ng && !(s >= kSpecLo && s <= kSpecHi));
+  while (redo) {
+    const int k = __ffs(redo) - 1;
+    redo &= redo - 1;
+    const Entry& e = loop_entry(sh, g.which, g.g0 + k);
+    const Seg& sg = sh.seg[g.dir];
+    const float2 ms = exact_row(sg.C + (int64_t)(sh.row0[g.dir] + i) * sg.ldc, sg.ldc, e.w, e.nk2, sg.cols, lane);
+    if (lane == k) sh.ms[i - g.r0][k] = ms;
+  }
+}
+__device__ __forceinline__ void loop_sums(const LoopGroup& g, LoopShared& sh, const float (&o)[kLoopRW],
+                                          const float (&s)[kLoopRW]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < kLoopRW; ++r) {
+    const int i = loop_row_of(g, r);
+    if (i >= sh.rows[g.dir]) continue;
+    if (lane < g.ng) sh.ms[i - g.r0][lane] = make_float2(o[r], s[r]);
+    if (__any_sync(0xffffffffu, lane < g.ng && !(s[r] >= kSpecLo && s[r] <= kSpecHi))) {
+      __syncwarp();
+      loop_redo(g, sh, r, s[r]);
+    }
+  }
+}
+
+// run_group's sums of a warp's rows; the weights of `cs` columns at a time (staged here
+// when that is not all of them).
+__device__ __noinline__ void loop_rows(const LoopGroup g, LoopShared& sh, int cs, int steps) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Seg& sg = sh.seg[g.dir];
+  const int nv = (int)(sg.ldc >> 2), nch = (sg.cols + kChunk - 1) / kChunk;
+  const float* const W = reinterpret_cast<float*>(loop_smem + kLoopHeader);
+  float o[kLoopRW];
+  loop_offsets(g, sh, o);
+  float2 (*const nko)[kLoopKG] = sh.nko + warp * kLoopRW;
+  const float4* crow[kLoopRW];
+  bool valid[kLoopRW];
+  float acc[kLoopRW][kLoopKG];
+#pragma unroll
+  for (int r = 0; r < kLoopRW; ++r) {
+    const int i = loop_row_of(g, r);
+    valid[r] = i < sh.rows[g.dir];
+    crow[r] = reinterpret_cast<const float4*>(sg.C + (int64_t)(sh.row0[g.dir] + (valid[r] ? i : 0)) * sg.ldc) + lane;
+    if (lane < g.ng) nko[r][lane] = make_float2(loop_entry(sh, g.which, g.g0 + lane).nk2, -o[r]);
+#pragma unroll
+    for (int k = 0; k < kLoopKG; ++k) acc[r][k] = 0.f;
+  }
+  __syncwarp();
+  for (int st = 0; st < steps; ++st) {
+    const int ch0 = st * (cs / kChunk), ch1 = min(nch, ch0 + cs / kChunk);
+    if (steps > 1) {
+      __syncthreads();
+      loop_stage(const_cast<float*>(W), sh, g.which, g.g0, g.ng, ch0 * kChunk, cs, sg.cols);
+      loop_staged();
+    }
+    if (!valid[0]) continue;
+    float4 nx[kLoopAhead][kLoopRW];
+#pragma unroll
+    for (int t = 0; t < kLoopAhead; ++t)
+#pragma unroll
+      for (int r = 0; r < kLoopRW; ++r)
+        nx[t][r] = load_cost(crow[r], (ch0 + t) * 32, nv - lane, valid[r] && ch0 + t < ch1);
+    for (int ch = ch0; ch < ch1; ch += kLoopAhead) {
+#pragma unroll
+      for (int t = 0; t < kLoopAhead; ++t) {
+        if (ch + t >= ch1) break;
+        uint64_t c01[kLoopRW], c23[kLoopRW];
+#pragma unroll
+        for (int r = 0; r < kLoopRW; ++r) {
+          c01[r] = pk(nx[t][r].x, nx[t][r].y);
+          c23[r] = pk(nx[t][r].z, nx[t][r].w);
+          const int nc = ch + t + kLoopAhead;
+          nx[t][r] = load_cost(crow[r], nc * 32, nv - lane, valid[r] && nc < ch1);
+        }
+        const float* wb = W + (ch + t - ch0) * kChunk + lane * 4;
+#pragma unroll
+        for (int k = 0; k < kLoopKG; ++k) {
+          if (k < g.ng) {
+            const float4 w = *reinterpret_cast<const float4*>(wb + k * cs);
+            const uint64_t w01 = pk(w.x, w.y), w23 = pk(w.z, w.w);
+#pragma unroll
+            for (int r = 0; r < kLoopRW; ++r) {
+              const float2 p = nko[r][k];
+              const uint64_t kk = pk(p.x, p.x), mo = pk(p.y, p.y);
+              const uint64_t e01 = ex2_off(fma2(kk, c01[r], w01), mo);
+              const uint64_t e23 = ex2_off(fma2(kk, c23[r], w23), mo);
+              const float2 e = upk(add2(e01, e23));
+              acc[r][k] += e.x + e.y;
+            }
+          }
+        }
+      }
+    }
+  }
+  float s[kLoopRW];
+#pragma unroll
+  for (int r = 0; r < kLoopRW; ++r) {
+    s[r] = 0.f;
+#pragma unroll
+    for (int k = 0; k < kLoopKG; ++k)
+      if (k < g.ng) {
+        const float x = warp_sumf(acc[r][k]);
+        if (k == lane) s[r] = x;
+      }
+  }
+  loop_sums(g, sh, o, s);
+}
+// run_single's sums of a warp's rows; weights in shared memory, or (too many columns)
+// in global memory.
+template <bool STAGED>
+__device__ __noinline__ void loop_rows_single(const LoopGroup g, LoopShared& sh) {
+  const int lane = threadIdx.x & 31;
+  const Seg& sg = sh.seg[g.dir];
+  const int nq = (sg.cols + 3) >> 2;
+  const Entry& e = loop_entry(sh, g.which, g.g0);
+  const float nk2 = e.nk2;
+  const uint64_t kk = pk(nk2, nk2);
+  const float4* const wg = reinterpret_cast<const float4*>(e.w);
+  auto weight = [&](int q) { return STAGED ? reinterpret_cast<const float4*>(loop_smem + kLoopHeader)[q] : wg[q]; };
+  float o[kLoopRW], s0[kLoopRW], s1[kLoopRW];
+  loop_offsets(g, sh, o);
+  const float4* crow[kLoopRW];
+#pragma unroll
+  for (int r = 0; r < kLoopRW; ++r) {
+    const int i = loop_row_of(g, r);
+    crow[r] = reinterpret_cast<const float4*>(sg.C + (int64_t)(sh.row0[g.dir] + (i < sh.rows[g.dir] ? i : 0)) * sg.ldc);
+    o[r] = __shfl_sync(0xffffffffu, o[r], 0);
+    s0[r] = s1[r] = 0.f;
+  }
+  if (loop_row_of(g, 0) < sh.rows[g.dir]) {
+    float4 nx[kLoopRW][4];
+    int q = lane;
+    if (q + 96 < nq) {
+#pragma unroll
+      for (int r = 0; r < kLoopRW; ++r)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) nx[r][t] = ld_stream(crow[r] + q + 32 * t);
+    }
+    for (; q + 96 < nq; q += 128) {
+      const bool more = q + 128 + 96 < nq;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float4 ww = weight(q + 32 * t);
+#pragma unroll
+        for (int r = 0; r < kLoopRW; ++r) {
+          const uint64_t mo = pk(-o[r], -o[r]);
+          const float4 cc = nx[r][t];
+          if (more) nx[r][t] = ld_stream(crow[r] + q + 128 + 32 * t);
+          const uint64_t e01 = ex2_off(fma2(kk, pk(cc.x, cc.y), pk(ww.x, ww.y)), mo);
+          const uint64_t e23 = ex2_off(fma2(kk, pk(cc.z, cc.w), pk(ww.z, ww.w)), mo);
+          const float2 e = upk(add2(e01, e23));
+          s0[r] += e.x;
+          s1[r] += e.y;
+        }
+      }
+    }
+    for (; q < nq; q += 32) {
+      const float4 ww = weight(q);
+#pragma unroll
+      for (int r = 0; r < kLoopRW; ++r) {
+        const float4 cc = ld_stream(crow[r] + q);
+        s0[r] += ex2(fmaf(nk2, cc.x, ww.x) - o[r]) + ex2(fmaf(nk2, cc.y, ww.y) - o[r]);
+        s1[r] += ex2(fmaf(nk2, cc.z, ww.z) - o[r]) + ex2(fmaf(nk2, cc.w, ww.w) - o[r]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kLoopRW; ++r) s0[r] = warp_sumf(s0[r] + s1[r]);
+  loop_sums(g, sh, o, s0);
+}
+
+// The state of the (row, entry) pairs in hand, on its way to shared memory.
+__device__ __noinline__ void loop_fetch(const LoopGroup g, LoopShared& sh) {
+  const int total = min(kLoopRows, sh.rows[g.dir] - g.r0) * g.ng, base = sh.row0[g.dir] + g.r0;
+  for (int t = threadIdx.x; t < total; t += kLoopThreads) {
+    const int r = t / g.ng, i = base + r;
+    const LoopEntry& e = sh.list[g.which][g.g0 + t - r * g.ng];
+    cp_async8(smem_addr(&sh.state[0][t]), e.pot + i);
+    cp_async8(smem_addr(&sh.state[1][t]), e.ls + i);
+    if (g.dir == 0) cp_async8(smem_addr(&sh.state[2][t]), e.logp + i);
+  }
+}
+// The updates of the pairs in hand, a thread per pair: item_a_update and item_b_update
+// on the state read ahead.
+__device__ __noinline__ void loop_update(const LoopGroup g, LoopShared& sh, Item* items) {
+  const int total = min(kLoopRows, sh.rows[g.dir] - g.r0) * g.ng, base = sh.row0[g.dir] + g.r0;
+  for (int t = threadIdx.x; t < total; t += kLoopThreads) {
+    const int r = t / g.ng, k = t - r * g.ng, i = base + r;
+    const float2 ms = sh.ms[r][k];
+    const double L2 = lse2(ms.x, ms.y);
+    if (g.which == 2) {
+      entry_epilogue(items, sh.chk[g.g0 + k], i, L2);
+      continue;
+    }
+    const LoopEntry& e = sh.list[g.which][g.g0 + k];
+    const double pot = sh.state[0][t], logp = g.dir == 0 ? sh.state[2][t] : e.logq, L = L2 * kLn2;
+    e.L[i] = L;
+    e.e.o[i] = (float)L2;
+    const double logs = pot * e.inv_eps + L - e.logn;
+    const double x = e.alpha * (logp - logs) - pot * e.inv_le;
+    e.ls_old[i] = sh.state[1][t];
+    e.ls[i] = x;
+    e.wout[i] = (float)((pot * e.inv_eps + x) * kLog2e);
+    if (x > e.ltau_lo && note_scaling(items[e.e.item], x)) sh.over = 1;
+  }
+}
+
+// One pass over the CTA's rows of a direction. `fresh`: lists anew.
+__device__ __noinline__ void loop_pass(const BatchArgs& B, int dir, int mode, bool fresh, LoopShared& sh) {
+  if (sh.rows[dir] == 0) return;
+  LoopGroup g;
+  g.dir = dir;
+  g.which = mode == kFresh ? 2 : dir;
+  if (fresh) {
+    __syncthreads();
+    if (threadIdx.x < 32) pick_entries(B, sh.pair[dir], mode, sh);
+    __syncthreads();
+  }
+  for (g.g0 = 0; g.g0 < sh.n[g.which];) {
+    const int n = sh.n[g.which], main = n - (n % sh.kg[dir] == 1 ? 1 : 0);
+    const bool single = g.g0 == main;
+    g.ng = single ? 1 : min(kLoopKG, main - g.g0);
+    // columns staged at once: all, or as many chunks as fit
+    const int nch = (sh.seg[dir].cols + kChunk - 1) / kChunk, fit = sh.wcap / (g.ng * kChunk);
+    const int steps = (nch + fit - 1) / fit, cs = (nch + steps - 1) / steps * kChunk;
+    for (g.r0 = 0; g.r0 < sh.rows[dir]; g.r0 += kLoopRows) {
+      if (g.which != 2) loop_fetch(g, sh);
+      if (steps == 1 && g.r0 == 0)
+        loop_stage(reinterpret_cast<float*>(loop_smem + kLoopHeader), sh, g.which, g.g0, g.ng, 0, cs, sh.seg[dir].cols);
+      else
+        cp_async_commit();
+      loop_staged();
+      if (!single)
+        loop_rows(g, sh, cs, steps);
+      else if (steps == 1)
+        loop_rows_single<true>(g, sh);
+      else
+        loop_rows_single<false>(g, sh);
+      __syncthreads();
+      loop_update(g, sh, B.items);
+      __syncthreads();
+    }
+    g.g0 += g.ng;
+  }
+}
+
+// The CTA's tiles.
+__device__ void loop_load(const LoopArgs& A, LoopShared& sh) {
+  if (threadIdx.x == 0) {
+    for (int dir = 0; dir < 2; ++dir) {
+      sh.rows[dir] = 0;
+      if ((int)blockIdx.x < A.dir[dir].ntiles) {
+        const LoopTile t = A.dir[dir].tiles[blockIdx.x];
+        sh.pair[dir] = t.pair_rows & (kLoopMaxPairs - 1);
+        sh.rows[dir] = t.pair_rows / kLoopMaxPairs;
+        sh.row0[dir] = t.row0;
+        sh.seg[dir] = A.segs[2 * sh.pair[dir] + dir];
+      }
+      sh.kg[dir] = A.dir[dir].kg;
+    }
+    sh.wcap = A.wcap;
+    sh.n[0] = sh.n[1] = sh.n[2] = 0;
+    sh.target = sh.seen = sh.seen2 = 0;
+    sh.over = 0;
+    sh.ok = 1;
+  }
+  __syncthreads();
+}
+
+// Whether an item of this CTA asks for more than a plain iteration (thread 0).
+__device__ bool loop_wants(const BatchArgs& B, int nblk, int plain) {
+  bool f = false;
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    if (B.blk[b].rank != 0) continue;
+    const Item& it = B.items[B.blk[b].item];
+    if (__ldcg(&it.status) != kActive) continue;
+    const int nb = __ldcg(&it.stage) == kScalings ? it.batch_size : 5;
+    f |= __ldcg(&it.batch_cnt) + plain + 1 >= nb || (double)(__ldcg(&it.it) + plain + 1) >= it.max_iter ||
+         __ldcg(&it.skip_row) != 0 || __ldcg(&it.need_sumk) == 1 || !(it.tau > 0.0);
+  }
+  return f;
+}
+// Whether an item of this CTA needs the check pass or a test; whether one still runs.
+__device__ void loop_status(const BatchArgs& B, int nblk, bool* check, bool* active) {
+  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
+    if (B.blk[b].rank != 0) continue;
+    const Item& it = B.items[B.blk[b].item];
+    const int st = __ldcg(&it.status);
+    *check |= st == kMaxIterPending || (st == kActive && (__ldcg(&it.due) || __ldcg(&it.need_sumk) == 1));
+    *active |= st == kActive || st == kMaxIterPending;
+  }
+}
+
+__global__ void __launch_bounds__(kLoopThreads, 1) loop_kernel(const __grid_constant__ LoopArgs A, int nblk) {
+  LoopShared& sh = *reinterpret_cast<LoopShared*>(loop_smem);
+  const BatchArgs& B = A.B;
+  const bool items = threadIdx.x < kThreads;   // the threads of the per-item work
+  loop_load(A, sh);
+  int plain = 0;
+  bool running = true;
+  for (int n = 0; n < kLoopIters && running; ++n) {
+    const bool fresh = plain == 0;   // the items' state may have changed since the last pass
+    loop_pass(B, 0, kRowA, fresh, sh);
+    if (!loop_barrier(A, sh, false, false)) return;
+    loop_pass(B, 1, kColB, fresh, sh);
+    __syncthreads();
+    // the last iteration leaves nothing pending
+    const bool wants = threadIdx.x == 0 && (sh.over || n == kLoopIters - 1 || loop_wants(B, nblk, plain));
+    if (!loop_barrier(A, sh, wants, false)) return;
+    if (threadIdx.x == 0) sh.over = 0;
+    if (!sh.any) {
+      ++plain;
+      continue;
+    }
+    if (items)
+      for (int b = blockIdx.x; b < nblk; b += gridDim.x) item_body(B, b, plain);
+    plain = 0;
+    // the items' last CTAs decided: read the outcome after the barrier
+    if (!loop_barrier(A, sh, false, false)) return;
+    bool check = false, active = false;
+    if (threadIdx.x == 0) loop_status(B, nblk, &check, &active);
+    if (!loop_barrier(A, sh, check, active)) return;
+    running = sh.any2 != 0;
+    if (!sh.any) continue;
+    loop_pass(B, 0, kFresh, true, sh);
+    if (!loop_barrier(A, sh, false, false)) return;
+    if (items)
+      for (int b = blockIdx.x; b < nblk; b += gridDim.x) test_body(B, b);
+    if (!loop_barrier(A, sh, false, false)) return;
+    if (items)
+      for (int b = blockIdx.x; b < nblk; b += gridDim.x) apply_body(B, b);
+    if (!loop_barrier(A, sh, false, false)) return;
+    check = active = false;
+    if (threadIdx.x == 0) loop_status(B, nblk, &check, &active);
+    if (!loop_barrier(A, sh, false, active)) return;
+    running = sh.any2 != 0;
+  }
+  if (blockIdx.x == 0) {   // the count of active items for the host
+    int c = 0;
+    for (int k = threadIdx.x; k < B.n_items; k += kLoopThreads) {
+      const int st = __ldcg(&B.items[k].status);
+      c += st == kActive || st == kMaxIterPending ? 1 : 0;
+    }
+    c = __syncthreads_count(c != 0);
+    if (threadIdx.x == 0) B.active[0] = c;
+  }
+}
+
+// Rows of a direction dealt out evenly to at most `ctas` tiles of whole rows of one
+// pair, at least 8 rows each (the tiles' memory). A pass is mostly latency, the same for
+// 10 rows as for 40 (a round), so a row counts as its columns and another 2000. Empty
+// when there are too many pairs, or rows for a tile's word.
+static std::vector<LoopTile> loop_tiles(const std::vector<int>& rows, const std::vector<int>& cols, int ctas) {
+  double total = 0.0;
+  for (size_t p = 0; p < rows.size(); ++p) total += (double)rows[p] * (cols[p] + 2000.0);
+  const int spare = ctas - (int)rows.size();   // every pair has one tile at least
+  std::vector<LoopTile> out;
+  if (spare < 0 || *std::max_element(rows.begin(), rows.end()) >= 1 << 17) return out;
+  for (size_t p = 0; p < rows.size(); ++p) {
+    const int n = std::min((rows[p] + 7) / 8, 1 + (int)(spare * ((double)rows[p] * (cols[p] + 2000.0) / total)));
+    for (int k = 0; k < n; ++k) {
+      const int r0 = (int)((int64_t)rows[p] * k / n), r1 = (int)((int64_t)rows[p] * (k + 1) / n);
+      out.push_back(LoopTile{(int)p | (r1 - r0) * kLoopMaxPairs, r0});
+    }
+  }
+  return out;
 }
 
 // ---------------------------------------------------------------------------
@@ -1062,7 +1631,7 @@ static std::vector<Tile> make_tiles(const std::vector<int>& rows, const std::vec
 
 // CTAs of the per-item kernels for an item of I + J points.
 static inline int item_blocks(int64_t I, int64_t J) {
-  return (int)std::min<int64_t>(32, std::max<int64_t>(1, (I + J + 2047) / 2048));
+  return (int)std::min<int64_t>(32, std::max<int64_t>(1, (I + J + 511) / 512));
 }
 
 struct Layout {
@@ -1297,6 +1866,9 @@ extern "C" size_t wotg_batch_workspace_bytes(const wotg_pair* pairs, int32_t n_p
 
 namespace {
 constexpr int kBodies = 8;  // iterations of the whole batch per graph launch
+// Exponentials of a pass up to which the batch runs in the loop kernel: about 60 us of
+// them at this part's rate, where the six launches' fixed 40 us are most of an iteration.
+constexpr double kLoopMaxExps = 5e8;
 }
 
 extern "C" int wotg_solve_batched(const wotg_pair* pairs, int32_t n_pairs, const wotg_item* items, int32_t n_items,
@@ -1462,67 +2034,130 @@ extern "C" int wotg_solve_batched(const wotg_pair* pairs, int32_t n_pairs, const
   init_kernel<<<nblk, kThreads, 0, cs>>>(B, L.G);
   WOTG_LAUNCHED();
 
-  const PassCfg& c0 = kCfgs[cfg[0]];
-  const PassCfg& c1 = kCfgs[cfg[1]];
-  PassArgs Arow{L.segs, 0, L.tiles[0][rw_slot(c0.rw)], L.ntiles[0][rw_slot(c0.rw)], L.row_n, L.row_list, L.pair_off,
-                L.items, L.counters + 0};
-  PassArgs Acol{L.segs, 1, L.tiles[1][rw_slot(c1.rw)], L.ntiles[1][rw_slot(c1.rw)], L.col_n, L.col_list, L.pair_off,
-                L.items, L.counters + 1};
-  PassArgs Achk{L.segs, 0, L.tiles[0][rw_slot(c0.rw)], L.ntiles[0][rw_slot(c0.rw)], L.chk_n, L.chk_list, chk_off,
-                L.items, L.counters + 2};
-  const int grid_row = pass_grid(c0.spec), grid_col = pass_grid(c1.spec);
-
-  WOTG_BCUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-  for (int b = 0; b < kBodies; ++b) {
-    c0.spec<<<grid_row, kThreads, 0, cs>>>(Arow);
-    c1.spec<<<grid_col, kThreads, 0, cs>>>(Acol);
-    item_kernel<<<nblk, kThreads, 0, cs>>>(B);
-    c0.spec<<<grid_row, kThreads, 0, cs>>>(Achk);
-    test_kernel<<<nblk, kThreads, 0, cs>>>(B);
-    apply_kernel<<<nblk, kThreads, 0, cs>>>(B);
-  }
-  {
-    cudaError_t e = cudaStreamEndCapture(cs, &graph);
-    if (e != cudaSuccess) {
-      set_last_error("cudaStreamEndCapture", e);
-      cleanup();
-      return WOTG_CUDA_ERROR;
-    }
-  }
-  WOTG_BCUDA(cudaGetLastError());
-  WOTG_BCUDA(cudaGraphInstantiate(&exec, graph, 0));
-
-  // Replay until no item is active; the active count of launch n is read while
-  // launch n + 1 runs.
   double max_iters = 0.0;
   for (int k = 0; k < ni; ++k)
     max_iters = std::max(max_iters, items[k].params.max_iter * std::max(1, items[k].params.growth_iters));
-  const double max_launches = std::min(max_iters, 1e12) / kBodies + 4;
-  long long launched = 0;
   g_replay_prof.clear();
   auto t_last = std::chrono::steady_clock::now();
-  for (;;) {
-    const int slot = (int)(launched & 1);
-    WOTG_BCUDA(cudaGraphLaunch(exec, cs));
-    for (int q = 0; q < kBodies * 6; ++q) count_launch();
-    WOTG_BCUDA(cudaMemcpyAsync(pinned + slot, L.active, sizeof(int), cudaMemcpyDeviceToHost, cs));
-    WOTG_BCUDA(cudaEventRecord(ev_done[slot], cs));
-    ++launched;
-    if (launched >= 2) {
-      const int prev = slot ^ 1;
-      WOTG_BCUDA(cudaEventSynchronize(ev_done[prev]));
-      // replay profile: the host waits on replay n - 1 while replay n runs, so the
-      // interval between these waits is one replay's device time once GPU-bound
-      const auto t_now = std::chrono::steady_clock::now();
-      g_replay_prof.push_back(std::make_pair(pinned[prev],
-                                             std::chrono::duration<float, std::milli>(t_now - t_last).count()));
-      t_last = t_now;
-      if (pinned[prev] == 0) break;
+  // Small batches run in the loop kernel.
+  const int g = sm_count();
+  std::vector<LoopTile> lt[2] = {loop_tiles(rows0, cols0, g), loop_tiles(cols0, rows0, g)};
+  double exps = 0.0;
+  for (int k = 0; k < ni; ++k) exps += (double)hi[k].I * hi[k].J;
+  bool in_loop = !lt[0].empty() && !lt[1].empty() && exps <= kLoopMaxExps &&
+                 *std::max_element(kp.begin(), kp.end()) <= kLoopMaxItems;
+  if (in_loop) {
+    int room = 0, dev = 0;
+    WOTG_BCUDA(cudaGetDevice(&dev));
+    WOTG_BCUDA(cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes attr{};
+    WOTG_BCUDA(cudaFuncGetAttributes(&attr, loop_kernel));
+    const int smem = (room - (int)attr.sharedSizeBytes) / 128 * 128;
+    WOTG_BCUDA(cudaFuncSetAttribute(loop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    LoopArgs A{};
+    A.B = B;
+    A.segs = L.segs;
+    A.wcap = (smem - (int)kLoopHeader) / (int)sizeof(float);
+    for (int d = 0; d < 2; ++d) {
+      WOTG_BCUDA(cudaMemcpyAsync(L.tiles[d][0], lt[d].data(), sizeof(LoopTile) * lt[d].size(), cudaMemcpyHostToDevice, cs));
+      A.dir[d] = LoopDir{reinterpret_cast<const LoopTile*>(L.tiles[d][0]), (int)lt[d].size(), kCfgs[cfg[d]].kg};
     }
-    if ((double)launched > max_launches) {
-      set_last_message("wotg_solve_batched: iteration bound exceeded");
-      status = WOTG_CUDA_ERROR;
-      break;
+    A.bar = reinterpret_cast<unsigned long long*>(L.active + 2);
+    A.err = L.active + 1;
+    int nb = nblk;
+    const double max_launches = std::min(max_iters, 1e12) / kLoopIters + 4;
+    for (double launched = 0.0;; launched += 1.0) {
+      WOTG_BCUDA(cudaMemsetAsync(L.active, 0, 4 * sizeof(int), cs));
+      void* args[] = {&A, &nb};
+      cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(loop_kernel), dim3(g), dim3(kLoopThreads),
+                                                  args, smem, cs);
+      if (e == cudaErrorCooperativeLaunchTooLarge && launched == 0.0) {
+        // fewer SMs than the device has: the launches below, with their own tiles
+        cudaGetLastError();
+        in_loop = false;
+        for (int d = 0; d < 2; ++d)
+          WOTG_BCUDA(cudaMemcpyAsync(L.tiles[d][0], tiles[d][0].data(), sizeof(Tile) * tiles[d][0].size(),
+                                     cudaMemcpyHostToDevice, cs));
+        break;
+      }
+      WOTG_BCUDA(e);
+      count_launch();
+      WOTG_BCUDA(cudaMemcpyAsync(pinned, L.active, 2 * sizeof(int), cudaMemcpyDeviceToHost, cs));
+      WOTG_BCUDA(cudaStreamSynchronize(cs));
+      const auto t_now = std::chrono::steady_clock::now();
+      g_replay_prof.push_back(std::make_pair(pinned[0], std::chrono::duration<float, std::milli>(t_now - t_last).count()));
+      t_last = t_now;
+      if (pinned[1]) {
+        set_last_message("wotg_solve_batched: a bounded grid barrier ran out");
+        status = WOTG_CUDA_ERROR;
+        break;
+      }
+      if (pinned[0] == 0) break;
+      if (launched > max_launches) {
+        set_last_message("wotg_solve_batched: iteration bound exceeded");
+        status = WOTG_CUDA_ERROR;
+        break;
+      }
+    }
+  }
+  if (!in_loop) {
+    const PassCfg& c0 = kCfgs[cfg[0]];
+    const PassCfg& c1 = kCfgs[cfg[1]];
+    PassArgs Arow{L.segs, 0, L.tiles[0][rw_slot(c0.rw)], L.ntiles[0][rw_slot(c0.rw)], L.row_n, L.row_list, L.pair_off,
+                  L.items, L.counters + 0};
+    PassArgs Acol{L.segs, 1, L.tiles[1][rw_slot(c1.rw)], L.ntiles[1][rw_slot(c1.rw)], L.col_n, L.col_list, L.pair_off,
+                  L.items, L.counters + 1};
+    PassArgs Achk{L.segs, 0, L.tiles[0][rw_slot(c0.rw)], L.ntiles[0][rw_slot(c0.rw)], L.chk_n, L.chk_list, chk_off,
+                  L.items, L.counters + 2};
+    const int grid_row = pass_grid(c0.spec), grid_col = pass_grid(c1.spec);
+
+    WOTG_BCUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+    for (int b = 0; b < kBodies; ++b) {
+      c0.spec<<<grid_row, kThreads, 0, cs>>>(Arow);
+      c1.spec<<<grid_col, kThreads, 0, cs>>>(Acol);
+      item_kernel<<<nblk, kThreads, 0, cs>>>(B);
+      c0.spec<<<grid_row, kThreads, 0, cs>>>(Achk);
+      test_kernel<<<nblk, kThreads, 0, cs>>>(B);
+      apply_kernel<<<nblk, kThreads, 0, cs>>>(B);
+    }
+    {
+      cudaError_t e = cudaStreamEndCapture(cs, &graph);
+      if (e != cudaSuccess) {
+        set_last_error("cudaStreamEndCapture", e);
+        cleanup();
+        return WOTG_CUDA_ERROR;
+      }
+    }
+    WOTG_BCUDA(cudaGetLastError());
+    WOTG_BCUDA(cudaGraphInstantiate(&exec, graph, 0));
+
+    // Replay until no item is active; the active count of launch n is read while
+    // launch n + 1 runs.
+    const double max_launches = std::min(max_iters, 1e12) / kBodies + 4;
+    long long launched = 0;
+    for (;;) {
+      const int slot = (int)(launched & 1);
+      WOTG_BCUDA(cudaGraphLaunch(exec, cs));
+      for (int q = 0; q < kBodies * 6; ++q) count_launch();
+      WOTG_BCUDA(cudaMemcpyAsync(pinned + slot, L.active, sizeof(int), cudaMemcpyDeviceToHost, cs));
+      WOTG_BCUDA(cudaEventRecord(ev_done[slot], cs));
+      ++launched;
+      if (launched >= 2) {
+        const int prev = slot ^ 1;
+        WOTG_BCUDA(cudaEventSynchronize(ev_done[prev]));
+        // replay profile: the host waits on replay n - 1 while replay n runs, so the
+        // interval between these waits is one replay's device time once GPU-bound
+        const auto t_now = std::chrono::steady_clock::now();
+        g_replay_prof.push_back(std::make_pair(pinned[prev],
+                                               std::chrono::duration<float, std::milli>(t_now - t_last).count()));
+        t_last = t_now;
+        if (pinned[prev] == 0) break;
+      }
+      if ((double)launched > max_launches) {
+        set_last_message("wotg_solve_batched: iteration bound exceeded");
+        status = WOTG_CUDA_ERROR;
+        break;
+      }
     }
   }
   WOTG_BCUDA(cudaMemcpyAsync(hi.data(), L.items, sizeof(Item) * ni, cudaMemcpyDeviceToHost, cs));
