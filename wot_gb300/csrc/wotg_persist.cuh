@@ -64,6 +64,7 @@ struct PersistArgs {
   double scale_factor;            // exp(-log(epsilon) / kScalings)
   int batch_size, scaling_iter, inner_iter_max, extra_iter, n_iter, mode;
   long long budget;               // iterations of this launch (a batch is not split)
+  int wfloats;                    // streamed: floats of a weight vector kept in shared memory, 0: none are
 };
 
 // The solver's control state during a launch; thread 0 of every CTA keeps the
@@ -505,9 +506,45 @@ struct Owned : PersistBase {
   }
 };
 
+__device__ __forceinline__ void async16(void* to, const void* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // The streamed variant: C read from L2 or HBM in both passes, the FP64 state in
 // global memory (own rows and columns only), any size.
+//
+// What bounds it: the instructions per element. A pass over 4001 x 5003 took 44000
+// cycles of each SM for its rows and 34000 for its columns, of which the exponentials
+// are 5400, whether its costs came ahead of use through a ring in shared memory or
+// not; 23000 and 24000 with the arithmetic on packed FP32 pairs (wotg_state.cuh) and
+// the weights and their low parts, twice the bytes of the costs, in shared memory
+// (22.3 -> 18.4 ms a solve). Two rows per warp, or 24 or 32 warps, were no faster.
 struct Streamed : Owned {
+  __device__ static __forceinline__ float* wstage() { return reinterpret_cast<float*>(persist_smem + kMergeHeaderBytes); }
+  // Copies a pass's weights and their low parts (n floats each) to shared memory.
+  __device__ static __forceinline__ void stage(const float* w, const float* wl, int n) {
+    if (!A().wfloats) return;
+    float* to = wstage();
+    for (int k = threadIdx.x * 4; k < n; k += kPersistThreads * 4) {
+      if (k + 4 <= n) {
+        async16(to + k, w + k);
+        async16(to + A().wfloats + k, wl + k);
+      } else {
+        for (int q = k; q < n; ++q) {
+          to[q] = w[q];
+          to[A().wfloats + q] = wl[q];
+        }
+      }
+    }
+    async_commit();
+    async_wait<0>();
+  }
   __device__ static __forceinline__ int c0() { return sh().c0; }
   __device__ static __forceinline__ int c1() { return sh().c1; }
   // I row offsets (on the weight grid) in rowc's memory, free during the solve; J
@@ -552,33 +589,36 @@ struct Streamed : Owned {
     return over_tau(lb);
   }
 
+  // Row sums of rows [b, e) into res, a warp per row.
+  template <bool STAGED>
+  __device__ static __noinline__ void row_sums(int b, int e) {
+    const int lane = threadIdx.x & 31, nv = (int)(A().g.ldc >> 2);
+    const float4* const w4 = reinterpret_cast<const float4*>(STAGED ? wstage() : A().V.wcol);
+    const float4* const wl4 = reinterpret_cast<const float4*>(STAGED ? wstage() + A().wfloats : A().V.wcol_lo);
+    for (int i = b + (threadIdx.x >> 5); i < e; i += kPersistWarps) {
+      float m, s, cmp, h, l;
+      const float4* row = reinterpret_cast<const float4*>(A().C + (int64_t)i * A().g.ldc);
+      row_lse<true>([row](int k) { return ld_stream(row + k); }, [w4](int k) { return w4[k]; },
+                    [wl4](int k) { return wl4[k]; }, nv, lane, orow()[i], sh().c.kappa2, sh().c.kappa2_lo, m, s, cmp);
+      two_sum(s, -cmp, h, l);
+      df_merge_lanes<16, 1>(m, h, l);
+      if (lane == 0) mg().res[i - b] = make_float4(m, h, l, 0.f);
+    }
+  }
+
   // Row phase. FRESH: the row sums with the current b only (a gap check), kept
   // for the a-update of the next iteration.
   template <bool FRESH>
   __device__ static bool row_phase() {
-    const int lane = threadIdx.x & 31;
-    const float k2 = sh().c.kappa2, k2l = sh().c.kappa2_lo;
-    const float4* w4 = reinterpret_cast<const float4*>(A().V.wcol);
-    const float4* wl4 = reinterpret_cast<const float4*>(A().V.wcol_lo);
     bool over = false;
     for (int b = r0(); b < r1(); b += kPersistBlk) {
       const int e = min(r1(), b + kPersistBlk);
-      if (threadIdx.x == 0) sh().ticket = b;
+      stage(A().V.wcol, A().V.wcol_lo, (int)A().g.ldc);
       __syncthreads();
-      for (;;) {
-        int i = 0;
-        if (lane == 0) i = atomicAdd(&sh().ticket, 1);
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i >= e) break;
-        float m, s, cmp, h, l;
-        // plain loads of the weights: other CTAs wrote them before the last barrier
-        const float4* row = reinterpret_cast<const float4*>(A().C + (int64_t)i * A().g.ldc);
-        row_lse<true>([row](int k) { return ld_stream(row + k); }, [w4](int k) { return w4[k]; },
-                      [wl4](int k) { return wl4[k]; }, (int)(A().g.ldc >> 2), lane, orow()[i], k2, k2l, m, s, cmp);
-        two_sum(s, -cmp, h, l);
-        df_merge_lanes<16, 1>(m, h, l);
-        if (lane == 0) mg().res[i - b] = make_float4(m, h, l, 0.f);
-      }
+      if (A().wfloats)
+        row_sums<true>(b, e);
+      else
+        row_sums<false>(b, e);
       __syncthreads();
       for (int i = b + threadIdx.x; i < e; i += kPersistThreads) {
         const float4 r = mg().res[i - b];
@@ -600,28 +640,41 @@ struct Streamed : Owned {
     return over;
   }
 
-  // Column phase: partials of (float4 column, row block) at part[(c4 nrb + r) 4 + q].
-  __device__ static void col_phase() {
+  // Column phase: partials of (float4 column, row block) at part[(c4 nrb + r) 4 + q], a
+  // warp per unit (row block, 128 columns).
+  template <bool STAGED>
+  __device__ static __noinline__ void col_sums() {
     const int lane = threadIdx.x & 31;
-    const int nv = (int)(A().g.ldc >> 2), ncg = (nv + 31) >> 5;
-    const int units = ncg * A().g.nrb, nw = gridDim.x * kPersistWarps;
-    const float k2 = sh().c.kappa2, k2l = sh().c.kappa2_lo;
-    for (int u = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; u < units; u += nw) {
-      const int r = u / ncg, c4 = (u % ncg) * 32 + lane;
+    const int64_t ld4 = A().g.ldc >> 2;
+    const int nv = (int)ld4, ncg = (nv + 31) >> 5, rows_per = (int)A().g.rows_per, I = (int)A().g.I;
+    // the CTA's units: about the rows it has in the row phase, so that it reads them
+    // through the same die's L2 (any other order has each die keep its own copy)
+    const int64_t all = (int64_t)ncg * A().g.nrb;
+    const int units = (int)(all * (blockIdx.x + 1) / gridDim.x), first = (int)(all * blockIdx.x / gridDim.x) + (threadIdx.x >> 5);
+    const float* const w = STAGED ? wstage() : A().V.wrow;
+    const float* const wl = STAGED ? wstage() + A().wfloats : A().V.wrow_lo;
+    for (int u = first; u < units; u += kPersistWarps) {
+      const int r = u / ncg, c4 = (u - r * ncg) * 32 + lane;
       if (c4 >= nv) continue;
       float o[4], m[4], s[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A().g.J ? l2col()[c4 * 4 + q].x : 0.f;
-      const int64_t a = (int64_t)r * A().g.rows_per;
+      const int a = r * rows_per;
       const float4* col = reinterpret_cast<const float4*>(A().C) + c4;
-      const int64_t ld4 = A().g.ldc >> 2;
-      const float *wr = A().V.wrow, *wrl = A().V.wrow_lo;
-      col_lse<true>([=](int64_t i) { return ld_stream(col + i * ld4); }, [wr](int64_t i) { return wr[i]; },
-                    [wrl](int64_t i) { return wrl[i]; }, a, min(A().g.I, a + A().g.rows_per), o, k2, k2l, m, s);
+      col_lse<true>([=](int i) { return ld_stream(col + i * ld4); }, [w](int i) { return w[i]; },
+                    [wl](int i) { return wl[i]; }, a, min(I, a + rows_per), o, sh().c.kappa2, sh().c.kappa2_lo, m, s);
       float4* out = reinterpret_cast<float4*>(A().V.part + ((int64_t)c4 * A().g.nrb + r) * 4);
       out[0] = make_float4(m[0], s[0], m[1], s[1]);
       out[1] = make_float4(m[2], s[2], m[3], s[3]);
     }
+  }
+  __device__ static void col_phase() {
+    stage(A().V.wrow, A().V.wrow_lo, (int)A().g.I);
+    __syncthreads();
+    if (A().wfloats)
+      col_sums<true>();
+    else
+      col_sums<false>();
   }
 
   // Merge phase: eight lanes per column over its row blocks, then the b-update.

@@ -366,21 +366,26 @@ struct SolveResult {
   Coef final_coef{};
 };
 
-// Shared memory the resident kernels may use beside their static part; their
-// limit is raised to it once per device.
+// Shared memory the solvers on a cost may use beside their static part; their limit
+// is raised to it once per device.
 static int resident_room(int* room) {
   static std::atomic<int> known[64] = {};
   int dev = 0;
   WOTG_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && (*room = known[dev].load(std::memory_order_acquire)) > 0) return WOTG_OK;
   int limit = 0;
-  cudaFuncAttributes a{}, b{};
   WOTG_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  WOTG_CUDA(cudaFuncGetAttributes(&a, resident_kernel<true>));
-  WOTG_CUDA(cudaFuncGetAttributes(&b, resident_kernel<false>));
-  *room = limit - (int)std::max(a.sharedSizeBytes, b.sharedSizeBytes);
-  WOTG_CUDA(cudaFuncSetAttribute(resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, *room));
-  WOTG_CUDA(cudaFuncSetAttribute(resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, *room));
+  const void* const kernels[] = {reinterpret_cast<const void*>(resident_kernel<true>),
+                                 reinterpret_cast<const void*>(resident_kernel<false>),
+                                 reinterpret_cast<const void*>(persist_kernel<true>),
+                                 reinterpret_cast<const void*>(persist_kernel<false>)};
+  *room = limit;
+  for (const void* k : kernels) {
+    cudaFuncAttributes a{};
+    WOTG_CUDA(cudaFuncGetAttributes(&a, k));
+    *room = std::min(*room, limit - (int)a.sharedSizeBytes);
+  }
+  for (const void* k : kernels) WOTG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, *room));
   if (dev < 64) known[dev].store(*room, std::memory_order_release);
   return WOTG_OK;
 }
@@ -423,7 +428,7 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
   // one CTA per SM; fewer only where the device grants the process fewer SMs
   int grid = std::min(sm_count(), kRedBlocks);
   int rows_cap = 0, cols_cap = 0;
-  size_t smem = kMergeHeaderBytes;
+  size_t streamed_smem = kMergeHeaderBytes, smem = streamed_smem;
   const bool gap = mode == kModeGap;
   const void* streamed = gap ? reinterpret_cast<const void*>(persist_kernel<true>)
                              : reinterpret_cast<const void*>(persist_kernel<false>);
@@ -468,6 +473,12 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
       kernel = gap ? reinterpret_cast<const void*>(resident_kernel<true>)
                    : reinterpret_cast<const void*>(resident_kernel<false>);
     }
+    const int64_t longest = (std::max(S.g.ldc, S.g.I) + 3) & ~int64_t(3);
+    if (streamed_smem + 8 * longest <= room) {
+      A.wfloats = (int)longest;
+      streamed_smem += 8 * longest;
+    }
+    if (kernel == streamed) smem = streamed_smem;
   }
   for (;;) {
     WOTG_CUDA(cudaMemsetAsync(&A.ctl->bar, 0, 2 * sizeof(unsigned long long), S.st));
@@ -480,7 +491,7 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
       if (threads == kResidentThreads) {
         kernel = streamed;
         threads = kPersistThreads;
-        smem = kMergeHeaderBytes;
+        smem = streamed_smem;
       } else {
         grid /= 2;
         T.vctas = std::min(T.vctas, kTcHalves * grid);

@@ -55,22 +55,32 @@ __device__ __forceinline__ double absorb_key(double la, const Coef& c) {
   return exp(la);
 }
 
-// Exponent of one element: plain (w - k2 C, one rounding) or precise (relative
-// to the grid offset o with the weight's and kappa2's low parts, see
-// split_weight).
+// Exponents of two elements: plain (w - k2 C, one rounding) or precise (relative
+// to the grid offset o with the weight's and kappa2's low parts, see split_weight),
+// from -o, -k2 and -k2l. As packed FP32 pairs: the passes are bound by instruction
+// issue (24 instructions per element in scalar form, of which the exponential is one).
 template <bool PREC>
-__device__ __forceinline__ float expo(float cc, float w, float wl, float o, float k2, float k2l) {
-  if (PREC) return fmaf(-k2, cc, w - o) + fmaf(-k2l, cc, wl);
-  return fmaf(-k2, cc, w);
+__device__ __forceinline__ float2 expo2(float2 cc, float2 w, float2 wl, float2 no, float2 nk2, float2 nk2l) {
+  if (PREC) return __fadd2_rn(__ffma2_rn(nk2, cc, __fadd2_rn(w, no)), __ffma2_rn(nk2l, cc, wl));
+  return __ffma2_rn(nk2, cc, w);
 }
+__device__ __forceinline__ float2 pair_of(float x) { return make_float2(x, x); }
+// a - b of pairs (the product by -1 is exact; a negated pair costs two instructions)
+__device__ __forceinline__ float2 sub2_rn(float2 a, float2 b) { return __ffma2_rn(b, pair_of(-1.f), a); }
 
 // One step of an online base-2 LSE: the partial (m, s) (with PREC the sum
-// compensated, s - cmp) takes in the four exponents x.
+// compensated, s - cmp) takes in four columns of a row.
 template <bool PREC>
-__device__ __forceinline__ void lse_step(float x0, float x1, float x2, float x3, float& m, float& s, float& cmp) {
-  const float mn = fmaxf(m, fmaxf(fmaxf(x0, x1), fmaxf(x2, x3)));
+__device__ __forceinline__ void lse_step(const float4& cc, const float4& w, const float4& wl, float2 no, float2 nk2,
+                                         float2 nk2l, float& m, float& s, float& cmp) {
+  const float2 x01 = expo2<PREC>(make_float2(cc.x, cc.y), make_float2(w.x, w.y), make_float2(wl.x, wl.y), no, nk2, nk2l);
+  const float2 x23 = expo2<PREC>(make_float2(cc.z, cc.w), make_float2(w.z, w.w), make_float2(wl.z, wl.w), no, nk2, nk2l);
+  const float mn = fmaxf(m, fmaxf(fmaxf(x01.x, x01.y), fmaxf(x23.x, x23.y)));
   const float r = ex2(m - mn);
-  const float v = (ex2(x0 - mn) + ex2(x1 - mn)) + (ex2(x2 - mn) + ex2(x3 - mn));
+  const float2 z01 = sub2_rn(x01, pair_of(mn)), z23 = sub2_rn(x23, pair_of(mn));
+  // (e0 + e1) + (e2 + e3)
+  const float2 e = __fadd2_rn(make_float2(ex2(z01.x), ex2(z23.x)), make_float2(ex2(z01.y), ex2(z23.y)));
+  const float v = e.x + e.y;
   if (PREC) {
     s = __fmul_rn(s, r);
     cmp = __fmul_rn(cmp, r);
@@ -91,10 +101,7 @@ __device__ __forceinline__ void row_lse(const Cost& cost, const W& w, const Wl& 
   m = kNegBig;
   s = 0.f;
   cmp = 0.f;
-  auto step = [&](const float4& cc, const float4& ww, const float4& wlo) {
-    lse_step<PREC>(expo<PREC>(cc.x, ww.x, wlo.x, o, k2, k2l), expo<PREC>(cc.y, ww.y, wlo.y, o, k2, k2l),
-                   expo<PREC>(cc.z, ww.z, wlo.z, o, k2, k2l), expo<PREC>(cc.w, ww.w, wlo.w, o, k2, k2l), m, s, cmp);
-  };
+  const float2 no = pair_of(-o), nk2 = pair_of(-k2), nk2l = pair_of(-k2l);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   // the cost loads of the next 128-float4 chunk are issued before this
   // chunk's arithmetic (two chunks of loads in flight per lane)
@@ -116,27 +123,88 @@ __device__ __forceinline__ void row_lse(const Cost& cost, const W& w, const Wl& 
 #pragma unroll
     for (int t = 0; t < 4; ++t) wlo[t] = PREC ? wl(k + 32 * t) : zero;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) step(cc[t], ww[t], wlo[t]);
+    for (int t = 0; t < 4; ++t) lse_step<PREC>(cc[t], ww[t], wlo[t], no, nk2, nk2l, m, s, cmp);
   }
 #pragma unroll
   for (int t = 0; t < 4; ++t)
-    if (k + 32 * t < nv) step(cn[t], w(k + 32 * t), PREC ? wl(k + 32 * t) : zero);
+    if (k + 32 * t < nv) lse_step<PREC>(cn[t], w(k + 32 * t), PREC ? wl(k + 32 * t) : zero, no, nk2, nk2l, m, s, cmp);
 }
 
-// One thread's share of a column pass: the online base-2 LSE of 4 columns over
-// rows [r0, r1), in chunks of kColRowChunk rows. cost(i) loads the columns'
-// float4 of row i, w(i) and wl(i) the row's weight; o the columns' offsets (PREC).
+// One thread's share of a column pass: the online base-2 LSE (m, s) of 4 columns (as
+// two pairs), with PREC compensated by cmp, over rows.
 constexpr int kColRowChunk = 4;
+struct ColSums {
+  float2 m[2], s[2], cmp[2];
+};
+__device__ __forceinline__ void col_clear(ColSums& c) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    c.m[q] = pair_of(kNegBig);
+    c.s[q] = c.cmp[q] = pair_of(0.f);
+  }
+}
+// Takes v, the sum of the new exponentials against the new maximum mn, into pair q.
+template <bool PREC>
+__device__ __forceinline__ void col_take(ColSums& c, int q, float2 mn, float2 v) {
+  const float2 d = sub2_rn(c.m[q], mn);
+  const float2 r = make_float2(ex2(d.x), ex2(d.y));
+  if (PREC) {
+    // kahan_add of both columns
+    const float2 s = __fmul2_rn(c.s[q], r), cm = __fmul2_rn(c.cmp[q], r);
+    const float2 y = sub2_rn(v, cm), t = __fadd2_rn(s, y);
+    c.cmp[q] = sub2_rn(sub2_rn(t, s), y);
+    c.s[q] = t;
+  } else {
+    c.s[q] = __ffma2_rn(c.s[q], r, v);
+  }
+  c.m[q] = mn;
+}
+// NR rows of costs cc with their weights; no the columns' -offsets (PREC).
+template <bool PREC, int NR>
+__device__ __forceinline__ void col_rows(const float4 (&cc)[NR], const float (&ww)[NR], const float (&wlo)[NR],
+                                         const float2 (&no)[2], float2 nk2, float2 nk2l, ColSums& c) {
+  float2 x[2][NR];
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    x[0][t] = expo2<PREC>(make_float2(cc[t].x, cc[t].y), pair_of(ww[t]), pair_of(wlo[t]), no[0], nk2, nk2l);
+    x[1][t] = expo2<PREC>(make_float2(cc[t].z, cc[t].w), pair_of(ww[t]), pair_of(wlo[t]), no[1], nk2, nk2l);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    float2 mn = c.m[q];
+#pragma unroll
+    for (int t = 0; t < NR; ++t) mn = make_float2(fmaxf(mn.x, x[q][t].x), fmaxf(mn.y, x[q][t].y));
+    float2 v = pair_of(0.f);
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      const float2 z = sub2_rn(x[q][t], mn);
+      const float2 e = make_float2(ex2(z.x), ex2(z.y));
+      v = t == 0 ? e : __fadd2_rn(v, e);
+    }
+    col_take<PREC>(c, q, mn, v);
+  }
+}
 
+template <bool PREC>
+__device__ __forceinline__ void col_result(const ColSums& c, float (&m)[4], float (&s)[4]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    m[2 * q] = c.m[q].x;
+    m[2 * q + 1] = c.m[q].y;
+    s[2 * q] = PREC ? c.s[q].x - c.cmp[q].x : c.s[q].x;
+    s[2 * q + 1] = PREC ? c.s[q].y - c.cmp[q].y : c.s[q].y;
+  }
+}
+
+// The same over rows [r0, r1): cost(i) loads the columns' float4 of row i, w(i) and
+// wl(i) the row's weight; o the columns' offsets (PREC).
 template <bool PREC, class I, class Cost, class W, class Wl>
 __device__ __forceinline__ void col_lse(const Cost& cost, const W& w, const Wl& wl, I r0, I r1, const float (&o)[4],
                                         float k2, float k2l, float (&m)[4], float (&s)[4]) {
-  float cmp[4] = {0.f, 0.f, 0.f, 0.f};   // PREC: compensated sums s - cmp
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    m[q] = kNegBig;
-    s[q] = 0.f;
-  }
+  ColSums c;
+  col_clear(c);
+  const float2 no[2] = {make_float2(-o[0], -o[1]), make_float2(-o[2], -o[3])};
+  const float2 nk2 = pair_of(-k2), nk2l = pair_of(-k2l);
   I i = r0;
   // the next chunk's cost loads are issued before this chunk's arithmetic
   float4 cn[kColRowChunk];
@@ -157,58 +225,14 @@ __device__ __forceinline__ void col_lse(const Cost& cost, const W& w, const Wl& 
     for (int t = 0; t < kColRowChunk; ++t) ww[t] = w(i + t);
 #pragma unroll
     for (int t = 0; t < kColRowChunk; ++t) wlo[t] = PREC ? wl(i + t) : 0.f;
-    float x[4][kColRowChunk];
-#pragma unroll
-    for (int t = 0; t < kColRowChunk; ++t) {
-      x[0][t] = expo<PREC>(cc[t].x, ww[t], wlo[t], o[0], k2, k2l);
-      x[1][t] = expo<PREC>(cc[t].y, ww[t], wlo[t], o[1], k2, k2l);
-      x[2][t] = expo<PREC>(cc[t].z, ww[t], wlo[t], o[2], k2, k2l);
-      x[3][t] = expo<PREC>(cc[t].w, ww[t], wlo[t], o[3], k2, k2l);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float mx = x[q][0];
-#pragma unroll
-      for (int t = 1; t < kColRowChunk; ++t) mx = fmaxf(mx, x[q][t]);
-      const float mn = fmaxf(m[q], mx);
-      const float r = ex2(m[q] - mn);
-      float v = 0.f;
-#pragma unroll
-      for (int t = 0; t < kColRowChunk; ++t) v += ex2(x[q][t] - mn);
-      if (PREC) {
-        s[q] = __fmul_rn(s[q], r);
-        cmp[q] = __fmul_rn(cmp[q], r);
-        kahan_add(s[q], cmp[q], v);
-      } else {
-        s[q] = s[q] * r + v;
-      }
-      m[q] = mn;
-    }
+    col_rows<PREC, kColRowChunk>(cc, ww, wlo, no, nk2, nk2l, c);
   }
   for (; i < r1; ++i) {
-    const float4 cc = cost(i);
-    const float ww = w(i);
-    const float wlo = PREC ? wl(i) : 0.f;
-    const float xs[4] = {expo<PREC>(cc.x, ww, wlo, o[0], k2, k2l), expo<PREC>(cc.y, ww, wlo, o[1], k2, k2l),
-                         expo<PREC>(cc.z, ww, wlo, o[2], k2, k2l), expo<PREC>(cc.w, ww, wlo, o[3], k2, k2l)};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float mn = fmaxf(m[q], xs[q]);
-      const float r = ex2(m[q] - mn);
-      if (PREC) {
-        s[q] = __fmul_rn(s[q], r);
-        cmp[q] = __fmul_rn(cmp[q], r);
-        kahan_add(s[q], cmp[q], ex2(xs[q] - mn));
-      } else {
-        s[q] = s[q] * r + ex2(xs[q] - mn);
-      }
-      m[q] = mn;
-    }
+    const float4 cc[1] = {cost(i)};
+    const float ww[1] = {w(i)}, wlo[1] = {PREC ? wl(i) : 0.f};
+    col_rows<PREC, 1>(cc, ww, wlo, no, nk2, nk2l, c);
   }
-  if (PREC) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s[q] -= cmp[q];
-  }
+  col_result<PREC>(c, m, s);
 }
 
 // The gap terms of one point: x = exp(t) its marginal sum (t = log x), p its
