@@ -166,9 +166,12 @@ __global__ void __launch_bounds__(kPcaThreads) csr_tfill_kernel(const int64_t* _
 // Y (n x r) = X Q - 1 a^T - c b^T (a, b: r; c: n; any may be NULL). A group of
 // G warps per row of the CSR X (G = 1 for short rows, 8 for the thousands of
 // entries of a gene's row in the transpose): warp w of the group takes entries
-// w, w + G, ... four at a time (independent loads in flight), lane l owns
-// output columns l and l + 32; the group's partial rows are summed in warp
-// order through shared memory, so the result does not depend on timing.
+// w, w + G, ... eight at a time (independent loads in flight), a lane per output
+// column of the CTA's 32 (blockIdx.y); the group's partial rows are summed in warp
+// order through shared memory, so the result does not depend on timing. What bounds
+// it: the longest row, 64 cycles an entry on its warp's FP64 unit (128 when a warp
+// did both halves of 40 columns: 164 us for 1000 genes of 4500 cells).
+constexpr int64_t kLongRows = 256;   // entries per row on average from which a row takes a CTA
 template <int G>
 __global__ void __launch_bounds__(kPcaThreads) spmm_centred_kernel(const int64_t* __restrict__ rowptr,
                                                                    const int32_t* __restrict__ colidx,
@@ -179,86 +182,75 @@ __global__ void __launch_bounds__(kPcaThreads) spmm_centred_kernel(const int64_t
                                                                    const double* __restrict__ b,
                                                                    double* __restrict__ Y) {
   constexpr int kGroups = kPcaThreads / 32 / G;
-  __shared__ double red[kPcaThreads / 32][2][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ double red[kPcaThreads / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.y * 32 + lane;
   const int grp = warp / G, w = warp % G;
-  const bool h0 = lane < r, h1 = lane + 32 < r;
+  if ((rowptr[n] > kLongRows * n) != (G > 1)) return;   // the other launch's matrix
+  const bool mine = col < r;
+  const double* const Qc = Q + (mine ? col : 0);
   for (int64_t i0 = (int64_t)blockIdx.x * kGroups; i0 < n; i0 += (int64_t)gridDim.x * kGroups) {
     const int64_t i = i0 + grp;
-    double y0 = 0.0, y1 = 0.0;
+    double y = 0.0;
     if (i < n) {
       const int64_t e = rowptr[i + 1];
       int64_t k = rowptr[i] + w;
-      for (; k + 3 * G < e; k += 4 * G) {
-        int64_t j[4];
-        double v[4];
+      for (; k + 7 * G < e; k += 8 * G) {
+        double v[8], q[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          j[u] = colidx[k + u * G];
+        for (int u = 0; u < 8; ++u) {
           v[u] = vals[k + u * G];
+          q[u] = Qc[(int64_t)colidx[k + u * G] * r];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (h0) y0 = fma(v[u], Q[j[u] * r + lane], y0);
-          if (h1) y1 = fma(v[u], Q[j[u] * r + lane + 32], y1);
-        }
+        for (int u = 0; u < 8; ++u) y = fma(v[u], q[u], y);
       }
-      for (; k < e; k += G) {
-        const int64_t j = colidx[k];
-        const double v = vals[k];
-        if (h0) y0 = fma(v, Q[j * r + lane], y0);
-        if (h1) y1 = fma(v, Q[j * r + lane + 32], y1);
-      }
+      for (; k < e; k += G) y = fma(vals[k], Qc[(int64_t)colidx[k] * r], y);
     }
     if (G > 1) {
-      red[warp][0][lane] = y0;
-      red[warp][1][lane] = y1;
+      red[warp][lane] = y;
       __syncthreads();
-      if (w == 0) {
-        for (int q = 1; q < G; ++q) {
-          y0 += red[warp + q][0][lane];
-          y1 += red[warp + q][1][lane];
-        }
-      }
+      if (w == 0)
+        for (int q = 1; q < G; ++q) y += red[warp + q][lane];
       __syncthreads();
     }
-    if (i < n && w == 0) {
-      const double ci = c ? c[i] : 0.0;
-      if (h0) Y[i * r + lane] = y0 - (a ? a[lane] : 0.0) - ci * (b ? b[lane] : 0.0);
-      if (h1) Y[i * r + lane + 32] = y1 - (a ? a[lane + 32] : 0.0) - ci * (b ? b[lane + 32] : 0.0);
-    }
+    if (i < n && w == 0 && mine) Y[i * r + col] = y - (a ? a[col] : 0.0) - (c ? c[i] : 0.0) * (b ? b[col] : 0.0);
   }
 }
 
 // Partial Gram matrices of row blocks: part[blk] = sum over its rows of a_i^T a_i.
-__global__ void __launch_bounds__(kPcaThreads) gram_partial_kernel(const double* __restrict__ A, int64_t n, int r,
-                                                                   int64_t rpb, double* __restrict__ part) {
+// A CTA takes kGramThreads entries (k <= l) of the upper triangle over its row block,
+// a warp per FP64 unit; the lower triangle is the same sums. What bounds it: an FP64
+// FMA holds its unit 64 cycles, so a row block costs 64 cycles per row however many
+// blocks there are. All of an r = 40 matrix in one CTA of 8 warps took 138 us on
+// 18 CTAs; 820 entries in seven CTAs per row block take the SMs that idled.
+constexpr int kGramThreads = 128;
+__global__ void __launch_bounds__(kGramThreads) gram_partial_kernel(const double* __restrict__ A, int64_t n, int r,
+                                                                    int64_t rpb, double* __restrict__ part) {
   __shared__ double row[32][kPcaMaxR];
   const int64_t r0 = (int64_t)blockIdx.x * rpb, r1 = min(n, r0 + rpb);
-  const int rr = r * r;
-  double acc[16];   // entries e = threadIdx.x + 256 t of the r x r matrix (r <= 64)
-#pragma unroll
-  for (int t = 0; t < 16; ++t) acc[t] = 0.0;
+  // entry e of the triangle: row k of it holds r - k entries
+  int k = 0, l = blockIdx.y * kGramThreads + threadIdx.x;
+  while (k < r && l >= r - k) l -= r - k++;
+  l += k;
+  const bool mine = k < r;
+  if (!mine) k = l = 0;
+  double s = 0.0;
   for (int64_t i0 = r0; i0 < r1; i0 += 32) {
     const int rows = (int)((r1 - i0) < 32 ? (r1 - i0) : 32);
-    for (int e = threadIdx.x; e < rows * r; e += blockDim.x) row[e / r][e % r] = A[(i0 + e / r) * r + e % r];
+    for (int e = threadIdx.x; e < rows * r; e += kGramThreads) row[e / r][e % r] = A[i0 * r + e];
     __syncthreads();
+    if (rows == 32) {
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      const int e = threadIdx.x + kPcaThreads * t;
-      if (e < rr) {
-        const int k = e / r, l = e % r;
-        double s = acc[t];
-        for (int q = 0; q < rows; ++q) s = fma(row[q][k], row[q][l], s);
-        acc[t] = s;
-      }
+      for (int q = 0; q < 32; ++q) s = fma(row[q][k], row[q][l], s);
+    } else {
+      for (int q = 0; q < rows; ++q) s = fma(row[q][k], row[q][l], s);
     }
     __syncthreads();
   }
-#pragma unroll
-  for (int t = 0; t < 16; ++t) {
-    const int e = threadIdx.x + kPcaThreads * t;
-    if (e < rr) part[(int64_t)blockIdx.x * rr + e] = acc[t];
+  if (mine) {
+    double* out = part + (int64_t)blockIdx.x * r * r;
+    out[k * r + l] = s;
+    if (k != l) out[l * r + k] = s;
   }
 }
 
@@ -273,29 +265,34 @@ __global__ void gram_final_kernel(const double* __restrict__ part, int64_t nb, i
 // Partial vector-matrix products of K ranges: part[blk] = sum over its k of w_k Q_k
 // (Q row-major, r <= 64 columns; lane l owns columns l and l + 32, warps take
 // interleaved rows, summed in warp order).
+// A CTA takes 32 columns (blockIdx.y), its loads eight rows at a time: read one after
+// another, a trip to L2 per row of each warp, a vector of 1024 took 57 us.
 __global__ void __launch_bounds__(kPcaThreads) vecmat_partial_kernel(const double* __restrict__ w,
                                                                      const double* __restrict__ Q, int64_t K, int r,
                                                                      int64_t kpb, double* __restrict__ part) {
-  __shared__ double red[kPcaThreads / 32][2][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kPcaThreads / 32, kAhead = 8;
+  __shared__ double red[kWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.y * 32 + lane;
   const int64_t k0 = (int64_t)blockIdx.x * kpb, k1 = min(K, k0 + kpb);
-  const bool h0 = lane < r, h1 = lane + 32 < r;
-  double y0 = 0.0, y1 = 0.0;
-  for (int64_t k = k0 + warp; k < k1; k += kPcaThreads / 32) {
-    const double wk = w[k];
-    if (h0) y0 = fma(wk, Q[k * r + lane], y0);
-    if (h1) y1 = fma(wk, Q[k * r + lane + 32], y1);
+  const bool mine = col < r;
+  double y = 0.0;
+  for (int64_t k = k0 + warp; k < k1; k += kAhead * kWarps) {
+    double wk[kAhead], q[kAhead];
+#pragma unroll
+    for (int t = 0; t < kAhead; ++t) {
+      const int64_t kt = k + t * kWarps;
+      wk[t] = kt < k1 ? w[kt] : 0.0;
+      q[t] = kt < k1 && mine ? Q[kt * r + col] : 0.0;
+    }
+#pragma unroll
+    for (int t = 0; t < kAhead; ++t)
+      if (k + t * kWarps < k1) y = fma(wk[t], q[t], y);
   }
-  red[warp][0][lane] = y0;
-  red[warp][1][lane] = y1;
+  red[warp][lane] = y;
   __syncthreads();
   if (warp == 0) {
-    for (int q = 1; q < kPcaThreads / 32; ++q) {
-      y0 += red[q][0][lane];
-      y1 += red[q][1][lane];
-    }
-    if (h0) part[(int64_t)blockIdx.x * r + lane] = y0;
-    if (h1) part[(int64_t)blockIdx.x * r + lane + 32] = y1;
+    for (int q = 1; q < kWarps; ++q) y += red[q][lane];
+    if (mine) part[(int64_t)blockIdx.x * r + col] = y;
   }
 }
 
@@ -372,17 +369,15 @@ extern "C" int wotg_spmm_centred(const int64_t* rowptr, const int32_t* colidx, c
                                  double* Y, void* stream) {
   if (!rowptr || !colidx || !vals || !Q || !Y || n <= 0 || r < 1 || r > kPcaMaxR) return WOTG_BADARG;
   cudaStream_t st = (cudaStream_t)stream;
-  // rows longer than a few hundred entries (a gene's row of the transpose) get a whole CTA each
-  int64_t nnz = 0;
-  WOTG_CUDA(cudaMemcpyAsync(&nnz, rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  WOTG_CUDA(cudaStreamSynchronize(st));
-  if (nnz > 256 * n) {
-    const int grid = (int)std::min<int64_t>(n, (int64_t)sm_count() * 8);
-    spmm_centred_kernel<8><<<grid, kPcaThreads, 0, st>>>(rowptr, colidx, vals, n, Q, r, a, c, b, Y);
-  } else {
-    const int grid = (int)std::min<int64_t>((n + 7) / 8, (int64_t)sm_count() * 16);
-    spmm_centred_kernel<1><<<grid, kPcaThreads, 0, st>>>(rowptr, colidx, vals, n, Q, r, a, c, b, Y);
-  }
+  // rows longer than a few hundred entries (a gene's row of the transpose) get a whole
+  // CTA each; which of the two launches works is for the device to see (rowptr[n]): the
+  // host would wait for the stream
+  const unsigned halves = (r + 31) / 32;
+  spmm_centred_kernel<8><<<dim3((unsigned)std::min<int64_t>(n, (int64_t)sm_count() * 8), halves), kPcaThreads, 0, st>>>(
+      rowptr, colidx, vals, n, Q, r, a, c, b, Y);
+  WOTG_LAUNCHED();
+  spmm_centred_kernel<1><<<dim3((unsigned)std::min<int64_t>((n + 7) / 8, (int64_t)sm_count() * 16), halves), kPcaThreads, 0,
+                           st>>>(rowptr, colidx, vals, n, Q, r, a, c, b, Y);
   WOTG_LAUNCHED();
   return WOTG_OK;
 }
@@ -402,7 +397,8 @@ extern "C" int wotg_gram_f64(const double* A, int64_t n, int32_t r, double* G, v
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t rpb = gram_rpb(n), nb = (n + rpb - 1) / rpb;
   double* part = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  gram_partial_kernel<<<(unsigned)nb, kPcaThreads, 0, st>>>(A, n, r, rpb, part);
+  gram_partial_kernel<<<dim3((unsigned)nb, (r * (r + 1) / 2 + kGramThreads - 1) / kGramThreads), kGramThreads, 0, st>>>(
+      A, n, r, rpb, part);
   WOTG_LAUNCHED();
   gram_final_kernel<<<(r * r + 255) / 256, 256, 0, st>>>(part, nb, r * r, G);
   WOTG_LAUNCHED();
@@ -423,7 +419,7 @@ extern "C" int wotg_vecmat_f64(const double* w, const double* Q, int64_t K, int3
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t kpb = vecmat_kpb(K), nb = (K + kpb - 1) / kpb;
   double* part = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  vecmat_partial_kernel<<<(unsigned)nb, kPcaThreads, 0, st>>>(w, Q, K, r, kpb, part);
+  vecmat_partial_kernel<<<dim3((unsigned)nb, (r + 31) / 32), kPcaThreads, 0, st>>>(w, Q, K, r, kpb, part);
   WOTG_LAUNCHED();
   gram_final_kernel<<<1, 64, 0, st>>>(part, nb, r, out);   // fixed-order sum of the block partials
   WOTG_LAUNCHED();
