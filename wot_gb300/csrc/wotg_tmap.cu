@@ -7,6 +7,7 @@
 // Accumulation is FP64 like the reference (k populations at a time, k <= 16 per
 // pass); X is read once per pass with coalesced loads.
 #include <algorithm>
+#include <type_traits>
 
 #include "wotg_common.cuh"
 
@@ -14,11 +15,16 @@ namespace wotg {
 
 constexpr int kMaxK = 16;
 
-// out[r][i] = sum_j X[i][j] P[r][j]; one warp per row i of X.
+// Both kernels take exactly KC populations (P and out at the first of them). What
+// bounds them is FP64 FMAs, 64 cycles each on an SM's quarter: with KC = 16 and the
+// populations past k predicated off, eight of them cost as much as sixteen (5003 x
+// 7001: 1.5 ms pull, 1.1 ms push; the FMAs of eight take 0.5 ms).
+
+// out[r][i] = sum_j X[i][j] P[r][j]; one warp per row i of X, the loads of two steps
+// ahead of their FMAs.
 template <int KC>
 __global__ void __launch_bounds__(256) pull_kernel(const double* __restrict__ X, int64_t I, int64_t J,
-                                                   const double* __restrict__ P, int k0, int k,
-                                                   double* __restrict__ out) {
+                                                   const double* __restrict__ P, double* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -27,16 +33,29 @@ __global__ void __launch_bounds__(256) pull_kernel(const double* __restrict__ X,
 #pragma unroll
     for (int r = 0; r < KC; ++r) acc[r] = 0.0;
     const double* row = X + i * J;
-    for (int64_t j = lane; j < J; j += 32) {
+    int64_t j = lane;
+    for (; j + 32 < J; j += 64) {
+      const double x0 = row[j], x1 = row[j + 32];
+      double p0[KC], p1[KC];
+#pragma unroll
+      for (int r = 0; r < KC; ++r) {
+        p0[r] = __ldg(P + r * J + j);
+        p1[r] = __ldg(P + r * J + j + 32);
+      }
+#pragma unroll
+      for (int r = 0; r < KC; ++r) acc[r] = fma(x0, p0[r], acc[r]);
+#pragma unroll
+      for (int r = 0; r < KC; ++r) acc[r] = fma(x1, p1[r], acc[r]);
+    }
+    if (j < J) {
       const double x = row[j];
 #pragma unroll
-      for (int r = 0; r < KC; ++r)
-        if (k0 + r < k) acc[r] = fma(x, __ldg(P + (int64_t)(k0 + r) * J + j), acc[r]);
+      for (int r = 0; r < KC; ++r) acc[r] = fma(x, __ldg(P + r * J + j), acc[r]);
     }
 #pragma unroll
     for (int r = 0; r < KC; ++r) {
       const double t = warp_sum(acc[r]);
-      if (lane == 0 && k0 + r < k) out[(int64_t)(k0 + r) * I + i] = t;
+      if (lane == 0) out[r * I + i] = t;
     }
   }
 }
@@ -45,8 +64,8 @@ __global__ void __launch_bounds__(256) pull_kernel(const double* __restrict__ X,
 // splits the rows, FP64 atomics merge the row blocks.
 template <int KC>
 __global__ void __launch_bounds__(256) push_kernel(const double* __restrict__ X, int64_t I, int64_t J,
-                                                   const double* __restrict__ P, int k0, int k,
-                                                   int64_t rows_per, double* __restrict__ out) {
+                                                   const double* __restrict__ P, int64_t rows_per,
+                                                   double* __restrict__ out) {
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t r0 = (int64_t)blockIdx.y * rows_per;
   const int64_t r1 = min(I, r0 + rows_per);
@@ -54,15 +73,24 @@ __global__ void __launch_bounds__(256) push_kernel(const double* __restrict__ X,
   double acc[KC];
 #pragma unroll
   for (int r = 0; r < KC; ++r) acc[r] = 0.0;
-  for (int64_t i = r0; i < r1; ++i) {
-    const double x = X[i * J + j];
+  const double* x = X + r0 * J + j;
+#pragma unroll 2
+  for (int64_t i = r0; i < r1; ++i, x += J) {
+    const double xi = *x;
 #pragma unroll
-    for (int r = 0; r < KC; ++r)
-      if (k0 + r < k) acc[r] = fma(__ldg(P + (int64_t)(k0 + r) * I + i), x, acc[r]);
+    for (int r = 0; r < KC; ++r) acc[r] = fma(__ldg(P + r * I + i), xi, acc[r]);
   }
 #pragma unroll
-  for (int r = 0; r < KC; ++r)
-    if (k0 + r < k) atomicAdd(out + (int64_t)(k0 + r) * J + j, acc[r]);
+  for (int r = 0; r < KC; ++r) atomicAdd(out + r * J + j, acc[r]);
+}
+
+// Calls f with the number of populations as a compile-time constant.
+template <int KC = kMaxK, class F>
+static void with_count(int k, const F& f) {
+  if constexpr (KC > 1) {
+    if (k < KC) return with_count<KC - 1>(k, f);
+  }
+  f(std::integral_constant<int, KC>{});
 }
 
 // Divide each of the k rows (length n) by its sum; one CTA per row.
@@ -96,7 +124,9 @@ extern "C" int wotg_apply_coupling_f64(const double* X, int64_t I, int64_t J, co
   if (transpose) {
     const int grid = (int)std::min<int64_t>((I + 7) / 8, (int64_t)sms * 8);
     for (int k0 = 0; k0 < k; k0 += kMaxK) {
-      pull_kernel<kMaxK><<<grid, 256, 0, st>>>(X, I, J, P, k0, k, out);
+      with_count(std::min(k - k0, kMaxK), [&](auto kc) {
+        pull_kernel<kc><<<grid, 256, 0, st>>>(X, I, J, P + k0 * J, out + k0 * I);
+      });
       WOTG_LAUNCHED();
     }
     if (normalize) {
@@ -112,7 +142,9 @@ extern "C" int wotg_apply_coupling_f64(const double* X, int64_t I, int64_t J, co
     const int64_t rows_per = (I + nrb - 1) / nrb;
     nrb = (I + rows_per - 1) / rows_per;
     for (int k0 = 0; k0 < k; k0 += kMaxK) {
-      push_kernel<kMaxK><<<dim3((unsigned)ncb, (unsigned)nrb), 256, 0, st>>>(X, I, J, P, k0, k, rows_per, out);
+      with_count(std::min(k - k0, kMaxK), [&](auto kc) {
+        push_kernel<kc><<<dim3((unsigned)ncb, (unsigned)nrb), 256, 0, st>>>(X, I, J, P + k0 * I, rows_per, out + k0 * J);
+      });
       WOTG_LAUNCHED();
     }
     if (normalize) {
