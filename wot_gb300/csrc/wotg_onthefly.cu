@@ -165,11 +165,11 @@ int tc_lse_launch(const __half* Pt, int n_ptiles, const __half* Qt, int nq, int 
   if (kp == 32) {
     WOTG_CUDA(tc_set_smem_attr<32>());
     lse_tc_kernel<32, 0><<<ctas, kTcThreads, TcSmem<32>::kAlloc, st>>>(Pt, Qt, n_ptiles, nq, part, off, err,
-                                                                        wait_tries, nullptr, 0, 0, nullptr, NoFin{});
+                                                                        wait_tries, nullptr, 0, nullptr);
   } else if (kp == 64) {
     WOTG_CUDA(tc_set_smem_attr<64>());
     lse_tc_kernel<64, 0><<<ctas, kTcThreads, TcSmem<64>::kAlloc, st>>>(Pt, Qt, n_ptiles, nq, part, off, err,
-                                                                        wait_tries, nullptr, 0, 0, nullptr, NoFin{});
+                                                                        wait_tries, nullptr, 0, nullptr);
   } else {
     return WOTG_BADARG;
   }
@@ -200,14 +200,14 @@ __global__ void lse_points_finish_kernel(int64_t n, int nq, int ctas, int nparts
 }
 
 // Population weights of columns [0, J) of k populations (FP64, row stride ldp),
-// from population k0 on, as FP32 rows of jpad entries (zero past J).
+// from population k0 on, as FP32, npop_max per column (zero past J and k).
 __global__ void pop_pack_kernel(const double* __restrict__ P, int64_t ldp, int k0, int k, int64_t J, int64_t jpad,
                                 int npop_max, float* __restrict__ popw) {
   const int64_t total = (int64_t)npop_max * jpad;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
-    const int kk = (int)(idx / jpad);
-    const int64_t j = idx % jpad;
+    const int kk = (int)(idx % npop_max);
+    const int64_t j = idx / npop_max;
     popw[idx] = (kk < k && j < J) ? (float)P[(int64_t)(k0 + kk) * ldp + j] : 0.f;
   }
 }
@@ -450,12 +450,12 @@ extern "C" int wotg_apply_points(const float* X, int64_t I, int64_t ldx, const f
     WOTG_LAUNCHED();
     if (P.kp == 32) {
       WOTG_CUDA((tc_set_smem_attr<32, kTcPops>()));
-      lse_tc_kernel<32, kTcPops><<<P.ctas, kTcThreads, TcSmem<32>::kAlloc, st>>>(
-          P.Xa, P.Yb, P.n_xt, P.n_yt, P.part, nullptr, P.err, kTcWaitTries, popw, kc, (int)jpad, psum, NoFin{});
+      lse_tc_kernel<32, kTcPops><<<P.ctas, kTcThreads, TcSmem<32, kTcPops>::kAlloc, st>>>(
+          P.Xa, P.Yb, P.n_xt, P.n_yt, P.part, nullptr, P.err, kTcWaitTries, popw, kc, psum);
     } else {
       WOTG_CUDA((tc_set_smem_attr<64, kTcPops>()));
-      lse_tc_kernel<64, kTcPops><<<P.ctas, kTcThreads, TcSmem<64>::kAlloc, st>>>(
-          P.Xa, P.Yb, P.n_xt, P.n_yt, P.part, nullptr, P.err, kTcWaitTries, popw, kc, (int)jpad, psum, NoFin{});
+      lse_tc_kernel<64, kTcPops><<<P.ctas, kTcThreads, TcSmem<64, kTcPops>::kAlloc, st>>>(
+          P.Xa, P.Yb, P.n_xt, P.n_yt, P.part, nullptr, P.err, kTcWaitTries, popw, kc, psum);
     }
     WOTG_LAUNCHED();
     pop_finish_kernel<<<(unsigned)((I + 255) / 256), 256, 0, st>>>(I, P.n_yt, P.ctas, kTcParts, P.part, psum,

@@ -1,8 +1,7 @@
 // wotg_tc_kernel.cuh — the tensor-core half-step kernel (tcgen05 cost tiles,
-// log-sum-exp epilogue from TMEM), shared by the standalone entry points and
-// the solvers. Its `Fin` policy lets a solver finish each row tile inside the
-// kernel (merge of the partials and the FP64 update, see lse_tc_kernel);
-// NoFin leaves the partials to a separate pass.
+// log-sum-exp epilogue from TMEM) of the standalone entry points, whose parts the
+// on-the-fly solver shares (wotg_tc_persist.cuh). The partials are merged by a
+// separate pass.
 #pragma once
 
 #include <stdint.h>
@@ -14,13 +13,6 @@
 namespace wotg {
 
 constexpr uint32_t kTcWaitTries = kTcDefaultWaitTries;  // x up to 1 us per try: about 4 s
-
-// The partials stay in `part` for a separate merge.
-struct NoFin {
-  static constexpr bool kActive = false;
-  __device__ __forceinline__ void start() const {}
-  __device__ __forceinline__ void quarter_done(const float2* part, int t, int wq, int lane) const {}
-};
 
 // ---------------------------------------------------------------------------
 // On-the-fly half-step: base-2 log-sum-exp partials
@@ -37,12 +29,6 @@ struct NoFin {
 // 32-column quarters, one partial at part[((cta + tile) * 128 + row) * 4 + quarter].
 // Along the walk (cta, tile) only ever steps up, so cta + tile indexes every
 // (CTA, row tile) segment uniquely.
-//
-// Fin (a solver's policy): once a warp has written its partial of a segment,
-// fin.quarter_done() counts it for its row tile and lane quarter; the warp
-// that brings the count to 2 x (CTAs covering the tile) merges those 32 rows'
-// partials and applies the solver's update (no barrier, no wait: per-warp
-// counters in global memory, reset by that warp for the next launch).
 //
 // Warp roles (10 warps, two CTAs per SM):
 //   warp 0      producer: bulk asynchronous copies of A tiles (one per segment,
@@ -71,18 +57,21 @@ constexpr int kTcColsPerWarp = 128 / kTcParts;
 constexpr int kTcCtasPerSm = 2;
 constexpr int kTcThreads = 32 * (2 + kTcEpiWarps);
 
-template <int KP>
+template <int KP, int NPOP = 0>
 struct TcSmem {
   static constexpr uint32_t kHalfBytes = 128u * KP * 2u;      // one of hi / lo
   static constexpr uint32_t kTileBytes = 2u * kHalfBytes;      // packed 128-point tile (hi + lo)
   // Two CTAs per SM in 96 KB each: 32 columns double-buffer the row tile (A) and
   // keep a 4-deep ring of column tiles (B); 64 columns single-buffer A (it
   // changes only at the few row-tile boundaries of a CTA's stretch) and keep 2 B stages.
-  static constexpr int kStages = KP == 32 ? kTcStages : 2;     // B ring depth
+  // The population form adds the weights of each column tile (and one stage less).
+  static constexpr int kStages = KP == 32 ? (NPOP ? kTcStages - 1 : kTcStages) : 2;   // B ring depth
   static constexpr int kABuf = KP == 32 ? 2 : 1;               // A buffers
   static constexpr uint32_t kA = 0;                            // kABuf buffers
   static constexpr uint32_t kB = kABuf * kTileBytes;           // kStages buffers
-  static constexpr uint32_t kBar = kB + kStages * kTileBytes;
+  static constexpr uint32_t kPopBytes = NPOP * 128u * 4u;
+  static constexpr uint32_t kW = kB + kStages * kTileBytes;    // kStages weight tiles
+  static constexpr uint32_t kBar = kW + kStages * kPopBytes;
   // barriers: full[S], empty[S], a_full[kABuf], a_empty[kABuf], acc_full[kTcAcc], acc_empty[kTcAcc],
   // drain; then the TMEM slot and the abort flag
   static constexpr uint32_t kBytes = kBar + 8 * (2 * kStages + 2 * kABuf + 2 * kTcAcc + 1) + 16;
@@ -156,28 +145,41 @@ __device__ __forceinline__ void sum32_off(const float (&d)[32], float o, float2 
 
 // Weighted sums of 32 exponents for up to NPOP populations at once (the
 // population form of the epilogue): one exp2 per element against the running
-// maximum m, then s[k] += 2^(d - m) w[k][col] for every population k, the
-// weights w (npop rows of ldw floats, 16-byte aligned) read as warp-uniform
-// 128-bit loads. The sums are rescaled when the maximum moves.
+// maximum m, then s[k] += 2^(d - m) w[col][k] for every population k, two at a time as
+// packed FP32 pairs; the weights (NPOP floats per column, in shared memory beside the
+// column tile) are read as warp-uniform 128-bit loads. The sums are rescaled when
+// the maximum moves. (Weights read from global memory, one row per population, waited
+// for L2 at every tile: 0.93 ms for eight populations at 22001 x 30011, d = 50, of
+// which the products are 0.14.)
 template <int NPOP>
-__device__ __forceinline__ void multi32(const float (&d)[32], const float* __restrict__ w, int npop, int ldw,
-                                        int col0, float& m, float (&s)[NPOP]) {
-  float mx = d[0];
+__device__ __forceinline__ void multi32(const float (&d)[32], const float* w, float& m,
+                                        float2 (&s)[NPOP / 2]) {
+  static_assert(NPOP % 4 == 0, "weights by float4");
+  float mx[8];
 #pragma unroll
-  for (int c = 1; c < 32; ++c) mx = fmaxf(mx, d[c]);
-  const float mn = fmaxf(m, mx);
+  for (int c = 0; c < 8; ++c) mx[c] = fmaxf(fmaxf(d[4 * c], d[4 * c + 1]), fmaxf(d[4 * c + 2], d[4 * c + 3]));
+#pragma unroll
+  for (int h = 4; h >= 1; h >>= 1)
+#pragma unroll
+    for (int c = 0; c < h; ++c) mx[c] = fmaxf(mx[c], mx[c + h]);
+  const float mn = fmaxf(m, mx[0]);
   const float r = ex2(m - mn);
 #pragma unroll
-  for (int k = 0; k < NPOP; ++k) s[k] *= r;
+  for (int k = 0; k < NPOP / 2; ++k) s[k] = __fmul2_rn(s[k], make_float2(r, r));
   m = mn;
 #pragma unroll
   for (int c = 0; c < 32; c += 4) {
-    const float e0 = ex2(d[c] - mn), e1 = ex2(d[c + 1] - mn), e2 = ex2(d[c + 2] - mn), e3 = ex2(d[c + 3] - mn);
+    float e[4];
 #pragma unroll
-    for (int k = 0; k < NPOP; ++k) {
-      if (k < npop) {
-        const float4 pw = __ldg(reinterpret_cast<const float4*>(w + (int64_t)k * ldw + col0 + c));
-        s[k] = fmaf(e0, pw.x, fmaf(e1, pw.y, fmaf(e2, pw.z, fmaf(e3, pw.w, s[k]))));
+    for (int t = 0; t < 4; ++t) e[t] = ex2(d[c + t] - mn);
+#pragma unroll
+    for (int t = 3; t >= 0; --t) {
+      const float2 et = make_float2(e[t], e[t]);
+#pragma unroll
+      for (int k = 0; k < NPOP; k += 4) {
+        const float4 pw = *reinterpret_cast<const float4*>(w + (c + t) * NPOP + k);
+        s[k / 2] = __ffma2_rn(et, make_float2(pw.x, pw.y), s[k / 2]);
+        s[k / 2 + 1] = __ffma2_rn(et, make_float2(pw.z, pw.w), s[k / 2 + 1]);
       }
     }
   }
@@ -186,15 +188,15 @@ __device__ __forceinline__ void multi32(const float (&d)[32], const float* __res
 // NPOP = 0: the log-sum-exp half-step (partials (m, s) in part). NPOP > 0: the
 // population form, npop <= NPOP weighted sums per row (maxima in part[].x,
 // sums in psum[slot * NPOP + k]) with the population weights popw.
-template <int KP, int NPOP, class Fin = NoFin>
+template <int KP, int NPOP>
 __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const __half* __restrict__ Pt,
                                                                const __half* __restrict__ Qt,
                                                                int n_pt, int nq, float2* __restrict__ part,
                                                                const float* off,
                                                                int* __restrict__ err, uint32_t wait_tries,
                                                                const float* __restrict__ popw, int npop,
-                                                               int ldpw, float* __restrict__ psum, Fin fin) {
-  using L = TcSmem<KP>;
+                                                               float* __restrict__ psum) {
+  using L = TcSmem<KP, NPOP>;
   constexpr int S = L::kStages;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
   if (tid == 0) {
     for (int b = 0; b < S; ++b) {
       tc::mbar_init(&full[b], 1);
-      tc::mbar_init(&empty[b], 1);
+      tc::mbar_init(&empty[b], NPOP > 0 ? 1 + kTcEpiWarps : 1);   // its weights are the epilogue's
     }
     for (int b = 0; b < NA; ++b) {
       tc::mbar_init(&a_full[b], 1);
@@ -242,11 +244,6 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  // launched as a dependent of the previous half-step's combine: everything
-  // above is this CTA's own set-up; global memory only from here on
-  pdl_wait();
-  pdl_trigger();
-  if (Fin::kActive && blockIdx.x == 0 && tid == 0) fin.start();
   const uint32_t tmem = *tmem_slot;
   const uint32_t sA = tc::smem_u32(smem + L::kA);
   const uint32_t sB = tc::smem_u32(smem + L::kB);
@@ -276,9 +273,12 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
                        &a_full[seg % NA]);
           seg_last = seg;
         }
-        tc::mbar_expect_tx(&full[stage], L::kTileBytes);
+        tc::mbar_expect_tx(&full[stage], L::kTileBytes + L::kPopBytes);
         tc::bulk_g2s(sB + (uint32_t)stage * L::kTileBytes, Qt + (int64_t)q * tile_halfs, L::kTileBytes,
                      &full[stage]);
+        if (NPOP > 0)
+          tc::bulk_g2s(tc::smem_u32(smem + L::kW) + (uint32_t)stage * L::kPopBytes, popw + (int64_t)q * 128 * NPOP,
+                       L::kPopBytes, &full[stage]);
         j_last = j;
         if (++q == nq) {
           q = 0;
@@ -373,9 +373,9 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
     const int row = 32 * wq + lane;
     float m = kNegBig, s = 0.f;
     float2 acc[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-    float sp[NPOP > 0 ? NPOP : 1];
+    float2 sp[NPOP > 0 ? NPOP / 2 : 1];
 #pragma unroll
-    for (int k = 0; k < (NPOP > 0 ? NPOP : 1); ++k) sp[k] = 0.f;
+    for (int k = 0; k < (NPOP > 0 ? NPOP / 2 : 1); ++k) sp[k] = make_float2(0.f, 0.f);
     int t = t_first, q = q_first;
     // speculative form: the row's offset for the current row tile
     if (off) m = off[(int64_t)t * 128 + row];
@@ -393,31 +393,40 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
       tc::fence_after_sync();
       static_assert(kTcColsPerWarp == 64, "two 32-column TMEM blocks per warp and tile");
       const uint32_t taddr = tmem + ((uint32_t)(32 * wq) << 16) + (uint32_t)(128 * b + kTcColsPerWarp * cq);
-      float d0[32], d1[32];
-      const int col0 = q * 128 + kTcColsPerWarp * cq;   // first column of d0 within the column set
+      float d0[32];
       if constexpr (NPOP > 0) {
-        // first block, then the second block's load runs under the first
-        // block's sums (fewer live registers beside the population sums)
-        tc::tmem_ld32(taddr, d0);
-        tc::tmem_wait_ld();
-        tc::tmem_hold(d0);
-        tc::tmem_ld32(taddr + 32, d1);
-        multi32<NPOP>(d0, popw, npop, ldpw, col0, m, sp);
-        tc::tmem_wait_ld();
-        tc::tmem_hold(d1);
+        const int stage = j % S;
+        // complete already (the products waited for it): this warp's own view of the weights
+        const bool have = __all_sync(0xffffffffu, tc::mbar_wait(&full[stage], (uint32_t)((j / S) & 1), wait_tries));
+        if (!have) {
+          if (lane == 0) {
+            *abort_flag = 1;
+            atomicExch(err, 1);
+          }
+          break;
+        }
+        const float* w = reinterpret_cast<const float*>(smem + L::kW + (uint32_t)stage * L::kPopBytes) +
+                         kTcColsPerWarp * cq * NPOP;
+        // one 32-column block after the other: both at once leave no registers for the sums
+        tc::tmem_read32(taddr, d0);
+        multi32<NPOP>(d0, w, m, sp);
+        tc::tmem_read32(taddr + 32, d0);
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&acc_empty[b]);
-        multi32<NPOP>(d1, popw, npop, ldpw, col0 + 32, m, sp);
+        multi32<NPOP>(d0, w + 32 * NPOP, m, sp);
+        // the weights' loads have returned before the next copy may overwrite them: without
+        // the fence the last sums, and with them the wait for their loads, moved below
+        // the arrival
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty[stage]);
       } else {
         // both 32-column blocks loaded at once and the accumulator handed back
         // to the MMA issuer before any sums (measured 3 % faster than
         // overlapping the second load with the first block's sums)
-        tc::tmem_ld32(taddr, d0);
-        tc::tmem_ld32(taddr + 32, d1);
-        tc::tmem_wait_ld();
-        tc::tmem_hold(d0);
-        tc::tmem_hold(d1);
+        float d1[32];
+        tc::tmem_read64(taddr, d0, d1);
         tc::fence_before_sync();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&acc_empty[b]);
@@ -440,14 +449,11 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
         part[slot] = make_float2(m, s);
         if constexpr (NPOP > 0) {
 #pragma unroll
-          for (int k = 0; k < NPOP; ++k) {
-            psum[slot * NPOP + k] = sp[k];
-            sp[k] = 0.f;
+          for (int k = 0; k < NPOP / 2; ++k) {
+            reinterpret_cast<float2*>(psum + slot * NPOP)[k] = sp[k];
+            sp[k] = make_float2(0.f, 0.f);
           }
         }
-        // the warp that writes the last partial of rows [t 128 + 32 wq, + 32)
-        // (over the CTAs and column halves covering the row tile) finishes them
-        if constexpr (Fin::kActive) fin.quarter_done(part, t, wq, lane);
         m = kNegBig;
         s = 0.f;
         if (q == nq) {
@@ -464,10 +470,10 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const 
 }
 
 
-template <int KP, int NPOP = 0, class Fin = NoFin>
+template <int KP, int NPOP = 0>
 static cudaError_t tc_set_smem_attr() {
-  static cudaError_t once = cudaFuncSetAttribute(lse_tc_kernel<KP, NPOP, Fin>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcSmem<KP>::kAlloc);
+  static cudaError_t once = cudaFuncSetAttribute(lse_tc_kernel<KP, NPOP>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcSmem<KP, NPOP>::kAlloc);
   return once;
 }
 

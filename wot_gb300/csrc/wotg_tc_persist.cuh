@@ -398,11 +398,7 @@ struct TcPersist : Owned {
       tc::fence_after_sync();
       const uint32_t taddr = tbase + (uint32_t)(128 * b);
       float d0[32], d1[32];
-      tc::tmem_ld32(taddr, d0);
-      tc::tmem_ld32(taddr + 32, d1);
-      tc::tmem_wait_ld();
-      tc::tmem_hold(d0);
-      tc::tmem_hold(d1);
+      tc::tmem_read64(taddr, d0, d1);
       tc::fence_before_sync();
       __syncwarp();
       if ((threadIdx.x & 31) == 0) tc::mbar_arrive(accempty + b);
