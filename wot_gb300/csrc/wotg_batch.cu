@@ -1243,18 +1243,18 @@ __device__ __noinline__ void loop_rows(const LoopGroup g, LoopShared& sh, int cs
   __syncwarp();
   for (int st = 0; st < steps; ++st) {
     const int ch0 = st * (cs / kChunk), ch1 = min(nch, ch0 + cs / kChunk);
-    if (steps > 1) {
-      __syncthreads();
-      loop_stage(const_cast<float*>(W), sh, g.which, g.g0, g.ng, ch0 * kChunk, cs, sg.cols);
-      loop_staged();
-    }
-    if (!valid[0]) continue;
     float4 nx[kLoopAhead][kLoopRW];
 #pragma unroll
     for (int t = 0; t < kLoopAhead; ++t)
 #pragma unroll
       for (int r = 0; r < kLoopRW; ++r)
         nx[t][r] = load_cost(crow[r], (ch0 + t) * 32, nv - lane, valid[r] && ch0 + t < ch1);
+    if (steps > 1) {
+      __syncthreads();
+      loop_stage(const_cast<float*>(W), sh, g.which, g.g0, g.ng, ch0 * kChunk, cs, sg.cols);
+    }
+    if (st == 0 || steps > 1) loop_staged();   // the first costs are on their way meanwhile
+    if (!valid[0]) continue;
     for (int ch = ch0; ch < ch1; ch += kLoopAhead) {
 #pragma unroll
       for (int t = 0; t < kLoopAhead; ++t) {
@@ -1322,15 +1322,16 @@ __device__ __noinline__ void loop_rows_single(const LoopGroup g, LoopShared& sh)
     o[r] = __shfl_sync(0xffffffffu, o[r], 0);
     s0[r] = s1[r] = 0.f;
   }
+  float4 nx[kLoopRW][4];
+  int q = lane;
+  if (q + 96 < nq) {
+#pragma unroll
+    for (int r = 0; r < kLoopRW; ++r)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) nx[r][t] = ld_stream(crow[r] + q + 32 * t);
+  }
+  loop_staged();   // the first costs are on their way meanwhile
   if (loop_row_of(g, 0) < sh.rows[g.dir]) {
-    float4 nx[kLoopRW][4];
-    int q = lane;
-    if (q + 96 < nq) {
-#pragma unroll
-      for (int r = 0; r < kLoopRW; ++r)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) nx[r][t] = ld_stream(crow[r] + q + 32 * t);
-    }
     for (; q + 96 < nq; q += 128) {
       const bool more = q + 128 + 96 < nq;
 #pragma unroll
@@ -1424,7 +1425,6 @@ __device__ __noinline__ void loop_pass(const BatchArgs& B, int dir, int mode, bo
         loop_stage(reinterpret_cast<float*>(loop_smem + kLoopHeader), sh, g.which, g.g0, g.ng, 0, cs, sh.seg[dir].cols);
       else
         cp_async_commit();
-      loop_staged();
       if (!single)
         loop_rows(g, sh, cs, steps);
       else if (steps == 1)
@@ -1541,21 +1541,40 @@ __global__ void __launch_bounds__(kLoopThreads, 1) loop_kernel(const __grid_cons
   }
 }
 
-// Rows of a direction dealt out evenly to at most `ctas` tiles of whole rows of one
-// pair, at least 8 rows each (the tiles' memory). A pass is mostly latency, the same for
-// 10 rows as for 40 (a round), so a row counts as its columns and another 2000. Empty
-// when there are too many pairs, or rows for a tile's word.
+// Rows of a direction dealt out to at most `ctas` tiles of whole rows of one pair, at
+// least 8 rows each (the tiles' memory). A pass is mostly latency, the same for 10 rows as
+// for a round (kLoopRows), so every pair gets the tiles for one round each if there are
+// as many, and the rest go where a row, counted as its columns and another 2000, is
+// worst off. Empty when there are too many pairs, or rows for a tile's word.
 static std::vector<LoopTile> loop_tiles(const std::vector<int>& rows, const std::vector<int>& cols, int ctas) {
-  double total = 0.0;
-  for (size_t p = 0; p < rows.size(); ++p) total += (double)rows[p] * (cols[p] + 2000.0);
-  const int spare = ctas - (int)rows.size();   // every pair has one tile at least
   std::vector<LoopTile> out;
-  if (spare < 0 || *std::max_element(rows.begin(), rows.end()) >= 1 << 17) return out;
-  for (size_t p = 0; p < rows.size(); ++p) {
-    const int n = std::min((rows[p] + 7) / 8, 1 + (int)(spare * ((double)rows[p] * (cols[p] + 2000.0) / total)));
-    for (int k = 0; k < n; ++k) {
-      const int r0 = (int)((int64_t)rows[p] * k / n), r1 = (int)((int64_t)rows[p] * (k + 1) / n);
-      out.push_back(LoopTile{(int)p | (r1 - r0) * kLoopMaxPairs, r0});
+  const int np = (int)rows.size();
+  if (np > ctas || *std::max_element(rows.begin(), rows.end()) >= 1 << 17) return out;
+  std::vector<int> n(np);
+  int used = 0;
+  for (int p = 0; p < np; ++p) used += n[p] = (rows[p] + kLoopRows - 1) / kLoopRows;
+  if (used > ctas) {
+    n.assign(np, 1);
+    used = np;
+  }
+  for (; used < ctas; ++used) {
+    int worst = -1;
+    double most = 0.0;
+    for (int p = 0; p < np; ++p) {
+      const double load = (double)rows[p] * (cols[p] + 2000.0) / n[p];
+      if (n[p] < (rows[p] + 7) / 8 && load > most) {
+        most = load;
+        worst = p;
+      }
+    }
+    if (worst < 0) break;
+    ++n[worst];
+  }
+  for (int p = 0; p < np; ++p) {
+    n[p] = std::min(n[p], (rows[p] + 7) / 8);
+    for (int k = 0; k < n[p]; ++k) {
+      const int r0 = (int)((int64_t)rows[p] * k / n[p]), r1 = (int)((int64_t)rows[p] * (k + 1) / n[p]);
+      out.push_back(LoopTile{p | (r1 - r0) * kLoopMaxPairs, r0});
     }
   }
   return out;
