@@ -138,11 +138,9 @@ int wotg_median(const float* C, int64_t I, int64_t J, int64_t ldc, double* media
  *                   v + eps log b) of the last solve, so that
  *                   tmap = exp((u_bar_i + v_bar_j - cost_scale C_ij) / eps) / J
  *                   with eps = stats->final_epsilon.
- * stats (host) may be NULL. The final epsilon stage's batches of iterations
- * between duality-gap checks run as CUDA graphs, captured once per stage on a
- * stream of the call's own (ordered with `stream` by events; the stream, two
- * events and at most two graphs live for the call); the no-alloc entry point
- * launches plainly on `stream`. Results are the same either way. */
+ * stats (host) may be NULL. A solve is one cooperative kernel on `stream`,
+ * launched again every 20 ms or so until its stopping test holds; the call waits
+ * for it. Results are the same with the no-alloc entry point. */
 size_t wotg_solve_workspace_bytes(int64_t I, int64_t J, int64_t ldc);   /* materialised form */
 size_t wotg_problem_workspace_bytes(const wotg_problem* problem);       /* any form */
 int wotg_compute_transport_matrix(const wotg_problem* problem, const wotg_params* params,
@@ -321,7 +319,8 @@ int wotg_gemm_f64(const double* A, int64_t lda, const double* B, int64_t ldb, co
  * over all pairs that reads a pair's cost once for all of its active items,
  * the reference's control flow (epsilon stages, batches, absorption, stage and
  * duality-gap tests, growth iterations) runs per item on the device, and the
- * iterations are replayed from a captured CUDA graph. Results per item are the
+ * iterations are replayed from a captured CUDA graph, or, for a small batch, run
+ * in one cooperative kernel. Results per item are the
  * reference's (duality-gap solver only), returned as potentials:
  *   tmap_ij = exp((u_bar_i + v_bar_j - cost_scale C_ij) / eps) * scale
  * with eps = stats.final_epsilon and scale = 1/J (or 1 when max_iter was hit).
@@ -422,9 +421,10 @@ int wotg_ot_adjoint(const float* X, int64_t I, int64_t ldx, const float* Y, int6
 
 /* Diagnostic (no counterpart in the reference): the replay profile of the last
  * wotg_solve_batched call on this host thread, one record per graph replay
- * (8 iterations of the whole batch): the number of items still active after
- * the previous replay and the host milliseconds between the waits on
- * successive replays (one replay's device time once the GPU is the bound).
+ * (8 iterations of the whole batch; a small batch: per launch of its loop, up to
+ * 200 iterations): the number of items still active after the previous replay (the
+ * launch) and the host milliseconds between the waits on successive replays (one
+ * replay's device time once the GPU is the bound).
  * Writes min(cap, n) records (either array may be NULL), returns n. */
 int32_t wotg_batch_replay_profile(int32_t* active, float* ms, int32_t cap);
 

@@ -27,7 +27,8 @@
 //    CTA of each of those kernels rebuilds the per-pair lists of items the next
 //    pass will see.
 //  * Six launches per iteration of the whole batch, captured B iterations at a
-//    time in a CUDA graph and replayed until no item is active.
+//    time in a CUDA graph and replayed until no item is active. Small batches run
+//    in one cooperative kernel instead (loop_kernel below).
 //
 // Item state and iteration counts follow the single-problem driver
 // (wotg_sinkhorn.cu) step for step, so every item gives the reference's
@@ -1536,8 +1537,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) loop_kernel(const __grid_cons
       const int st = __ldcg(&B.items[k].status);
       c += st == kActive || st == kMaxIterPending ? 1 : 0;
     }
-    c = __syncthreads_count(c != 0);
-    if (threadIdx.x == 0) B.active[0] = c;
+    if (threadIdx.x == 0) sh.n[2] = 0;
+    __syncthreads();
+    if (c) atomicAdd(&sh.n[2], c);
+    __syncthreads();
+    if (threadIdx.x == 0) B.active[0] = sh.n[2];
   }
 }
 

@@ -2,9 +2,9 @@
 //
 // Reference: wot/ot/optimal_transport.py (wot 1.0.8)
 //   compute_transport_matrix        :10-33   -> wotg_compute_transport_matrix (growth loop)
-//   optimal_transport_duality_gap   :67-164  -> solve_duality_gap
-//   transport_stablev2              :167-236 -> solve_fixed_iters
-//   primal / dual                   :45-62   -> gap_partial_kernel (O(I+J), see below)
+//   optimal_transport_duality_gap   :67-164  -> solve_persistent, kModeGap
+//   transport_stablev2              :167-236 -> solve_persistent, kModeFixed
+//   primal / dual                   :45-62   -> gap_test (O(I+J), see below)
 //
 // State. The reference keeps FP64 absorbed potentials u, v, scalings a, b and
 // the stabilised kernel K = exp((u_i - C_ij + v_j)/eps) as a dense matrix that
@@ -26,6 +26,11 @@
 //   primal = F1(x) + F2(y) + dx<ubar,x> + dy<vbar,y> + eps (sum(exp(-C/eps))/(IJ) - dx sum x).
 // The row sums with the current b are exactly the next iteration's first
 // half-step, so a gap check costs one row pass that the next iteration reuses.
+//
+// A solve is one cooperative kernel, launched anew every 20 ms of iterations:
+// wotg_resident.cuh (costs that fit in shared memory), wotg_persist.cuh (any cost, and
+// the control of all three) or wotg_tc_persist.cuh (costs formed on the fly). Here are
+// the entry points, the choice and the outputs.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -70,7 +75,6 @@ struct TcState {
   float* offY;
   int* redoX;
   int* redoY;
-  int* tile_ctr;                   // per (row tile, lane quarter): partials written
   unsigned long long* redo_total;  // rows recomputed exactly, over the solve (diagnostic)
 };
 
@@ -639,7 +643,7 @@ static void tc_layout(Bump& b, const wotg_problem* prob, TcState& tc) {
   tc.offY = b.take<float>(tc.J_pad);
   tc.redoX = b.take<int>(2 + prob->I);
   tc.redoY = b.take<int>(2 + prob->J);
-  tc.tile_ctr = b.take<int>((size_t)4 * std::max(tc.n_xt, tc.n_yt));
+  b.take<int>((size_t)4 * std::max(tc.n_xt, tc.n_yt));   // unused: the scratch need stays what callers sized for
   tc.redo_total = b.take<unsigned long long>(1);
 }
 

@@ -25,8 +25,8 @@ constexpr uint32_t kTcWaitTries = kTcDefaultWaitTries;  // x up to 1 us per try:
 // Persistent schedule: the n_pt x nq (row tile, column tile) pairs are walked
 // row-major and cut into gridDim.x contiguous, equal stretches, one per CTA. A
 // stretch covers one or more row tiles ("segments"); at the end of each
-// segment the CTA writes, for every row of that row tile and each of the four
-// 32-column quarters, one partial at part[((cta + tile) * 128 + row) * 4 + quarter].
+// segment the CTA writes, for every row of that row tile and each of the two
+// 64-column halves, one partial at part[((cta + tile) * 128 + row) * 2 + half].
 // Along the walk (cta, tile) only ever steps up, so cta + tile indexes every
 // (CTA, row tile) segment uniquely.
 //

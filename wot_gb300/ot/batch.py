@@ -5,7 +5,7 @@ wot/ot/ot_model.py:124-201) and a parameter sweep repeats that per parameter set
 ``solve_batched`` hands every item to ``wotg_solve_batched``: one persistent
 launch per Sinkhorn half-step over all items, each pair's cost read once for all
 of its items, the reference's control flow per item on the device, replayed from
-a CUDA graph. Each result is the reference's map for that item, held as
+a CUDA graph or, for a small batch, looped in one kernel. Each result is the reference's map for that item, held as
 potentials (an ``ImplicitMap``) instead of a dense I x J matrix.
 """
 from __future__ import annotations
