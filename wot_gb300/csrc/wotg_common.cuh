@@ -150,12 +150,6 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
-__device__ __forceinline__ double warp_maxd(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
-  return x;
-}
-
 // Max of non-negative doubles through their bit patterns (monotone for x >= 0).
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* slot, double x) {
   if (x > 0.0) atomicMax(slot, (unsigned long long)__double_as_longlong(x));

@@ -78,8 +78,7 @@ __global__ void __launch_bounds__(128) tc_selftest_kernel(const float* __restric
   if (ok) {
     for (int c = 0; c < kSelfN; c += 32) {
       float v[32];
-      tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-      tc::tmem_wait_ld();
+      tc::tmem_read32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
 #pragma unroll
       for (int t = 0; t < 32; ++t) D[(warp * 32 + lane) * kSelfN + c + t] = v[t];
     }

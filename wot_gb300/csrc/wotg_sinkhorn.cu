@@ -130,11 +130,6 @@ __global__ void col_combine_kernel(Geom g, const float2* __restrict__ part, doub
 // Zero state for a new solve; p = G; padding of wcol = 0.
 __global__ void init_kernel(Geom g, Vecs V, const double* __restrict__ G) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx == 0) {
-    V.maxslot[0] = 0ull;
-    V.maxslot[1] = 0ull;
-    V.counters[0] = 0;
-  }
   if (idx < g.I) {
     V.u[idx] = 0.0;
     V.la[idx] = 0.0;
@@ -566,10 +561,10 @@ static size_t layout(Bump& b, const Geom& g, Vecs& V) {
   V.wrow_lo = b.take<float>(g.I);
   V.wcol_lo = b.take<float>(g.ldc);
   V.part = b.take<float2>((size_t)g.nrb * g.ldc);
-  V.maxslot = b.take<unsigned long long>(2);
+  b.take<unsigned long long>(2);   // unused, like the ints below: the scratch need stays what callers sized for
   V.red = b.take<double>((size_t)kRedBlocks * kNq);
   V.scal = b.take<double>(16);
-  V.counters = b.take<int>(8);
+  b.take<int>(8);
   return b.off + 256;
 }
 
@@ -829,7 +824,7 @@ extern "C" int wotg_refine_potentials(const wotg_problem* prob, const wotg_param
 // again in the process. All calls share the array: calls whose work overlaps
 // on the GPU (other streams, other host threads) race on it, so serialise
 // them. The solver re-initialises everything it reads from the scratch at the
-// start of each solve (state vectors, max slots, counters, the tensor-core
+// start of each solve (state vectors, control words, the tensor-core
 // form's packed points and error word), so no clearing between calls is
 // needed.
 // ---------------------------------------------------------------------------

@@ -29,10 +29,8 @@ struct Vecs {
   float* wcol_lo;  // ldc
   float4* rowc;    // I   per-row constants of the dense coupling (coupling_rows_kernel)
   float2* part;    // nrb x ldc column-pass partials (m, s) in base 2
-  unsigned long long* maxslot;  // 2 slots of max(a, b) bits, alternating per iteration
   double* red;     // kRedBlocks x kNq reduction partials
   double* scal;    // kNq final sums + misc scalars
-  int* counters;   // [0] absorptions
 };
 
 constexpr int kNq = 8;
@@ -44,16 +42,6 @@ struct Geom {
   int ncb, nrb;             // column pass: blocks of 1024 columns x row blocks
   int64_t rows_per;         // rows per row block
 };
-
-// exp(la) as the absorption test needs it: the test only compares the largest
-// exp(la) with tau, so away from log(tau) the value is 0 (below) or +inf
-// (above) with the same outcome, and the FP64 exp (slow on this part) is formed
-// only within 1e-9 of log(tau). NaN stays NaN.
-__device__ __forceinline__ double absorb_key(double la, const Coef& c) {
-  if (la < c.ltau_lo) return 0.0;
-  if (la > c.ltau_hi) return INFINITY;
-  return exp(la);
-}
 
 // Exponents of two elements: plain (w - k2 C, one rounding) or precise (relative
 // to the grid offset o with the weight's and kappa2's low parts, see split_weight),

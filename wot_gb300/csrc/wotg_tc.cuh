@@ -110,36 +110,8 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// Warp-wide load of 32 TMEM lanes x 32 consecutive 32-bit columns: lane l of the
-// warp receives row (lane base + l), columns [col, col + 32).
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Ties 32 registers written by tmem_ld32 to the preceding tmem_wait_ld: the
-// compiler sees them redefined here, so no use of them moves above the wait.
-__device__ __forceinline__ void tmem_hold(float (&v)[32]) {
-  asm volatile(""
-               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
-                 "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),
-                 "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),
-                 "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),
-                 "+f"(v[29]), "+f"(v[30]), "+f"(v[31]));
-}
-
-// Loads of 32 or 64 consecutive columns with their wait in one statement: the
+// Warp-wide loads of 32 TMEM lanes x 32 or 64 consecutive 32-bit columns (lane l of the
+// warp receives row (lane base + l)) with their wait in one statement: the
 // registers of a tcgen05.ld are written until its wait, and the compiler, which takes
 // them as written by the load, may move or spill one of them in between.
 __device__ __forceinline__ void tmem_read32(uint32_t taddr, float (&v)[32]) {
