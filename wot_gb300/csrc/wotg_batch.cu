@@ -1889,9 +1889,12 @@ extern "C" size_t wotg_batch_workspace_bytes(const wotg_pair* pairs, int32_t n_p
 
 namespace {
 constexpr int kBodies = 8;  // iterations of the whole batch per graph launch
-// Exponentials of a pass up to which the batch runs in the loop kernel: about 60 us of
-// them at this part's rate, where the six launches' fixed 40 us are most of an iteration.
-constexpr double kLoopMaxExps = 5e8;
+// Exponentials of a pass up to which the batch runs in the loop kernel: where its time
+// meets the replayed launches', whose fixed 40 us an iteration no longer count. Measured
+// for 150 iterations, launches -> loop: 300 x 400, 4 pairs x 5 items 7.3 -> 4.7 ms; 1500 x
+// 2000, 8 x 5 (1.2e8) 22.6 -> 17.2 and 1 x 25 (7.5e7) 22.0 -> 22.3; 6000 x 8000, 2 x 5
+// (4.8e8) 54 -> 40 and 4 x 5 (9.6e8) 87 -> 76; 9000 x 11000, 1 x 10 (9.9e8) 92 -> 93.
+constexpr double kLoopMaxExps = 1e9;
 }
 
 extern "C" int wotg_solve_batched(const wotg_pair* pairs, int32_t n_pairs, const wotg_item* items, int32_t n_items,
