@@ -17,3 +17,16 @@ def test_weights_in_and_out_of_shared_memory(I, J):
     cfg = dict(CFG, max_iter=60)
     got, _ = ot.compute_transport_matrix(solver=ot.optimal_transport_duality_gap, C=C, G=G, **cfg)
     assert_parity(got, _reference(C, G, cfg), what=(I, J))
+
+
+@pytest.mark.parametrize('I,J', [(5003, 6001), (131, 200003)])
+def test_costs_past_l2_against_the_on_the_fly_form(I, J):
+    """Costs of more than 100 MB are loaded another way, lines asked for ahead: with
+    the weights in shared memory, and with more than fit there."""
+    from wot_gb300.ot import device as D
+    rng = np.random.default_rng(J)
+    x, y = rng.normal(size=(I, 12)).astype(np.float32), rng.normal(size=(J, 12)).astype(np.float32)
+    cost, g = D.default_cost(x, y), rng.lognormal(0, 0.3, I)
+    T = {form: D.solve(cost, g, dict(CFG, max_iter=45), 0, form=form).tmap.cpu().numpy()
+         for form in ('materialized', 'onthefly')}
+    assert_parity(T['onthefly'], T['materialized'], marginals=False, what=(I, J))

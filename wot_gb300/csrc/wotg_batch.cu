@@ -295,8 +295,9 @@ __device__ __forceinline__ void stage_weights(float (*dst)[kChunk], const Entry*
   }
 }
 
+template <bool KEEP>
 __device__ __forceinline__ float4 load_cost(const float4* crow, int64_t q, int64_t nv, bool valid) {
-  if (valid && q < nv) return ld_stream(crow + q);
+  if (valid && q < nv) return KEEP ? ld_stream(crow + q) : ld_once(crow + q);
   return make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
 }
 
@@ -335,7 +336,7 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
   cp_async_commit();
   float4 nxt[RW];
 #pragma unroll
-  for (int rr = 0; rr < RW; ++rr) nxt[rr] = load_cost(crow[rr], lane, nv, valid[rr]);
+  for (int rr = 0; rr < RW; ++rr) nxt[rr] = load_cost<false>(crow[rr], lane, nv, valid[rr]);
   for (int ch = 0; ch < nch; ++ch) {
     if (ch + 1 < nch) stage_weights<KG>(sW[(ch + 1) & 1], gp, ng, (int64_t)(ch + 1) * kChunk, sg.cols);
     cp_async_commit();
@@ -345,7 +346,7 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
 #pragma unroll
     for (int rr = 0; rr < RW; ++rr) {
       cc[rr] = nxt[rr];
-      if (ch + 1 < nch) nxt[rr] = load_cost(crow[rr], (int64_t)(ch + 1) * 32 + lane, nv, valid[rr]);
+      if (ch + 1 < nch) nxt[rr] = load_cost<false>(crow[rr], (int64_t)(ch + 1) * 32 + lane, nv, valid[rr]);
     }
     const float* wb = &sW[ch & 1][0][lane * 4];
     if (SPEC) {
@@ -466,7 +467,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
     for (; q + 96 < nq; q += 128) {
       float4 cc[4], ww[4];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) cc[t] = ld_stream(crow + q + 32 * t);
+      for (int t = 0; t < 4; ++t) cc[t] = ld_once(crow + q + 32 * t);
 #pragma unroll
       for (int t = 0; t < 4; ++t) ww[t] = w4[q + 32 * t];   // not __ldg: written by other CTAs before a barrier
 #pragma unroll
@@ -479,7 +480,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
       }
     }
     for (; q < nq; q += 32) {
-      const float4 cc = ld_stream(crow + q);
+      const float4 cc = ld_once(crow + q);
       const float4 ww = w4[q];
       s0 += ex2(fmaf(nk2, cc.x, ww.x) - o) + ex2(fmaf(nk2, cc.y, ww.y) - o);
       s1 += ex2(fmaf(nk2, cc.z, ww.z) - o) + ex2(fmaf(nk2, cc.w, ww.w) - o);
@@ -1249,7 +1250,7 @@ __device__ __noinline__ void loop_rows(const LoopGroup g, LoopShared& sh, int cs
     for (int t = 0; t < kLoopAhead; ++t)
 #pragma unroll
       for (int r = 0; r < kLoopRW; ++r)
-        nx[t][r] = load_cost(crow[r], (ch0 + t) * 32, nv - lane, valid[r] && ch0 + t < ch1);
+        nx[t][r] = load_cost<true>(crow[r], (ch0 + t) * 32, nv - lane, valid[r] && ch0 + t < ch1);
     if (steps > 1) {
       __syncthreads();
       loop_stage(const_cast<float*>(W), sh, g.which, g.g0, g.ng, ch0 * kChunk, cs, sg.cols);
@@ -1266,7 +1267,7 @@ __device__ __noinline__ void loop_rows(const LoopGroup g, LoopShared& sh, int cs
           c01[r] = pk(nx[t][r].x, nx[t][r].y);
           c23[r] = pk(nx[t][r].z, nx[t][r].w);
           const int nc = ch + t + kLoopAhead;
-          nx[t][r] = load_cost(crow[r], nc * 32, nv - lane, valid[r] && nc < ch1);
+          nx[t][r] = load_cost<true>(crow[r], nc * 32, nv - lane, valid[r] && nc < ch1);
         }
         const float* wb = W + (ch + t - ch0) * kChunk + lane * 4;
 #pragma unroll

@@ -99,10 +99,12 @@ __device__ __forceinline__ double lse2(float o, float s) {
   return (double)o + (double)e + (double)log2f(m);
 }
 
-// 128-bit load of a cost (never written while a kernel reads it). Not marked
-// evict-first: the next pass finds a cost of up to some 100 MB in L2 (a 4001 x 5003
-// solve took 22.3 ms with __ldcs, 20.9 with __ldg).
+// 128-bit loads of a cost (never written while a kernel reads it). ld_stream keeps it
+// in L2, where the next pass finds a cost of up to some 100 MB (a 4001 x 5003 solve
+// took 22.3 ms with __ldcs, 20.9 with __ldg); ld_once marks it evict-first, for costs
+// that do not stay there anyway.
 __device__ __forceinline__ float4 ld_stream(const float4* p) { return __ldg(p); }
+__device__ __forceinline__ float4 ld_once(const float4* p) { return __ldcs(p); }
 
 // Merge two base-2 log-sum-exp partials (m, s): value = s * 2^m.
 __device__ __forceinline__ void lse_merge(float& m, float& s, float m2, float s2) {

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(512) radix_hist_kernel(const float* __restrict
   for (int64_t i = blockIdx.x; i < I; i += gridDim.x) {
     const float4* row = reinterpret_cast<const float4*>(C + i * ldc);
     for (int64_t c4 = threadIdx.x; c4 < nv; c4 += blockDim.x) {
-      const float4 v = ld_stream(row + c4);
+      const float4 v = ld_once(row + c4);
       const float vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int t = 0; t < 4; ++t) {

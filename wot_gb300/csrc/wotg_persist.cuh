@@ -506,6 +506,13 @@ struct Owned : PersistBase {
   }
 };
 
+// Costs of more bytes than stay in L2 are loaded evict-first, and each warp's lines are
+// asked for kAhead chunks before their loads: 100 iterations at 20000 x 25000 82 -> 72 ms,
+// 40000 x 9000 66 -> 54, 6000 x 8000 (192 MB) 9.7 -> 7.8; at 4001 x 5003 (80 MB) it would
+// take 21.3 ms for a solve instead of 18.3.
+constexpr int64_t kKeptBytes = 100000000;
+constexpr int kAhead = 4;
+__device__ __forceinline__ void prefetch_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void async16(void* to, const void* from) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from)
                : "memory");
@@ -525,6 +532,7 @@ __device__ __forceinline__ void async_wait() {
 // not; 23000 and 24000 with the arithmetic on packed FP32 pairs (wotg_state.cuh) and
 // the weights and their low parts, twice the bytes of the costs, in shared memory
 // (22.3 -> 18.4 ms a solve). Two rows per warp, or 24 or 32 warps, were no faster.
+template <bool KEPT>
 struct Streamed : Owned {
   __device__ static __forceinline__ float* wstage() { return reinterpret_cast<float*>(persist_smem + kMergeHeaderBytes); }
   // Copies a pass's weights and their low parts (n floats each) to shared memory.
@@ -598,8 +606,23 @@ struct Streamed : Owned {
     for (int i = b + (threadIdx.x >> 5); i < e; i += kPersistWarps) {
       float m, s, cmp, h, l;
       const float4* row = reinterpret_cast<const float4*>(A().C + (int64_t)i * A().g.ldc);
-      row_lse<true>([row](int k) { return ld_stream(row + k); }, [w4](int k) { return w4[k]; },
-                    [wl4](int k) { return wl4[k]; }, nv, lane, orow()[i], sh().c.kappa2, sh().c.kappa2_lo, m, s, cmp);
+      // a 128-byte line per lane of the chunk kAhead chunks on, or of the warp's next row
+      const bool more = i + kPersistWarps < e;
+      auto ahead = [row, nv, lane, more](int k) {
+        int q = k + 128 * kAhead + lane * 8;
+        const float4* p = row + q;
+        if (q >= nv) {
+          q -= nv;
+          p = row + (int64_t)kPersistWarps * nv + q;
+          if (!more || q >= nv) return;
+        }
+        if (lane < 16) prefetch_line(p);
+      };
+      auto ask = [&ahead](int k) {
+        if constexpr (!KEPT) ahead(k);
+      };
+      row_lse<true>([row](int k) { return KEPT ? ld_stream(row + k) : ld_once(row + k); }, [w4](int k) { return w4[k]; },
+                    [wl4](int k) { return wl4[k]; }, nv, lane, orow()[i], sh().c.kappa2, sh().c.kappa2_lo, m, s, cmp, ask);
       two_sum(s, -cmp, h, l);
       df_merge_lanes<16, 1>(m, h, l);
       if (lane == 0) mg().res[i - b] = make_float4(m, h, l, 0.f);
@@ -661,8 +684,24 @@ struct Streamed : Owned {
       for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A().g.J ? l2col()[c4 * 4 + q].x : 0.f;
       const int a = r * rows_per;
       const float4* col = reinterpret_cast<const float4*>(A().C) + c4;
-      col_lse<true>([=](int i) { return ld_stream(col + i * ld4); }, [w](int i) { return w[i]; },
-                    [wl](int i) { return wl[i]; }, a, min(I, a + rows_per), o, sh().c.kappa2, sh().c.kappa2_lo, m, s);
+      // as for the rows: four lines of each of the four rows kAhead chunks on, or of the
+      // warp's next unit
+      const int last = min(I, a + rows_per), u2 = u + kPersistWarps, r2 = u2 / ncg;
+      const int line = (lane & 3) * 8, skew = lane >> 2;
+      auto ahead = [=](int i) {
+        int q = i + kColRowChunk * kAhead + skew, c = (u - r * ncg) * 32 + line;
+        if (q >= last) {
+          if (u2 >= units) return;
+          q = r2 * rows_per + (q - last);
+          c = (u2 - r2 * ncg) * 32 + line;
+        }
+        if (lane < 16 && q < I && c < nv) prefetch_line(reinterpret_cast<const float4*>(A().C) + q * ld4 + c);
+      };
+      auto ask = [&ahead](int i) {
+        if constexpr (!KEPT) ahead(i);
+      };
+      col_lse<true>([=](int i) { return KEPT ? ld_stream(col + i * ld4) : ld_once(col + i * ld4); }, [w](int i) { return w[i]; },
+                    [wl](int i) { return wl[i]; }, a, last, o, sh().c.kappa2, sh().c.kappa2_lo, m, s, ask);
       float4* out = reinterpret_cast<float4*>(A().V.part + ((int64_t)c4 * A().g.nrb + r) * 4);
       out[0] = make_float4(m[0], s[0], m[1], s[1]);
       out[1] = make_float4(m[2], s[2], m[3], s[3]);
@@ -937,10 +976,11 @@ __device__ void persist_run(P& p) {
 }
 
 // GAP: the duality-gap solver (kModeGap); else kModeFixed or kModeRefine.
-template <bool GAP>
+// KEPT: the cost stays in L2 (kKeptBytes).
+template <bool GAP, bool KEPT>
 __global__ void __launch_bounds__(kPersistThreads, 1) persist_kernel(const __grid_constant__ PersistArgs A) {
   PersistBase::begin(A);
-  Streamed p;
+  Streamed<KEPT> p;
   persist_run<GAP>(p);
 }
 

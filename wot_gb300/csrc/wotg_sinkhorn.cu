@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) row_pass_kernel(const float* __restrict__
     float m, s, cmp;
     const float4* row = reinterpret_cast<const float4*>(C + i * g.ldc);
     auto wk = [w4](int k) { return __ldg(w4 + k); };
-    row_lse<false>([row](int k) { return ld_stream(row + k); }, wk, wk, (int)(g.ldc >> 2), lane, 0.f, k2, 0.f, m, s, cmp);
+    row_lse<false>([row](int k) { return ld_once(row + k); }, wk, wk, (int)(g.ldc >> 2), lane, 0.f, k2, 0.f, m, s, cmp);
     warp_lse(m, s);
     if (lane == 0) L[i] = ((double)m + log2((double)s)) * kLn2;
   }
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) col_partial_kernel(const float* __restric
   const float4* col = reinterpret_cast<const float4*>(C) + c4;
   const int64_t ld4 = g.ldc >> 2;
   auto wi = [w](int64_t i) { return __ldg(w + i); };
-  col_lse<false>([=](int64_t i) { return ld_stream(col + i * ld4); }, wi, wi, r0, min(g.I, r0 + g.rows_per), o, k2, 0.f,
+  col_lse<false>([=](int64_t i) { return ld_once(col + i * ld4); }, wi, wi, r0, min(g.I, r0 + g.rows_per), o, k2, 0.f,
                  m, s);
   float4* out = reinterpret_cast<float4*>(part + (int64_t)blockIdx.y * g.ldc + c4 * 4);
   out[0] = make_float4(m[0], s[0], m[1], s[1]);
@@ -365,6 +365,11 @@ struct SolveResult {
   Coef final_coef{};
 };
 
+static const void* streamed_kernel(bool gap, bool kept) {
+  if (gap) return kept ? reinterpret_cast<const void*>(persist_kernel<true, true>) : reinterpret_cast<const void*>(persist_kernel<true, false>);
+  return kept ? reinterpret_cast<const void*>(persist_kernel<false, true>) : reinterpret_cast<const void*>(persist_kernel<false, false>);
+}
+
 // Shared memory the solvers on a cost may use beside their static part; their limit
 // is raised to it once per device.
 static int resident_room(int* room) {
@@ -376,8 +381,8 @@ static int resident_room(int* room) {
   WOTG_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const void* const kernels[] = {reinterpret_cast<const void*>(resident_kernel<true>),
                                  reinterpret_cast<const void*>(resident_kernel<false>),
-                                 reinterpret_cast<const void*>(persist_kernel<true>),
-                                 reinterpret_cast<const void*>(persist_kernel<false>)};
+                                 streamed_kernel(true, true), streamed_kernel(true, false),
+                                 streamed_kernel(false, true), streamed_kernel(false, false)};
   *room = limit;
   for (const void* k : kernels) {
     cudaFuncAttributes a{};
@@ -429,8 +434,7 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
   int rows_cap = 0, cols_cap = 0;
   size_t streamed_smem = kMergeHeaderBytes, smem = streamed_smem;
   const bool gap = mode == kModeGap;
-  const void* streamed = gap ? reinterpret_cast<const void*>(persist_kernel<true>)
-                             : reinterpret_cast<const void*>(persist_kernel<false>);
+  const void* streamed = streamed_kernel(gap, 4 * S.g.I * S.g.ldc <= kKeptBytes);
   const void* kernel = streamed;
   TcPersistArgs T{};
   int threads = kPersistThreads;

@@ -82,10 +82,14 @@ __device__ __forceinline__ void lse_step(const float4& cc, const float4& w, cons
 // One lane's share of a row's online base-2 LSE: float4 columns lane, lane + 32,
 // ... < nv, in order; (m, s) as partial s 2^m, with PREC the sum compensated,
 // s - cmp. cost(k), w(k), wl(k) load float4 k of the row, the weights and their
-// low parts (from global or shared memory).
-template <bool PREC, class Cost, class W, class Wl>
+// low parts (from global or shared memory); ahead(k) is told each whole chunk's first
+// float4 (of 128).
+struct NoAhead {
+  __device__ __forceinline__ void operator()(int) const {}
+};
+template <bool PREC, class Cost, class W, class Wl, class Ahead = NoAhead>
 __device__ __forceinline__ void row_lse(const Cost& cost, const W& w, const Wl& wl, int nv, int lane, float o, float k2,
-                                        float k2l, float& m, float& s, float& cmp) {
+                                        float k2l, float& m, float& s, float& cmp, const Ahead& ahead = Ahead()) {
   m = kNegBig;
   s = 0.f;
   cmp = 0.f;
@@ -101,6 +105,7 @@ __device__ __forceinline__ void row_lse(const Cost& cost, const W& w, const Wl& 
   const int full = nv & ~127;   // whole chunks; the last, partial one follows
   for (; k < full; k += 128) {
     float4 cc[4], ww[4], wlo[4];
+    ahead(k - lane);
 #pragma unroll
     for (int t = 0; t < 4; ++t) cc[t] = cn[t];
 #pragma unroll
@@ -185,10 +190,11 @@ __device__ __forceinline__ void col_result(const ColSums& c, float (&m)[4], floa
 }
 
 // The same over rows [r0, r1): cost(i) loads the columns' float4 of row i, w(i) and
-// wl(i) the row's weight; o the columns' offsets (PREC).
-template <bool PREC, class I, class Cost, class W, class Wl>
+// wl(i) the row's weight; o the columns' offsets (PREC); ahead(i) is told each whole
+// chunk's first row.
+template <bool PREC, class I, class Cost, class W, class Wl, class Ahead = NoAhead>
 __device__ __forceinline__ void col_lse(const Cost& cost, const W& w, const Wl& wl, I r0, I r1, const float (&o)[4],
-                                        float k2, float k2l, float (&m)[4], float (&s)[4]) {
+                                        float k2, float k2l, float (&m)[4], float (&s)[4], const Ahead& ahead = Ahead()) {
   ColSums c;
   col_clear(c);
   const float2 no[2] = {make_float2(-o[0], -o[1]), make_float2(-o[2], -o[3])};
@@ -203,6 +209,7 @@ __device__ __forceinline__ void col_lse(const Cost& cost, const W& w, const Wl& 
   for (; i + kColRowChunk <= r1; i += kColRowChunk) {
     float4 cc[kColRowChunk];
     float ww[kColRowChunk], wlo[kColRowChunk];
+    ahead((int)i);
 #pragma unroll
     for (int t = 0; t < kColRowChunk; ++t) cc[t] = cn[t];
     if (i + 2 * kColRowChunk <= r1) {
