@@ -43,6 +43,7 @@
 #include <tuple>
 #include <vector>
 
+#include "wotg_barrier.cuh"
 #include "wotg_coef.cuh"
 #include "wotg_common.cuh"
 #include "wotg_state.cuh"
@@ -1066,32 +1067,30 @@ struct LoopShared {
   Seg seg[2];                        // their costs
   int kg[2], wcap;
   int over, ok;
-  unsigned int target, seen, seen2, any, any2;
+  BarrierSeen seen;
+  int any, any2;                     // flags raised at the last barrier that took them
 };
 static_assert(sizeof(LoopTile) == sizeof(Tile), "kept in the tiles' memory");
 constexpr size_t kLoopHeader = (sizeof(LoopShared) + 127) / 128 * 128;
 extern __shared__ __align__(128) unsigned char loop_smem[];
 
-// All CTAs arrive; the flags of any CTA come back in sh.any and sh.any2.
-__device__ bool loop_barrier(const LoopArgs& A, LoopShared& sh, bool flag, bool flag2) {
+// All CTAs arrive; with `take`, the flags of any CTA come back in sh.any and sh.any2 (no
+// two such barriers in a row, see wotg_barrier.cuh).
+__device__ bool loop_barrier(const LoopArgs& A, LoopShared& sh, bool flag = false, bool flag2 = false, bool take = false) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(A.bar),
-                 "l"(1ull + ((unsigned long long)(flag ? 1 : 0) << 24) + ((unsigned long long)(flag2 ? 1 : 0) << 44))
-                 : "memory");
-    sh.target += gridDim.x;
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(A.bar), "l"(barrier_arrival(flag, flag2)) : "memory");
     unsigned long long v = 0;
     bool done = false;
     for (uint32_t t = 0; t < kLoopTries && !done; ++t) {
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(A.bar) : "memory");
-      done = (v & 0xFFFFFFu) >= sh.target;
+      done = barrier_complete(v, sh.seen);
       if ((t & 255) == 255 && *(volatile int*)A.err) break;
     }
-    const unsigned int f = (unsigned int)(v >> 24) & 0xFFFFFu, f2 = (unsigned int)(v >> 44);
-    sh.any = f != sh.seen;
-    sh.any2 = f2 != sh.seen2;
-    sh.seen = f;
-    sh.seen2 = f2;
+    bool f, f2;
+    barrier_pass(v, gridDim.x, take, sh.seen, &f, &f2);
+    sh.any = f;
+    sh.any2 = f2;
     if (!done) {
       atomicExch(A.err, 1);
       sh.ok = 0;
@@ -1457,7 +1456,7 @@ __device__ void loop_load(const LoopArgs& A, LoopShared& sh) {
     }
     sh.wcap = A.wcap;
     sh.n[0] = sh.n[1] = sh.n[2] = 0;
-    sh.target = sh.seen = sh.seen2 = 0;
+    sh.seen = BarrierSeen{gridDim.x, 0, 0};
     sh.over = 0;
     sh.ok = 1;
   }
@@ -1498,12 +1497,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1) loop_kernel(const __grid_cons
   for (int n = 0; n < kLoopIters && running; ++n) {
     const bool fresh = plain == 0;   // the items' state may have changed since the last pass
     loop_pass(B, 0, kRowA, fresh, sh);
-    if (!loop_barrier(A, sh, false, false)) return;
+    if (!loop_barrier(A, sh)) return;
     loop_pass(B, 1, kColB, fresh, sh);
     __syncthreads();
     // the last iteration leaves nothing pending
     const bool wants = threadIdx.x == 0 && (sh.over || n == kLoopIters - 1 || loop_wants(B, nblk, plain));
-    if (!loop_barrier(A, sh, wants, false)) return;
+    if (!loop_barrier(A, sh, wants, false, true)) return;
     if (threadIdx.x == 0) sh.over = 0;
     if (!sh.any) {
       ++plain;
@@ -1513,23 +1512,23 @@ __global__ void __launch_bounds__(kLoopThreads, 1) loop_kernel(const __grid_cons
       for (int b = blockIdx.x; b < nblk; b += gridDim.x) item_body(B, b, plain);
     plain = 0;
     // the items' last CTAs decided: read the outcome after the barrier
-    if (!loop_barrier(A, sh, false, false)) return;
+    if (!loop_barrier(A, sh)) return;
     bool check = false, active = false;
     if (threadIdx.x == 0) loop_status(B, nblk, &check, &active);
-    if (!loop_barrier(A, sh, check, active)) return;
+    if (!loop_barrier(A, sh, check, active, true)) return;
     running = sh.any2 != 0;
     if (!sh.any) continue;
     loop_pass(B, 0, kFresh, true, sh);
-    if (!loop_barrier(A, sh, false, false)) return;
+    if (!loop_barrier(A, sh)) return;
     if (items)
       for (int b = blockIdx.x; b < nblk; b += gridDim.x) test_body(B, b);
-    if (!loop_barrier(A, sh, false, false)) return;
+    if (!loop_barrier(A, sh)) return;
     if (items)
       for (int b = blockIdx.x; b < nblk; b += gridDim.x) apply_body(B, b);
-    if (!loop_barrier(A, sh, false, false)) return;
+    if (!loop_barrier(A, sh)) return;
     check = active = false;
     if (threadIdx.x == 0) loop_status(B, nblk, &check, &active);
-    if (!loop_barrier(A, sh, false, active)) return;
+    if (!loop_barrier(A, sh, false, active, true)) return;
     running = sh.any2 != 0;
   }
   if (blockIdx.x == 0) {   // the count of active items for the host

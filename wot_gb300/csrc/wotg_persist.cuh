@@ -32,6 +32,7 @@
 
 #include <stddef.h>
 
+#include "wotg_barrier.cuh"
 #include "wotg_df.cuh"
 #include "wotg_state.cuh"
 
@@ -94,9 +95,8 @@ struct PersistShared {
   double dx, dy;                  // 1 / I, 1 / J
   float a1h, a1l, a2h, a2l;       // alpha1, alpha2 as pairs
   RunState rs;
-  unsigned int target;            // barrier arrivals that complete the next barrier
-  unsigned int flags, flags2;     // barrier flags seen so far (absorption; rows to recompute)
-  int flagged, flagged2;          // raised at the last barrier
+  BarrierSeen seen;               // its flags: absorption; rows to recompute
+  int flagged, flagged2;          // raised at the last barrier that took them
   int ok, decision, ticket;
   int r0, r1, j0, j1, c0, c1;     // owned rows, columns, float4 columns
   int row_flag, over_flag;        // a row to recompute / a scaling above tau, since the half-step began
@@ -167,8 +167,7 @@ struct PersistBase {
       PersistShared& s = sh();
       const Geom& g = A().g;
       const int n = gridDim.x, b = blockIdx.x;
-      s.target = n;
-      s.flags = s.flags2 = 0;
+      s.seen = BarrierSeen{(unsigned int)n, 0, 0};
       s.ok = 1;
       s.r0 = (int)(g.I * b / n);
       s.r1 = (int)(g.I * (b + 1) / n);
@@ -183,23 +182,21 @@ struct PersistBase {
     for (int i = threadIdx.x; i < kLogTable; i += blockDim.x) mg().tab[i] = log_table_entry(i);
   }
 
-  // All CTAs arrive; `flag` and `flag2` are or-ed over the CTAs into *flagged and
-  // *flagged2. The word counts arrivals in its low 24 bits and flags in 20 bits
-  // each above: enough for the 2000 iterations of a launch at 304 CTAs.
-  __device__ static __noinline__ bool barrier(bool flag, bool flag2) {
+  // All CTAs arrive; with `take`, `flag` and `flag2` are or-ed over the CTAs into
+  // sh().flagged and sh().flagged2 (wotg_barrier.cuh). The counts are enough for the 2000
+  // iterations of a launch at 304 CTAs.
+  __device__ static __noinline__ bool barrier(bool flag, bool flag2, bool take) {
     __syncthreads();
     if (threadIdx.x == 0) {
       PersistShared& s = sh();
       PersistCtl* ctl = A().ctl;
-      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->bar),
-                   "l"(1ull + ((unsigned long long)(flag ? 1 : 0) << 24) + ((unsigned long long)(flag2 ? 1 : 0) << 44))
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->bar), "l"(barrier_arrival(flag, flag2))
                    : "memory");
       unsigned long long v = 0;
-      const unsigned int want = s.target;
       bool done = false;
       for (uint32_t t = 0; t < kBarrierTries; ++t) {
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&ctl->bar) : "memory");
-        if (((unsigned int)v & 0xFFFFFFu) >= want) {
+        if (barrier_complete(v, s.seen)) {
           done = true;
           break;
         }
@@ -209,20 +206,21 @@ struct PersistBase {
         atomicExch(&ctl->err, 1);
         s.ok = 0;
       }
-      const unsigned int f = (unsigned int)(v >> 24) & 0xFFFFFu, f2 = (unsigned int)(v >> 44);
-      s.flagged = f != s.flags;
-      s.flagged2 = f2 != s.flags2;
-      s.flags = f;
-      s.flags2 = f2;
-      s.target = want + gridDim.x;
+      bool f, f2;
+      barrier_pass(v, gridDim.x, take, s.seen, &f, &f2);
+      s.flagged = f;
+      s.flagged2 = f2;
     }
     __syncthreads();
     return sh().ok != 0;
   }
-  __device__ static __forceinline__ bool sync(bool flag, bool* flagged = nullptr, bool flag2 = false,
-                                              bool* flagged2 = nullptr) {
-    const bool ok = barrier(flag, flag2);
-    if (flagged) *flagged = sh().flagged != 0;
+  // A barrier without flags.
+  __device__ static __forceinline__ bool sync() { return barrier(false, false, false); }
+  // One whose flags are taken. No two in a row, but where the second only adds to the
+  // first's `flagged` (TcPersist::side).
+  __device__ static __forceinline__ bool sync(bool flag, bool* flagged, bool flag2 = false, bool* flagged2 = nullptr) {
+    const bool ok = barrier(flag, flag2, true);
+    *flagged = sh().flagged != 0;
     if (flagged2) *flagged2 = sh().flagged2 != 0;
     return ok;
   }
@@ -280,7 +278,7 @@ struct PersistBase {
   // V.red: one barrier, then every CTA adds them in the same order into sh().tot.
   template <int NQ>
   __device__ static bool reduce_ctas() {
-    if (!sync(false)) return false;
+    if (!sync()) return false;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w < NQ) {
       double t = 0.0;
@@ -363,7 +361,7 @@ struct PersistBase {
   // q = mean(p) from its sum, and the constants of the coefficients.
   __device__ static bool publish_mean() {
     if (threadIdx.x == 0 && blockIdx.x == 0) A().ctl->q = sh().tot[0] / (double)A().g.I;
-    return sync(false);
+    return sync();
   }
   __device__ static void constants() {
     if (threadIdx.x < 32) {
@@ -783,9 +781,9 @@ struct Streamed : Owned {
   // One iteration; *absorb_now when max(a, b) > tau.
   __device__ static bool iterate(bool lrow_valid, bool* absorb_now) {
     bool over = lrow_valid ? row_update_cached() : row_phase<false>();
-    if (!sync(false)) return false;
+    if (!sync()) return false;
     col_phase();
-    if (!sync(false)) return false;
+    if (!sync()) return false;
     over |= merge_phase();
     over = __syncthreads_or(over);
     return sync(over, absorb_now);
@@ -801,11 +799,11 @@ struct Streamed : Owned {
     set_coef(eps);
     reset_gap();
     absorb<true>(eps_old);
-    return sync(false);
+    return sync();
   }
   __device__ static bool absorb_now(double eps) {
     absorb<false>(eps);
-    return sync(false);
+    return sync();
   }
   __device__ static bool fresh() {
     row_phase<true>();

@@ -616,7 +616,7 @@ struct Resident : PersistBase {
       split_weight(vn * sh().c.inv_eps * kLog2e, &w.x, &w.y, 0);
       publish(t, w.x, w.y, pc(t).x, !RESCALE);
     }
-    return sync(false) && stage_weights(nullptr);
+    return sync() && stage_weights(nullptr);
   }
   __device__ static bool start_stage(double eps_old, double eps) {
     set_coef(eps);
@@ -629,7 +629,7 @@ struct Resident : PersistBase {
     fold_all();
     for (int t = threadIdx.x; t < nc(); t += kResidentThreads)
       publish(t, A().V.wcol[j0() + t], A().V.wcol_lo[j0() + t], 0.f, false);
-    return sync(false) && stage_weights(nullptr);
+    return sync() && stage_weights(nullptr);
   }
   __device__ static bool resume(double eps) {
     set_coef(eps);
@@ -650,7 +650,7 @@ struct Resident : PersistBase {
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) A().ctl->epoch = (int)sh().epoch;
     if (!done) return true;
-    if (!sync(false)) return false;   // nobody polls the offset words any more
+    if (!sync()) return false;   // nobody polls the offset words any more
     for (int t = threadIdx.x; t < nc(); t += kResidentThreads) {
       A().V.wcol[j0() + t] = F(kWhi, j0() + t);
       A().V.wcol_lo[j0() + t] = F(kWlo, j0() + t);

@@ -211,7 +211,7 @@ struct TcPersist : Owned {
       w = span<ROW>(i);
       p = load<ROW>(i);
     }
-    if (!sync(false)) return false;
+    if (!sync()) return false;
     while (i < end) {
       float m = kNegBig, sum = 0.f;
       for (int c = 0; c < w.n; c += 8) {
@@ -579,7 +579,7 @@ struct TcPersist : Owned {
       if (threadIdx.x == 0) sh().row_ok = sh().col_ok = 0;
     }
     async_fence();
-    return sync(false);
+    return sync();
   }
   // Row forms of both sides for the current epsilon: gamma = 2 kappa log2 e /
   // sqrt(cost_scale) times the points (the column forms hold sqrt(cost_scale) y).
