@@ -51,7 +51,8 @@ struct PersistCtl {
   double eps, q, sumk;            // current epsilon, mean(p), sum exp(-C/eps) / (I J) at the final stage
   double gap_num, gap_den;        // the last relative gap as a quotient
   long long it, checks, absorptions;
-  int stage, status, lrow_valid, started, since, index, epoch, pad_;
+  int stage, status, lrow_valid, started, since, index, epoch;
+  int batch;                      // iterations done of a batch that the launch ended in
   unsigned long long bar;         // grid barrier: arrivals and flags (PersistBase::sync); zeroed per launch
   int err, pad2_;                 // zeroed per launch
 };
@@ -64,7 +65,7 @@ struct PersistArgs {
   double epsilon, lambda1, lambda2, epsilon0, tau, tolerance, max_iter, cost_scale;
   double scale_factor;            // exp(-log(epsilon) / kScalings)
   int batch_size, scaling_iter, inner_iter_max, extra_iter, n_iter, mode;
-  long long budget;               // iterations of this launch (a batch is not split)
+  long long budget;               // iterations of this launch
   int wfloats;                    // streamed: floats of a weight vector kept in shared memory, 0: none are
 };
 
@@ -73,7 +74,7 @@ struct PersistArgs {
 struct RunState {
   double eps, sumk;
   long long it, checks, absorptions, used;
-  int stage, status, lrow_valid, since, index, stage_done;
+  int stage, status, lrow_valid, since, index, stage_done, batch;
 };
 
 // A virtual CTA's tiles in a tensor-core half-step (wotg_tc_persist.cuh).
@@ -183,8 +184,10 @@ struct PersistBase {
   }
 
   // All CTAs arrive; with `take`, `flag` and `flag2` are or-ed over the CTAs into
-  // sh().flagged and sh().flagged2 (wotg_barrier.cuh). The counts are enough for the 2000
-  // iterations of a launch at 304 CTAs.
+  // sh().flagged and sh().flagged2 (wotg_barrier.cuh). The counts last a launch: its
+  // budget keeps the flags below 2^20 (barriers that take flags: one per iteration
+  // streamed, up to four on the fly), and the arrivals, at most nine barriers per
+  // iteration with its tests, below 2^24.
   __device__ static __noinline__ bool barrier(bool flag, bool flag2, bool take) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -851,6 +854,7 @@ __device__ void persist_run(P& p) {
     rs.since = ctl->since;
     rs.index = ctl->index;
     rs.stage_done = 0;
+    rs.batch = ctl->batch;
   });
   if (rs.status != kRunning) return;
   if (!started && !p.mean_growth()) return;
@@ -880,9 +884,12 @@ __device__ void persist_run(P& p) {
         }
       }
       const int nb = rs.stage == kScalings ? A.batch_size : 5;
+      // a batch may be longer than the launch, which then ends inside it (the next one
+      // runs at least one of its iterations before the test)
+      const int t0 = rs.batch;
       bool cached = rs.lrow_valid != 0, last = false;
-      int t = 0;
-      while (t < nb && !last) {
+      int t = t0;
+      while (t < nb && !last && rs.used + (t - t0) < A.budget) {
         bool over = false;
         if (!p.iterate(cached, &over)) return;
         cached = false;
@@ -891,17 +898,20 @@ __device__ void persist_run(P& p) {
           change([&] { ++rs.absorptions; });
           if (!p.absorb_now(rs.eps)) return;
         }
-        last = (double)(rs.it + t) >= A.max_iter;
+        last = (double)(rs.it + (t - t0)) >= A.max_iter;
       }
+      const bool part = !last && t < nb;
       change([&] {
-        rs.it += t;
-        rs.used += t;
+        rs.it += t - t0;
+        rs.used += t - t0;
         rs.lrow_valid = 0;
+        rs.batch = part ? t : 0;
         if (last)
           rs.status = kMaxIter;
-        else
+        else if (!part)
           ++rs.checks;
       });
+      if (part) break;
       if (last) {
         if (!p.fresh()) return;
         break;
@@ -970,6 +980,7 @@ __device__ void persist_run(P& p) {
     ctl->started = 1;
     ctl->since = rs.since;
     ctl->index = rs.index;
+    ctl->batch = rs.batch;
   }
 }
 

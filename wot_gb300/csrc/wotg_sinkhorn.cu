@@ -422,7 +422,10 @@ static int solve_persistent(Solver& S, const wotg_params& P, int mode, double ep
   A.n_iter = n_iter;
   A.mode = mode;
   const double per_iter = 8e-6 + (S.tc.on ? 4e-13 : 2.5e-12) * (double)S.g.I * (double)S.g.J;
-  A.budget = std::max<long long>(8, std::min<long long>(2000, (long long)(0.02 / per_iter)));
+  // at most 2000, or as many as the barrier's flag counts last
+  const int flagged = S.tc.on ? 4 : 1;
+  A.budget = std::min<long long>(2000, ((1 << kBarrierFlagBits) - 1) / (flagged * std::min(sm_count(), kRedBlocks)));
+  A.budget = std::max<long long>(8, std::min<long long>(A.budget, (long long)(0.02 / per_iter)));
   PersistCtl h{};
   if (S.tc.on) {
     int s = S.mean_of(S.V.p, S.g.I, &h.q);
