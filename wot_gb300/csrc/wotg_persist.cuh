@@ -878,6 +878,11 @@ __device__ void persist_run(P& p) {
         });
         if (!p.start_stage(old, rs.eps)) return;
         if (rs.stage == kScalings) {
+          if (!(INFINITY > A.tolerance)) {   // `while gap > tolerance` from gap = inf: no iteration
+            if (!p.fresh()) return;
+            change([&] { rs.status = kConverged; });
+            break;
+          }
           double sumk;
           if (!p.sum_exp(&sumk)) return;
           change([&] { rs.sumk = sumk; });
