@@ -556,10 +556,11 @@ struct Streamed : Owned {
   }
   __device__ static __forceinline__ int c0() { return sh().c0; }
   __device__ static __forceinline__ int c1() { return sh().c1; }
-  // I row offsets (on the weight grid) in rowc's memory, free during the solve; J
-  // base-2 log-sum-exps of the columns (offset on the grid + remainder) in Lcol's.
+  // Offsets on the weight grid: the rows' in rowc's memory, free during the solve, the
+  // columns' in Lcol's. The columns' base-2 log-sum-exps stay FP64 for the gap test: in
+  // the final stage they take the place of the old scalings, which its tests don't read.
   __device__ static __forceinline__ float* orow() { return reinterpret_cast<float*>(A().V.rowc); }
-  __device__ static __forceinline__ float2* l2col() { return reinterpret_cast<float2*>(A().V.Lcol); }
+  __device__ static __forceinline__ float* ocol() { return reinterpret_cast<float*>(A().V.Lcol); }
 
   __device__ Streamed() {
     fill_table();
@@ -590,7 +591,7 @@ struct Streamed : Owned {
   __device__ static __forceinline__ bool update_col(int64_t j, double L2) {
     const double vj = A().V.v[j];
     const double lb = fma(-sh().a2ln2, L2, fma(vj, sh().kv, sh().bconst));
-    A().V.lb_old[j] = A().V.lb[j];
+    A().V.lb_old[j] = sh().rs.stage == kScalings ? L2 : A().V.lb[j];
     A().V.lb[j] = lb;
     const float2 w = split_pair(fma(lb, kLog2e, vj * sh().iel2));
     A().V.wcol[j] = w.x;
@@ -682,7 +683,7 @@ struct Streamed : Owned {
       if (c4 >= nv) continue;
       float o[4], m[4], s[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A().g.J ? l2col()[c4 * 4 + q].x : 0.f;
+      for (int q = 0; q < 4; ++q) o[q] = c4 * 4 + q < A().g.J ? ocol()[c4 * 4 + q] : 0.f;
       const int a = r * rows_per;
       const float4* col = reinterpret_cast<const float4*>(A().C) + c4;
       // as for the rows: four lines of each of the four rows kAhead chunks on, or of the
@@ -750,9 +751,8 @@ struct Streamed : Owned {
         const int j = b * 4 + t;
         if (j >= A().g.J) break;
         const float4 r = mg().res[t];
-        const double L2 = lse2_pair(l2col()[j].x, r.x, r.y, r.z, mg().tab);
-        const float o = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
-        l2col()[j] = make_float2(o, (float)(L2 - (double)o));
+        const double L2 = lse2_pair(ocol()[j], r.x, r.y, r.z, mg().tab);
+        ocol()[j] = fabs(L2) < 1e30 ? grid_near(L2) : 0.f;
         over |= update_col(j, L2);
       }
       __syncthreads();
@@ -793,8 +793,8 @@ struct Streamed : Owned {
   }
 
   __device__ static bool gap_test(double sumk, bool* go_on, bool* nan) {
-    const float2* l2 = l2col();
-    return gap_test_with([l2](int j) { return ((double)l2[j].x + (double)l2[j].y) * kLn2; }, sumk, go_on, nan);
+    const double* l2 = A().V.lb_old;
+    return gap_test_with([l2](int j) { return l2[j] * kLn2; }, sumk, go_on, nan);
   }
 
   // Absorbs with the old epsilon and starts a stage at `eps`.
