@@ -64,8 +64,9 @@ struct TcSmem {
   // Two CTAs per SM in 96 KB each: 32 columns double-buffer the row tile (A) and
   // keep a 4-deep ring of column tiles (B); 64 columns single-buffer A (it
   // changes only at the few row-tile boundaries of a CTA's stretch) and keep 2 B stages.
-  // The population form adds the weights of each column tile (and one stage less).
-  static constexpr int kStages = KP == 32 ? (NPOP ? kTcStages - 1 : kTcStages) : 2;   // B ring depth
+  // The population form adds the weights of each column tile (and, for eight
+  // populations at 32 columns, has one stage less).
+  static constexpr int kStages = KP == 32 ? (NPOP > 4 ? kTcStages - 1 : kTcStages) : 2;   // B ring depth
   static constexpr int kABuf = KP == 32 ? 2 : 1;               // A buffers
   static constexpr uint32_t kA = 0;                            // kABuf buffers
   static constexpr uint32_t kB = kABuf * kTileBytes;           // kStages buffers
@@ -186,15 +187,15 @@ __device__ __forceinline__ void multi32(const float (&d)[32], const float* w, fl
 }
 
 // NPOP = 0: the log-sum-exp half-step (partials (m, s) in part). NPOP > 0: the
-// population form, npop <= NPOP weighted sums per row (maxima in part[].x,
-// sums in psum[slot * NPOP + k]) with the population weights popw.
+// population form, NPOP weighted sums per row (maxima in part[].x, sums in
+// psum[slot * NPOP + k]) with the population weights popw (zero past the last one).
 template <int KP, int NPOP>
 __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) lse_tc_kernel(const __half* __restrict__ Pt,
                                                                const __half* __restrict__ Qt,
                                                                int n_pt, int nq, float2* __restrict__ part,
                                                                const float* off,
                                                                int* __restrict__ err, uint32_t wait_tries,
-                                                               const float* __restrict__ popw, int npop,
+                                                               const float* __restrict__ popw,
                                                                float* __restrict__ psum) {
   using L = TcSmem<KP, NPOP>;
   constexpr int S = L::kStages;
