@@ -129,12 +129,23 @@ __global__ void __launch_bounds__(kNarrowThreads) gemm_narrow_kernel(const doubl
 
 using namespace wotg;
 
+// Whether the rows x cols block at x (leading dimension ld) shares memory with the one at c.
+static bool overlaps(const double* x, int64_t ld, int64_t rows, int64_t cols, const double* c, int64_t ldc,
+                     int64_t c_rows, int64_t c_cols) {
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), c0 = reinterpret_cast<uintptr_t>(c);
+  const uintptr_t x1 = x0 + 8 * (uint64_t)((rows - 1) * ld + cols), c1 = c0 + 8 * (uint64_t)((c_rows - 1) * ldc + c_cols);
+  return x0 < c1 && c0 < x1;
+}
+
 extern "C" int wotg_gemm_f64(const double* A, int64_t lda, const double* B, int64_t ldb, const int64_t* b_rows,
                              double* C, int64_t ldc, int64_t M, int64_t N, int64_t K, void* stream) {
   if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0 || lda < K || ldb < N || ldc < N) return WOTG_BADARG;
   const int64_t gx = (N + kGemmTile - 1) / kGemmTile, gy = (M + kGemmTile - 1) / kGemmTile;
   if (gx > 2147483647LL || gy > 65535) return WOTG_BADARG;
-  if (N <= kNarrow && K <= kNarrow) {
+  // a product in place stays with the tiles: with N <= 64 a CTA has read its rows of A when
+  // it writes them, while the narrow kernel's threads share them with others'
+  if (N <= kNarrow && K <= kNarrow && !overlaps(A, lda, M, K, C, ldc, M, N) &&
+      (b_rows || !overlaps(B, ldb, K, N, C, ldc, M, N))) {
     const int64_t blocks = std::min<int64_t>((M * N + kNarrowThreads - 1) / kNarrowThreads, (int64_t)sm_count() * 12);
     gemm_narrow_kernel<<<(unsigned)blocks, kNarrowThreads, 0, (cudaStream_t)stream>>>(A, lda, B, ldb, b_rows, C, ldc, M,
                                                                                      (int)N, (int)K);
