@@ -1037,7 +1037,6 @@ struct LoopTile {
 struct LoopDir {
   const LoopTile* tiles;   // CTA b's tile at b
   int ntiles;
-  int kg;   // the tuned pass's group: an entry alone in its group is summed by run_single
 };
 struct LoopArgs {
   BatchArgs B;
@@ -1065,7 +1064,7 @@ struct LoopShared {
   int n[3];                          // entries of the row, column and check lists
   int pair[2], row0[2], rows[2];     // the CTA's tiles
   Seg seg[2];                        // their costs
-  int kg[2], wcap;
+  int wcap;
   int over, ok;
   BarrierSeen seen;
   int any, any2;                     // flags raised at the last barrier that took them
@@ -1414,7 +1413,9 @@ __device__ __noinline__ void loop_pass(const BatchArgs& B, int dir, int mode, bo
     __syncthreads();
   }
   for (g.g0 = 0; g.g0 < sh.n[g.which];) {
-    const int n = sh.n[g.which], main = n - (n % sh.kg[dir] == 1 ? 1 : 0);
+    // an entry alone after the full groups is summed as a single one (whatever group the
+    // tuner found fastest for the launches, so that a call's bits don't depend on timing)
+    const int n = sh.n[g.which], main = n - (n % kLoopKG == 1 ? 1 : 0);
     const bool single = g.g0 == main;
     g.ng = single ? 1 : min(kLoopKG, main - g.g0);
     // columns staged at once: all, or as many chunks as fit
@@ -1452,7 +1453,6 @@ __device__ void loop_load(const LoopArgs& A, LoopShared& sh) {
         sh.row0[dir] = t.row0;
         sh.seg[dir] = A.segs[2 * sh.pair[dir] + dir];
       }
-      sh.kg[dir] = A.dir[dir].kg;
     }
     sh.wcap = A.wcap;
     sh.n[0] = sh.n[1] = sh.n[2] = 0;
@@ -2086,7 +2086,7 @@ extern "C" int wotg_solve_batched(const wotg_pair* pairs, int32_t n_pairs, const
     A.wcap = (smem - (int)kLoopHeader) / (int)sizeof(float);
     for (int d = 0; d < 2; ++d) {
       WOTG_BCUDA(cudaMemcpyAsync(L.tiles[d][0], lt[d].data(), sizeof(LoopTile) * lt[d].size(), cudaMemcpyHostToDevice, cs));
-      A.dir[d] = LoopDir{reinterpret_cast<const LoopTile*>(L.tiles[d][0]), (int)lt[d].size(), kCfgs[cfg[d]].kg};
+      A.dir[d] = LoopDir{reinterpret_cast<const LoopTile*>(L.tiles[d][0]), (int)lt[d].size()};
     }
     A.bar = reinterpret_cast<unsigned long long*>(L.active + 2);
     A.err = L.active + 1;
