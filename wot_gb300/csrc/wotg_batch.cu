@@ -223,37 +223,39 @@ __device__ __forceinline__ bool note_scaling(Item& it, double l) {
   return true;
 }
 
-// L2 = base-2 log-sum-exp of row r for entry e; true when an absorption may be due.
-__device__ __forceinline__ bool entry_epilogue(Item* items, const Entry& e, int64_t r, double L2) {
+// L2 = base-2 log-sum-exp of row r for entry e.
+__device__ __forceinline__ void entry_epilogue(Item* items, const Entry& e, int64_t r, double L2) {
   const double L = L2 * kLn2;
   switch (e.mode) {
     case kOut:
       e.out[r] = L;
       if (e.o) e.o[r] = (float)L2;
-      return false;
+      return;
     case kFresh: {
       Item& it = items[e.item];
       it.Lrow[r] = L;
       it.orow[r] = (float)L2;
-      return false;
+      return;
     }
     case kSumK:
       items[e.item].rsum[r] = exp(L);
-      return false;
+      return;
     case kRowA: {
       Item& it = items[e.item];
       it.Lrow[r] = L;
       it.orow[r] = (float)L2;
-      return note_scaling(it, item_a_update(it, r, L));
+      note_scaling(it, item_a_update(it, r, L));
+      return;
     }
     case kColB: {
       Item& it = items[e.item];
       it.Lcol[r] = L;
       it.ocol[r] = (float)L2;
-      return note_scaling(it, item_b_update(it, r, L));
+      note_scaling(it, item_b_update(it, r, L));
+      return;
     }
     default:
-      return false;
+      return;
   }
 }
 
@@ -306,8 +308,7 @@ __device__ __forceinline__ float4 load_cost(const float4* crow, int64_t q, int64
 // row0 + w * RW + [0, RW)). SPEC: offset sums with exact fallback; else running max.
 template <int KG, int RW, bool SPEC>
 __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int row0, int ng, const Entry* gp,
-                                          float (*sW)[KG][kChunk], float2 (*s_ms)[KG], int* s_over, int warp,
-                                          int lane) {
+                                          float (*sW)[KG][kChunk], float2 (*s_ms)[KG], int warp, int lane) {
   float nk2[KG];
   float acc[RW][KG], off[RW][KG];
   bool valid[RW];
@@ -441,7 +442,7 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
   for (int idx = threadIdx.x; idx < total; idx += kThreads) {
     const int r = idx / ng, k = idx - r * ng;
     const float2 ms = s_ms[r][k];
-    if (entry_epilogue(A.items, gp[k], row0 + r, lse2(ms.x, ms.y))) *s_over = 1;
+    entry_epilogue(A.items, gp[k], row0 + r, lse2(ms.x, ms.y));
   }
 }
 
@@ -450,8 +451,8 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
 // and the weights (L1/L2-resident), no shared-memory staging and no barrier.
 // Columns past `cols` in the last float4 meet the cost's +inf padding.
 template <int RW>
-__device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int row0, const Entry* gp, int* s_over,
-                                           int warp, int lane) {
+__device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int row0, const Entry* gp, int warp,
+                                           int lane) {
   const Entry e = gp[0];
   const float nk2 = e.nk2;
   const float4* w4 = reinterpret_cast<const float4*>(e.w);
@@ -493,7 +494,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
       oo = ms.x;
       s = ms.y;
     }
-    if (lane == 0 && entry_epilogue(A.items, e, row, lse2(oo, s))) *s_over = 1;
+    if (lane == 0) entry_epilogue(A.items, e, row, lse2(oo, s));
   }
 }
 
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(PassArgs A) {
   __shared__ __align__(16) float sW[2][KG][kChunk];
   __shared__ Entry gp[KG];
   __shared__ float2 s_ms[kWarps * RW][KG];
-  __shared__ int s_tile, s_over;
+  __shared__ int s_tile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
     if (threadIdx.x == 0) s_tile = atomicAdd(A.counter, 1);
@@ -519,9 +520,9 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(PassArgs A) {
       if (threadIdx.x < ng) gp[threadIdx.x] = lst[g0 + threadIdx.x];
       __syncthreads();
       if (SPEC && ng == 1)
-        run_single<RW>(A, sg, tile.row0, gp, &s_over, warp, lane);
+        run_single<RW>(A, sg, tile.row0, gp, warp, lane);
       else
-        run_group<KG, RW, SPEC>(A, sg, tile.row0, ng, gp, sW, s_ms, &s_over, warp, lane);
+        run_group<KG, RW, SPEC>(A, sg, tile.row0, ng, gp, sW, s_ms, warp, lane);
       __syncthreads();
     }
   }

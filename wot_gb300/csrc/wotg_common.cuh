@@ -33,9 +33,6 @@ void set_last_message(const char* msg);
 
 // Host-side count of kernels this library launched (wotg_launch_count).
 void count_launch();
-// n kernels launched by one replay of a captured graph; the count so far.
-void count_launches(unsigned long long n);
-unsigned long long launches_so_far();
 
 #define WOTG_LAUNCHED()                                   \
   do {                                                    \
@@ -119,20 +116,6 @@ __device__ __forceinline__ void warp_lse(float& m, float& s) {
     float m2 = __shfl_xor_sync(0xffffffffu, m, o);
     float s2 = __shfl_xor_sync(0xffffffffu, s, o);
     lse_merge(m, s, m2, s2);
-  }
-}
-
-// Merge of base-2 partials (m, s) in FP64 across a warp: every lane ends with
-// the warp's total as (m, S), value S 2^m (S in FP64).
-__device__ __forceinline__ void warp_lse_f64(float& m, double& S) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float m2 = __shfl_xor_sync(0xffffffffu, m, o);
-    const double S2 = __shfl_xor_sync(0xffffffffu, S, o);
-    const float mn = fmaxf(m, m2);
-    // the scale factors by the FP32 ex2 (2 ulp), the sums themselves in FP64
-    S = S * (double)ex2(m - mn) + S2 * (double)ex2(m2 - mn);
-    m = mn;
   }
 }
 

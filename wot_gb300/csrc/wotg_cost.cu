@@ -24,8 +24,6 @@ static char g_last_error[512] = "";
 static std::atomic<unsigned long long> g_launches{0};
 
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
-void count_launches(unsigned long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
-unsigned long long launches_so_far() { return g_launches.load(std::memory_order_relaxed); }
 
 void set_last_error(const char* what, cudaError_t err) {
   snprintf(g_last_error, sizeof(g_last_error), "%s: %s", what, cudaGetErrorString(err));

@@ -41,7 +41,7 @@ __device__ __forceinline__ void df_add(float& h, float& l, float h2, float l2) {
 
 // Merge of base-2 partials (m, h + l) over the lanes that differ in the bits of
 // `FROM` .. `TO` (powers of two): every lane ends with the group's total. The
-// scale factors are the FP32 ex2 of warp_lse_f64.
+// scale factors are the FP32 ex2 (2 ulp).
 template <int FROM, int TO>
 __device__ __forceinline__ void df_merge_lanes(float& m, float& h, float& l) {
 #pragma unroll

@@ -66,7 +66,6 @@ struct TcState {
   double* normX;            // |x_i|^2 (FP64)
   double* normY;
   float2* part;
-  int* err;
   // Speculative half-steps: each row's base-2 log-sum-exp of the MMA exponents
   // from the previous half-step (row side offX, column side offY), valid while
   // epsilon is unchanged; rows whose sum left the safe range are listed in
@@ -640,7 +639,7 @@ static void tc_layout(Bump& b, const wotg_problem* prob, TcState& tc) {
   tc.normY = b.take<double>(prob->J);
   tc.part = b.take<float2>((size_t)(std::max(tc.ctas_row, tc.ctas_col) + std::max(tc.n_xt, tc.n_yt)) * 128 *
                            tc_parts());
-  tc.err = b.take<int>(4);
+  b.take<int>(4);   // unused, as below
   tc.offX = b.take<float>(tc.I_pad);
   tc.offY = b.take<float>(tc.J_pad);
   tc.redoX = b.take<int>(2 + prob->I);
@@ -832,8 +831,7 @@ extern "C" int wotg_refine_potentials(const wotg_problem* prob, const wotg_param
 // on the GPU (other streams, other host threads) race on it, so serialise
 // them. The solver re-initialises everything it reads from the scratch at the
 // start of each solve (state vectors, control words, the tensor-core
-// form's packed points and error word), so no clearing between calls is
-// needed.
+// form's packed points), so no clearing between calls is needed.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;
