@@ -223,39 +223,38 @@ __device__ __forceinline__ bool note_scaling(Item& it, double l) {
   return true;
 }
 
-// L2 = base-2 log-sum-exp of row r for entry e.
-__device__ __forceinline__ void entry_epilogue(Item* items, const Entry& e, int64_t r, double L2) {
+// L2 = base-2 log-sum-exp of row r for entry e; returns the log-scaling whose maximum
+// over the rows feeds the absorption test (log a_i or log b_j), else -inf.
+__device__ __forceinline__ double entry_epilogue(Item* items, const Entry& e, int64_t r, double L2) {
   const double L = L2 * kLn2;
   switch (e.mode) {
     case kOut:
       e.out[r] = L;
       if (e.o) e.o[r] = (float)L2;
-      return;
+      return -INFINITY;
     case kFresh: {
       Item& it = items[e.item];
       it.Lrow[r] = L;
       it.orow[r] = (float)L2;
-      return;
+      return -INFINITY;
     }
     case kSumK:
       items[e.item].rsum[r] = exp(L);
-      return;
+      return -INFINITY;
     case kRowA: {
       Item& it = items[e.item];
       it.Lrow[r] = L;
       it.orow[r] = (float)L2;
-      note_scaling(it, item_a_update(it, r, L));
-      return;
+      return item_a_update(it, r, L);
     }
     case kColB: {
       Item& it = items[e.item];
       it.Lcol[r] = L;
       it.ocol[r] = (float)L2;
-      note_scaling(it, item_b_update(it, r, L));
-      return;
+      return item_b_update(it, r, L);
     }
     default:
-      return;
+      return -INFINITY;
   }
 }
 
@@ -308,7 +307,7 @@ __device__ __forceinline__ float4 load_cost(const float4* crow, int64_t q, int64
 // row0 + w * RW + [0, RW)). SPEC: offset sums with exact fallback; else running max.
 template <int KG, int RW, bool SPEC>
 __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int row0, int ng, const Entry* gp,
-                                          float (*sW)[KG][kChunk], float2 (*s_ms)[KG], int warp, int lane) {
+                                          float (*sW)[KG][kChunk], double (*s_vmax)[KG], int warp, int lane) {
   float nk2[KG];
   float acc[RW][KG], off[RW][KG];
   bool valid[RW];
@@ -408,7 +407,11 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
           warp_lse(off[rr][k], acc[rr][k]);
       }
     }
-  // Lane k holds entry k.
+  // Lane k finishes entry k. (Spread over a thread per (row, entry) after a barrier, as in
+  // the loop kernel, the FP64 updates cost a third, but the column loop came out with
+  // 105 registers instead of 80, one CTA per SM less: five items at 20000 x 25000 took
+  // 179 ms for 120 iterations instead of 162, ten pairs x 25 items 472 instead of 448.)
+  double vmax = -INFINITY;
 #pragma unroll
   for (int rr = 0; rr < RW; ++rr) {
     float s = 0.f, o = 0.f;
@@ -432,31 +435,23 @@ __device__ __forceinline__ void run_group(const PassArgs& A, const Seg& sg, int 
         }
       }
     }
-    if (mine) s_ms[warp * RW + rr][lane] = make_float2(o, s);
+    if (mine) vmax = fmax(vmax, entry_epilogue(A.items, gp[lane], row[rr], lse2(o, s)));
   }
-  __syncthreads();
-  // The FP64 updates, a thread per (row, entry): an FP64 instruction takes 64 cycles
-  // however few of a warp's lanes are active, so ten entries of each warp's rows in
-  // turn cost three times as much.
-  const int total = min(kWarps * RW, sg.rows - row0) * ng;
-  for (int idx = threadIdx.x; idx < total; idx += kThreads) {
-    const int r = idx / ng, k = idx - r * ng;
-    const float2 ms = s_ms[r][k];
-    entry_epilogue(A.items, gp[k], row0 + r, lse2(ms.x, ms.y));
-  }
+  if (lane < KG) s_vmax[warp][lane] = vmax;
 }
 
 // One entry over the tile's rows (a pair with a single active item, as in the
 // tail of a batch): each warp streams its rows with 128-bit loads of the cost
 // and the weights (L1/L2-resident), no shared-memory staging and no barrier.
 // Columns past `cols` in the last float4 meet the cost's +inf padding.
-template <int RW>
-__device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int row0, const Entry* gp, int warp,
-                                           int lane) {
+template <int RW, int KG>
+__device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int row0, const Entry* gp,
+                                           double (*s_vmax)[KG], int warp, int lane) {
   const Entry e = gp[0];
   const float nk2 = e.nk2;
-  const float4* w4 = reinterpret_cast<const float4*>(e.w);
+  const float4* __restrict__ w4 = reinterpret_cast<const float4*>(e.w);
   const int64_t nq = ((int64_t)sg.cols + 3) >> 2;
+  double vmax = -INFINITY;
 #pragma unroll 1
   for (int rr = 0; rr < RW; ++rr) {
     const int64_t row = (int64_t)row0 + warp * RW + rr;
@@ -471,7 +466,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
 #pragma unroll
       for (int t = 0; t < 4; ++t) cc[t] = ld_once(crow + q + 32 * t);
 #pragma unroll
-      for (int t = 0; t < 4; ++t) ww[t] = w4[q + 32 * t];   // not __ldg: written by other CTAs before a barrier
+      for (int t = 0; t < 4; ++t) ww[t] = __ldg(w4 + q + 32 * t);
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         const uint64_t e01 = ex2_off(fma2(kk, pk(cc[t].x, cc[t].y), pk(ww[t].x, ww[t].y)), mo);
@@ -483,7 +478,7 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
     }
     for (; q < nq; q += 32) {
       const float4 cc = ld_once(crow + q);
-      const float4 ww = w4[q];
+      const float4 ww = __ldg(w4 + q);
       s0 += ex2(fmaf(nk2, cc.x, ww.x) - o) + ex2(fmaf(nk2, cc.y, ww.y) - o);
       s1 += ex2(fmaf(nk2, cc.z, ww.z) - o) + ex2(fmaf(nk2, cc.w, ww.w) - o);
     }
@@ -494,15 +489,16 @@ __device__ __forceinline__ void run_single(const PassArgs& A, const Seg& sg, int
       oo = ms.x;
       s = ms.y;
     }
-    if (lane == 0) entry_epilogue(A.items, e, row, lse2(oo, s));
+    if (lane == 0) vmax = fmax(vmax, entry_epilogue(A.items, e, row, lse2(oo, s)));
   }
+  if (lane == 0) s_vmax[warp][0] = vmax;
 }
 
 template <int KG, int RW, bool SPEC>
 __global__ void __launch_bounds__(kThreads) pass_kernel(PassArgs A) {
   __shared__ __align__(16) float sW[2][KG][kChunk];
   __shared__ Entry gp[KG];
-  __shared__ float2 s_ms[kWarps * RW][KG];
+  __shared__ double s_vmax[kWarps][KG];
   __shared__ int s_tile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (;;) {
@@ -520,9 +516,20 @@ __global__ void __launch_bounds__(kThreads) pass_kernel(PassArgs A) {
       if (threadIdx.x < ng) gp[threadIdx.x] = lst[g0 + threadIdx.x];
       __syncthreads();
       if (SPEC && ng == 1)
-        run_single<RW>(A, sg, tile.row0, gp, warp, lane);
+        run_single<RW, KG>(A, sg, tile.row0, gp, s_vmax, warp, lane);
       else
-        run_group<KG, RW, SPEC>(A, sg, tile.row0, ng, gp, sW, s_ms, warp, lane);
+        run_group<KG, RW, SPEC>(A, sg, tile.row0, ng, gp, sW, s_vmax, warp, lane);
+      __syncthreads();
+      // absorption maxima of this group: one test per item
+      if (threadIdx.x < ng) {
+        const Entry& e = gp[threadIdx.x];
+        if (e.mode == kRowA || e.mode == kColB) {
+          double v = -INFINITY;
+#pragma unroll
+          for (int w = 0; w < kWarps; ++w) v = fmax(v, s_vmax[w][threadIdx.x]);
+          note_scaling(A.items[e.item], v);
+        }
+      }
       __syncthreads();
     }
   }
