@@ -1592,6 +1592,63 @@ static std::vector<LoopTile> loop_tiles(const std::vector<int>& rows, const std:
   return out;
 }
 
+// Exponentials of a direction's pass per CTA: evenly dealt (`even`; a tile has at least
+// min(8, rows) rows), and as the loop's longest tile takes them, whose last round costs
+// three fifths of a full one when it is at most one row per warp. A single round is
+// latency however full it is.
+static void loop_share(const std::vector<LoopTile>& tiles, const std::vector<int>& rows, const std::vector<int>& cols,
+                       const std::vector<int>& items, int ctas, double* even, double* worst) {
+  double all = 0.0;
+  *even = *worst = 0.0;
+  for (size_t p = 0; p < rows.size(); ++p) {
+    const double per_row = (double)cols[p] * items[p];
+    all += rows[p] * per_row;
+    *even = std::max(*even, std::min(8, rows[p]) * per_row);
+  }
+  *even = std::max(*even, all / ctas);
+  int longest = 0;
+  for (const LoopTile& t : tiles) longest = std::max(longest, t.pair_rows / kLoopMaxPairs);
+  for (const LoopTile& t : tiles) {
+    const int p = t.pair_rows & (kLoopMaxPairs - 1), n = t.pair_rows / kLoopMaxPairs, rest = n % kLoopRows;
+    const int taken = longest <= kLoopRows || rest == 0 ? n : n - rest + (rest <= kLoopWarps ? kLoopRows * 3 / 5 : kLoopRows);
+    *worst = std::max(*worst, (double)taken * cols[p] * items[p]);
+  }
+  *worst = std::max(*worst, *even);
+}
+
+// Whether the loop kernel is the faster form for a batch. It saves the launches' fixed 40 us
+// an iteration and loses to them where (ms for 120 iterations, launches -> loop)
+//  * its tiles come out uneven or its rounds half full, unless that costs less than the
+//    40 us: `waste`, in exponentials and three more per entry of a cost for its loads. 77
+//    pairs x 5 items of 1000 x 1000 59.5 -> 85.6, 20 items of 7000 x 7000 65.5 -> 82.9 (46
+//    rows a tile, rounds of 40); but four pairs x 5 of 1560 x 1560 12.3 -> 10.6;
+//  * one item streams a cost that does not stay in L2, of which it has fewer bytes under
+//    way than the launches: 9000 x 11000 22.0 -> 26.2, 20000 x 25000 79.7 -> 118.5 (two
+//    items 34.8 -> 26.9 and 140 -> 112);
+//  * a pair has so many items that they take a pass by themselves, over 2e8 exponentials
+//    and 20 items a pair: 25 of 1700 x 1700, 12 pairs, 81.7 -> 87.1 (20 of 4000 x 4000, 3
+//    pairs, 69.9 -> 63.3);
+//  * a pass has over 1e9 exponentials.
+// Elsewhere it gains: three pairs x 5 of 1500 x 1800 to convergence 15.4 -> 10.0, five
+// items of 4000 x 5000 23.7 -> 18.7, of 12000 x 15000 103 -> 93.
+constexpr double kLoopMaxExps = 1e9, kLoopManyExps = 2e8, kLoopManyItems = 20, kLoopL2Entries = 2.5e7,
+                 kLoopShare = 0.8, kLoopWaste = 3.5e7;
+static bool loop_pays(const std::vector<LoopTile> (&tiles)[2], const std::vector<int>& I, const std::vector<int>& J,
+                      const std::vector<int>& items, int ctas) {
+  double exps = 0.0, entries = 0.0;
+  for (size_t p = 0; p < I.size(); ++p) {
+    entries += (double)I[p] * J[p];
+    exps += (double)I[p] * J[p] * items[p];
+  }
+  if (exps > kLoopMaxExps || (exps > kLoopManyExps && exps > kLoopManyItems * entries)) return false;
+  if (entries > kLoopL2Entries && exps < 2.0 * entries) return false;
+  double even[2], worst[2];
+  loop_share(tiles[0], I, J, items, ctas, even, worst);
+  loop_share(tiles[1], J, I, items, ctas, even + 1, worst + 1);
+  const double waste = (exps + 3.0 * entries) * ((worst[0] + worst[1]) / (even[0] + even[1]) - 1.0 / kLoopShare);
+  return waste <= kLoopWaste;
+}
+
 // ---------------------------------------------------------------------------
 // Cost transpose, dense coupling from potentials.
 // ---------------------------------------------------------------------------
@@ -1897,12 +1954,6 @@ extern "C" size_t wotg_batch_workspace_bytes(const wotg_pair* pairs, int32_t n_p
 
 namespace {
 constexpr int kBodies = 8;  // iterations of the whole batch per graph launch
-// Exponentials of a pass up to which the batch runs in the loop kernel: where its time
-// meets the replayed launches', whose fixed 40 us an iteration no longer count. Measured
-// for 150 iterations, launches -> loop: 300 x 400, 4 pairs x 5 items 7.3 -> 4.7 ms; 1500 x
-// 2000, 8 x 5 (1.2e8) 22.6 -> 17.2 and 1 x 25 (7.5e7) 22.0 -> 22.3; 6000 x 8000, 2 x 5
-// (4.8e8) 54 -> 40 and 4 x 5 (9.6e8) 87 -> 76; 9000 x 11000, 1 x 10 (9.9e8) 92 -> 93.
-constexpr double kLoopMaxExps = 1e9;
 }
 
 extern "C" int wotg_solve_batched(const wotg_pair* pairs, int32_t n_pairs, const wotg_item* items, int32_t n_items,
@@ -2073,13 +2124,11 @@ extern "C" int wotg_solve_batched(const wotg_pair* pairs, int32_t n_pairs, const
     max_iters = std::max(max_iters, items[k].params.max_iter * std::max(1, items[k].params.growth_iters));
   g_replay_prof.clear();
   auto t_last = std::chrono::steady_clock::now();
-  // Small batches run in the loop kernel.
+  // Small batches run in the loop kernel, where that is the faster form.
   const int g = sm_count();
   std::vector<LoopTile> lt[2] = {loop_tiles(rows0, cols0, g), loop_tiles(cols0, rows0, g)};
-  double exps = 0.0;
-  for (int k = 0; k < ni; ++k) exps += (double)hi[k].I * hi[k].J;
-  bool in_loop = !lt[0].empty() && !lt[1].empty() && exps <= kLoopMaxExps &&
-                 *std::max_element(kp.begin(), kp.end()) <= kLoopMaxItems;
+  bool in_loop = !lt[0].empty() && !lt[1].empty() && *std::max_element(kp.begin(), kp.end()) <= kLoopMaxItems &&
+                 loop_pays(lt, rows0, cols0, kp, g);
   if (in_loop) {
     int room = 0, dev = 0;
     WOTG_BCUDA(cudaGetDevice(&dev));
