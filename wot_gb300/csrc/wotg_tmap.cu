@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) pull_kernel(const double* __restrict__ X,
     for (int r = 0; r < KC; ++r) acc[r] = 0.0;
     const double* row = X + i * J;
     int64_t j = lane;
-    for (; j + 32 < J; j += 64) {
+    for (; j - lane + 64 <= J; j += 64) {   // whole steps of the warp: a split one would take its FMAs twice
       const double x0 = row[j], x1 = row[j + 32];
       double p0[KC], p1[KC];
 #pragma unroll
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) pull_kernel(const double* __restrict__ X,
 #pragma unroll
       for (int r = 0; r < KC; ++r) acc[r] = fma(x1, p1[r], acc[r]);
     }
-    if (j < J) {
+    for (; j < J; j += 32) {
       const double x = row[j];
 #pragma unroll
       for (int r = 0; r < KC; ++r) acc[r] = fma(x, __ldg(P + r * J + j), acc[r]);
