@@ -64,8 +64,8 @@ struct TcSmem {
   // Two CTAs per SM in 96 KB each: 32 columns double-buffer the row tile (A) and
   // keep a 4-deep ring of column tiles (B); 64 columns single-buffer A (it
   // changes only at the few row-tile boundaries of a CTA's stretch) and keep 2 B stages.
-  // The population form adds the weights of each column tile (and, for eight
-  // populations at 32 columns, has one stage less).
+  // The population form adds the weights of each column tile: 104 and 100 KB for four
+  // populations at 32 and 64 columns, 92 (one stage less) and 104 KB for eight.
   static constexpr int kStages = KP == 32 ? (NPOP > 4 ? kTcStages - 1 : kTcStages) : 2;   // B ring depth
   static constexpr int kABuf = KP == 32 ? 2 : 1;               // A buffers
   static constexpr uint32_t kA = 0;                            // kABuf buffers

@@ -138,13 +138,15 @@ FORMS = {'materialized': N.FORM_MATERIALIZED, 'onthefly': N.FORM_ONTHEFLY}
 TC_MAX_DIM = 62   # point dimensions the tensor-core half-step packs (two bias columns in 64)
 
 
-# Below this many cost entries the two forms take about the same time (measured
-# on GB300 at 30 dimensions: 1500 x 1800 cells 24 ms streamed against 30 ms on
-# the tensor cores per solve, 2500 x 3000 32 ms against 30 ms, 9000 x 10800
-# 93 ms against 43 ms), so 'auto' keeps the streamed form there: its exponents
-# are exact to the FP32 storage of C, while the tensor-core form's carry the
-# error of the points' 22-bit FP16 hi/lo split accumulated in FP32 (about
-# kappa |x| |y| 2^-22 per exponent).
+# From this many cost entries 'auto' takes the tensor cores. The forms' times (ms per solve
+# of some 455 iterations on GB300, materialised / on the fly, 30 dimensions): 1500 x 1800
+# 5.6 / 10.6, 2000 x 2500 10.4 / 11.7, 2500 x 3000 11.8 / 12.1, 3000 x 3600 12.8 / 12.6,
+# 4000 x 4800 15.3 / 13.4, 5000 x 6000 26.6 / 15.3, 9000 x 10800 69 / 25; at 50 dimensions
+# 3000 x 3600 12.7 / 13.5, 4000 x 4800 15.1 / 14.6. They meet near 1e7 entries; the line
+# stays where it lies although the materialised form is up to 15 % faster just above it,
+# because a pair's map would change with the form: the materialised form's exponents are
+# exact to the FP32 storage of C, the tensor cores' carry the error of the points' 22-bit
+# FP16 hi/lo split accumulated in FP32 (about kappa |x| |y| 2^-22 per exponent).
 TC_AUTO_MIN_ENTRIES = 4_000_000
 
 
@@ -152,7 +154,7 @@ def resolve_form(cost: DeviceCost, form: str) -> int:
     """'materialized' streams the FP32 cost; 'onthefly' recomputes cost tiles
     from the points on the tensor cores; 'auto' picks the latter when the cost
     was built from points of at most TC_MAX_DIM dimensions and has at least
-    TC_AUTO_MIN_ENTRIES entries (where it is the faster form)."""
+    TC_AUTO_MIN_ENTRIES entries (well above which it is the faster form)."""
     if form == 'auto':
         tc = (cost.X is not None and cost.X.shape[1] <= TC_MAX_DIM
               and cost.I * cost.J >= TC_AUTO_MIN_ENTRIES)
